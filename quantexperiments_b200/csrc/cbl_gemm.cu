@@ -28,6 +28,17 @@ constexpr int GM_SMEM = 65536 + GM_A_STAGES * 2 * GM_A_BYTES + GM_B_STAGES * GM_
 constexpr int GM_DECODE_WARPS = 8, GM_THREADS = (GM_DECODE_WARPS + 2) * 32;
 constexpr uint32_t GM_WAIT_LIMIT = 1u << 24;   // mbarrier polls (a few tens of cycles each) before a wait gives up
 
+// The issuing thread of a warp, chosen by elect.sync, and a warp index the compiler knows to be uniform.  With a
+// plain `lane == 0` the compiler must assume that several threads could get here and wraps every tcgen05.mma (whose
+// descriptors live in uniform registers) in a loop over the active lanes: 97 clocks per MMA issued, whatever its size,
+// against 21 (N = 16) .. 75 (N = 128) for the MMA itself (A in tensor memory, M = 128, measured on B200).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ int uniform_warp(int tid) { return __shfl_sync(0xffffffffu, tid >> 5, 0); }
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
@@ -135,7 +146,7 @@ k_gemm_l8(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* __res
     __shared__ __align__(8) unsigned long long s_bar[2 * GM_A_STAGES + 2 * GM_B_STAGES + 1];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     // row tiles vary fastest across the grid: blocks that run together share one activation tile in L2
     const int r0 = blockIdx.x * GM_BN, tok0 = blockIdx.y * GM_BM;
     // one tile of the l8 layout per k-block; a second (summed) book is a second pass over the same activation
@@ -174,7 +185,7 @@ k_gemm_l8(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* __res
     if (warp == GM_DECODE_WARPS) {
         // ---------------- TMA producer of the activations (its ring is deeper than the weights': the
         // round trip through L2 is several k-blocks long)
-        if (lane == 0) {
+        if (elect_one()) {
             for (int kb = 0; kb < nkb; kb++) {
                 const int s = kb % GM_A_STAGES;
                 if (!mbar_wait(empty_a(s), ((kb / GM_A_STAGES) & 1) ^ 1)) { s_abort = 1; break; }
@@ -187,7 +198,7 @@ k_gemm_l8(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* __res
         }
     } else if (warp == GM_DECODE_WARPS + 1) {
         // ---------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // f16 x f16 -> f32, K-major both
             for (int kb = 0; kb < nkb; kb++) {
                 const int sa = kb % GM_A_STAGES, sb = kb % GM_B_STAGES;
@@ -337,7 +348,7 @@ k_gemm_l8_2sm(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* _
     __shared__ __align__(8) unsigned long long s_bar[3 * G2_STAGES + 1];   // full_a, full_b, empty per stage; tmem_full
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int r0 = (blockIdx.x >> 1) * GM_BN, tok_base = blockIdx.y * 512;
@@ -375,7 +386,7 @@ k_gemm_l8_2sm(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* _
 
     if (warp == G2_DECODE_WARPS) {
         // ---------------- TMA producer: this block's 2 x 128 tokens; completion lands on the leader's barrier
-        if (lane == 0) {
+        if (elect_one()) {
             for (int kb = 0; kb < nkb; kb++) {
                 const int s = kb % G2_STAGES;
                 if (!mbar_wait(empty(s), ((kb / G2_STAGES) & 1) ^ 1)) { s_abort = 1; break; }
@@ -388,7 +399,7 @@ k_gemm_l8_2sm(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* _
         }
     } else if (warp == G2_DECODE_WARPS + 1) {
         // ---------------- MMA issuer (leader block only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             for (int kb = 0; kb < nkb; kb++) {
                 const int s = kb % G2_STAGES;
@@ -519,7 +530,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GR
     __shared__ __align__(8) unsigned long long s_bar[3 * GR_STAGES + 1];    // full_a, full_x, empty per stage; tmem_full
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     int mi = 0;
     while (mi + 1 < P.n && (int)blockIdx.x >= P.tile0[mi + 1]) mi++;
@@ -566,7 +577,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GR
     };
 
     if (warp == GR_DECODE_WARPS) {
-        if (lane == 0) {                                      // TMA producer of the activations
+        if (elect_one()) {                                      // TMA producer of the activations
             int it = 0;
             for (int sg = 0; sg < 2; sg++) {
                 for (int kb = seg_lo[sg]; kb < seg_hi[sg]; kb += GR_KBS, it++) {
@@ -580,7 +591,7 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GR
             }
         }
     } else if (warp == GR_DECODE_WARPS + 1) {
-        if (lane == 0) {                                      // MMA issuer
+        if (elect_one()) {                                      // MMA issuer
             const uint32_t idesc = (1u << 4) | ((uint32_t)(P.npad >> 3) << 17) | ((uint32_t)(GR_ROWS >> 4) << 24);
             int it = 0;
             uint32_t accumulate = 0;
@@ -701,8 +712,6 @@ k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GR
 // registers into its TMEM lane (tcgen05.st) and the MMA takes A from TMEM, so neither the store of the A tile nor
 // the tensor cores' read of it touch shared memory - only the codeword gathers do.  TMEM columns: 0..31 the
 // accumulator, then GT_STAGES stages of 4 k-blocks x 32 columns (a k-block = 64 fp16 per row = 32 columns).
-// What bounds it now is the tensor pipe itself: an MMA of 128 rows x 16 k takes about 170 cycles however few the
-// tokens (independent accumulators and a software-pipelined decode loop changed nothing), i.e. 1.4 us per stage.
 constexpr int GT_STAGES = 3;
 constexpr int GT_A_COL0 = 32, GT_A_STAGE_COLS = GR_KBS * 32;
 constexpr int GT_SMEM = 65536 + GT_STAGES * GR_X_STAGE;
@@ -732,7 +741,7 @@ k_gemm_rows_ta(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     __shared__ __align__(8) unsigned long long s_bar[3 * GT_STAGES + 1];    // full_a, full_x, empty per stage; tmem_full
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     int mi = 0;
     while (mi + 1 < P.n && (int)blockIdx.x >= P.tile0[mi + 1]) mi++;
@@ -779,7 +788,7 @@ k_gemm_rows_ta(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
     };
 
     if (warp == GR_DECODE_WARPS) {
-        if (lane == 0) {                                      // TMA producer of the activations
+        if (elect_one()) {                                      // TMA producer of the activations
             int it = 0;
             for (int sg = 0; sg < 2; sg++) {
                 for (int kb = seg_lo[sg]; kb < seg_hi[sg]; kb += GR_KBS, it++) {
@@ -793,7 +802,7 @@ k_gemm_rows_ta(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
             }
         }
     } else if (warp == GR_DECODE_WARPS + 1) {
-        if (lane == 0) {                                      // MMA issuer
+        if (elect_one()) {                                      // MMA issuer
             const uint32_t idesc = (1u << 4) | ((uint32_t)(P.npad >> 3) << 17) | ((uint32_t)(GR_ROWS >> 4) << 24);
             int it = 0;
             uint32_t accumulate = 0;
@@ -942,7 +951,7 @@ k_gemm_dense(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ C
     __shared__ __align__(8) unsigned long long s_bar[2 * GD_STAGES + 1];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     // token tiles vary fastest across the grid: blocks that run together share weight rows in L2
     const int r0 = blockIdx.y * GM_BN, tok0 = blockIdx.x * GM_BM;
     const int nkb = (m.C + GM_BK - 1) / GM_BK;
@@ -966,7 +975,7 @@ k_gemm_dense(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ C
     const uint32_t tmem = s_tmem;
 
     if (warp == GD_EPI_WARPS) {
-        if (lane == 0) {                                      // TMA producer: activations (2 x 128 tokens) and weights (256 rows)
+        if (elect_one()) {                                      // TMA producer: activations (2 x 128 tokens) and weights (256 rows)
             for (int kb = 0; kb < nkb; kb++) {
                 const int s = kb % GD_STAGES;
                 if (!mbar_wait(empty(s), ((kb / GD_STAGES) & 1) ^ 1)) { s_abort = 1; break; }
@@ -978,7 +987,7 @@ k_gemm_dense(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ C
             }
         }
     } else if (warp == GD_EPI_WARPS + 1) {
-        if (lane == 0) {                                      // MMA issuer
+        if (elect_one()) {                                      // MMA issuer
             constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
             for (int kb = 0; kb < nkb; kb++) {
                 const int s = kb % GD_STAGES;
@@ -1042,7 +1051,7 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     __shared__ __align__(8) unsigned long long s_bar[2 * G3_STAGES + 4];   // full, empty per stage; acc_full[2], acc_empty[2]
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     // a decode kernel of the next matrix (launched with programmatic serialization) may share the SMs with this GEMM
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t rank;
@@ -1072,7 +1081,7 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     const uint32_t tmem = s_tmem;
 
     if (warp == G3_EPI_WARPS) {
-        if (lane == 0) {                                      // TMA producer: this block's 128 tokens and 128 weight rows
+        if (elect_one()) {                                      // TMA producer: this block's 128 tokens and 128 weight rows
             int it = 0;
             for (int t = cluster; t < ntiles && !s_abort; t += nclusters) {
                 const int tok0 = (t % ntt) * 256 + (int)rank * 128, r0 = (t / ntt) * GM_BN + (int)rank * 128;
@@ -1088,7 +1097,7 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             }
         }
     } else if (warp == G3_EPI_WARPS + 1) {
-        if (lane == 0 && rank == 0) {                         // MMA issuer (leader block)
+        if (rank == 0 && elect_one()) {                         // MMA issuer (leader block)
             constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             int it = 0, li = 0;
             for (int t = cluster; t < ntiles && !s_abort; t += nclusters, li++) {
