@@ -27,35 +27,101 @@ __device__ __forceinline__ int cbl_scale_exp(float mx) {
     return k < -100 ? -100 : (k > 110 ? 110 : k);
 }
 
-__global__ void __launch_bounds__(256) k_prep_x(const void* __restrict__ x, int xdtype, int B, int C, int64_t ldx,
-                                                const int32_t* __restrict__ perms, int Bpad, int Cpad, __half* __restrict__ xp,
-                                                float* __restrict__ xinv) {
-    __shared__ float s_max[8];
+// Eight values of an activation row as fp32.  VEC: one or two 16-byte loads of consecutive columns (no column order,
+// 16-byte aligned rows); otherwise element by element, through the column order when there is one.
+template <bool VEC>
+__device__ __forceinline__ void prep_load8(const void* __restrict__ x, int xdtype, int64_t row, int c, int C, const int32_t* __restrict__ perm,
+                                           float (&v)[8]) {
+    if (VEC) {
+        if (xdtype == CBL_F32) {
+            const float4 a = __ldg((const float4*)((const float*)x + row + c)), b = __ldg((const float4*)((const float*)x + row + c) + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+            const uint4 u = __ldg((const uint4*)((const char*)x + (row + c) * 2));
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float2 f = xdtype == CBL_BF16 ? __bfloat1622float2(*(const __nv_bfloat162*)&w[k]) : __half22float2(*(const __half2*)&w[k]);
+                v[2 * k] = f.x;
+                v[2 * k + 1] = f.y;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = c + k < C ? cbl_load_in(x, xdtype, row + (perm ? __ldg(perm + c + k) : c + k)) : 0.f;
+    }
+}
+
+// One block per (column order, token).  The row is read ONCE, 8 columns per thread and load, and stays in registers
+// between the search for its largest magnitude and the conversion (the element-wise two-pass form took 60 us for
+// 2048 tokens x 3584 columns, this one 9).  Rows longer than PREP_NV x 8 x NT columns read their tail twice.
+constexpr int PREP_NV = 5;
+template <int NT, bool VEC>
+__global__ void __launch_bounds__(NT) k_prep_x(const void* __restrict__ x, int xdtype, int B, int C, int64_t ldx,
+                                               const int32_t* __restrict__ perms, int Bpad, int Cpad, __half* __restrict__ xp,
+                                               float* __restrict__ xinv) {
+    __shared__ float s_max[NT / 32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int b = blockIdx.x % Bpad, m = blockIdx.x / Bpad;
+    const int b = blockIdx.x % Bpad, m = blockIdx.x / Bpad, tid = threadIdx.x;
+    const int32_t* perm = perms ? perms + (int64_t)m * C : nullptr;
+    const int64_t row = (int64_t)b * ldx;
     __half* dst = xp + (int64_t)blockIdx.x * Cpad;
+    constexpr int STEP = NT * 8;
+    float v[PREP_NV][8];
     float mx = 0.f;
-    if (b < B)
-        for (int c = threadIdx.x; c < C; c += 256) mx = fmaxf(mx, fabsf(cbl_load_in(x, xdtype, (int64_t)b * ldx + c)));
+#pragma unroll
+    for (int j = 0; j < PREP_NV; j++) {
+        const int c = (j * NT + tid) * 8;
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[j][k] = 0.f;
+        if (b < B && c < C) prep_load8<VEC>(x, xdtype, row, c, C, perm, v[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < PREP_NV; j++)
+#pragma unroll
+        for (int k = 0; k < 8; k++) mx = fmaxf(mx, fabsf(v[j][k]));
+    for (int c = PREP_NV * STEP + tid * 8; b < B && c < C; c += STEP) {
+        float t[8];
+        prep_load8<VEC>(x, xdtype, row, c, C, perm, t);
+#pragma unroll
+        for (int k = 0; k < 8; k++) mx = fmaxf(mx, fabsf(t[k]));
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
     __syncthreads();
     mx = s_max[0];
 #pragma unroll
-    for (int i = 1; i < 8; i++) mx = fmaxf(mx, s_max[i]);
-    const int k = cbl_scale_exp(mx);
-    const float sc = ldexpf(1.f, -k);
-    if (threadIdx.x == 0) xinv[blockIdx.x] = ldexpf(1.f, k);
-    for (int c = threadIdx.x; c < Cpad; c += 256) {
-        float v = 0.f;
-        if (b < B && c < C) {
-            int src = perms ? perms[(int64_t)m * C + c] : c;
-            v = cbl_load_in(x, xdtype, (int64_t)b * ldx + src) * sc;
-        }
-        dst[c] = __float2half_rn(v);
+    for (int i = 1; i < NT / 32; i++) mx = fmaxf(mx, s_max[i]);
+    const int k2 = cbl_scale_exp(mx);
+    const float sc = ldexpf(1.f, -k2);
+    if (tid == 0) xinv[blockIdx.x] = ldexpf(1.f, k2);
+    auto put = [&](int c, const float (&t)[8]) {
+        uint4 o;
+        __half2 h0 = __floats2half2_rn(t[0] * sc, t[1] * sc), h1 = __floats2half2_rn(t[2] * sc, t[3] * sc);
+        __half2 h2 = __floats2half2_rn(t[4] * sc, t[5] * sc), h3 = __floats2half2_rn(t[6] * sc, t[7] * sc);
+        o.x = *(uint32_t*)&h0; o.y = *(uint32_t*)&h1; o.z = *(uint32_t*)&h2; o.w = *(uint32_t*)&h3;
+        *(uint4*)(dst + c) = o;
+    };
+#pragma unroll
+    for (int j = 0; j < PREP_NV; j++) {
+        const int c = (j * NT + tid) * 8;
+        if (c < Cpad) put(c, v[j]);
     }
+    for (int c = PREP_NV * STEP + tid * 8; c < Cpad; c += STEP) {
+        float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (b < B && c < C) prep_load8<VEC>(x, xdtype, row, c, C, perm, t);
+        put(c, t);
+    }
+}
+
+template <int NT>
+static cudaError_t prep_launch(bool vec, cudaLaunchConfig_t& cfg, const void* x, int xdtype, int B, int C, int64_t ldx, const int32_t* perms,
+                               int Bpad, int Cpad, __half* xp, float* xinv) {
+    cfg.blockDim = dim3(NT);
+    if (vec) return cudaLaunchKernelEx(&cfg, k_prep_x<NT, true>, x, xdtype, B, C, ldx, perms, Bpad, Cpad, xp, xinv);
+    return cudaLaunchKernelEx(&cfg, k_prep_x<NT, false>, x, xdtype, B, C, ldx, perms, Bpad, Cpad, xp, xinv);
 }
 
 extern "C" int cbl_prep_x(const void* x, int xdtype, int32_t B, int32_t C, int64_t ldx, const int32_t* perms, int32_t M,
@@ -63,6 +129,7 @@ extern "C" int cbl_prep_x(const void* x, int xdtype, int32_t B, int32_t C, int64
     if (!x || !xp || B <= 0 || C <= 0 || M <= 0 || ldx < C) return CBL_EINVAL;
     if (xdtype != CBL_F16 && xdtype != CBL_BF16 && xdtype != CBL_F32) return CBL_EINVAL;
     if (M > 1 && !perms) return CBL_EINVAL;
+    if ((uintptr_t)xp % 16) return CBL_EINVAL;
     int Bpad = (B + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
     float* xinv = (float*)((__half*)xp + (int64_t)M * Bpad * Cpad);
     cudaLaunchAttribute attr[1];
@@ -73,9 +140,15 @@ extern "C" int cbl_prep_x(const void* x, int xdtype, int32_t B, int32_t C, int64
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(M * Bpad);
-    cfg.blockDim = dim3(256);
-    CBL_CUDA(cudaLaunchKernelEx(&cfg, k_prep_x, x, xdtype, (int)B, (int)C, ldx, M > 1 ? perms : (const int32_t*)nullptr, Bpad, Cpad,
-                                (__half*)xp, xinv));
+    const int esz = xdtype == CBL_F32 ? 4 : 2;
+    const bool vec = M == 1 && C % 8 == 0 && (uintptr_t)x % 16 == 0 && (B == 1 || (ldx * esz) % 16 == 0);
+    const int32_t* pp = M > 1 ? perms : nullptr;
+    // about three to five loads per thread: enough in flight to hide their latency, few enough to keep the row in registers
+    cudaError_t e;
+    if (C <= 4096) e = prep_launch<128>(vec, cfg, x, xdtype, B, C, ldx, pp, Bpad, Cpad, (__half*)xp, xinv);
+    else if (C <= 8192) e = prep_launch<256>(vec, cfg, x, xdtype, B, C, ldx, pp, Bpad, Cpad, (__half*)xp, xinv);
+    else e = prep_launch<512>(vec, cfg, x, xdtype, B, C, ldx, pp, Bpad, Cpad, (__half*)xp, xinv);
+    CBL_CUDA(e);
     return cbl_check_launch();
 }
 
