@@ -328,6 +328,37 @@ int cbl_repack_x16(const cbl_packed* m, void* out, cbl_stream s);
 size_t cbl_gemv_x16_workspace_bytes(int32_t R);
 int cbl_gemv_x16(const cbl_x16* m, const void* xp, int32_t B, void* y, int ydtype, int64_t ldy, void* workspace, cbl_stream s);
 
+/* ------------------------------------------------------------------------------------------
+ * Book-in-copies layout ("b3") for 1..128 tokens on tcgen05.mma with the weight rows as the M side: tiles of 128
+ * row positions (rows grouped by column order, padded per order), k-blocks of 64 columns; a tag is stored as the slot
+ * of its codeword in one of two or three rotated copies of the book in shared memory, the copies chosen at load time so that
+ * the eight rows read together hit different banks.  16 bits per tag.  d = 8, bits = 12, G = 1; books = 2 stored as
+ * a second run; M >= 1 column orders.
+ * replaces shapequant/kernels/gemv.py:107-170 and batched_runs.py:745-771 for these token counts.
+ * ------------------------------------------------------------------------------------------ */
+typedef struct cbl_b3 {
+    int32_t R, C, books, M, ntile, copies;
+    const void* words;                 /* uint32 [books][ntile][ceil(C / 64)][128][4] */
+    const int32_t* tile_rows;          /* int32 [ntile * 128] source row per position, -1 = padding; NULL (M == 1): the position itself */
+    const int32_t* tile_order;         /* int32 [ntile] column order of a tile when M > 1 */
+    const void* table;                 /* fp16 [4096, 8] */
+    const void* table2;                /* fp16 [4096, 8] when books == 2 */
+    const void* row_scale;             /* fp16 [R] */
+    const void* bias;                  /* [R] in y's type, or NULL: y = round(round(product) + bias) */
+} cbl_b3;
+
+int32_t cbl_gemm_b3_max_tokens(int32_t copies);     /* 3 copies: 16; 2 copies: 128 (the activations need the room) */
+size_t cbl_b3_bytes(int32_t ntile, int32_t C, int32_t books);
+int cbl_repack_b3(const cbl_packed* m, const int32_t* tile_rows, int32_t ntile, int32_t copies, void* out, cbl_stream s);
+/* Up to 4 matrices that share the input x [ntok, >= C] (row stride ldx) and its column orders (perms int32 [M, C] when
+ * M > 1): ys[i][t * ldy + r] = round(row_scale[r] * sum_c W_i[r, c] x[t, c]), ntok up to cbl_gemm_b3_max_tokens.  stage: cbl_prep_x_bytes(ntok, C,
+ * M) bytes, 16-byte aligned.  workspace: cbl_gemm_b3_workspace_bytes bytes (arrival counters, zero before the first call
+ * and left zero, then partial sums).  Results do not depend on timing: partial sums are added in a fixed order. */
+size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int32_t ntok);
+int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
+                int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s);
+int cbl_gemm_b3_status(void* workspace, cbl_stream s);
+
 /* Two-phase prefill for many tokens and for matrices with several column orders: decode the matrix ONCE
  * into a 16-bit scratch, then multiply with a TMA-fed tcgen05 GEMM (both operands by TMA, accumulators in
  * tensor memory).

@@ -44,6 +44,13 @@ class X16(Structure):
                 ("words", c_void_p), ("table", c_void_p), ("table2", c_void_p), ("row_scale", c_void_p)]
 
 
+class B3(Structure):
+    """struct cbl_b3: book-in-copies layout for 1..128 tokens."""
+    _fields_ = [("R", c_int32), ("C", c_int32), ("books", c_int32), ("M", c_int32), ("ntile", c_int32), ("copies", c_int32),
+                ("words", c_void_p), ("tile_rows", c_void_p), ("tile_order", c_void_p), ("table", c_void_p),
+                ("table2", c_void_p), ("row_scale", c_void_p), ("bias", c_void_p)]
+
+
 L8_MAX_ORDERS = 16
 
 
@@ -77,6 +84,13 @@ SIGNATURES = {
     "cbl_repack_x16": (c_int, [POINTER(Packed), c_void_p, c_void_p]),
     "cbl_gemv_x16_workspace_bytes": (c_size_t, [c_int32]),
     "cbl_gemv_x16": (c_int, [POINTER(X16), c_void_p, c_int32, c_void_p, c_int, c_int64, c_void_p, c_void_p]),
+    "cbl_gemm_b3_max_tokens": (c_int32, [c_int32]),
+    "cbl_b3_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
+    "cbl_repack_b3": (c_int, [POINTER(Packed), c_void_p, c_int32, c_int32, c_void_p, c_void_p]),
+    "cbl_gemm_b3_workspace_bytes": (c_size_t, [POINTER(B3), c_int32, c_int32]),
+    "cbl_gemm_b3": (c_int, [POINTER(B3), c_int32, c_void_p, c_int, c_int32, c_int64, c_void_p, POINTER(c_void_p), c_int, c_int64, c_void_p,
+                            c_void_p, c_void_p]),
+    "cbl_gemm_b3_status": (c_int, [c_void_p, c_void_p]),
     "cbl_l8_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "cbl_repack_l8": (c_int, [POINTER(Packed), c_void_p, c_void_p]),
     "cbl_l8r_bytes": (c_size_t, [c_int32, c_int32, c_int32]),

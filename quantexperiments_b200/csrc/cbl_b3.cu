@@ -1,0 +1,795 @@
+// Products of 1..64 tokens straight from the packed tags (d = 8, 12-bit tags, 4096-entry fp16 books, one or two summed
+// books, any number of column orders) with the weight rows as the M side of tcgen05.mma.
+//
+// A decode thread owns a weight row.  Per k-block (64 columns = 8 chunks) it gathers the row's eight 16-byte codewords
+// from shared memory and writes them from registers into its lane of tensor memory (tcgen05.st); the MMA takes the
+// decoded tile from there (A, 128 rows x 16) and the staged fp16 activations from shared memory (B, N = tokens).
+//
+// What bounds it is the gather: eight lanes' 16-byte reads go through the shared-memory banks at a time, and eight
+// random codewords hit the fullest of the eight 16-byte bank groups 2.6 times on average (2.95 lookups per clock and
+// SM measured).  So shared memory holds the book THREE times, copy j with the codewords of every group of eight
+// rotated by {0, 1, 3}[j], and the load-time re-layout picks, for every eight rows that are read together, the copies
+// that spread their codewords over the bank groups (a maximum matching; 1.24 reads of the fullest group are left):
+// 5.7 lookups per clock and SM.  A tag becomes a 16-bit slot number of the three copies.  The MMAs (M = 128, K = 16: 21 clocks at
+// 16 tokens, 27 at 32, 43 at 64) hide behind the gathers up to 64 tokens.
+//
+// Work split: the (tile of 128 rows, k-block) units of all matrices of a group form one sequence that is cut into equal
+// ranges, one per block (one block per SM).  Two summed books are two such sequences over the same output tiles.  A
+// block's share of a tile is a piece; pieces of a tile that several blocks share are written to a slot of the
+// work space each, and the block that arrives last adds them in a fixed order and writes the outputs (so results are
+// reproducible bit for bit; nobody waits for anybody).
+//
+// Decoding does not depend on the activations: it starts while the kernel before this one is still running, as far as
+// the ring of decoded k-blocks in tensor memory reaches.
+#include <type_traits>
+#include "cbl_tc.cuh"
+
+namespace {
+
+constexpr int B3_ROWS = 128;                     // weight rows per tile
+constexpr int B3_KB = 64;                        // columns per k-block
+constexpr int B3_NMAX = 128;                     // tokens per launch
+constexpr int B3_3COPIES_MAX = 16;               // tokens up to which the book has three copies, two above
+constexpr int B3_DEC_WARPS = 16, B3_DEC = B3_DEC_WARPS * 32;
+constexpr int B3_EPI_WARP = 16, B3_X_WARP = 20, B3_MMA_WARP = 21, B3_X2_WARP = 22, B3_THREADS = 23 * 32;
+constexpr int B3_BAR_STAGE = 4;                  // named barriers of the stages: 4, 5, 6
+constexpr int B3_SMEM = 229376;                  // copies of the book and the ring of the activations
+constexpr int B3_MAX_RX = 8, B3_MAX_ST = 3;
+constexpr int B3_MAX_MATS = 4, B3_MAX_SEGS = 2 * B3_MAX_MATS;
+constexpr int B3_MAX_TILES = 16320;              // output tiles of a launch: one arrival counter each
+constexpr int B3_CTL_WORDS = 16384;              // status word at 0, counters from 64
+constexpr int B3_MAX_PIECES = 128;               // pieces of a block
+constexpr uint32_t B3_WAIT_LIMIT = 1u << 18;
+
+struct B3Seg {                                   // one book of one matrix: tiles gi0 .. gi1 - 1 of the sequence
+    const uint4* words;
+    const uint4* table;
+    int gi0, gi1, mi;
+};
+struct B3Mat {
+    const __half* row_scale;
+    const int32_t* tile_rows;                    // source row of every row position, -1 = padding; NULL: the position itself
+    const int32_t* tile_order;                   // column order of a tile; NULL: one order
+    const void* bias;                            // in y's type, or NULL
+    void* y;
+    int R, ntile, gi0, books, ctr0;
+};
+struct B3Launch {
+    int nseg, nkb, npad, xrows, ntok, NST, RX, XU, PP, Bpad;
+    int ks, q, rem;                              // ks > 0: ks blocks share a tile; else blocks have q units, the first rem one more
+    int64_t ldy;
+    const float* xinv;
+    float* partial;
+    unsigned int* counters;
+    unsigned int* status;
+    B3Seg seg[B3_MAX_SEGS];
+    B3Mat mat[B3_MAX_MATS];
+};
+
+__device__ __forceinline__ bool b3_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Bounded wait.  One that expires marks the block aborted (the launch reports it) and the roles go on in step: the named
+// barriers between them need every arrival.
+__device__ __forceinline__ void b3_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+    for (uint32_t i = 0; i < B3_WAIT_LIMIT; i++)
+        if (b3_test(bar, parity)) return;
+    *abort = 1;
+}
+// k-blocks kb .. of 64 columns of the staged rows c1 .. (the map's third dimension counts k-blocks).
+__device__ __forceinline__ void b3_tma_3d(uint32_t dst, const CUtensorMap* map, int c1, int kb, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(map), "r"(0), "r"(c1), "r"(kb), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void b3_sts128(uint32_t addr, const uint4& v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void b3_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void b3_tmem_st16(uint32_t taddr, const uint4 (&c)[4]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(c[0].x), "r"(c[0].y), "r"(c[0].z), "r"(c[0].w), "r"(c[1].x), "r"(c[1].y), "r"(c[1].z), "r"(c[1].w), "r"(c[2].x), "r"(c[2].y),
+        "r"(c[2].z), "r"(c[2].w), "r"(c[3].x), "r"(c[3].y), "r"(c[3].z), "r"(c[3].w)
+        : "memory");
+}
+// Outputs round once to y's type; a bias is added to the rounded product and the sum rounded again, as two operators would.
+template <typename T>
+__device__ __forceinline__ T b3_round(float v, bool bias, float b) {
+    const T o = cbl_cvt_out<T>(v);
+    return bias ? cbl_cvt_out<T>((float)o + b) : o;
+}
+
+// Copy j of the book holds codeword e of the group of eight e / 8 at position (e + b3_rot(e / 8, j)) mod 8 of the group.
+__device__ __forceinline__ uint32_t b3_rot(uint32_t group, int j) {
+    const uint32_t r1 = group % 7u;
+    return j == 0 ? 0u : j == 1 ? 1u + r1 : 1u + (r1 + 1u + group % 42u / 7u) % 7u;
+}
+
+template <int COPIES, typename T>
+__global__ void __launch_bounds__(B3_THREADS, 1)
+k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap xmap1, const __grid_constant__ B3Launch P) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long s_bar[B3_MAX_ST + 2 * B3_MAX_RX + 4];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort, s_nfin;
+    __shared__ int s_fin[B3_MAX_PIECES];                       // tiles (as gi of their first book) that this block has to finish
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
+    const int cta = (int)blockIdx.x;
+    const int nkb = P.nkb;
+    auto start = [&](int c) { return P.ks > 0 ? c / P.ks * nkb + c % P.ks * nkb / P.ks : P.q * c + min(c, P.rem); };      // first unit of block c
+    auto owner = [&](int u) {                                  // block that has unit u
+        if (P.ks > 0) return u / nkb * P.ks + ((u % nkb + 1) * P.ks - 1) / nkb;
+        const int big = P.rem * (P.q + 1);
+        return u < big ? u / (P.q + 1) : P.rem + (u - big) / P.q;
+    };
+    const int u0 = start(cta), u1 = start(cta + 1), nu = u1 - u0, nq = (nu + 3) / 4;
+    const uint32_t sbase = cbl_smem_u32(smem), bar0 = cbl_smem_u32(s_bar);
+    const int NST = P.NST, RX = P.RX, XU = P.XU;
+    auto empty_a = [&](int s) { return bar0 + 8u * s; };
+    auto full_x = [&](int s) { return bar0 + 8u * (B3_MAX_ST + s); };
+    auto empty_x = [&](int s) { return bar0 + 8u * (B3_MAX_ST + B3_MAX_RX + s); };
+    auto acc_full = [&](int b) { return bar0 + 8u * (B3_MAX_ST + 2 * B3_MAX_RX + b); };
+    auto acc_empty = [&](int b) { return bar0 + 8u * (B3_MAX_ST + 2 * B3_MAX_RX + 2 + b); };
+    const uint32_t x_base = sbase + COPIES * 65536u;
+    const uint32_t xbytes = (uint32_t)P.xrows * 128u, xstage = xbytes * (uint32_t)XU, a_col0 = 2u * (uint32_t)P.npad;
+    auto seg_of = [&](int gi) { int s = 0; while (s + 1 < P.nseg && gi >= P.seg[s].gi1) s++; return s; };
+    auto wait = [&](uint32_t bar, uint32_t parity) { return b3_wait(bar, parity, &s_abort); };
+    auto slot_of = [&](int c, int gi) { return P.partial + (size_t)(c * P.PP + gi - start(c) / nkb) * (size_t)(P.npad * B3_ROWS); };
+
+    if (tid == 0) {
+        s_abort = s_nfin = 0;
+        for (int s = 0; s < NST; s++) mbar_init(empty_a(s), 1);
+        for (int s = 0; s < RX; s++) { mbar_init(full_x(s), 1); mbar_init(empty_x(s), 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == B3_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cbl_smem_u32(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // the rotated copies of a book, by the decode threads (blocks start at different places: all of them read the same 64 KB)
+    auto load_book = [&](const uint4* __restrict__ tb) {
+        uint4 v[4096 / B3_DEC];
+#pragma unroll
+        for (int k = 0; k < 4096 / B3_DEC; k++) v[k] = __ldg(tb + ((k + cta) & (4096 / B3_DEC - 1)) * B3_DEC + tid);
+#pragma unroll
+        for (int k = 0; k < 4096 / B3_DEC; k++) {
+            const uint32_t e = (uint32_t)(((k + cta) & (4096 / B3_DEC - 1)) * B3_DEC + tid);
+#pragma unroll
+            for (int j = 0; j < COPIES; j++) b3_sts128(sbase + (uint32_t)j * 65536u + ((e & ~7u) | ((e + b3_rot(e >> 3, j)) & 7u)) * 16u, v[k]);
+        }
+    };
+    // decode thread = row (tid & 127) of a tile; a warpgroup takes every fourth unit of the block's range.  A run is the
+    // part of the range in one book: its tags lie back to back, 16 bytes per row and unit.
+    const int wg = warp >> 2;
+    const uint4* tp = nullptr;                                 // this thread's tags of the run's first unit
+    int rn = 0, rj = 0;                                        // units of the run; this warpgroup's first
+    uint4 q0, q1, q2, q3;
+    auto tags = [&](int j) { return j < rn ? cbl_ldg_stream(tp + (int64_t)j * B3_ROWS) : make_uint4(0, 0, 0, 0); };
+    auto begin_run = [&](const B3Seg& sg, int u) {
+        rn = min(u1, sg.gi1 * nkb) - u;
+        rj = (wg - (u - u0)) & 3;
+        tp = sg.words + (int64_t)(u - sg.gi0 * nkb) * B3_ROWS + (tid & (B3_ROWS - 1));
+        q0 = tags(rj); q1 = tags(rj + 4); q2 = tags(rj + 8); q3 = tags(rj + 12);
+    };
+    if (warp < B3_DEC_WARPS) {
+        const B3Seg& sg = P.seg[seg_of(u0 / nkb)];
+        begin_run(sg, u0);
+        load_book(sg.table);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    // The stages of the ring that are free, seen from its next one on: every lane tests one barrier, how many in a row
+    // have completed their phase (at least one, also when the wait has expired).  A test queues behind the gathers, some
+    // hundred clocks, so it is made for all stages at once.
+    auto free_stages = [&](auto&& barrier, int stage, uint32_t par, int len) {
+        const int sl = stage + lane;
+        const bool wr = sl >= len;
+        const uint32_t bar = barrier(lane < len ? (wr ? sl - len : sl) : 0), ph = par ^ (uint32_t)wr;
+        for (uint32_t i = 0; i < B3_WAIT_LIMIT; i++) {
+            const uint32_t m = __ballot_sync(0xffffffffu, lane < len && b3_test(bar, ph));
+            if (m & 1u) return __ffs(~m) - 1;
+        }
+        s_abort = 1;
+        return 1;
+    };
+
+    if (warp < B3_DEC_WARPS) {
+        // ---------------- decode
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + a_col0 + (uint32_t)wg * 32u;
+        int st = 0, credit = 0;                                // stage of this warpgroup's next unit, stages known to be free
+        uint32_t par = 1;
+        auto room = [&]() {
+            if (credit == 0) credit = free_stages(empty_a, st, par, NST);
+            credit--;
+        };
+        auto done = [&]() {                                    // this warp's part of the stage is in tensor memory
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            asm volatile("bar.arrive %0, %1;" ::"r"(B3_BAR_STAGE + st), "n"(B3_DEC + 64) : "memory");
+            if (++st == NST) { st = 0; par ^= 1u; }
+        };
+        // A unit is gathered in two halves of four codewords; the next half is always on its way while one is stored.
+        auto gather = [&](uint32_t w0, uint32_t w1, uint4 (&cw)[4]) {
+            cw[0] = cbl_lds128(sbase + (w0 & 0x3FFF0u));
+            cw[1] = cbl_lds128(sbase + ((w0 >> 14) & 0x3FFF0u));
+            cw[2] = cbl_lds128(sbase + (w1 & 0x3FFF0u));
+            cw[3] = cbl_lds128(sbase + ((w1 >> 14) & 0x3FFF0u));
+        };
+        uint4 ca[4], cb[4];
+        auto unit = [&](const uint4& e, const uint4& next) {
+            gather(e.z, e.w, cb);
+            room();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            b3_tmem_st16(lane_addr + (uint32_t)st * 128u, ca);
+            gather(next.x, next.y, ca);
+            b3_tmem_st16(lane_addr + (uint32_t)st * 128u + 16u, cb);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            done();
+        };
+        int mine = 0;                                          // units this warpgroup has decoded
+        for (int u = u0; u < u1;) {
+            if (rj < rn) gather(q0.x, q0.y, ca);
+            for (int j = rj; j < rn; j += 16) {                // (beyond the run the tags are zero: slot 0)
+                uint4 c = q0;
+                q0 = tags(j + 16);
+                unit(c, q1);
+                if (j + 4 < rn) { c = q1; q1 = tags(j + 20); unit(c, q2); }
+                if (j + 8 < rn) { c = q2; q2 = tags(j + 24); unit(c, q3); }
+                if (j + 12 < rn) { c = q3; q3 = tags(j + 28); unit(c, q0); }
+            }
+            if (rj < rn) mine += (rn - rj + 3) / 4;
+            u += rn;
+            if (u < u1) {                                      // another book: everybody is done with the one before
+                const B3Seg& sg = P.seg[seg_of(u / nkb)];
+                begin_run(sg, u);
+                asm volatile("bar.sync 1, %0;" ::"n"(B3_DEC) : "memory");
+                load_book(sg.table);
+                asm volatile("bar.sync 1, %0;" ::"n"(B3_DEC) : "memory");
+            }
+        }
+        if (mine < nq) { room(); done(); }                     // no unit of the last stage: arrive all the same
+    } else if (warp == B3_MMA_WARP) {
+        // ---------------- MMA issue, four units at a time.  A stage is announced through a named barrier, which does not
+        // queue with the gathers; counters depend on nothing but the block's range, so that they stay in uniform registers.
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(P.npad >> 3) << 17) | ((uint32_t)(B3_ROWS >> 4) << 24);
+        int st = 0, xs = 0, xk = 0, pc = 0, kb = u0 % nkb;
+        for (int i = 0; i < nu; i += 4) {
+            asm volatile("bar.sync %0, %1;" ::"r"(B3_BAR_STAGE + st), "n"(B3_DEC + 64) : "memory");
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int n = min(4, nu - i);
+            for (int k = 0; k < n;) {                          // the units of one piece at a time
+                const int m = min(n - k, nkb - kb), b = pc & 1;
+                const bool first = kb == 0 || (i == 0 && k == 0), end = i + k + m == nu, last = kb + m == nkb || end;
+                if (first && pc > 1) {
+                    wait(acc_empty(b), ((pc >> 1) & 1) ^ 1);
+                    __syncwarp();
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+                // nothing but straight code in here: with a wait inside, the compiler no longer sees a single thread and issues an
+                // MMA every 130 clocks (measured) instead of every 20
+                const uint32_t d = tmem + (uint32_t)(b * P.npad);
+                if (m == 4) {                                  // all of a stage: no loop either
+                    const int xs1 = XU == 4 ? xs : (xs + 1 == RX ? 0 : xs + 1);
+                    const uint64_t x0 = umma_desc_sw128(x_base + (uint32_t)xs * xstage), x1 = umma_desc_sw128(x_base + (uint32_t)xs1 * xstage + (XU == 4 ? 2 * xbytes : 0u));
+                    const uint32_t a = tmem + a_col0 + (uint32_t)(st * 128), xw = xbytes >> 4;
+                    const uint32_t acc0 = first ? 0u : 1u;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + kk * 8, x0 + kk * 2, idesc, kk == 0 ? acc0 : 1u);
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 32 + kk * 8, x0 + xw + kk * 2, idesc, 1u);
+                        if (XU == 2) umma_commit(empty_x(xs));
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 64 + kk * 8, x1 + kk * 2, idesc, 1u);
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 96 + kk * 8, x1 + xw + kk * 2, idesc, 1u);
+                        umma_commit(empty_x(xs1));
+                        umma_commit(empty_a(st));
+                        if (last) umma_commit(acc_full(b));
+                    }
+                } else if (elect_one()) {
+                    int x = xs, xi = xk;
+                    for (int t = 0; t < m; t++) {
+                        const uint64_t xd = umma_desc_sw128(x_base + (uint32_t)x * xstage + (uint32_t)xi * xbytes);
+                        const uint32_t a = tmem + a_col0 + (uint32_t)(st * 128 + (k + t) * 32);
+#pragma unroll
+                        for (int kk = 0; kk < B3_KB / 16; kk++) umma_f16_ta(d, a + kk * 8, xd + kk * 2, idesc, (first && t == 0 && kk == 0) ? 0u : 1u);
+                        if (++xi == XU || (end && t == m - 1)) {
+                            umma_commit(empty_x(x));
+                            xi = 0;
+                            if (++x == RX) x = 0;
+                        }
+                    }
+                    if (last) umma_commit(acc_full(b));
+                    if (k + m == n) umma_commit(empty_a(st));
+                }
+                __syncwarp();
+                kb += m;
+                if (last) { kb = 0; pc++; }
+                for (xk += m; xk >= XU; xk -= XU) xs = xs + 1 == RX ? 0 : xs + 1;
+                k += m;
+            }
+            if (++st == NST) st = 0;
+        }
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next kernel's blocks may take the SMs as they empty
+    } else if (warp == B3_X_WARP) {
+        // ---------------- activations by TMA: XU units per stage, in order
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        int xs = 0, credit = 0, kb = u0 % nkb, gi = u0 / nkb;
+        uint32_t par = 1;
+        auto row_of = [&](int g) {                             // first activation row of the tile's column order
+            const B3Seg& sg = P.seg[seg_of(g)];
+            const B3Mat& m = P.mat[sg.mi];
+            return m.tile_order ? __ldg(m.tile_order + g - sg.gi0) * P.Bpad : 0;
+        };
+        int c1 = row_of(gi);
+        for (int i = 0; i < nu; i += XU) {
+            if (credit == 0) credit = free_stages(empty_x, xs, par, RX);
+            credit--;
+            const int n = min(XU, nu - i);
+            const uint32_t dst = x_base + (uint32_t)xs * xstage;
+            if (kb + n <= nkb) {                               // one copy brings XU k-blocks (at the end of the range more than are used)
+                if (elect_one()) {
+                    mbar_expect_tx(full_x(xs), xstage);
+                    b3_tma_3d(dst, &xmap, c1, kb, full_x(xs));
+                }
+                kb += n;
+            } else {                                           // across the border of a tile: one by one
+                if (elect_one()) mbar_expect_tx(full_x(xs), (uint32_t)n * xbytes);
+                __syncwarp();
+                for (int k = 0; k < n; k++) {
+                    if (kb == nkb) { kb = 0; c1 = row_of(++gi); }
+                    if (elect_one()) b3_tma_3d(dst + (uint32_t)k * xbytes, &xmap1, c1, kb, full_x(xs));
+                    __syncwarp();
+                    kb++;
+                }
+            }
+            if (kb == nkb && i + n < nu) { kb = 0; c1 = row_of(++gi); }
+            __syncwarp();
+            if (++xs == RX) { xs = 0; par ^= 1u; }
+        }
+    } else if (warp == B3_X2_WARP) {
+        // ---------------- tells the MMA warp that a stage's activations have landed (and, like the decode warps, only when the
+        // stage NST before it has been multiplied: a barrier takes one arrival of everybody at a time)
+        int st = 0, xs = 0, credit = 0;
+        uint32_t par = 0, pst = 1;
+        for (int i = 0; i < nu; i += 4) {
+            if (credit == 0) credit = free_stages(empty_a, st, pst, NST);
+            credit--;
+            for (int k = 0; k < 4 && i + k < nu; k += XU) {
+                wait(full_x(xs), par);
+                if (++xs == RX) { xs = 0; par ^= 1u; }
+            }
+            __syncwarp();
+            asm volatile("bar.arrive %0, %1;" ::"r"(B3_BAR_STAGE + st), "n"(B3_DEC + 64) : "memory");
+            if (++st == NST) { st = 0; pst ^= 1u; }
+        }
+    } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        float xv[B3_NMAX / 32];                                // factors that undo the token scales: tokens lane, lane + 32, ..
+        // ---------------- epilogue: warp w reads TMEM lanes 32 (w & 3) .. (= rows of the tile); columns = tokens
+        const int q = warp & 3, row = q * 32 + lane;
+        int pc = 0;
+        for (int u = u0; u < u1; pc++) {
+            const int gi = u / nkb, n = min((gi + 1) * nkb, u1) - u, b = pc & 1;
+            const B3Seg& sg = P.seg[seg_of(gi)];
+            const B3Mat& m = P.mat[sg.mi];
+            const int tile = gi - sg.gi0, p = tile * B3_ROWS + row;
+            const bool whole = n == nkb && m.books == 1;
+            int r = -1;
+            float rs = 0.f;
+            if (whole) {
+                r = m.tile_rows ? __ldg(m.tile_rows + p) : p;
+                if (r >= m.R) r = -1;
+                rs = r >= 0 ? __half2float(__ldg(m.row_scale + r)) : 0.f;
+            }
+            if (pc == 0 || m.tile_order) {
+                const float* xi = P.xinv + (m.tile_order ? __ldg(m.tile_order + tile) * P.Bpad : 0);
+#pragma unroll
+                for (int k = 0; k < B3_NMAX / 32; k++) xv[k] = lane + 32 * k < P.ntok ? __ldcg(xi + lane + 32 * k) : 0.f;
+            }
+            float* mine = whole ? nullptr : slot_of(cta, gi) + row;
+            int np = 0;                                        // pieces of this output tile
+            if (!whole)
+                for (int k = 0; k < m.books; k++) {
+                    const int g = (m.gi0 + k * m.ntile + tile) * nkb;
+                    np += owner(g + nkb - 1) - owner(g) + 1;
+                }
+            unsigned int* const ctr = P.counters + m.ctr0 + tile;
+            T* const yr = (T*)m.y + max(r, 0);
+            const bool put = whole && r >= 0;
+            const float brow = put && m.bias ? (float)((const T*)m.bias)[r] : 0.f;
+            const bool bias = m.bias != nullptr;
+            const int64_t ldy = P.ldy;
+            const int ntok = P.ntok;
+            wait(acc_full(b), (pc >> 1) & 1);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int n0 = 0; n0 < ntok; n0 += 16) {
+                uint32_t v[16];
+                const float xw = n0 < 32 ? xv[0] : n0 < 64 ? xv[1] : n0 < 96 ? xv[2] : xv[3];
+                b3_tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * P.npad + n0), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) * __shfl_sync(0xffffffffu, xw, (n0 + j) & 31));
+                const int nn = ntok - n0;
+                if (!whole) {
+                    float* o = mine + n0 * B3_ROWS;
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (j < nn) __stcg(o + j * B3_ROWS, __uint_as_float(v[j]));
+                } else if (put) {
+                    T* o = yr + n0 * ldy;
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        if (j < nn) *o = b3_round<T>(__uint_as_float(v[j]) * rs, bias, brow);
+                        o += ldy;
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty(b));
+            if (!whole) {
+                asm volatile("bar.sync 2, 128;" ::: "memory");
+                if (warp == B3_EPI_WARP && lane == 0) {
+                    unsigned int before;                       // release: this block's pieces, acquire: the others' (read after the barrier below)
+                    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(ctr) : "memory");
+                    if (before == (unsigned)(np - 1)) {
+                        *ctr = 0;
+                        s_fin[s_nfin++] = m.gi0 + tile;
+                    }
+                }
+            }
+            u += n;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (s_abort && tid == 0) atomicExch(P.status, 1u);
+    if (warp == B3_MMA_WARP) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+    // ---------------- tiles whose last piece came from this block: all of its threads add the pieces (five groups of 128 rows
+    // share the tokens; book after book, block after block - the order does not depend on who came last) and write y
+    const int nfin = s_abort ? 0 : s_nfin;
+    if (nfin && warp < 20) {
+        __threadfence();
+        const int row = tid & (B3_ROWS - 1), grp = tid >> 7;
+        for (int f = 0; f < nfin; f++) {
+            const int gi = s_fin[f];
+            const B3Mat& m = P.mat[P.seg[seg_of(gi)].mi];
+            const int tile = gi - m.gi0;
+            int r = m.tile_rows ? __ldg(m.tile_rows + tile * B3_ROWS + row) : tile * B3_ROWS + row;
+            if (r >= m.R) r = -1;
+            const float rs = r >= 0 ? __half2float(__ldg(m.row_scale + r)) : 0.f;
+            const bool bias = m.bias != nullptr;
+            const float brow = r >= 0 && bias ? (float)((const T*)m.bias)[r] : 0.f;
+            T* const yr = (T*)m.y + max(r, 0);
+            const size_t slot = (size_t)(P.npad * B3_ROWS);
+            const int ntok = P.ntok;
+            // eight loads in flight: eight pieces of a token, or two pieces of four tokens
+            auto add = [&](auto tokens) {
+                constexpr int TJ = decltype(tokens)::value, H = 8 / TJ;
+                for (int n = grp; n < ntok; n += 5 * TJ) {
+                    float sum[TJ];
+#pragma unroll
+                    for (int j = 0; j < TJ; j++) sum[j] = 0.f;
+                    for (int k = 0; k < m.books; k++) {
+                        const int g = gi + k * m.ntile, c0 = owner(g * nkb), ce = owner(g * nkb + nkb - 1);
+                        // a tile is the last piece of its first block and the first piece of the others
+                        const int ord = g - start(c0) / nkb;
+                        for (int c = c0; c <= ce; c += H) {
+                            float v[H][TJ];
+#pragma unroll
+                            for (int h = 0; h < H; h++) {
+                                const int cc = min(c + h, ce);
+                                const float* src = P.partial + row + (size_t)(cc * P.PP + (cc == c0 ? ord : 0)) * slot;
+#pragma unroll
+                                for (int j = 0; j < TJ; j++) v[h][j] = __ldcg(src + min(n + 5 * j, ntok - 1) * B3_ROWS);
+                            }
+#pragma unroll
+                            for (int h = 0; h < H; h++)
+                                if (c + h <= ce) {
+#pragma unroll
+                                    for (int j = 0; j < TJ; j++) sum[j] += v[h][j];
+                                }
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < TJ; j++)
+                        if (r >= 0 && n + 5 * j < ntok) yr[(int64_t)(n + 5 * j) * P.ldy] = b3_round<T>(sum[j] * rs, bias, brow);
+                }
+            };
+            if (ntok <= 5) add(std::integral_constant<int, 1>());
+            else add(std::integral_constant<int, 4>());
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------ re-layout
+//
+// uint32 [book][tile][k-block][128 rows][4]: word k of a row and k-block holds the slots of its chunks 2k and 2k + 1 as
+// byte offsets / 16 at bits 4..17 and 18..31 (the reader masks and shifts, nothing more).  A thread places two chunks of
+// eight consecutive row positions, the rows whose codewords one shared-memory pass reads.
+// bk[j]: nibble i = bank group of row i's codeword in copy j; result: nibble i = copy chosen for row i.
+__device__ __forceinline__ uint32_t b3_match(const uint32_t (&bk)[3], int copies) {
+    uint32_t own = 0x88888888u, choice = 0;                            // bank group -> row (8 = free)
+    uint32_t left = 0;                                                 // rows without a bank group of their own
+    auto bank = [&](int i, int j) { return ((j == 0 ? bk[0] : j == 1 ? bk[1] : bk[2]) >> (4 * i)) & 7u; };
+    for (int i = 0; i < 8; i++) {
+        // augmenting path by depth-first search: stack of (row, copy tried), a bank group is visited once
+        uint32_t rows = (uint32_t)i, tried = 0, seen = 0;
+        int depth = 0;
+        while (true) {
+            const int cur = (rows >> (4 * depth)) & 15, j = (tried >> (4 * depth)) & 15;
+            if (j == copies) {
+                if (depth == 0) { left |= 1u << i; break; }
+                depth--;
+                tried += 1u << (4 * depth);
+                continue;
+            }
+            const uint32_t b = bank(cur, j);
+            if (seen >> b & 1u) { tried += 1u << (4 * depth); continue; }
+            seen |= 1u << b;
+            const int o = (own >> (4 * b)) & 15;
+            if (o == 8) {
+                for (int k = 0; k <= depth; k++) {
+                    const int rk = (rows >> (4 * k)) & 15, jk = (tried >> (4 * k)) & 15;
+                    const uint32_t bk = bank(rk, jk);
+                    own = (own & ~(15u << (4 * bk))) | ((uint32_t)rk << (4 * bk));
+                    choice = (choice & ~(15u << (4 * rk))) | ((uint32_t)jk << (4 * rk));
+                }
+                break;
+            }
+            depth++;
+            rows = (rows & ~(15u << (4 * depth))) | ((uint32_t)o << (4 * depth));
+            tried &= ~(15u << (4 * depth));
+        }
+    }
+    uint32_t twice = 0;                                                // the rows left over double up on different groups
+    for (int i = 0; i < 8; i++)
+        if (left >> i & 1u) {
+            int jb = 0;
+            for (int j = copies - 1; j >= 0; j--)
+                if (!(twice >> bank(i, j) & 1u)) jb = j;
+            twice |= 1u << bank(i, jb);
+            choice = (choice & ~(15u << (4 * i))) | ((uint32_t)jb << (4 * i));
+        }
+    return choice;
+}
+
+__global__ void __launch_bounds__(256) k_repack_b3(cbl_packed m, const int32_t* __restrict__ tile_rows, int ntile, int nkb, int copies,
+                                                   uint32_t* __restrict__ out, int64_t nthreads) {
+    const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= nthreads) return;
+    const int cp = (int)(gid % (nkb * 4));
+    int64_t rest = gid / (nkb * 4);
+    const int g = (int)(rest & 15);
+    rest >>= 4;
+    const int tile = (int)(rest % ntile), book = (int)(rest / ntile);
+    const int nch = m.C / 8;
+    const int32_t* words = book ? m.tags2 : m.tags;
+    uint32_t word[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) word[i] = 0;
+    for (int h = 0; h < 2; h++) {
+        const int chunk = 2 * cp + h;
+        uint32_t tag[8], bk[3] = {0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int p = tile * B3_ROWS + g * 8 + i;
+            const int r = tile_rows ? tile_rows[p] : p;
+            // padding reads codeword 8 k + i: any will do (its activations are zero or its row is not written)
+            tag[i] = (r >= 0 && r < m.R && chunk < nch) ? cbl_read_tag(words + (int64_t)r * m.W, m.W, chunk, 12) : (uint32_t)i;
+#pragma unroll
+            for (int j = 0; j < 3; j++) bk[j] |= ((tag[i] + b3_rot(tag[i] >> 3, j)) & 7u) << (4 * i);
+        }
+        const uint32_t choice = b3_match(bk, copies);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t j = (choice >> (4 * i)) & 15u;
+            const uint32_t b = (j == 0 ? bk[0] : j == 1 ? bk[1] : bk[2]) >> (4 * i) & 7u, s = j * 4096u + ((tag[i] & ~7u) | b);
+            word[i] |= s << (h ? 18 : 4);
+        }
+    }
+    uint32_t* o = out + ((((int64_t)book * ntile + tile) * nkb + (cp >> 2)) * B3_ROWS + g * 8) * 4 + (cp & 3);
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i * 4] = word[i];
+}
+
+struct B3Plan { int T, U, G, PP, ks, npad, rows, NST, RX, XU; };
+
+int b3_plan(const cbl_b3* mats, int n, int ntok, B3Plan& pl) {
+    pl.T = 0;
+    int tiles = 0;
+    for (int i = 0; i < n; i++) { pl.T += mats[i].ntile * mats[i].books; tiles += mats[i].ntile; }
+    if (tiles > B3_MAX_TILES) return CBL_EUNSUPPORTED;
+    const int nkb = cbl_ceil_div(mats[0].C, B3_KB), S = cbl_sm_count();
+    if ((int64_t)pl.T * nkb > (1 << 30)) return CBL_EUNSUPPORTED;
+    pl.U = pl.T * nkb;
+    pl.npad = (ntok + 15) / 16 * 16;
+    pl.NST = (512 - 2 * pl.npad) / 128;                        // stages of four decoded k-blocks in tensor memory, beside two accumulators
+    if (pl.NST > B3_MAX_ST) pl.NST = B3_MAX_ST;
+    const int ring = B3_SMEM - mats[0].copies * 65536;
+    pl.XU = ring / (pl.npad * 512) >= 3 ? 4 : 2;               // units per stage of the activations' ring
+    // up to 8 tokens only 8 rows are brought in; the MMA (N = 16) reads the 8 rows after them as well, whatever they are, into
+    // columns that nobody looks at: the ring's last unit needs 1 KB behind it
+    pl.rows = ntok <= 8 ? 8 : pl.npad;
+    pl.RX = (ring - (pl.npad - pl.rows) * 128) / (pl.rows * 128 * pl.XU);
+    if (pl.RX > B3_MAX_RX) pl.RX = B3_MAX_RX;
+    // Blocks: as many as there are SMs, at least six k-blocks each (below that the book and the hand-over
+    // of partial sums, which grows with the tokens, cost more than the lookups).  Where whole tiles, or equal fractions of a tile, fill 85 % of the
+    // SMs the cut follows them, so that a block has one piece; otherwise ranges run across tile borders.
+    int G = S;
+    pl.ks = 0;
+    if (pl.T < S) {
+        int ks = S / pl.T;
+        const int least = 6 + ntok / 8, most = nkb / least > 1 ? nkb / least : 1;
+        if (ks > most) ks = most;
+        if (ks == most || pl.T * ks * 100 >= 85 * S) { G = pl.T * ks; pl.ks = ks; }
+    } else {
+        const int waves = cbl_ceil_div(pl.T, S), g = cbl_ceil_div(pl.T, waves);
+        if (pl.T % g == 0 && g * 100 >= 85 * S) G = g;
+    }
+    if (G > pl.U) { G = pl.U; pl.ks = 0; }
+    pl.G = G;
+    pl.PP = pl.U == 0 ? 1 : cbl_ceil_div(cbl_ceil_div(pl.U, G), nkb) + 1;
+    return pl.PP > B3_MAX_PIECES ? CBL_EUNSUPPORTED : CBL_OK;
+}
+
+int b3_check(const cbl_b3* m, const cbl_b3* first) {
+    if (!m->words || !m->table || !m->row_scale) return CBL_EINVAL;
+    if (m->books != 1 && m->books != 2) return CBL_EINVAL;
+    if (m->books == 2 && !m->table2) return CBL_EINVAL;
+    if (m->R < 0 || m->C <= 0 || m->C % 8 || m->ntile < 0 || m->M < 1) return CBL_EINVAL;
+    if (m->M > 1 && (!m->tile_rows || !m->tile_order)) return CBL_EINVAL;
+    if (!m->tile_rows && m->ntile != cbl_ceil_div(m->R, B3_ROWS)) return CBL_EINVAL;
+    if (m->copies != 2 && m->copies != 3) return CBL_EINVAL;
+    if (m->C != first->C || m->M != first->M || m->copies != first->copies) return CBL_EINVAL;      // one staged activation serves the group
+    if (((uintptr_t)m->words % 16) || ((uintptr_t)m->table % 16) || (m->table2 && (uintptr_t)m->table2 % 16)) return CBL_EINVAL;
+    return CBL_OK;
+}
+
+}  // namespace
+
+extern "C" int32_t cbl_gemm_b3_max_tokens(int32_t copies) { return copies == 3 ? B3_3COPIES_MAX : copies == 2 ? B3_NMAX : 0; }
+
+extern "C" size_t cbl_b3_bytes(int32_t ntile, int32_t C, int32_t books) {
+    if (ntile < 0 || C <= 0 || books < 1) return 0;
+    return (size_t)books * ntile * cbl_ceil_div(C, B3_KB) * B3_ROWS * 16;
+}
+
+extern "C" int cbl_repack_b3(const cbl_packed* m, const int32_t* tile_rows, int32_t ntile, int32_t copies, void* out, cbl_stream s) {
+    if (!m || !m->tags || !out || ((uintptr_t)out % 16) || ntile < 0 || (copies != 2 && copies != 3)) return CBL_EINVAL;
+    if (m->d != 8 || m->bits != 12 || m->G != 1) return CBL_EUNSUPPORTED;
+    if (m->books != 1 && m->books != 2) return CBL_EINVAL;
+    if (m->books == 2 && !m->tags2) return CBL_EINVAL;
+    if (m->R < 0 || m->C <= 0 || m->C % 8 || (int64_t)m->W * 32 < (int64_t)(m->C / 8) * 12) return CBL_EINVAL;
+    if (!tile_rows && ntile != cbl_ceil_div(m->R, B3_ROWS)) return CBL_EINVAL;
+    const int nkb = cbl_ceil_div(m->C, B3_KB);
+    const int64_t n = (int64_t)m->books * ntile * 16 * nkb * 4;
+    if (n == 0) return CBL_OK;
+    k_repack_b3<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)s>>>(*m, tile_rows, ntile, nkb, copies, (uint32_t*)out, n);
+    return cbl_check_launch();
+}
+
+extern "C" size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int32_t ntok) {
+    if (!mats || n < 1 || n > B3_MAX_MATS || ntok < 1 || ntok > cbl_gemm_b3_max_tokens(mats[0].copies) || mats[0].C <= 0) return 0;
+    B3Plan pl;
+    if (b3_plan(mats, n, ntok, pl)) return 0;
+    return (size_t)B3_CTL_WORDS * 4 + (size_t)pl.G * pl.PP * pl.npad * B3_ROWS * 4;
+}
+
+extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
+                           int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
+    if (!mats || !x || !ys || !stage || !workspace || n < 1) return CBL_EINVAL;
+    if (n > B3_MAX_MATS || ntok > cbl_gemm_b3_max_tokens(mats[0].copies)) return CBL_EUNSUPPORTED;
+    if (ntok < 1 || ldx < mats[0].C) return CBL_EINVAL;
+    if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
+    if (((uintptr_t)stage % 16) || ((uintptr_t)workspace % 16)) return CBL_EINVAL;
+    for (int i = 0; i < n; i++) {
+        int rc = b3_check(mats + i, mats);
+        if (rc) return rc;
+        if (!ys[i] || (ntok > 1 && ldy < mats[i].R)) return CBL_EINVAL;
+    }
+    const int C = mats[0].C, M = mats[0].M;
+    if (M > 1 && !perms) return CBL_EINVAL;
+    B3Plan pl;
+    int rc = b3_plan(mats, n, ntok, pl);
+    if (rc) return rc;
+    if (pl.U == 0) return CBL_OK;
+    rc = cbl_prep_x(x, xdtype, ntok, C, ldx, perms, M, stage, s);
+    if (rc) return rc;
+    const int Bpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
+    B3Launch P;
+    P.nkb = cbl_ceil_div(C, B3_KB);
+    P.ks = pl.ks; P.q = pl.U / pl.G; P.rem = pl.U % pl.G; P.npad = pl.npad; P.xrows = pl.rows; P.ntok = ntok; P.NST = pl.NST; P.RX = pl.RX; P.XU = pl.XU; P.PP = pl.PP; P.Bpad = Bpad;
+    P.ldy = ldy;
+    P.xinv = (const float*)((const __half*)stage + (int64_t)M * Bpad * Cpad);
+    P.status = (unsigned int*)workspace;
+    P.counters = P.status + 64;
+    P.partial = (float*)((char*)workspace + (size_t)B3_CTL_WORDS * 4);
+    P.nseg = 0;
+    int gi = 0, ctr = 0;
+    for (int i = 0; i < n; i++) {
+        const cbl_b3& m = mats[i];
+        B3Mat& o = P.mat[i];
+        o.row_scale = (const __half*)m.row_scale; o.tile_rows = m.tile_rows; o.tile_order = M > 1 ? m.tile_order : nullptr;
+        o.bias = m.bias; o.y = ys[i]; o.R = m.R; o.ntile = m.ntile; o.gi0 = gi; o.books = m.books; o.ctr0 = ctr;
+        ctr += m.ntile;
+        for (int k = 0; k < m.books && m.ntile > 0; k++) {
+            B3Seg& sg = P.seg[P.nseg++];
+            sg.words = (const uint4*)m.words + (size_t)k * m.ntile * P.nkb * B3_ROWS;
+            sg.table = (const uint4*)(k ? m.table2 : m.table);
+            sg.gi0 = gi; sg.gi1 = gi + m.ntile; sg.mi = i;
+            gi += m.ntile;
+        }
+    }
+    encode_tiled_fn enc = get_encode();
+    if (!enc) return CBL_ECUDA;
+    // the maps of the staged activations are a function of these values; a caller that reuses its buffer finds them made
+    struct MapKey { void* p; int Cpad, rows, box, XU; };
+    static thread_local MapKey key = {nullptr, 0, 0, 0, 0};
+    static thread_local CUtensorMap xmap, xmap1;
+    if (key.p != stage || key.Cpad != Cpad || key.rows != M * Bpad || key.box != pl.rows || key.XU != pl.XU) {
+        const cuuint64_t dims[3] = {B3_KB, (cuuint64_t)M * Bpad, (cuuint64_t)Cpad / B3_KB};
+        const cuuint64_t strides[2] = {(cuuint64_t)Cpad * 2, B3_KB * 2};
+        const cuuint32_t box[3] = {B3_KB, (cuuint32_t)pl.rows, (cuuint32_t)pl.XU}, box1[3] = {B3_KB, (cuuint32_t)pl.rows, 1};
+        const cuuint32_t estr[3] = {1, 1, 1};
+        key.p = nullptr;
+        for (int k = 0; k < 2; k++) {
+            CUresult cr = enc(k ? &xmap1 : &xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, stage, dims, strides, k ? box1 : box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
+        }
+        key = {stage, Cpad, M * Bpad, pl.rows, pl.XU};
+    }
+    typedef void (*kernel_fn)(const CUtensorMap, const CUtensorMap, const B3Launch);
+    static const kernel_fn fns[6] = {k_gemm_b3<2, float>, k_gemm_b3<2, __half>, k_gemm_b3<2, __nv_bfloat16>,
+                                     k_gemm_b3<3, float>, k_gemm_b3<3, __half>, k_gemm_b3<3, __nv_bfloat16>};      // by cbl_dtype
+    static bool attr_set[64] = {};
+    int dev = 0;
+    CBL_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        for (int k = 0; k < 6; k++) CBL_CUDA(cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, B3_SMEM));
+        attr_set[dev] = true;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = (cudaStream_t)s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(pl.G);
+    cfg.blockDim = dim3(B3_THREADS);
+    cfg.dynamicSmemBytes = B3_SMEM;
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[(mats[0].copies - 2) * 3 + ydtype], xmap, xmap1, P));
+    return cbl_check_launch();
+}
+
+extern "C" int cbl_gemm_b3_status(void* workspace, cbl_stream s) {
+    if (!workspace) return CBL_EINVAL;
+    unsigned int v = 0;
+    CBL_CUDA(cudaMemcpyAsync(&v, workspace, 4, cudaMemcpyDeviceToHost, (cudaStream_t)s));
+    CBL_CUDA(cudaStreamSynchronize((cudaStream_t)s));
+    if (v) CBL_CUDA(cudaMemsetAsync(workspace, 0, (size_t)B3_CTL_WORDS * 4, (cudaStream_t)s));
+    return v ? CBL_ETIMEOUT : CBL_OK;
+}

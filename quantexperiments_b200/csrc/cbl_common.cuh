@@ -90,3 +90,10 @@ __device__ __forceinline__ float cbl_load_in(const void* x, int dtype, int64_t i
     if (dtype == CBL_F16) return __half2float(((const __half*)x)[i]);
     return ((const float*)x)[i];
 }
+
+// Power-of-two exponent k such that |v| * 2^-k < 2^14 for the largest magnitude mx (k may be negative).
+__device__ __forceinline__ int cbl_scale_exp(float mx) {
+    if (!(mx > 0.f) || !(mx < 3.0e38f)) return 0;
+    int k = ilogbf(mx) - 13;
+    return k < -100 ? -100 : (k > 110 ? 110 : k);
+}

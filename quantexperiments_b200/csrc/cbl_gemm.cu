@@ -12,8 +12,7 @@
 // The epilogue reads TMEM with tcgen05.ld, applies the fp16 row scale and the token's power-of-two
 // activation scale, rounds once and writes Y.  Every wait is bounded; a wait that expires sets the
 // status word and lets the block drain and free its tensor memory.
-#include <cuda.h>
-#include "cbl_common.cuh"
+#include "cbl_tc.cuh"
 
 namespace {
 
@@ -28,26 +27,6 @@ constexpr int GM_SMEM = 65536 + GM_A_STAGES * 2 * GM_A_BYTES + GM_B_STAGES * GM_
 constexpr int GM_DECODE_WARPS = 8, GM_THREADS = (GM_DECODE_WARPS + 2) * 32;
 constexpr uint32_t GM_WAIT_LIMIT = 1u << 24;   // mbarrier polls (a few tens of cycles each) before a wait gives up
 
-// The issuing thread of a warp, chosen by elect.sync, and a warp index the compiler knows to be uniform.  With a
-// plain `lane == 0` the compiler must assume that several threads could get here and wraps every tcgen05.mma (whose
-// descriptors live in uniform registers) in a loop over the active lanes: 97 clocks per MMA issued, whatever its size,
-// against 21 (N = 16) .. 75 (N = 128) for the MMA itself (A in tensor memory, M = 128, measured on B200).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(e));
-    return e != 0;
-}
-__device__ __forceinline__ int uniform_warp(int tid) { return __shfl_sync(0xffffffffu, tid >> 5, 0); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
 // Bounded wait for a phase of an mbarrier: a non-blocking test in a spin loop (the blocking try_wait form
 // adds wake-up latency to every pipeline hand-off); false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
@@ -61,30 +40,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(map), "r"(c0), "r"(c1), "r"(bar)
-                 : "memory");
-}
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// K-major, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart (descriptor version 1).
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-    d |= (uint64_t)1 << 16;                 // leading byte offset (unused with swizzle): 1
-    d |= (uint64_t)(1024 >> 4) << 32;       // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                 // descriptor version
-    d |= (uint64_t)2 << 61;                 // SWIZZLE_128B
-    return d;
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
@@ -716,24 +677,6 @@ constexpr int GT_STAGES = 3;
 constexpr int GT_A_COL0 = 32, GT_A_STAGE_COLS = GR_KBS * 32;
 constexpr int GT_SMEM = 65536 + GT_STAGES * GR_X_STAGE;
 
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint4 (&c)[8]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(c[0].x), "r"(c[0].y), "r"(c[0].z), "r"(c[0].w), "r"(c[1].x), "r"(c[1].y), "r"(c[1].z), "r"(c[1].w), "r"(c[2].x),
-          "r"(c[2].y), "r"(c[2].z), "r"(c[2].w), "r"(c[3].x), "r"(c[3].y), "r"(c[3].z), "r"(c[3].w), "r"(c[4].x), "r"(c[4].y), "r"(c[4].z),
-          "r"(c[4].w), "r"(c[5].x), "r"(c[5].y), "r"(c[5].z), "r"(c[5].w), "r"(c[6].x), "r"(c[6].y), "r"(c[6].z), "r"(c[6].w), "r"(c[7].x),
-          "r"(c[7].y), "r"(c[7].z), "r"(c[7].w)
-        : "memory");
-}
-
 __global__ void __launch_bounds__(GR_THREADS, 1)
 k_gemm_rows_ta(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GRLaunch P, const float* __restrict__ xinv, int ntok, int ydtype,
             int64_t ldy, unsigned int* __restrict__ status) {
@@ -1224,21 +1167,6 @@ __global__ void __maxnreg__(56) k_decode_raw(cbl_packed m, __half* __restrict__ 
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");          // later kernels that wait for this one also wait for its predecessors
-}
-
-typedef CUresult (*encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-encode_tiled_fn get_encode() {
-    static encode_tiled_fn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = (encode_tiled_fn)p;
-    }
-    return fn;
 }
 
 }  // namespace

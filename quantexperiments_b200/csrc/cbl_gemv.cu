@@ -20,13 +20,6 @@ extern "C" size_t cbl_prep_x_bytes(int32_t B, int32_t C, int32_t M) {
     return (size_t)M * Bpad * Cpad * 2 + (size_t)M * Bpad * 4;
 }
 
-// Power-of-two exponent k such that |v| * 2^-k < 2^14 for the largest magnitude mx (k may be negative).
-__device__ __forceinline__ int cbl_scale_exp(float mx) {
-    if (!(mx > 0.f) || !(mx < 3.0e38f)) return 0;
-    int k = ilogbf(mx) - 13;
-    return k < -100 ? -100 : (k > 110 ? 110 : k);
-}
-
 // Eight values of an activation row as fp32.  VEC: one or two 16-byte loads of consecutive columns (no column order,
 // 16-byte aligned rows); otherwise element by element, through the column order when there is one.
 template <bool VEC>
@@ -34,10 +27,10 @@ __device__ __forceinline__ void prep_load8(const void* __restrict__ x, int xdtyp
                                            float (&v)[8]) {
     if (VEC) {
         if (xdtype == CBL_F32) {
-            const float4 a = __ldg((const float4*)((const float*)x + row + c)), b = __ldg((const float4*)((const float*)x + row + c) + 1);
+            const float4 a = __ldcg((const float4*)((const float*)x + row + c)), b = __ldcg((const float4*)((const float*)x + row + c) + 1);
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
-            const uint4 u = __ldg((const uint4*)((const char*)x + (row + c) * 2));
+            const uint4 u = __ldcg((const uint4*)((const char*)x + (row + c) * 2));
             const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int k = 0; k < 4; k++) {

@@ -359,6 +359,120 @@ class X16Matrix:
         return self.run_prepped(self.prep(X, B), Y, B)
 
 
+def order_tiles(dm: DeviceMatrix, rows: int) -> tuple[torch.Tensor | None, torch.Tensor | None, int]:
+    """Rows grouped by column order into tiles of `rows` positions, every order padded with -1 to whole tiles (the reference
+    groups rows by order the same way, shapequant/kernels/proto_runs.py:380-388): (tile_rows, tile_order, tiles).  One
+    column order needs no table: (None, None, ceil(R / rows))."""
+    if dm.M == 1:
+        return None, None, -(-dm.R // rows)
+    mask = dm.row_mask.to(torch.int64)
+    count = torch.bincount(mask, minlength=dm.M)
+    padded = (count + rows - 1) // rows * rows
+    start = torch.cumsum(padded, 0) - padded
+    by_order = torch.argsort(mask, stable=True)
+    rank = torch.arange(dm.R, device=dm.device) - torch.repeat_interleave(torch.cumsum(count, 0) - count, count)
+    n = int(padded.sum())
+    tile_rows = torch.full((n,), -1, dtype=torch.int32, device=dm.device)
+    tile_rows[start[mask[by_order]] + rank] = by_order.to(torch.int32)
+    tile_order = torch.repeat_interleave(torch.arange(dm.M, dtype=torch.int32, device=dm.device), padded // rows)
+    return tile_rows, tile_order, n // rows
+
+
+class B3Matrix:
+    """Layout for 1..16 (three copies of the book in shared memory) or 1..128 tokens (two): tags as slots of the copies
+    (cbl_b3.cu).  d = 8, 12-bit tags, one or two books, any number of column orders."""
+
+    def __init__(self, dm: DeviceMatrix, copies: int = 3, alloc=None):
+        _need_fast(dm)
+        self.dm, self.R, self.C, self.M, self.books, self.device = dm, dm.R, dm.C, dm.M, dm.books, dm.device
+        self.copies, self.bmax = copies, lib.cbl_gemm_b3_max_tokens(copies)
+        self.tile_rows, self.tile_order, self.ntile = order_tiles(dm, 128)
+        nbytes = lib.cbl_b3_bytes(self.ntile, dm.C, dm.books)
+        self.words = _alloc_i32(max(nbytes, 16) // 4, dm.device, alloc)
+        with torch.cuda.device(dm.device):
+            _lib.check("cbl_repack_b3", lib.cbl_repack_b3(ctypes.byref(dm.struct()), _ptr(self.tile_rows), self.ntile, copies,
+                                                          self.words.data_ptr(), _stream()))
+
+    def struct(self, bias: torch.Tensor | None = None) -> _lib.B3:
+        dm = self.dm
+        return _lib.B3(self.R, self.C, self.books, self.M, self.ntile, self.copies, _ptr(self.words), _ptr(self.tile_rows), _ptr(self.tile_order),
+                       _ptr(dm.table), _ptr(dm.table2), _ptr(dm.row_scale), _ptr(bias))
+
+    def nbytes(self) -> int:
+        return self.words.numel() * 4 + (0 if self.tile_rows is None else (self.tile_rows.numel() + self.tile_order.numel()) * 4)
+
+
+class B3Group:
+    """Up to four matrices that read the same activations through the same column orders (q|k|v, gate|up), run as one
+    launch: run(X [B, >= C], ys) writes ys[i] [B, R_i]; the outputs share one row stride."""
+
+    MAX = 4
+    _scratch: dict = {}
+    _retired: list = []                     # outgrown buffers stay alive: a captured graph may still point at them
+
+    def __init__(self, mats: list[B3Matrix], biases: list | None = None):
+        if not 1 <= len(mats) <= self.MAX:
+            raise ValueError(f"a group holds 1..{self.MAX} matrices")
+        if len({(m.C, m.M, m.device, m.copies) for m in mats}) != 1:
+            raise ValueError("grouped matrices share the input size, the column orders, the number of book copies and the device")
+        self.bmax = mats[0].bmax
+        self.mats, self.C, self.M, self.device = mats, mats[0].C, mats[0].M, mats[0].device
+        self.biases = biases if biases is not None else [None] * len(mats)
+        self.perms = mats[0].dm.perms
+        self._built = None
+        self._ws_bytes: dict = {}
+        self._ys = (ctypes.c_void_p * len(mats))()
+
+    @property
+    def _structs(self):
+        key = tuple(m.words.data_ptr() for m in self.mats)
+        if self._built is None or self._built[0] != key:
+            self._built = (key, (_lib.B3 * len(self.mats))(*[m.struct(b) for m, b in zip(self.mats, self.biases)]))
+        return self._built[1]
+
+    @classmethod
+    def buffers(cls, device: torch.device, stage_bytes: int, ws_bytes: int) -> tuple[torch.Tensor, torch.Tensor]:
+        """Staging buffer and work space of the products on (device, current stream)."""
+        key = (device.index, _stream())
+        st, ws = cls._scratch.get(key, (None, None))
+        if st is None or st.numel() < stage_bytes or ws.numel() < ws_bytes:
+            if st is not None:
+                cls._retired.append((st, ws))
+            st = torch.empty(max(stage_bytes, 4 << 20), dtype=torch.uint8, device=device)
+            ws = torch.zeros(max(ws_bytes, 16 << 20), dtype=torch.uint8, device=device)
+            cls._scratch[key] = (st, ws)
+        return st, ws
+
+    def run(self, X: torch.Tensor, ys: list[torch.Tensor]) -> list[torch.Tensor]:
+        B = X.shape[0]
+        if X.dim() != 2 or X.shape[1] < self.C or (self.M == 1 and X.shape[1] != self.C) or X.stride(1) != 1 or X.device != self.device:
+            raise ValueError("X must be [B, C] with unit column stride on the matrices' device")
+        if not 1 <= B <= self.bmax:
+            raise ValueError(f"batch {B} outside 1..{self.bmax}")
+        if len(ys) != len(self.mats) or len({y.dtype for y in ys}) != 1:
+            raise ValueError("one output per matrix, one dtype")
+        ldy = ys[0].stride(0) if B > 1 else max(m.R for m in self.mats)
+        for i, (y, m) in enumerate(zip(ys, self.mats)):
+            if y.shape != (B, m.R) or y.stride(1) != 1 or (B > 1 and y.stride(0) != ldy):
+                raise ValueError("outputs must be [B, R_i] with unit column stride and a common row stride")
+            self._ys[i] = y.data_ptr()
+        st = self._structs
+        need = self._ws_bytes.get(B)
+        if need is None:
+            need = self._ws_bytes[B] = (lib.cbl_prep_x_bytes(B, self.C, self.M), lib.cbl_gemm_b3_workspace_bytes(st, len(self.mats), B))
+        stage, ws = self.buffers(self.device, *need)
+        with torch.cuda.device(self.device):
+            _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1], _ptr(self.perms),
+                                                      self._ys, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
+        return ys
+
+    def status(self) -> None:
+        """Synchronises and raises CblError if a bounded device-side wait of an earlier run() expired."""
+        _, ws = self._scratch.get((self.device.index, _stream()), (None, None))
+        if ws is not None:
+            _lib.check("cbl_gemm_b3_status", lib.cbl_gemm_b3_status(ws.data_ptr(), _stream()))
+
+
 class DenseStack:
     """Matrices that multiply the same activations (q|k|v, gate|up, or a single matrix), for many tokens or
     for matrices with several column orders: every matrix is decoded ONCE into a 16-bit scratch shared by

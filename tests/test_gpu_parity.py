@@ -795,3 +795,68 @@ def test_large_decode_with_the_book_in_shared_memory_equals_the_generic_decode(R
     _lib.check("cbl_dequant", _lib.lib.cbl_dequant(ctypes.byref(dm.struct()), big.data_ptr(), _lib.BF16, C + 8, 0, R,
                                                    torch.cuda.current_stream().cuda_stream))
     assert torch.equal(big[:R, :C], dm.dequant(dtype=torch.bfloat16)) and torch.isnan(big[:R, C:]).all() and torch.isnan(big[R:]).all()
+
+
+# ------------------------------------------------------------------------------------------ 1..64 tokens, book in three copies
+@pytest.mark.parametrize("Rs,C,books,M", [((1,), 8, 1, 1), ((130,), 64, 1, 1), ((300,), 264, 2, 1), ((1000, 129, 40), 520, 1, 1), ((260, 130), 1032, 2, 4),
+                                          ((2304,), 8200, 1, 16), ((3584, 512, 512), 3584, 1, 1), ((20000,), 456, 1, 1), ((9000, 9000), 904, 2, 1),
+                                          ((19000,), 128, 2, 16), ((18950,), 2248, 1, 1)])
+def test_three_copy_product_matches_fp32_matmul(Rs, C, books, M):
+    """cbl_gemm_b3: groups, whole tiles and tiles shared by several blocks, ranges that cross matrices and books, ragged rows
+    and columns, column orders; token counts at the edges of the 16-token steps; fp32 / bf16 outputs as column slices; bias."""
+    from quantexperiments_b200.kernels import B3Group, B3Matrix
+    ms = [orc.synth_matrix(R, C, seed=R + C + i, books=books, M=M) for i, R in enumerate(Rs)]
+    dms = [_dm(m) for m in ms]
+    if M > 1:
+        for m, dm in zip(ms[1:], dms[1:]):
+            m["perms"], dm.perms = ms[0]["perms"], dms[0].perms
+    w = torch.cat([torch.from_numpy(orc.synth_decode(m)) for m in ms]).cuda()
+    b3 = {k: [B3Matrix(dm, k) for dm in dms] for k in (2, 3)}
+    g = torch.Generator(device="cuda").manual_seed(C)
+    for B, copies in ((1, 3), (2, 3), (8, 2), (9, 3), (16, 3), (17, 2), (32, 2), (33, 2), (64, 2), (90, 2), (128, 2)):
+        X = torch.randn(B, C, device="cuda", generator=g)
+        X[0, 3] = 2.0e4
+        X = X.bfloat16()
+        ref = X.float() @ w.t()
+        for ydt in (torch.float32, torch.bfloat16):
+            biases = [torch.randn(R, device="cuda", generator=g).to(ydt) if i == 0 and B == 9 else None for i, R in enumerate(Rs)]
+            want = ref.clone()
+            if biases[0] is not None:
+                want[:, :Rs[0]] += biases[0].float()
+            grp = B3Group(b3[copies], biases)
+            Y = torch.full((B, sum(Rs) + 8), 3.0, device="cuda", dtype=ydt)
+            ys, o = [], 0
+            for R in Rs:
+                ys.append(Y[:, o:o + R])
+                o += R
+            first = None
+            for _ in range(2):
+                grp.run(X, ys)
+                got = Y[:, :sum(Rs)].float()
+                for t in range(B):
+                    assert (got[t] - want[t]).abs().max() / max(ref[t].abs().max(), want[t].abs().max()) <= 2 * _out_tol(ydt), (B, ydt, t)
+                assert (Y[:, sum(Rs):] == 3.0).all()
+                assert first is None or torch.equal(first, Y)
+                first = Y.clone()
+        grp.status()
+
+
+@pytest.mark.parametrize("copies,limit", [(3, 1.25), (2, 1.8)])
+def test_copy_layout_is_the_matrix_and_spreads_the_banks(copies, limit):
+    """Every 16-bit slot names a copy of the tag's codeword; eight rows read together hit the fullest of the eight bank groups
+    1.2 times on average with three copies, 1.7 with two (2.6 without)."""
+    from quantexperiments_b200.kernels import B3Matrix
+    m = orc.synth_matrix(600, 1000, seed=9)
+    b = B3Matrix(_dm(m), copies)
+    w = b.words.cpu().numpy().view(np.uint32).astype(np.int64).reshape(b.ntile, -1, 128, 4)
+    slots = np.stack([(w & 0x3FFF0) >> 4, w >> 18], -1).reshape(b.ntile, -1, 128, 8)          # [tile][k-block][row][chunk]
+    copy, at = slots // 4096, slots % 4096
+    assert copy.max() == copies - 1
+    group = at // 8
+    rot = np.stack([0 * group, 1 + group % 7, 1 + (group % 7 + 1 + group % 42 // 7) % 7])
+    tag = group * 8 + ((at - np.take_along_axis(rot, copy[None], 0)[0]) & 7)
+    got = tag.transpose(0, 2, 1, 3).reshape(b.ntile * 128, -1)
+    assert np.array_equal(got[:600, :125], orc.unpack_bits(m["words"][0], 12, 125))
+    banks = (slots & 7).reshape(b.ntile, -1, 16, 8, 8)                                         # groups of eight rows
+    fullest = np.max([(banks == k).sum(3) for k in range(8)], axis=0)
+    assert fullest[:4].mean() < limit
