@@ -223,6 +223,9 @@ int cbl_gemv_l8_plan(const cbl_l8* mats, int32_t n, int32_t max_blocks, int32_t*
  *          (merge_runs) and the per-piece loop of shapequant/vllm_ext/core.py:376-384 (_small). */
 int cbl_gemv_l8_multi(const cbl_l8* mats, int32_t n, const void* x, int xdtype, void* const* ys, int ydtype,
                       void* workspace, cbl_stream s);
+/* The same with a bias per matrix (an entry, or biases itself, may be NULL), in y's type: y = round(round(product) + bias). */
+int cbl_gemv_l8_bias(const cbl_l8* mats, int32_t n, const void* x, int xdtype, void* const* ys, int ydtype, const void* const* biases,
+                     void* workspace, cbl_stream s);
 
 /* Row-split (tensor-parallel o / down) batch-1 product fused with the sum over ranks, without a
  * collective library: each rank accumulates its chunk range locally, then one kernel per rank
@@ -386,6 +389,9 @@ int cbl_decode_raw(const cbl_packed* m, void* out, cbl_stream s);
 int cbl_decode_raw_wide(const cbl_packed* m, void* out, int32_t C_out, cbl_stream s);
 int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok, int64_t ldx,
                    void* y, int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s);
+/* The same plus a bias [R] in y's type: y = round(round(product) + bias). */
+int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok, int64_t ldx,
+                   void* y, int ydtype, int64_t ldy, const void* bias, void* stage, void* workspace, cbl_stream s);
 
 /* ------------------------------------------------------------------------------------------------
  * Decode-step operators between the packed linears (Qwen2-style blocks).  `dtype` is the model's

@@ -108,6 +108,7 @@ SIGNATURES = {
     "cbl_gemm_l8": (c_int, [POINTER(L8), c_void_p, c_int, c_int32, c_int64, c_void_p, c_int, c_int64, c_void_p, c_void_p, c_void_p]),
     "cbl_gemm_l8_2sm": (c_int, [POINTER(L8), c_void_p, c_int, c_int32, c_int64, c_void_p, c_int, c_int64, c_void_p, c_void_p, c_void_p]),
     "cbl_gemv_l8_multi": (c_int, [POINTER(L8), c_int32, c_void_p, c_int, POINTER(c_void_p), c_int, c_void_p, c_void_p]),
+    "cbl_gemv_l8_bias": (c_int, [POINTER(L8), c_int32, c_void_p, c_int, POINTER(c_void_p), c_int, POINTER(c_void_p), c_void_p, c_void_p]),
     "cbl_gemv_l8_ar_workspace_bytes": (c_size_t, [c_int32]),
     "cbl_gemv_l8_ar": (c_int, [POINTER(L8), c_void_p, c_int, c_void_p, c_int, POINTER(c_void_p), c_int32, c_int32, c_void_p]),
     "cbl_gemv_l8_ar_status": (c_int, [c_void_p, c_int32, c_void_p]),
@@ -121,6 +122,8 @@ SIGNATURES = {
     "cbl_decode_raw_wide": (c_int, [POINTER(Packed), c_void_p, c_int32, c_void_p]),
     "cbl_gemm_dense": (c_int, [c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_int, c_int32, c_int64, c_void_p, c_int, c_int64, c_void_p,
                                c_void_p, c_void_p]),
+    "cbl_gemm_dense_bias": (c_int, [c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_int, c_int32, c_int64, c_void_p, c_int, c_int64, c_void_p,
+                                    c_void_p, c_void_p, c_void_p]),
     "cbl_embed_rows": (c_int, [c_void_p, c_int, c_int64, c_int32, c_void_p, c_int32, c_void_p, c_void_p]),
     "cbl_add_rmsnorm": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int, c_float, c_int32, c_int32, c_void_p, c_void_p]),
     "cbl_rope_kv": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_float,

@@ -1,4 +1,5 @@
-"""In-tree build of libcbl.so (hand-written CUDA for sm_100a behind a C ABI).
+"""In-tree build of libcbl.so (hand-written CUDA for sm_100a behind a C ABI) and of _cblhost.so (the native call path
+between torch and it, csrc/host.cpp).
 
     python -m quantexperiments_b200.build [--force] [--verbose]
 
@@ -14,6 +15,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libcbl.so"
+HOST = PKG / "_cblhost.so"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -29,9 +31,31 @@ def _stale() -> bool:
     return any(p.stat().st_mtime > t for p in deps)
 
 
+def build_host(force: bool = False, verbose: bool = False) -> Path:
+    """Compile csrc/host.cpp against the installed torch; returns the extension module's path."""
+    src, deps = CSRC / "host.cpp", [CSRC / "host.cpp", PKG.parent / "include" / "cbl.h"]
+    if not force and HOST.exists() and all(p.stat().st_mtime <= HOST.stat().st_mtime for p in deps):
+        return HOST
+    import sysconfig
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path("/usr/local/cuda")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-isystem", str(root / "include"),
+           "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda / "include"),
+           "-isystem", sysconfig.get_paths()["include"], str(src), "-o", str(HOST), f"-L{PKG}", "-l:libcbl.so", "-Wl,-rpath,$ORIGIN", f"-L{root / 'lib'}",
+           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", f"-L{cuda / 'lib64'}", "-lcudart"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+    if r.returncode:
+        raise RuntimeError(f"g++ failed ({r.returncode}): {' '.join(cmd)}")
+    return HOST
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every kernel for sm_100a into libcbl.so; returns its path."""
+    """Compile every kernel for sm_100a into libcbl.so, and the host extension; returns the library's path."""
     if not force and not _stale():
+        build_host(False, verbose)
         return LIB
     cmd = ["nvcc", *ARCH, "-O3", "-std=c++17", "-lineinfo", "-shared", "-Xcompiler", "-fPIC", "--threads", "0",
            "-I", str(PKG.parent / "include"), *(["-Xptxas", "-v"] if verbose else []),
@@ -41,6 +65,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         sys.stderr.write(r.stdout + r.stderr)
     if r.returncode:
         raise RuntimeError(f"nvcc failed ({r.returncode}): {' '.join(cmd)}")
+    build_host(force, verbose)
     return LIB
 
 

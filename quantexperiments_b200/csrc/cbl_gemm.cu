@@ -58,9 +58,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         : "r"(taddr));
 }
 
+// The product rounded to y's type plus the bias, to be rounded again: what two operators would give.
+__device__ __forceinline__ float gemm_add_bias(float v, const void* __restrict__ bias, int ydtype, int r) {
+    if (ydtype == CBL_BF16) v = __bfloat162float(__float2bfloat16_rn(v));
+    else if (ydtype == CBL_F16) v = __half2float(__float2half_rn(v));
+    return v + cbl_load_in(bias, ydtype, r);
+}
+
 // One token's 32 consecutive outputs: row scales as four 16-byte loads, outputs as 16-byte stores when aligned.
 __device__ __forceinline__ void gemm_store_row32(const uint32_t (&v)[32], int tok, int ntok, int rbase, const cbl_l8& m, float tsc,
-                                                 void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok) {
+                                                 void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok, const void* __restrict__ bias = nullptr) {
     if (tok >= ntok || rbase >= m.R) return;
     if (vec_ok && rbase + 32 <= m.R) {
         union { uint4 u[4]; __half h[32]; } rsv;
@@ -70,6 +77,10 @@ __device__ __forceinline__ void gemm_store_row32(const uint32_t (&v)[32], int to
         float o[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) o[j] = __uint_as_float(v[j]) * tsc * __half2float(rsv.h[j]);
+        if (bias) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) o[j] = gemm_add_bias(o[j], bias, ydtype, rbase + j);
+        }
         if (ydtype == CBL_F32) {
             float4* dst = (float4*)((float*)y + (int64_t)tok * ldy + rbase);
 #pragma unroll
@@ -93,7 +104,8 @@ __device__ __forceinline__ void gemm_store_row32(const uint32_t (&v)[32], int to
             const int r = rbase + j;
             if (r < m.R) {
                 const float rs = __half2float(__ldg((const __half*)m.row_scale + r));
-                cbl_store_out(y, ydtype, (int64_t)tok * ldy + r, __uint_as_float(v[j]) * tsc * rs);
+                const float o = __uint_as_float(v[j]) * tsc * rs;
+                cbl_store_out(y, ydtype, (int64_t)tok * ldy + r, bias ? gemm_add_bias(o, bias, ydtype, r) : o);
             }
         }
     }
@@ -989,7 +1001,7 @@ constexpr int G3_EPI_WARPS = 8, G3_THREADS = (G3_EPI_WARPS + 2) * 32;
 
 __global__ void __launch_bounds__(G3_THREADS, 1)
 k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, cbl_l8 m, const float* __restrict__ xinv,
-                 int ntok, void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok, unsigned int* __restrict__ status) {
+                 int ntok, void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok, const void* __restrict__ bias, unsigned int* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long s_bar[2 * G3_STAGES + 4];   // full, empty per stage; acc_full[2], acc_empty[2]
     __shared__ uint32_t s_tmem;
@@ -1075,7 +1087,7 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * GM_BN + c0), v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                gemm_store_row32(v, tok, ntok, r0 + c0, m, tsc, y, ydtype, ldy, vec_ok);
+                gemm_store_row32(v, tok, ntok, r0 + c0, m, tsc, y, ydtype, ldy, vec_ok, bias);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -1307,6 +1319,11 @@ extern "C" int cbl_decode_raw_wide(const cbl_packed* m, void* out, int32_t C_out
 
 extern "C" int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok,
                               int64_t ldx, void* y, int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
+    return cbl_gemm_dense_bias(w16, R, C, row_scale, x, xdtype, ntok, ldx, y, ydtype, ldy, nullptr, stage, workspace, s);
+}
+
+extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok,
+                              int64_t ldx, void* y, int ydtype, int64_t ldy, const void* bias, void* stage, void* workspace, cbl_stream s) {
     if (!w16 || !row_scale || !x || !y || !stage || !workspace) return CBL_EINVAL;
     if (R <= 0 || C <= 0 || C % 8 || ntok <= 0 || ldx < C || ldy < R) return CBL_EINVAL;
     if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
@@ -1351,6 +1368,7 @@ extern "C" int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void*
     const int esz = ydtype == CBL_F32 ? 4 : 2;
     const int vec_ok = ((uintptr_t)y % 16 == 0) && ((ldy * esz) % 16 == 0) && ((uintptr_t)row_scale % 16 == 0);
 #ifdef CBL_DENSE_1SM
+    if (bias) return CBL_EUNSUPPORTED;
     const int variant = 1;                                    // build option: the one-block kernel (for comparisons)
 #else
     const int variant = 2;
@@ -1385,7 +1403,7 @@ extern "C" int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void*
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, (unsigned int*)workspace));
+        CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, bias, (unsigned int*)workspace));
         return cbl_check_launch();
     }
     dim3 grid(cbl_ceil_div(ntok, GM_BM), cbl_ceil_div(R, GM_BN));

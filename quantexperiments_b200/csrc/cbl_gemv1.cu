@@ -142,6 +142,7 @@ struct L8Launch {
     unsigned long long* partial;       // L8_MAX_BLOCKS slots of L8_SLOT_ROWS words {valid << 32 | fp32 partial sum} (zero on entry, left zero)
     float* fsum[L8_MAX_GROUP];         // mode 1: fp32 sums by source row
     void* y[L8_MAX_GROUP];
+    const void* bias[L8_MAX_GROUP];    // mode 0: added to the rounded product, in y's type (NULL: none)
     unsigned int* status;              // set to 1 when a bounded wait expired
     const uint32_t* calls;             // optional: completed-call counter; call e = *calls + 1 writes its sums to
     int64_t fsum_stride;               // fsum[0] + (e & 1) * fsum_stride (two alternating buffers, see cbl_gemv_l8_ar)
@@ -408,8 +409,17 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
         const int r = rix ? rix[p] : p;
         return r < mm.R ? r : -1;
     };
+    // y = round(row scale * sum), or round(that + bias): two roundings, as by two operators
+    auto put = [&](int r, float v) {
+        if (P.bias[mi]) {
+            if (P.ydtype == CBL_BF16) v = __bfloat162float(__float2bfloat16_rn(v));
+            else if (P.ydtype == CBL_F16) v = __half2float(__float2half_rn(v));
+            v += cbl_load_in(P.bias[mi], P.ydtype, r);
+        }
+        cbl_store_out(P.y[mi], P.ydtype, r, v);
+    };
     auto emit = [&](int r, float v) {
-        if (P.mode == 0) cbl_store_out(P.y[mi], P.ydtype, r, v * __half2float(((const __half*)mm.row_scale)[r]));
+        if (P.mode == 0) put(r, v * __half2float(((const __half*)mm.row_scale)[r]));
         else fsum[r] = v;
     };
     const int n512 = (nrows + L8_NT - 1) / L8_NT;
@@ -486,7 +496,7 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
             }
         }
         if (grp == 0 && rr >= 0 && !late) {
-            if (P.mode == 0) cbl_store_out(P.y[mi], P.ydtype, rr, sum * rsc);
+            if (P.mode == 0) put(rr, sum * rsc);
             else fsum[rr] = sum;
         }
     }
@@ -785,7 +795,7 @@ static int launch_l8(L8Launch& P, const void* x, int xdtype, cudaStream_t st, in
 // Fills the launch descriptor of a group.  Work space: partial-sum slots | status word | fp32 sums of matrix 0,
 // matrix 1, ... (l8_rows_max(R_i) floats each).
 static int l8_group(const cbl_l8* mats, int32_t n, const void* x, int xdtype, void* const* ys, int ydtype, int mode, void* workspace,
-                    L8Launch& P) {
+                    L8Launch& P, const void* const* biases = nullptr) {
     if (!mats || !x || !workspace || n < 1) return CBL_EINVAL;
     if (n > L8_MAX_GROUP) return CBL_EUNSUPPORTED;
     if (xdtype != CBL_F16 && xdtype != CBL_BF16 && xdtype != CBL_F32) return CBL_EINVAL;
@@ -807,6 +817,7 @@ static int l8_group(const cbl_l8* mats, int32_t n, const void* x, int xdtype, vo
         P.m[P.n] = mats[i];
         P.fsum[P.n] = (float*)reg;
         P.y[P.n] = ys ? ys[i] : nullptr;
+        P.bias[P.n] = biases ? biases[i] : nullptr;
         P.n++;
     }
     P.calls = nullptr;
@@ -816,10 +827,15 @@ static int l8_group(const cbl_l8* mats, int32_t n, const void* x, int xdtype, vo
 
 extern "C" int cbl_gemv_l8_multi(const cbl_l8* mats, int32_t n, const void* x, int xdtype, void* const* ys, int ydtype,
                                  void* workspace, cbl_stream s) {
+    return cbl_gemv_l8_bias(mats, n, x, xdtype, ys, ydtype, nullptr, workspace, s);
+}
+
+extern "C" int cbl_gemv_l8_bias(const cbl_l8* mats, int32_t n, const void* x, int xdtype, void* const* ys, int ydtype,
+                                const void* const* biases, void* workspace, cbl_stream s) {
     if (!ys) return CBL_EINVAL;
     if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
-    L8Launch P;
-    int rc = l8_group(mats, n, x, xdtype, ys, ydtype, 0, workspace, P);
+    L8Launch P = {};
+    int rc = l8_group(mats, n, x, xdtype, ys, ydtype, 0, workspace, P, biases);
     if (rc) return rc;
     if (P.n == 0) return CBL_OK;
     return launch_l8(P, x, xdtype, (cudaStream_t)s);
@@ -1004,7 +1020,7 @@ static int l8_finish_launch(void (*kern)(KA...), dim3 grid, dim3 block, int clus
 extern "C" int cbl_gemv_l8_silu_mul(const cbl_l8* gate_up, const void* x, int xdtype, void* out, void* y_gate, void* y_up, int dtype,
                                     void* workspace, cbl_stream s) {
     if (!out || (dtype != CBL_F16 && dtype != CBL_BF16)) return CBL_EINVAL;
-    L8Launch P;
+    L8Launch P = {};
     int rc = l8_group(gate_up, 2, x, xdtype, nullptr, dtype, 1, workspace, P);
     P.y[0] = y_gate;
     P.y[1] = y_up;
@@ -1024,7 +1040,7 @@ extern "C" int32_t cbl_gemv_l8_add_norm_max_rows(void) { return L8_NORM_MAX_CTAS
 extern "C" int cbl_gemv_l8_add_norm(const cbl_l8* m, const void* x, int xdtype, float* h, const void* w, float eps, void* xout, void* y,
                                     int dtype, void* workspace, cbl_stream s) {
     if (!h || !w || !xout || (dtype != CBL_F16 && dtype != CBL_BF16)) return CBL_EINVAL;
-    L8Launch P;
+    L8Launch P = {};
     int rc = l8_group(m, 1, x, xdtype, nullptr, dtype, 1, workspace, P);
     P.y[0] = y;
     if (rc) return rc;
@@ -1044,7 +1060,7 @@ extern "C" int cbl_gemv_l8_rope_kv(const cbl_l8* qkv, const void* x, int xdtype,
                                    cbl_stream s) {
     if (!pos || !q_out || !kc || !vc || (dtype != CBL_F16 && dtype != CBL_BF16) || NH < 1 || NKV < 1 || max_len < 1) return CBL_EINVAL;
     if (HD < 2 || HD > 128 || (HD & 1)) return CBL_EUNSUPPORTED;
-    L8Launch P;
+    L8Launch P = {};
     int rc = l8_group(qkv, 3, x, xdtype, nullptr, dtype, 1, workspace, P);
     if (rc) return rc;
     if (qkv[0].R != NH * HD || qkv[1].R != NKV * HD || qkv[2].R != NKV * HD) return CBL_EINVAL;
@@ -1160,7 +1176,7 @@ extern "C" int cbl_gemv_l8_ar(const cbl_l8* m, const void* x, int xdtype, void* 
     const size_t rmax = l8_rows_max(m->R);
     char* own = (char*)peer_ws[rank];
     uint32_t* ctl = (uint32_t*)(own + 2 * rmax * 4 + L8_AR_MAX_RANKS * 4);
-    L8Launch P;
+    L8Launch P = {};
     P.n = 1;
     P.ydtype = ydtype;
     P.mode = 1;
@@ -1258,7 +1274,7 @@ extern "C" int cbl_gemv_l8_static(const cbl_l8* m, const void* x, int xdtype, vo
     // Every call shares the array and finds whatever the previous call left.  The array starts zero (static
     // storage) and a product that ran to its end has cleared every word it used, so nothing needs clearing here;
     // a product that gave up (status word set) leaves words behind, which cbl_gemv_l8_static_status clears.
-    L8Launch P;
+    L8Launch P = {};
     P.n = 1;
     P.ydtype = ydtype;
     P.mode = 0;

@@ -1,0 +1,286 @@
+// Native call path of the packed linears: one function call from Python to the launch.
+//
+// A layer keeps a Plan (a capsule) with the C-ABI descriptors of the layouts that exist; forward(plan, x) checks the
+// activations, picks the product for their token count, allocates the output and launches on torch's current stream.  It
+// returns None for whatever it does not handle (a layout that is not built yet, an unusual dtype): the Python path then
+// does the work and fills the plan.  Per call the Python path spends 20 (one token) to 45 us (many tokens) on the host, which is more
+// than most products of a decode step run on the GPU; this one spends 4 to 8.
+//
+// Scratch buffers (staged activations, partial sums, decoded weights) belong to a (device, stream) pair, grow on demand and
+// live as long as the process; an outgrown one stays alive because a captured graph may still point at it.
+#include <Python.h>
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/empty.h>
+#include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <map>
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "../../include/cbl.h"
+
+namespace {
+
+constexpr const char* PLAN = "cbl.plan";
+constexpr int MAX_PIECES = 4;
+
+struct Plan {
+    int device = 0, n = 0, orders = 1;                    // n matrices that read the same activations
+    int64_t in = 0, C = 0, R = 0;                         // activations per token, columns, rows of all matrices
+    int64_t rows[MAX_PIECES] = {}, first[MAX_PIECES] = {};
+    const int32_t* perms = nullptr;
+    bool has_l8 = false, has_b3[2] = {false, false}, has_dense = false;      // b3[0]: two copies of the book, b3[1]: three
+    cbl_l8 l8[MAX_PIECES];
+    cbl_b3 b3[2][MAX_PIECES];
+    cbl_packed packed[MAX_PIECES];
+    const void* row_scale = nullptr;                      // of the stacked rows
+    at::Tensor bias;
+    size_t ws_bytes[2][129] = {};
+    size_t l8_bytes = 0;
+    int dense_from = 0;                                   // tokens from which the two-phase product runs
+};
+
+struct Scratch {
+    at::Tensor l8, stage, partial, weights[2], dense_stage;
+    int turn = 0;
+};
+
+std::mutex g_mu;
+std::map<std::pair<int, void*>, Scratch> g_scratch;
+std::vector<at::Tensor> g_retired;
+
+Scratch& scratch_of(int device, void* stream) {           // (call with g_mu held; the reference stays valid)
+    return g_scratch[{device, stream}];
+}
+
+void* need(at::Tensor& t, size_t bytes, size_t least, bool zero, int device) {
+    if (!t.defined() || (size_t)t.numel() < bytes) {
+        if (t.defined()) g_retired.push_back(t);
+        const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device);
+        const int64_t n = (int64_t)std::max(bytes, least);
+        t = zero ? at::zeros({n}, opt) : at::empty({n}, opt);
+    }
+    return t.data_ptr();
+}
+
+PyObject* fail(const char* fn, int rc) {
+    PyErr_Format(PyExc_RuntimeError, "%s: %s (status %d)", fn, cbl_status_string(rc), rc);
+    return nullptr;
+}
+
+int dtype_of(at::ScalarType t) { return t == at::kBFloat16 ? CBL_BF16 : t == at::kHalf ? CBL_F16 : t == at::kFloat ? CBL_F32 : -1; }
+
+Plan* plan_of(PyObject* o) { return (Plan*)PyCapsule_GetPointer(o, PLAN); }
+
+// One product of `tokens` tokens into y [tokens, R] (row stride ldy); CBL_EUNSUPPORTED when the plan has no layout for them.
+int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* y, int ydt, int64_t ldy, const void* bias, void* stream, const char** fn) {
+    const int esz = ydt == CBL_F32 ? 4 : 2;
+    void* ys[MAX_PIECES];
+    for (int i = 0; i < p.n; i++) ys[i] = y + p.first[i] * esz;
+    const cbl_stream s = (cbl_stream)stream;
+    if (tokens == 1 && p.has_l8) {
+        void* ws;
+        {
+            std::lock_guard<std::mutex> lock(g_mu);
+            ws = need(scratch_of(p.device, stream).l8, p.l8_bytes, 16 << 20, true, p.device);
+        }
+        const void* biases[MAX_PIECES] = {};
+        if (bias) for (int i = 0; i < p.n; i++) biases[i] = (const char*)bias + p.first[i] * esz;
+        *fn = "cbl_gemv_l8_bias";
+        return cbl_gemv_l8_bias(p.l8, p.n, x, xdt, ys, ydt, bias ? biases : nullptr, ws, s);
+    }
+    const int k = tokens <= cbl_gemm_b3_max_tokens(3) ? 1 : 0;
+    if (tokens <= cbl_gemm_b3_max_tokens(2)) {
+        if (!p.has_b3[k]) return CBL_EUNSUPPORTED;
+        size_t& wb = p.ws_bytes[k][tokens];
+        if (!wb) wb = cbl_gemm_b3_workspace_bytes(p.b3[k], p.n, (int32_t)tokens);
+        void *stage, *ws;
+        {
+            std::lock_guard<std::mutex> lock(g_mu);
+            Scratch& sc = scratch_of(p.device, stream);
+            stage = need(sc.stage, cbl_prep_x_bytes((int32_t)tokens, (int32_t)p.C, p.orders), 4 << 20, false, p.device);
+            ws = need(sc.partial, wb, 16 << 20, true, p.device);
+        }
+        cbl_b3 mats[MAX_PIECES];
+        for (int i = 0; i < p.n; i++) {
+            mats[i] = p.b3[k][i];
+            mats[i].bias = bias ? (const char*)bias + p.first[i] * esz : nullptr;
+        }
+        *fn = "cbl_gemm_b3";
+        return cbl_gemm_b3(mats, p.n, x, xdt, (int32_t)tokens, ldx, p.perms, ys, ydt, ldy, stage, ws, s);
+    }
+    if (!p.has_dense || tokens < p.dense_from) return CBL_EUNSUPPORTED;
+    char *w, *stage, *status;
+    {
+        // two scratch buffers alternate: the decode of this product may run beside the GEMM of the one before
+        std::lock_guard<std::mutex> lock(g_mu);
+        Scratch& sc = scratch_of(p.device, stream);
+        sc.turn ^= 1;
+        w = (char*)need(sc.weights[sc.turn], cbl_dense_scratch_bytes((int32_t)p.R, (int32_t)p.C), 0, false, p.device);
+        stage = (char*)need(sc.dense_stage, cbl_gemm_stage_bytes((int32_t)tokens, (int32_t)p.C) + 16, 0, true, p.device);
+        status = stage + sc.dense_stage.numel() - 16;
+    }
+    const int64_t ld = (p.C + 7) / 8 * 8;
+    for (int i = 0; i < p.n; i++) {
+        *fn = "cbl_decode_raw";
+        const int rc = cbl_decode_raw(&p.packed[i], w + p.first[i] * ld * 2, s);
+        if (rc) return rc;
+    }
+    *fn = "cbl_gemm_dense";
+    return cbl_gemm_dense_bias(w, (int32_t)p.R, (int32_t)p.C, p.row_scale, x, xdt, (int32_t)tokens, ldx, y, ydt, ldy, bias, stage, status, s);
+}
+
+bool layout_for(const Plan& p, int64_t tokens) {
+    if (tokens == 1 && p.has_l8) return true;
+    if (tokens <= cbl_gemm_b3_max_tokens(2)) return p.has_b3[tokens <= cbl_gemm_b3_max_tokens(3) ? 1 : 0];
+    return p.has_dense && tokens >= p.dense_from;
+}
+
+// forward(plan or tuple of plans, x): x [..., in] -> y [..., sum of R] in x's dtype (+ bias), or None.  Several plans write
+// column slices of one output (pieces of a stacked layer with column orders of their own).
+PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "forward(plan, x)"); return nullptr; }
+    Plan* plans[16];
+    int np = 1;
+    if (PyTuple_Check(args[0])) {
+        np = (int)PyTuple_GET_SIZE(args[0]);
+        if (np < 1 || np > 16) Py_RETURN_NONE;
+        for (int i = 0; i < np; i++) plans[i] = plan_of(PyTuple_GET_ITEM(args[0], i));
+    } else plans[0] = plan_of(args[0]);
+    for (int i = 0; i < np; i++)
+        if (!plans[i]) return nullptr;
+    if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
+    const at::Tensor& x = THPVariable_Unpack(args[1]);
+    const int dim = (int)x.dim();
+    const Plan& p = *plans[0];
+    if (!x.is_cuda() || x.get_device() != p.device || dim < 1 || dim > 8 || x.size(-1) != p.in || !x.is_contiguous()) Py_RETURN_NONE;
+    const int dt = dtype_of(x.scalar_type());
+    const int64_t tokens = x.numel() / p.in;
+    if (dt < 0 || tokens < 1 || tokens > 65535) Py_RETURN_NONE;
+    int64_t R = 0;
+    for (int i = 0; i < np; i++) {
+        const Plan& q = *plans[i];
+        if (!layout_for(q, tokens) || (q.bias.defined() && (q.bias.scalar_type() != x.scalar_type() || !q.bias.is_contiguous()))) Py_RETURN_NONE;
+        R += q.R;
+    }
+    try {
+        const c10::cuda::OptionalCUDAGuard guard(x.device());
+        void* stream = (void*)c10::cuda::getCurrentCUDAStream(p.device).stream();
+        int64_t shape[8];
+        for (int i = 0; i + 1 < dim; i++) shape[i] = x.size(i);
+        shape[dim - 1] = R;
+        at::Tensor y = at::detail::empty_cuda(c10::IntArrayRef(shape, dim), x.scalar_type(), x.device(), std::nullopt);
+        char* out = (char*)y.mutable_data_ptr();
+        for (int i = 0; i < np; i++) {
+            Plan& q = *plans[i];
+            const char* fn = "";
+            const int rc = product(q, x.const_data_ptr(), dt, tokens, q.in, out, dt, R, q.bias.defined() ? q.bias.const_data_ptr() : nullptr, stream, &fn);
+            if (rc) return fail(fn, rc);
+            out += q.R * (dt == CBL_F32 ? 4 : 2);
+        }
+        return THPVariable_Wrap(std::move(y));
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+void free_plan(PyObject* o) { delete plan_of(o); }
+
+// plan(device, in, C, orders, rows: list, perms pointer, dense_from, bias or None) -> capsule
+PyObject* py_plan(PyObject*, PyObject* args) {
+    int device, orders, dense_from;
+    long long in, C;
+    unsigned long long perms;
+    PyObject *rows, *bias;
+    if (!PyArg_ParseTuple(args, "iLLiOKiO", &device, &in, &C, &orders, &rows, &perms, &dense_from, &bias)) return nullptr;
+    const Py_ssize_t n = PyList_Size(rows);
+    if (n < 1 || n > MAX_PIECES) { PyErr_SetString(PyExc_ValueError, "a plan holds 1..4 matrices"); return nullptr; }
+    Plan* p = new Plan;
+    p->device = device; p->in = in; p->C = C; p->orders = orders; p->n = (int)n; p->perms = (const int32_t*)perms; p->dense_from = dense_from;
+    for (Py_ssize_t i = 0; i < n; i++) {
+        p->first[i] = p->R;
+        p->rows[i] = PyLong_AsLongLong(PyList_GetItem(rows, i));
+        p->R += p->rows[i];
+        p->l8_bytes += cbl_gemv_l8_workspace_bytes((int32_t)p->rows[i]);
+    }
+    if (bias != Py_None && THPVariable_Check(bias)) p->bias = THPVariable_Unpack(bias);
+    return PyCapsule_New(p, PLAN, free_plan);
+}
+
+// set(plan, kind, descriptors, row_scale pointer): kind "l8", "b3" (two or three copies, as they say) or "dense"; the descriptors
+// are the ctypes structures' bytes, one per matrix
+PyObject* py_set(PyObject*, PyObject* args) {
+    PyObject* cap;
+    const char* kind;
+    Py_buffer buf;
+    unsigned long long row_scale = 0;
+    if (!PyArg_ParseTuple(args, "Osy*|K", &cap, &kind, &buf, &row_scale)) return nullptr;
+    Plan* p = plan_of(cap);
+    bool ok = p != nullptr;
+    if (ok) {
+        const std::string k = kind;
+        auto take = [&](auto* dst) {
+            if (buf.len != (Py_ssize_t)(sizeof(*dst) * p->n)) return false;
+            memcpy((void*)dst, buf.buf, buf.len);
+            return true;
+        };
+        if (k == "l8") ok = p->has_l8 = take(p->l8);
+        else if (k == "b3") {
+            const int copies = ((const cbl_b3*)buf.buf)->copies;
+            ok = (copies == 2 || copies == 3) && take(p->b3[copies - 2]);
+            if (ok) p->has_b3[copies - 2] = true;
+        } else if (k == "dense") {
+            ok = p->has_dense = take(p->packed);
+            p->row_scale = (const void*)row_scale;
+        } else ok = false;
+        if (!ok) PyErr_SetString(PyExc_ValueError, "unknown layout or wrong descriptor size");
+    }
+    PyBuffer_Release(&buf);
+    if (!ok) return nullptr;
+    Py_RETURN_NONE;
+}
+
+// status(device): synchronises the device and returns the or of the status words the products of its streams have left
+PyObject* py_status(PyObject*, PyObject* args) {
+    int device;
+    if (!PyArg_ParseTuple(args, "i", &device)) return nullptr;
+    long bad = 0;
+    try {
+        const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+        cudaDeviceSynchronize();
+        std::lock_guard<std::mutex> lock(g_mu);
+        for (auto& e : g_scratch) {
+            if (e.first.first != device) continue;
+            Scratch& s = e.second;
+            if (s.l8.defined() && cbl_gemv_l8_status(s.l8.data_ptr(), 0, nullptr)) bad |= 1;
+            if (s.partial.defined() && cbl_gemm_b3_status(s.partial.data_ptr(), nullptr)) bad |= 2;
+            if (s.dense_stage.defined()) {
+                unsigned int v = 0;
+                cudaMemcpy(&v, (char*)s.dense_stage.data_ptr() + s.dense_stage.numel() - 16, 4, cudaMemcpyDeviceToHost);
+                if (v) bad |= 4;
+            }
+        }
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+    return PyLong_FromLong(bad);
+}
+
+PyMethodDef methods[] = {
+    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "forward(plan, x) -> y or None"},
+    {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias)"},
+    {"set", py_set, METH_VARARGS, "set(plan, kind, descriptors, row_scale=0)"},
+    {"status", py_status, METH_VARARGS, "status(device) -> bits"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_cblhost", "native call path of the packed linears", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__cblhost(void) { return PyModule_Create(&module_def); }

@@ -24,8 +24,8 @@ import torch
 
 from . import _lib
 from ._lib import lib
-from .kernels import DenseStack, L8Group, _dt, _stream
-from .linear import DENSE_MIN_TOKENS, ROWS_MIN_TOKENS, PackedLinear, RunsLin
+from .kernels import DenseStack, _dt, _stream
+from .linear import PackedLinear, RunsLin, Stack
 
 NAMES = ("q", "k", "v", "o", "gate", "up", "down")
 
@@ -127,47 +127,17 @@ class Q4Embed:
 
 
 class _Stage:
-    """Linears that read the same input and write column slices of one [B, sum R] buffer (q|k|v, gate|up,
-    or a single matrix). One token and one column order: one grouped table-lookup launch."""
+    """A Stack of linears for B sequences and its [B, sum R] output buffer.  `group` is the grouped table-lookup launch of one
+    token (None where the stage runs otherwise)."""
 
-    def __init__(self, lins: list, out: torch.Tensor):
-        self.lins = [_lin(l) for l in lins]
-        self.out, self.B = out, out.shape[0]
-        self.offs, o = [], 0
-        for l in self.lins:
-            self.offs.append(o)
-            o += l.R
-        assert o == out.shape[1]
-        self.group = self.rows = None
-        one_order = all(l.dm.M == 1 for l in self.lins) and len(self.lins) <= L8Group.MAX and len({l.dm.books for l in self.lins}) == 1
-        if self.B == 1 and one_order:
-            self.group = L8Group([l.l8 for l in self.lins])
-            self.ys = [out[0, o:o + l.R] for o, l in zip(self.offs, self.lins)]
-        elif self.B >= ROWS_MIN_TOKENS and one_order:
-            # a few dozen sequences: the tensor-core kernel with the weight rows as the M side, all matrices in one launch
-            self.rows = L8Group([l.l8 for l in self.lins])
-            self.ys = [out[:, o:o + l.R] for o, l in zip(self.offs, self.lins)]
-        else:
-            for l in self.lins:
-                l.small_batch(self.B).xp_buffer(self.B)
-            # one staging pass of the activations serves every matrix of the stage when they share the column orders
-            p0 = self.lins[0].dm.perms
-            self.share = all(l.dm.M == self.lins[0].dm.M and (l.dm.perms is p0 or (p0 is not None and l.dm.perms is not None
-                                                                                     and torch.equal(l.dm.perms, p0)))
-                             for l in self.lins)
+    def __init__(self, stack: Stack, out: torch.Tensor):
+        self.stack, self.out, self.B = stack, out, out.shape[0]
+        stack.prepare(self.B)
+        self.group = stack.l8 if self.B == 1 and stack.tables else None
+        self.rows = stack.b3(self.B) if self.group is None and stack.shared else None     # the weight rows as the M side, one launch
 
     def run(self, x: torch.Tensor) -> None:
-        if self.group is not None:
-            self.group.run(x[0], self.ys)
-        elif self.rows is not None:
-            self.rows.gemm_rows(x, self.ys)
-        elif self.share:
-            xp = self.lins[0].small_batch(self.B).prep(x, self.B)
-            for o, l in zip(self.offs, self.lins):
-                l.small_batch(self.B).run_prepped(xp, self.out[:, o:o + l.R], self.B)
-        else:
-            for o, l in zip(self.offs, self.lins):
-                l.forward_into(x, self.out[:, o:o + l.R])
+        self.stack.run(x, self.out)
 
 
 class DecodeEngine:
@@ -218,13 +188,10 @@ class DecodeEngine:
             else:
                 sizes = (NH * HD, NKV * HD, NKV * HD)
                 self.biases.append(torch.cat([b.to(**a) if b is not None else torch.zeros(n, **a) for b, n in zip(bs, sizes)]))
-        self.stages = []
-        for L in layers:
-            self.stages.append({"qkv": _Stage([L["q"], L["k"], L["v"]], self.yqkv), "o": _Stage([L["o"]], self.yo),
-                                "gu": _Stage([L["gate"], L["up"]], self.ygu), "down": _Stage([L["down"]], self.yd)})
-        # prompts: q|k|v and gate|up as stacked two-phase GEMMs (decode once, one launch over the stacked rows)
-        self.stacks = [{"qkv": DenseStack([_lin(L[n]).dm for n in ("q", "k", "v")]), "gu": DenseStack([_lin(L[n]).dm for n in ("gate", "up")])}
-                       for L in layers]
+        self.stacks = [{"qkv": Stack([_lin(L[n]) for n in ("q", "k", "v")]), "o": Stack([_lin(L["o"])]),
+                        "gu": Stack([_lin(L[n]) for n in ("gate", "up")]), "down": Stack([_lin(L["down"])])} for L in layers]
+        self.stages = [{"qkv": _Stage(S["qkv"], self.yqkv), "o": _Stage(S["o"], self.yo), "gu": _Stage(S["gu"], self.ygu),
+                        "down": _Stage(S["down"], self.yd)} for S in self.stacks]
         self.graph = None
         self.only_linears = False
         # one token, one column order everywhere: the operator that follows a product runs on its fp32 sums (one small kernel)
@@ -289,19 +256,6 @@ class DecodeEngine:
             _lib.check("cbl_argmax", lib.cbl_argmax(self.logits.data_ptr(), _dt(self.logits.dtype), self.logits.stride(0), B, self.logits.shape[1],
                                                     self.tok.data_ptr(), self.pos.data_ptr(), s))
 
-    def _pieces(self, li: int, stack: str, names, x, y) -> None:
-        """Prompt tokens through stacked linears: one stacked two-phase GEMM for long prompts (or several column
-        orders), else piece by piece into column slices of y."""
-        L = self.layers[li]
-        if x.shape[0] >= DENSE_MIN_TOKENS or (x.shape[0] > 64 and any(_lin(L[n]).dm.M > 1 for n in names)):
-            self.stacks[li][stack].gemm(x, y)
-            return
-        o = 0
-        for n in names:
-            l = _lin(L[n])
-            l.forward_into(x, y[:, o:o + l.R])
-            o += l.R
-
     def _step_fused(self, s: int) -> None:
         """Batch-1 layers, each product followed by its step operator on the fp32 sums: q|k|v + rotary + cache
         write, attention, o + add + norm, gate|up + silu * up, down + add + norm (of the next layer)."""
@@ -350,7 +304,7 @@ class DecodeEngine:
             add = None
             for li, L in enumerate(self.layers):
                 self._addnorm(h, add, L["ln1"], x, T)
-                self._pieces(li, "qkv", ("q", "k", "v"), x, yqkv)
+                self.stacks[li]["qkv"].run(x, yqkv)
                 kc, vc = self.kc[li], self.vc[li]
                 self._rope(yqkv, self.biases[li], None, 0, seq, T, qr, kc, vc)
                 q4 = qr.view(T, NH, HD).transpose(0, 1)[None]
@@ -359,11 +313,11 @@ class DecodeEngine:
                     v4 = (v4 + self.biases[li][(NH + NKV) * HD:].view(1, NKV, 1, HD)).to(self.dtype)
                 ao = torch.nn.functional.scaled_dot_product_attention(q4, kc[seq, :, :T][None], v4, is_causal=True, enable_gqa=True)
                 ao = ao[0].transpose(0, 1).reshape(T, NH * HD)
-                _lin(L["o"]).forward_into(ao, yo)
+                self.stacks[li]["o"].run(ao, yo)
                 self._addnorm(h, yo, L["ln2"], x, T)
-                self._pieces(li, "gu", ("gate", "up"), x, ygu)
+                self.stacks[li]["gu"].run(x, ygu)
                 self._silu(ygu, act, T)
-                _lin(L["down"]).forward_into(act, yd)
+                self.stacks[li]["down"].run(act, yd)
                 add = yd
             hl, xl = h[T - 1:T].clone(), torch.empty(1, H, **a)
             self._addnorm(hl, yd[T - 1:T], self.final_norm, xl, 1)

@@ -418,7 +418,6 @@ class B3Group:
         self.bmax = mats[0].bmax
         self.mats, self.C, self.M, self.device = mats, mats[0].C, mats[0].M, mats[0].device
         self.biases = biases if biases is not None else [None] * len(mats)
-        self.perms = mats[0].dm.perms
         self._built = None
         self._ws_bytes: dict = {}
         self._ys = (ctypes.c_void_p * len(mats))()
@@ -429,6 +428,10 @@ class B3Group:
         if self._built is None or self._built[0] != key:
             self._built = (key, (_lib.B3 * len(self.mats))(*[m.struct(b) for m, b in zip(self.mats, self.biases)]))
         return self._built[1]
+
+    @property
+    def perms(self) -> torch.Tensor | None:
+        return self.mats[0].dm.perms
 
     @classmethod
     def buffers(cls, device: torch.device, stage_bytes: int, ws_bytes: int) -> tuple[torch.Tensor, torch.Tensor]:
@@ -530,6 +533,9 @@ class DenseStack:
         device = torch.device(device)
         key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
         st = cls._stage.get(key)
+        from . import _cblhost
+        if _cblhost.status(key[0]):
+            raise _lib.CblError("forward", _lib.ETIMEOUT, "a bounded device-side wait expired")
         if st is not None:
             torch.cuda.synchronize(device)
             if int(st[-16:].view(torch.int32)[0]) != 0:

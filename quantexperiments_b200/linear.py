@@ -1,7 +1,7 @@
 """The packed-linear call surfaces of the reference, backed by libcbl.
 
 PackedLinear   mirrors shapequant/kernels/gemv.py:107-175 (from_packed, gemv, dense, forward, stored_bytes);
-               more than 64 tokens run the fused decode + tcgen05 GEMM (the role of shapequant/kernels/runs_gemm.py:471-514)
+               more than 128 tokens run the two-phase decode + tcgen05 GEMM (the role of shapequant/kernels/runs_gemm.py:471-514)
 RunsLin        mirrors shapequant/kernels/decode_e2e.py:405-443 (run(x, y) into a caller-provided buffer)
 runs_linear    mirrors shapequant/runtime.py:41-51
 RunsBatch      mirrors shapequant/kernels/batched_runs.py:680-771 (run(X, Y, B))
@@ -19,34 +19,27 @@ import math
 
 import torch
 
-from .kernels import DeviceMatrix, L8Matrix, T16Matrix
+from . import _cblhost, _lib
+from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix
 
-# rows from which the batch-1 product uses activation-side tables instead of codeword lookups; with several column
-# orders every order needs its own tables, so the rule applies to the rows per order (measured on B200: a table build
-# costs as much as the lookups of ~1300 rows)
-L8_MIN_ROWS = 2048
+# One token, one column order: activation-side tables (L8Matrix) at every number of rows (64 x 3584: 5.8 us against 8.4 by
+# codeword gathers, 4096 x 3584: 6.8 against 10.1, 18944 x 3584: 13.2 against 14.5).  With several column orders every order
+# needs its own tables; those matrices gather codewords (B3Matrix) at every token count (5120 x 5120, 16 orders, two
+# books: 24 us against 47; 27648 x 5120: 55 against 59).  The rows per order from which the tables would still do are
+# what RowParallelLinear.attach() asks for.
+L8_MIN_ROWS = 1
 L8_MIN_ROWS_PER_ORDER = 1536
-# tokens from which the two-phase path runs (decode the matrix once into a 16-bit scratch + TMA-fed tensor-core
-# GEMM). Measured on B200 it beats the kernel that decodes weight tiles on the fly at every token count above the
-# small-batch kernel's 64 (12.1 vs 20.6 ms for the 196 Qwen2.5-7B matrices at 128 tokens, 30 vs 36 ms at 2048).
-DENSE_MIN_TOKENS = 65
-# tokens from which (up to 64) matrices with one column order run on the tensor-core kernel that takes the weight
-# rows as the M side (its cost does not grow with the token count; the mma.sync kernel wins below: 18944 x 3584 pair
-# 66 us at any count against 49 / 63 / 132 us at 8 / 16 / 32 tokens)
-ROWS_MIN_TOKENS = 17
-# 9..16 tokens, one column order: the activation-stationary mma.sync kernel (18944 x 3584 pair 45 us at any count up to
-# 16, against 72-75 us for the row-tile kernel at 12 / 16 tokens and 64 us for the rows-as-M kernel; up to 8 tokens the
-# row-tile kernel is as fast inside a step: 3.26 / 3.60 ms for the 196-matrix set at 4 / 8 tokens against 3.40 / 3.61)
-X16_MIN_TOKENS, X16_MAX_TOKENS = 9, 16
-
-
-def _is_capturing() -> bool:
-    return torch.cuda.is_current_stream_capturing()
+# Tokens up to which the book lies three times in shared memory (the activations of more tokens need the room: two copies).
+B3_MAX_3COPIES = 16
+# Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM.
+DENSE_MIN_TOKENS = 129
+# counts loader.pool_layouts() calls: native plans made before one hold old addresses
+pool_epoch = 0
 
 
 class PackedLinear(torch.nn.Module):
-    """A block linear run from packed tensors: one token -> batch-1 kernel, up to 64 tokens -> the
-    small-batch tensor-core kernel, more -> fused decode + tcgen05 GEMM. Constructor arguments follow the
+    """A block linear run from packed tensors: one token -> batch-1 kernel, up to 128 tokens -> the
+    codeword-gather tensor-core kernel, more -> decode once + tcgen05 GEMM. Constructor arguments follow the
     reference (words, table, row_scale, row_book, row_mask, perms, K, d, bias)."""
 
     def __init__(self, words, table, row_scale, row_book, row_mask, perms, K: int, d: int, bias=None,
@@ -68,6 +61,8 @@ class PackedLinear(torch.nn.Module):
         self.bias = bias
         self._t16: T16Matrix | None = None
         self._l8: L8Matrix | None = None
+        self._b3: dict[int, B3Group] = {}
+        self._host = None                       # native call plan (csrc/host.cpp), made after the first call of a kind
 
     @classmethod
     def from_packed(cls, pf, name: str, device="cuda", bias=None, **kw):
@@ -98,17 +93,33 @@ class PackedLinear(torch.nn.Module):
             self._x16 = X16Matrix(self.dm)
         return self._x16
 
-    def small_batch(self, n: int):
-        """The kernel layout that multiplies n <= 64 tokens by this matrix (prep / run_prepped / run / xp_buffer): the
-        activation-stationary one for 2..16 tokens and one column order, else the row-tile one."""
-        return self.x16 if (self.dm.M == 1 and X16_MIN_TOKENS <= n <= X16_MAX_TOKENS) else self.t16
+    def group(self, n: int) -> B3Group:
+        """The layout that multiplies n tokens (2..128, or 1 without the table layout), built on first use."""
+        copies = 3 if n <= B3_MAX_3COPIES else 2
+        g = self._b3.get(copies)
+        if g is None:
+            g = self._b3[copies] = B3Group([B3Matrix(self.dm, copies)])
+        return g
 
-    @property
-    def rows_group(self):
-        if getattr(self, "_rows_group", None) is None:
-            from .kernels import L8Group
-            self._rows_group = L8Group([self.l8])
-        return self._rows_group
+    def small_batch(self, n: int):
+        """The mma.sync layouts (prep / run_prepped / run / xp_buffer), kept for callers that stage activations themselves:
+        activation-stationary for 9..16 tokens and one column order, else row tiles."""
+        return self.x16 if (self.dm.M == 1 and 9 <= n <= 16) else self.t16
+
+    def _bind(self) -> None:
+        """(Re)makes the native call plan from the layouts that exist."""
+        dm = self.dm
+        if not dm.fast or (self.bias is not None and self.bias.requires_grad):
+            return
+        self._host_bias = self.bias
+        self._host = _cblhost.plan(dm.device.index, self.in_features, self.C, dm.M, [self.R], 0 if dm.perms is None else dm.perms.data_ptr(),
+                                   DENSE_MIN_TOKENS, self.bias)
+        if self._l8 is not None and self.use_l8() and dm.M == 1:
+            _cblhost.set(self._host, "l8", bytes(self._l8.struct()))
+        for g in self._b3.values():
+            _cblhost.set(self._host, "b3", bytes(g.mats[0].struct()))
+        if not self.wide:
+            _cblhost.set(self._host, "dense", bytes(dm.struct()), dm.row_scale.data_ptr())
 
     def use_l8(self) -> bool:
         """One token runs on the table-lookup kernel (any number of column orders up to its limit)."""
@@ -118,21 +129,16 @@ class PackedLinear(torch.nn.Module):
             return self.R >= L8_MIN_ROWS
         return self.dm.M <= L8Matrix.MAX_ORDERS and self.R >= L8_MIN_ROWS_PER_ORDER * self.dm.M
 
-    def use_gemm(self) -> bool:
-        """The tensor-core kernel that decodes weight tiles on the fly executes one column order (one or two
-        books); matrices with several orders take the two-phase path at every token count above 64."""
-        return self.dm.M == 1
-
     def gemv(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x [C] (fp16 / bf16 / fp32, contiguous) -> y [R] in x's dtype (or `out`'s)."""
         if not self.dm.fast:            # any d / tag width / several books per matrix: the generic product
             y = out if out is not None else torch.empty(self.R, dtype=x.dtype, device=x.device)
             self.dm.gemv_generic(x.reshape(1, -1), y.reshape(1, -1))
             return y
-        if self.use_l8():
-            return self.l8.run(x, out, wide=self.wide)
+        if self.dm.M == 1 and self.use_l8():
+            return self.l8.run(x, out)
         y = out if out is not None else torch.empty(self.R, dtype=x.dtype, device=x.device)
-        self.t16.run(x.reshape(1, -1), y.reshape(1, -1), 1, wide=self.wide)
+        self.group(1).run(x.reshape(1, -1), [y.reshape(1, -1)])
         return y
 
     def dense(self) -> torch.Tensor:
@@ -149,30 +155,117 @@ class PackedLinear(torch.nn.Module):
             # what the reference's own kernel is for them; a correctness path, whatever the token count
             self.dm.gemv_generic(x2 if x2.stride(1) == 1 else x2.contiguous(), y)
             return y
-        if n == 1 and self.use_l8() and y.is_contiguous():
-            self.l8.run(x2[0].contiguous(), y[0], wide=self.wide)
-        elif X16_MIN_TOKENS <= n <= X16_MAX_TOKENS and self.dm.M == 1:
-            self.x16.run(x2 if x2.stride(1) == 1 else x2.contiguous(), y)
-        elif n <= T16Matrix.BMAX and (n < ROWS_MIN_TOKENS or self.dm.M > 1):
-            self.t16.run(x2.contiguous(), y, n, wide=self.wide)
-        elif n <= T16Matrix.BMAX:
-            self.rows_group.gemm_rows(x2 if x2.stride(1) == 1 else x2.contiguous(), [y])
-        elif self.use_gemm() and n < DENSE_MIN_TOKENS:
-            self.l8.gemm(x2 if x2.stride(1) == 1 else x2.contiguous(), y)
+        x2 = x2 if x2.stride(1) == 1 else x2.contiguous()
+        if n == 1 and self.dm.M == 1 and self.use_l8() and y.is_contiguous():
+            self.l8.run(x2[0], y[0])
+        elif n < DENSE_MIN_TOKENS:
+            self.group(n).run(x2, [y])
         else:
-            # many tokens, or several column orders: decode once into the shared 16-bit scratch, then the TMA-fed GEMM
-            self.dm.gemm_dense(x2 if x2.stride(1) == 1 else x2.contiguous(), y)
+            # many tokens: decode once into the shared 16-bit scratch, then the TMA-fed GEMM
+            self.dm.gemm_dense(x2, y)
         return y
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if self._host is not None and self._host_bias is self.bias:
+            y = _cblhost.forward(self._host, x)
+            if y is not None:
+                return y
         lead = x.shape[:-1]
         n = math.prod(lead)
         y = self.forward_into(x.reshape(n, self.in_features), torch.empty(n, self.R, dtype=x.dtype, device=x.device))
         y = y.reshape(*lead, self.R)
+        if n:
+            self._bind()
         return y if self.bias is None else y + self.bias
 
     def stored_bytes(self) -> int:
         return self.dm.stored_bytes()
+
+
+class Stack:
+    """Linears that read the same activations (q|k|v, gate|up): run(x [n, C], y [n, sum R]) writes their outputs side by side.
+    One token: one table-lookup launch; up to 128 tokens: one codeword-gather launch where the pieces share their column
+    orders, else one per piece; more: every piece decoded once, one GEMM over the stacked rows.  Layouts are built on first
+    use of their token counts (or by prepare(), which a caller runs before it captures a graph)."""
+
+    def __init__(self, lins: list):
+        from .kernels import DenseStack, L8Group
+        self.lins, self.C, self.device = lins, lins[0].C, lins[0].dm.device
+        self.Rs = [l.R for l in lins]
+        self.R = sum(self.Rs)
+        p0 = lins[0].dm.perms
+        self.shared = len(lins) <= B3Group.MAX and all(l.dm.fast and l.dm.M == lins[0].dm.M and (l.dm.perms is p0 or (
+            p0 is not None and l.dm.perms is not None and torch.equal(l.dm.perms, p0))) for l in lins)
+        self.tables = all(l.dm.fast and l.dm.M == 1 for l in lins) and len(lins) <= L8Group.MAX
+        self.fast = all(l.dm.fast for l in lins)
+        self.dense = DenseStack([l.dm for l in lins]) if self.fast and len({l.C for l in lins}) == 1 and not any(l.wide for l in lins) else None
+        self._l8 = None
+        self._b3: dict[int, B3Group] = {}
+
+    @property
+    def l8(self):
+        from .kernels import L8Group
+        if self._l8 is None:
+            self._l8 = L8Group([l.l8 for l in self.lins])
+        return self._l8
+
+    def b3(self, n: int) -> B3Group:
+        copies = 3 if n <= B3_MAX_3COPIES else 2
+        if copies not in self._b3:
+            self._b3[copies] = B3Group([l.group(n).mats[0] for l in self.lins])
+        return self._b3[copies]
+
+    def ready(self, n: int) -> bool:
+        """Whether run() on n tokens builds no layout."""
+        if not self.fast or n >= DENSE_MIN_TOKENS:
+            return True
+        if n == 1 and self.tables:
+            return self._l8 is not None
+        copies = 3 if n <= B3_MAX_3COPIES else 2
+        return copies in self._b3 if self.shared else all(copies in l._b3 for l in self.lins)
+
+    def prepare(self, n: int) -> None:
+        if not self.fast or n >= DENSE_MIN_TOKENS:
+            return
+        if n == 1 and self.tables:
+            self.l8._structs
+        elif self.shared:
+            self.b3(n)._structs
+        else:
+            for l in self.lins:
+                l.group(n)
+
+    def run(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+        n = x.shape[0]
+        if n >= DENSE_MIN_TOKENS and self.dense is not None:
+            return self.dense.gemm(x, y)
+        ys = list(y.split(self.Rs, 1))
+        if n == 1 and self.tables:
+            self.l8.run(x[0], [t[0] for t in ys])
+        elif self.shared and n < DENSE_MIN_TOKENS:
+            self.b3(n).run(x, ys)
+        else:
+            for l, t in zip(self.lins, ys):
+                l.forward_into(x, t)
+        return y
+
+    def bind(self):
+        """Native call plan(s) of the layouts that exist: (for up to 128 tokens, for more)."""
+        if not self.fast or len(self.lins) > B3Group.MAX:
+            return None, None
+        dm = self.lins[0].dm
+        h = _cblhost.plan(dm.device.index, self.C, self.C, dm.M, self.Rs, 0 if dm.perms is None else dm.perms.data_ptr(), DENSE_MIN_TOKENS, None)
+        if self._l8 is not None:
+            _cblhost.set(h, "l8", bytes(self._l8._structs))
+        for g in self._b3.values():
+            _cblhost.set(h, "b3", bytes(g._structs))
+        if self.dense is not None:
+            _cblhost.set(h, "dense", b"".join(bytes(l.dm.struct()) for l in self.lins), self.dense.row_scale.data_ptr())
+        if self.shared:
+            return h, h
+        for l in self.lins:
+            l._bind()
+        return tuple(l._host for l in self.lins), h
 
 
 class RunsLin:
@@ -182,10 +275,10 @@ class RunsLin:
     def __init__(self, lin: PackedLinear):
         self.lin, self.R, self.C = lin, lin.R, lin.C
         self.perms = lin.dm.perms
-        if lin.use_l8():
+        if lin.dm.M == 1 and lin.use_l8():
             lin.l8          # build the layouts now, not inside a captured region
         else:
-            lin.t16.xp_buffer(1)
+            lin.group(1)
 
     def run(self, x: torch.Tensor, y: torch.Tensor, epi: dict | None = None):
         """y = W . x.  `epi` asks for the operator that follows the product in a decode step to run with it, as the
@@ -200,15 +293,14 @@ class RunsLin:
             if x.dim() == 1 or x.shape[0] == 1:
                 self.lin.gemv(x.reshape(-1), y.reshape(-1))
             else:
-                self.lin.t16.run(x, y, wide=self.lin.wide)
+                self.lin.forward_into(x, y)
             return y
         import ctypes
-        from . import _lib
         from .kernels import L8Group, _dt, _stream, l8_workspace
         if epi.get("perms") is not None:
             raise ValueError("epi['perms']: permuted copies of the output are not produced here (the next product applies its column orders itself)")
         if not self.lin.use_l8() or self.lin.dm.M != 1 or x.numel() != self.C:
-            raise ValueError("fused epilogues run one token through the table-lookup kernel (one column order, at least 2048 rows)")
+            raise ValueError("fused epilogues run one token through the table-lookup kernel (one column order)")
         mode, out = epi.get("mode"), epi["out"]
         xv = x.reshape(-1)
         if y.dtype not in (torch.float16, torch.bfloat16) or out.dtype != y.dtype:
@@ -264,8 +356,8 @@ class RunsBatch:
         if bmax > T16Matrix.BMAX:
             raise ValueError(f"bmax {bmax} over {T16Matrix.BMAX}")
         self.R, self.C, self.bmax = self.lin.R, self.lin.C, bmax
-        for b in range(1, bmax + 1):
-            self.lin.small_batch(b).xp_buffer(b)
+        for b in (1, min(bmax, B3_MAX_3COPIES), bmax):
+            self.lin.group(b)
 
     def run(self, X: torch.Tensor, Y: torch.Tensor, B: int | None = None) -> torch.Tensor:
         B = X.shape[0] if B is None else B
@@ -274,4 +366,4 @@ class RunsBatch:
             raise ValueError("RunsBatch.run: B <= bmax, X contiguous, X and Y fp16 or bf16")
         if Y.stride(-1) != 1 or Y.shape[-1] != self.R:
             raise ValueError("RunsBatch.run: Y must be [B, R] with unit column stride")
-        return self.lin.t16.run(X, Y, B, wide=True) if self.lin.wide else self.lin.small_batch(B).run(X, Y, B)
+        return self.lin.group(B).run(X[:B], [Y[:B]])[0]

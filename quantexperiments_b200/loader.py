@@ -224,19 +224,21 @@ def pool_layouts(linears) -> int:
     that use these matrices: single-matrix launchers and L8Group read the pointers at every call, but a captured
     graph, a PeerReduceGemv or a decode engine built earlier keeps the old addresses (build those afterwards).
     Returns the bytes now pooled."""
+    from . import linear
+    linear.pool_epoch += 1
     lins = [l for l in linears if not getattr(l, "_pooled", False)]
     pooled = 0
     for dev in {l.dm.device for l in lins}:
         slots = []
         for l in (x for x in lins if x.dm.device == dev):
-            objs = [l.dm] + [o for o in (l._l8, l._t16, getattr(l, "_x16", None)) if o is not None]
+            objs = [l.dm] + [o for o in (l._l8, l._t16, getattr(l, "_x16", None)) if o is not None] + [g.mats[0] for g in l._b3.values()]
             for o in objs:
                 for attr in ("tags", "tags2", "table", "table2", "row_scale", "row_book", "row_mask", "perms", "words", "words_c", "frag", "frag2",
-                             "row_index", "tile_rows", "tile_mask"):
+                             "row_index", "tile_rows", "tile_mask", "tile_order"):
                     v = getattr(o, attr, None)
                     if isinstance(v, torch.Tensor):
                         slots.append((o, attr, v))
-            l._pooled = True
+            l._pooled, l._host = True, None
         with torch.cuda.device(dev):
             arena = Arena(sum(_al(v.numel() * v.element_size()) for _, _, v in slots), dev)
             for o, attr, v in slots:

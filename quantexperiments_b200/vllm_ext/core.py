@@ -5,18 +5,17 @@ Mirrors shapequant/vllm_ext/core.py of the reference: PackedShards (:212-486: fr
 dense, nbytes, R, C), register (:622-624) and linear_op with its fake implementation (:693-702), so
 that vLLM's LinearMethod.apply can stay `torch.ops.shapequant.linear(x, handle)`.
 
-Dispatch on the number of tokens M: 1 -> batch-1 kernel per piece, <= bmax -> small-batch
-tensor-core kernel per piece, each writing its column slice of the stacked output; larger ->
-the fused decode + tcgen05 GEMM per piece into its slice (pieces with several column orders: decode
-to x's 16-bit dtype into a shared scratch followed by a library GEMM)."""
+Dispatch on the number of tokens: see linear.Stack (one token: table lookups; up to 128: codeword gathers on the tensor
+cores; more: decode once + GEMM over the stacked rows)."""
 
 from __future__ import annotations
 
 
 import torch
 
-from ..kernels import DenseStack, L8Group, T16Matrix
-from ..linear import DENSE_MIN_TOKENS, L8_MIN_ROWS, ROWS_MIN_TOKENS, PackedLinear
+from .. import _cblhost, linear
+from ..kernels import T16Matrix
+from ..linear import DENSE_MIN_TOKENS, PackedLinear, Stack
 
 BMAX = T16Matrix.BMAX
 
@@ -60,42 +59,22 @@ class PackedShards:
         self.bmax = self.cross = bmax
         self.device = lins[0].dm.device
         self.sq_name = ""
-        self.stack = DenseStack([lin.dm for lin in lins])     # many tokens / several column orders: decode once, one GEMM
         # Kernel layouts are second copies of the tags in a kernel's order: each is built when its token-count class
         # is first used (or by prepare()), so a layer that only ever decodes keeps one extra copy, not three.
-        self.group = self.rows = None
-        self._one_order = all(lin.dm.M == 1 for lin in lins) and len(lins) <= L8Group.MAX
-        self._ready: set = set()
+        self.stack = Stack(lins)
+        self._host = (None, None)               # native call plans: up to 128 tokens, more
         self.prepare(1)
 
-    def _class_of(self, M: int) -> str:
-        if M == 1:
-            return "one"
-        if M <= self.cross:
-            return "rows" if (M >= ROWS_MIN_TOKENS and self._one_order and len({lin.dm.books for lin in self.lins}) == 1) else f"small{M}"
-        return "many"
-
     def prepare(self, M: int) -> None:
-        """Build whatever forward() needs for M tokens (kernel layouts, staging buffers).  forward() calls it on
-        first use; call it yourself for every token count a CUDA graph will replay, before capturing."""
-        cls = self._class_of(M)
-        if cls in self._ready:
-            return
-        if torch.cuda.is_current_stream_capturing():
-            raise RuntimeError(f"PackedShards.prepare({M}) must run before the stream is captured (layouts are allocated on first use)")
-        if cls == "one":
-            if self._one_order and self.R >= L8_MIN_ROWS:
-                self.group = L8Group([lin.l8 for lin in self.lins])       # all pieces in one launch
-            else:
-                for lin in self.lins:
-                    lin.l8 if lin.use_l8() else lin.small_batch(1).xp_buffer(1)
-        elif cls == "rows":
-            self.rows = self.group if self.group is not None else L8Group([lin.l8 for lin in self.lins])
-            self.rows._structs_c                                      # (built by the first gemm_rows otherwise)
-        elif cls.startswith("small"):
-            for lin in self.lins:
-                lin.small_batch(M).xp_buffer(M)
-        self._ready.add(cls)
+        """Build whatever forward() needs for M tokens.  forward() calls it on first use; call it yourself for every token
+        count a CUDA graph will replay, before capturing."""
+        if not self.stack.ready(M):
+            if torch.cuda.is_current_stream_capturing():
+                raise RuntimeError(f"PackedShards.prepare({M}) must run before the stream is captured (layouts are allocated on first use)")
+            self.stack.prepare(M)
+            self._host = (None, None)
+        if self._host[1] is None or self._epoch != linear.pool_epoch:
+            self._host, self._epoch = self.stack.bind(), linear.pool_epoch
 
     @classmethod
     def from_packed(cls, pf, names: list[str], dev="cuda", **kw) -> "PackedShards":
@@ -108,6 +87,7 @@ class PackedShards:
             n += lin._t16.nbytes() if lin._t16 is not None else 0
             n += lin._x16.nbytes() if getattr(lin, "_x16", None) is not None else 0
             n += lin._l8.nbytes() if lin._l8 is not None else 0
+            n += sum(g.mats[0].nbytes() for g in lin._b3.values())
         return n
 
     def dense(self) -> torch.Tensor:
@@ -117,41 +97,19 @@ class PackedShards:
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """x [..., C] -> [..., R] in x's dtype."""
         shp = x.shape
+        M = x.numel() // self.C
+        host = self._host[M >= DENSE_MIN_TOKENS]
+        if host is not None and self._epoch == linear.pool_epoch and x.dtype in (torch.float16, torch.bfloat16):
+            y = _cblhost.forward(host, x)
+            if y is not None:
+                return y
         x2 = x.reshape(-1, self.C)
-        M = x2.shape[0]
         if M == 0:
-            y = x2.new_empty(0, self.R)
-        elif M <= self.cross:
-            self.prepare(M)
-            xin = x2 if x2.dtype in (torch.float16, torch.bfloat16) else x2.to(torch.bfloat16)
-            y = self._small(xin.contiguous(), M)
-        else:
-            xin = x2 if x2.dtype in (torch.float16, torch.bfloat16) else x2.to(torch.bfloat16)
-            y = self._large(xin.contiguous())
+            return x2.new_empty(0, self.R).view(*shp[:-1], self.R)
+        self.prepare(M)
+        xin = x2 if x2.dtype in (torch.float16, torch.bfloat16) else x2.to(torch.bfloat16)
+        y = self.stack.run(xin.contiguous(), torch.empty(M, self.R, dtype=xin.dtype, device=x.device))
         return y.to(x.dtype).view(*shp[:-1], self.R)
-
-    def _small(self, x: torch.Tensor, M: int) -> torch.Tensor:
-        y = torch.empty(M, self.R, dtype=x.dtype, device=x.device)
-        if M == 1 and self.group is not None:
-            self.group.run(x[0], [y[0, off:off + R] for off, R in zip(self.offs, self.Rs)])
-            return y
-        if self._class_of(M) == "rows":
-            self.rows.gemm_rows(x, [y[:, off:off + R] for off, R in zip(self.offs, self.Rs)])
-            return y
-        for lin, off, R in zip(self.lins, self.offs, self.Rs):
-            if M == 1 and lin.use_l8():
-                lin.l8.run(x[0], y[0, off:off + R])
-            else:
-                lin.small_batch(M).run(x, y[:, off:off + R], M)
-        return y
-
-    def _large(self, x: torch.Tensor) -> torch.Tensor:
-        y = torch.empty(x.shape[0], self.R, dtype=x.dtype, device=x.device)
-        if x.shape[0] >= DENSE_MIN_TOKENS or not all(lin.use_gemm() for lin in self.lins):
-            return self.stack.gemm(x, y)                  # all pieces decoded once, one TMA-fed tcgen05 GEMM over the stacked rows
-        for lin, off, R in zip(self.lins, self.offs, self.Rs):
-            lin.l8.gemm(x, y[:, off:off + R])             # fused decode + tcgen05 GEMM straight into the column slice
-        return y
 
 
 # ------------------------------------------------------------------ torch custom op
