@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(256) k_rows_finish(const __grid_constant__ GRL
 // The fused kernels above decode every weight tile once per 256 (or 512) tokens; their shared-memory pipe
 // carries the codeword gathers, the B-tile stores, the activation tiles and the tensor cores' operand
 // reads, and saturates before the tensor pipe does.  From about a thousand tokens on it is cheaper to
-// decode the matrix ONCE into a 16-bit scratch (k_decode_raw: raw codewords, or the sum of the two books'
+// decode the matrix ONCE into a 16-bit scratch (cbl_decode_raw: raw codewords, or the sum of the two books'
 // codewords, column orders undone) and to run a plain TMA-fed tcgen05 GEMM over it (k_gemm_dense: both
 // operands arrive by TMA, nothing but the tensor cores reads shared memory).  Row scales and the tokens'
 // power-of-two scales are applied in the epilogue exactly as in the fused kernel.  The scratch also
@@ -1104,83 +1104,6 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     }
 }
 
-// Raw 16-bit decode of a packed matrix (d = 8, 12-bit tags): out[r, col] = fp16(A[a] (+ B[b])) without the row
-// scale, col = the original column (column orders undone).  A warp walks one row 256 chunks at a time, lane l
-// taking chunks l, l + 32, ...: the 16-byte codewords of a warp-wide store are contiguous.  The book(s) sit in
-// shared memory.  One block of 512 threads per SM; it is launched with programmatic serialization and waits
-// for its predecessors only at its END, so that it decodes the next matrix beside a running GEMM (which
-// leaves shared memory for it) while everything after it still sees the stream's order.
-constexpr int DR_THREADS = 512;            // x 56 registers: fits beside the GEMM's 320 threads x 104 registers
-template <int BOOKS, bool PERM>
-__global__ void __maxnreg__(56) k_decode_raw(cbl_packed m, __half* __restrict__ out, int64_t ld) {
-    extern __shared__ __align__(16) unsigned char dsm[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    {
-        uint4* dst = (uint4*)dsm;
-        const uint4* t0 = (const uint4*)m.table;
-        for (int i = tid; i < 4096; i += DR_THREADS) dst[i] = __ldg(t0 + i);
-        if (BOOKS == 2) {
-            const uint4* t1 = (const uint4*)m.table2;
-            for (int i = tid; i < 4096; i += DR_THREADS) dst[4096 + i] = __ldg(t1 + i);
-        }
-    }
-    __syncthreads();
-    const uint32_t sb = cbl_smem_u32(dsm);
-    const int nch = m.C >> 3;
-    auto tag_of = [&](const int32_t* rw, int j) {
-        const uint32_t bit = 12u * (uint32_t)j, w = bit >> 5, sh = bit & 31u;
-        const uint32_t lo = (uint32_t)__ldg(rw + w);
-        const uint32_t hi = (sh > 20u && (int)(w + 1) < m.W) ? (uint32_t)__ldg(rw + w + 1) : 0u;
-        return (__funnelshift_r(lo, hi, sh) & 0xFFFu) << 4;
-    };
-    for (int r = blockIdx.x * (DR_THREADS / 32) + warp; r < m.R; r += gridDim.x * (DR_THREADS / 32)) {
-        const int32_t* rw = m.tags + (int64_t)r * m.W;
-        const int32_t* rw2 = BOOKS == 2 ? m.tags2 + (int64_t)r * m.W : nullptr;
-        const int32_t* perm = PERM ? m.perms + (int64_t)m.row_mask[r] * m.C : nullptr;
-        __half* orow = out + (int64_t)r * ld;
-        for (int j0 = 0; j0 < nch; j0 += 256) {
-            uint4 cw[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int j = j0 + 32 * i + lane;
-                cw[i] = make_uint4(0, 0, 0, 0);
-                if (j < nch) cw[i] = cbl_lds128(sb + tag_of(rw, j));
-            }
-            if (BOOKS == 2) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int j = j0 + 32 * i + lane;
-                    if (j < nch) {
-                        const uint4 o = cbl_lds128(sb + 65536u + tag_of(rw2, j));
-                        __half2* a = (__half2*)&cw[i];
-                        const __half2* b = (const __half2*)&o;
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float2 fa = __half22float2(a[e]), fb = __half22float2(b[e]);
-                            a[e] = __floats2half2_rn(fa.x + fb.x, fa.y + fb.y);
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int j = j0 + 32 * i + lane;
-                if (j < nch) {
-                    if (!PERM) {
-                        *(uint4*)(orow + j * 8) = cw[i];
-                    } else {
-                        const __half* hv = (const __half*)&cw[i];
-#pragma unroll
-                        for (int e = 0; e < 8; e++) orow[__ldg(perm + j * 8 + e)] = hv[e];
-                    }
-                }
-            }
-        }
-    }
-    asm volatile("griddepcontrol.wait;" ::: "memory");          // later kernels that wait for this one also wait for its predecessors
-}
-
 }  // namespace
 
 // Staging of the activations for cbl_gemm_l8: fp16 [Mpad8][Cpad512] followed by fp32 [Mpad8] inverse scales
@@ -1263,60 +1186,6 @@ extern "C" int cbl_gemm_l8_2sm(const cbl_l8* m, const void* x, int xdtype, int32
 }
 
 // ---- two-phase variant: host side
-extern "C" size_t cbl_dense_scratch_bytes(int32_t R, int32_t C) {
-    if (R < 0 || C < 0) return 0;
-    return (size_t)R * ((size_t)(C + 7) / 8 * 8) * 2;
-}
-
-static int decode_raw_impl(const cbl_packed* m, void* out, int32_t C_out, cbl_stream s) {
-    if (!m || !m->tags || !m->table || !out || ((uintptr_t)out % 16) || ((uintptr_t)m->table % 16)) return CBL_EINVAL;
-    if (C_out < m->C || (C_out > m->C && m->M <= 1)) return CBL_EINVAL;      // a wider output only makes sense with column orders
-    if (m->d != 8 || m->bits != 12 || m->G != 1) return CBL_EUNSUPPORTED;
-    if (m->R < 0 || m->C <= 0 || m->C % 8 || (int64_t)m->W * 32 < (int64_t)(m->C / 8) * 12) return CBL_EINVAL;
-    if (m->books != 1 && m->books != 2) return CBL_EINVAL;
-    if (m->books == 2 && (!m->tags2 || !m->table2 || ((uintptr_t)m->table2 % 16))) return CBL_EINVAL;
-    if (m->M > 1 && (!m->row_mask || !m->perms)) return CBL_EINVAL;
-    if (m->R == 0) return CBL_OK;
-    const int64_t ld = ((int64_t)C_out + 7) / 8 * 8;
-    const size_t smem = (size_t)65536 * m->books;
-    int grid = cbl_sm_count();
-    if (grid > cbl_ceil_div(m->R, DR_THREADS / 32)) grid = cbl_ceil_div(m->R, DR_THREADS / 32);
-    const cudaStream_t st = (cudaStream_t)s;
-    static bool attr_set[64][4] = {};
-    int dev = 0;
-    CBL_CUDA(cudaGetDevice(&dev));
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(DR_THREADS);
-    cfg.dynamicSmemBytes = smem;
-#define CBL_RAW(BK, PM, SLOT)                                                                                              \
-    do {                                                                                                                   \
-        if (dev >= 0 && dev < 64 && !attr_set[dev][SLOT]) {                                                                \
-            CBL_CUDA(cudaFuncSetAttribute(k_decode_raw<BK, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536 * BK)); \
-            attr_set[dev][SLOT] = true;                                                                                    \
-        }                                                                                                                  \
-        CBL_CUDA(cudaLaunchKernelEx(&cfg, k_decode_raw<BK, PM>, *m, (__half*)out, ld));                                    \
-    } while (0)
-    if (m->books == 1 && m->M == 1) CBL_RAW(1, false, 0);
-    else if (m->books == 1) CBL_RAW(1, true, 1);
-    else if (m->M == 1) CBL_RAW(2, false, 2);
-    else CBL_RAW(2, true, 3);
-#undef CBL_RAW
-    return cbl_check_launch();
-}
-
-extern "C" int cbl_decode_raw(const cbl_packed* m, void* out, cbl_stream s) { return decode_raw_impl(m, out, m ? m->C : 0, s); }
-
-// The same for a column shard of a matrix with several column orders, whose orders name positions of the FULL
-// activation vector (C_out of them): the scratch row is C_out wide and the shard's weights land at their positions.
-extern "C" int cbl_decode_raw_wide(const cbl_packed* m, void* out, int32_t C_out, cbl_stream s) { return decode_raw_impl(m, out, C_out, s); }
-
 extern "C" int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok,
                               int64_t ldx, void* y, int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
     return cbl_gemm_dense_bias(w16, R, C, row_scale, x, xdtype, ntok, ldx, y, ydtype, ldy, nullptr, stage, workspace, s);

@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes
 import math
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -120,7 +121,7 @@ class DeviceMatrix:
 
     def gemm_dense(self, X: torch.Tensor, Y: torch.Tensor | None = None) -> torch.Tensor:
         """Y [T, R] = X [T, C] . W^T through the two-phase path (see DenseStack).  A shard with x_cols takes X
-        [T, x_cols]: it is decoded once into a zeroed 16-bit scratch as wide as the activation vector (its orders name
+        [T, x_cols]: it is decoded once into a 16-bit scratch as wide as the activation vector (its orders name
         positions of that vector) and multiplied over all x_cols columns - every rank multiplies the full width, its rows
         being 1 / world dense, so for such shards this path buys tensor-core speed on long inputs, not a per-rank saving."""
         if self.x_cols is None:
@@ -147,7 +148,6 @@ class DeviceMatrix:
         if st is None or st.numel() < nst:
             st = DenseStack._stage[key] = torch.zeros(nst, dtype=torch.uint8, device=self.device)
         with torch.cuda.device(self.device):
-            sc[:need].zero_()
             s = _stream()
             _lib.check("cbl_decode_raw_wide", lib.cbl_decode_raw_wide(ctypes.byref(self.struct()), sc.data_ptr(), Cx, s))
             _lib.check("cbl_gemm_dense", lib.cbl_gemm_dense(sc.data_ptr(), self.R, Cx, self.row_scale.data_ptr(), X.data_ptr(), _dt(X.dtype), T,
@@ -365,17 +365,16 @@ def order_tiles(dm: DeviceMatrix, rows: int) -> tuple[torch.Tensor | None, torch
     column order needs no table: (None, None, ceil(R / rows))."""
     if dm.M == 1:
         return None, None, -(-dm.R // rows)
-    mask = dm.row_mask.to(torch.int64)
-    count = torch.bincount(mask, minlength=dm.M)
+    mask = dm.row_mask.cpu().numpy()
+    count = np.bincount(mask, minlength=dm.M)
     padded = (count + rows - 1) // rows * rows
-    start = torch.cumsum(padded, 0) - padded
-    by_order = torch.argsort(mask, stable=True)
-    rank = torch.arange(dm.R, device=dm.device) - torch.repeat_interleave(torch.cumsum(count, 0) - count, count)
-    n = int(padded.sum())
-    tile_rows = torch.full((n,), -1, dtype=torch.int32, device=dm.device)
-    tile_rows[start[mask[by_order]] + rank] = by_order.to(torch.int32)
-    tile_order = torch.repeat_interleave(torch.arange(dm.M, dtype=torch.int32, device=dm.device), padded // rows)
-    return tile_rows, tile_order, n // rows
+    start = np.cumsum(padded) - padded
+    by_order = np.argsort(mask, kind="stable")
+    rank = np.arange(dm.R) - np.repeat(np.cumsum(count) - count, count)
+    tile_rows = np.full(int(padded.sum()), -1, dtype=np.int32)
+    tile_rows[start[mask[by_order]] + rank] = by_order
+    tile_order = np.repeat(np.arange(dm.M, dtype=np.int32), padded // rows)
+    return torch.from_numpy(tile_rows).to(dm.device), torch.from_numpy(tile_order).to(dm.device), tile_order.size
 
 
 class B3Matrix:
