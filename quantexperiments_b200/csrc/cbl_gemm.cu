@@ -994,34 +994,37 @@ k_gemm_dense(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ C
 // tensor-memory columns: two buffers alternate, the epilogue warps drain one while the MMAs fill the other.
 // Barriers: "full" (leader block; TMA bytes of both blocks), "empty" and "accumulator full" (each block;
 // multicast commits from the leader), "accumulator empty" (leader; one arrival per epilogue warp of both blocks).
-constexpr int G3_STAGES = 4;              // 128 KB: leaves room for a decode block of the NEXT matrix on the same SM
-constexpr int G3_STAGE_BYTES = GM_A_BYTES + 128 * GM_BK * 2;                // 128 tokens + 128 rows of one k-block: 32 KB
-constexpr int G3_SMEM = G3_STAGES * G3_STAGE_BYTES + 1024;
+// Ring: as many stages of (128 tokens + half a tile's rows) x 64 columns as shared memory holds, 7 to 9.  A copy takes about
+// 1.5 us under load; with four stages (room for a decode block beside the GEMM) a k-block took 0.4 us whatever the tile.
+constexpr int G3_MAX_STAGES = 9;
+constexpr int G3_SMEM = 230400;
 constexpr int G3_EPI_WARPS = 8, G3_THREADS = (G3_EPI_WARPS + 2) * 32;
 
 __global__ void __launch_bounds__(G3_THREADS, 1)
 k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, cbl_l8 m, const float* __restrict__ xinv,
-                 int ntok, void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok, const void* __restrict__ bias, unsigned int* __restrict__ status) {
+                 int ntok, void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok, const void* __restrict__ bias, int bn, unsigned int* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long s_bar[2 * G3_STAGES + 4];   // full, empty per stage; acc_full[2], acc_empty[2]
+    __shared__ __align__(8) unsigned long long s_bar[2 * G3_MAX_STAGES + 4];   // full, empty per stage; acc_full[2], acc_empty[2]
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
-    // a decode kernel of the next matrix (launched with programmatic serialization) may share the SMs with this GEMM
+    // the decode of the next matrix (launched with programmatic serialization) takes the SMs as this GEMM leaves them
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int nkb = (m.C + GM_BK - 1) / GM_BK;
-    const int ntt = (ntok + 255) / 256, nrt = (m.R + GM_BN - 1) / GM_BN, ntiles = ntt * nrt;
+    const uint32_t stage_bytes = (uint32_t)(GM_A_BYTES + bn * 64);
+    const int nst = min(G3_MAX_STAGES, (int)((G3_SMEM - 1024) / stage_bytes));
+    const int ntt = (ntok + 255) / 256, nrt = (m.R + bn - 1) / bn, ntiles = ntt * nrt;
     const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
     const uint32_t sbase = (cbl_smem_u32(smem_raw) + 1023u) & ~1023u, bar0 = cbl_smem_u32(s_bar);
     auto full = [&](int s) { return bar0 + 8u * s; };
-    auto empty = [&](int s) { return bar0 + 8u * (G3_STAGES + s); };
-    auto acc_full = [&](int b) { return bar0 + 8u * (2 * G3_STAGES + b); };
-    auto acc_empty = [&](int b) { return bar0 + 8u * (2 * G3_STAGES + 2 + b); };
+    auto empty = [&](int s) { return bar0 + 8u * (G3_MAX_STAGES + s); };
+    auto acc_full = [&](int b) { return bar0 + 8u * (2 * G3_MAX_STAGES + b); };
+    auto acc_empty = [&](int b) { return bar0 + 8u * (2 * G3_MAX_STAGES + 2 + b); };
     if (tid == 0) {
         s_abort = 0;
-        for (int s = 0; s < G3_STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int s = 0; s < nst; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
         for (int b = 0; b < 2; b++) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 2 * G3_EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1035,55 +1038,65 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
 
+    // The producer and the issuing warp wait as whole warps and elect a thread only for straight code: with a wait inside
+    // the elected region the compiler wraps every copy and MMA in a loop over the active lanes (a few hundred clocks per copy).
     if (warp == G3_EPI_WARPS) {
-        if (elect_one()) {                                      // TMA producer: this block's 128 tokens and 128 weight rows
-            int it = 0;
-            for (int t = cluster; t < ntiles && !s_abort; t += nclusters) {
-                const int tok0 = (t % ntt) * 256 + (int)rank * 128, r0 = (t / ntt) * GM_BN + (int)rank * 128;
-                for (int kb = 0; kb < nkb; kb++, it++) {
-                    const int s = it % G3_STAGES;
-                    if (!mbar_wait(empty(s), ((it / G3_STAGES) & 1) ^ 1)) { s_abort = 1; break; }
-                    if (rank == 0) mbar_expect_tx(full(s), 2 * G3_STAGE_BYTES);
-                    const uint32_t dst = sbase + s * G3_STAGE_BYTES;
-                    const uint32_t lead_bar = mapa_u32(full(s), 0);
+        // TMA producer: this block's 128 tokens and its half of the weight rows
+        int s = 0;
+        uint32_t par = 1;
+        for (int t = cluster; t < ntiles && !s_abort; t += nclusters) {
+            const int tok0 = (t % ntt) * 256 + (int)rank * 128, r0 = (t / ntt) * bn + (int)rank * (bn >> 1);
+            for (int kb = 0; kb < nkb; kb++) {
+                if (!mbar_wait(empty(s), par)) { s_abort = 1; break; }
+                __syncwarp();
+                const uint32_t dst = sbase + s * stage_bytes, lead_bar = mapa_u32(full(s), 0);
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(full(s), 2u * stage_bytes);
                     tma_load_2d_2sm(dst, &xmap, kb * GM_BK, tok0, lead_bar);
                     tma_load_2d_2sm(dst + GM_A_BYTES, &wmap, kb * GM_BK, r0, lead_bar);
                 }
+                __syncwarp();
+                if (++s == nst) { s = 0; par ^= 1u; }
             }
         }
     } else if (warp == G3_EPI_WARPS + 1) {
-        if (rank == 0 && elect_one()) {                         // MMA issuer (leader block)
-            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-            int it = 0, li = 0;
+        if (rank == 0) {                                      // MMA issuer (leader block)
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+            int s = 0, li = 0;
+            uint32_t par = 0;
             for (int t = cluster; t < ntiles && !s_abort; t += nclusters, li++) {
                 const int buf = li & 1;
                 if (!mbar_wait(acc_empty(buf), ((li >> 1) & 1) ^ 1)) { s_abort = 1; break; }
+                __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int kb = 0; kb < nkb; kb++, it++) {
-                    const int s = it % G3_STAGES;
-                    if (!mbar_wait(full(s), (it / G3_STAGES) & 1)) { s_abort = 1; break; }
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (!mbar_wait(full(s), par)) { s_abort = 1; break; }
+                    __syncwarp();
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = sbase + s * G3_STAGE_BYTES, b_addr = a_addr + GM_A_BYTES;
+                    const uint32_t a_addr = sbase + s * stage_bytes, d = tmem + (uint32_t)(buf * GM_BN), acc = kb ? 1u : 0u;
+                    const uint64_t da = umma_desc_sw128(a_addr), db = umma_desc_sw128(a_addr + GM_A_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < GM_BK / 16; kk++)
-                        umma_f16_2sm(tmem + buf * GM_BN, umma_desc_sw128(a_addr + kk * 32), umma_desc_sw128(b_addr + kk * 32), idesc,
-                                     (kb | kk) ? 1u : 0u);
-                    umma_commit_2sm(empty(s));
+                        for (int kk = 0; kk < GM_BK / 16; kk++) umma_f16_2sm(d, da + kk * 2, db + kk * 2, idesc, kk ? 1u : acc);
+                        umma_commit_2sm(empty(s));
+                        if (kb == nkb - 1) umma_commit_2sm(acc_full(buf));
+                    }
+                    __syncwarp();
+                    if (++s == nst) { s = 0; par ^= 1u; }
                 }
-                umma_commit_2sm(acc_full(buf));
             }
         }
     } else {
-        // epilogue: warp w drains TMEM lanes 32 (w % 4).., columns 128 (w / 4).. of the tile's buffer
+        // epilogue: warp w drains TMEM lanes 32 (w % 4).., every other 32 columns of the tile's buffer
         const int q = warp & 3, ch = warp >> 2;
         int li = 0;
         for (int t = cluster; t < ntiles; t += nclusters, li++) {
             const int buf = li & 1;
             if (!mbar_wait(acc_full(buf), (li >> 1) & 1)) { s_abort = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int tok = (t % ntt) * 256 + (int)rank * 128 + q * 32 + lane, r0 = (t / ntt) * GM_BN;
+            const int tok = (t % ntt) * 256 + (int)rank * 128 + q * 32 + lane, r0 = (t / ntt) * bn;
             const float tsc = (tok < ntok) ? xinv[tok] : 0.f;
-            for (int c0 = ch * 128; c0 < ch * 128 + 128; c0 += 32) {
+            for (int c0 = ch * 32; c0 < bn; c0 += 64) {
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * GM_BN + c0), v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -1243,11 +1256,20 @@ extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const 
     const int variant = 2;
 #endif
     if (variant == 2) {
-        // box of the pair kernel: 128 tokens / 128 weight rows per block
+        // Rows per tile: the fewest waves of SM pairs, each as long as its tile is wide (plus a tile's start and end, about
+        // 40 rows' worth).  700 tokens x 3584 rows: 69 tiles of 160 rows in one wave instead of 42 of 256.
+        const int ntt = cbl_ceil_div(ntok, 256), pairs = cbl_sm_count() / 2;
+        int bn = 256;
+        long best = -1;
+        for (int b = 256; b >= 64; b -= 32) {
+            const long cost = (long)cbl_ceil_div(ntt * cbl_ceil_div(R, b), pairs) * (b + 40);
+            if (best < 0 || cost < best) { best = cost; bn = b; }
+        }
+        // box of the pair kernel: 128 tokens / half of the tile's weight rows per block
         {
             const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)R};
             const cuuint64_t strides[1] = {(cuuint64_t)((C + 7) / 8 * 8) * 2};
-            const cuuint32_t box[2] = {GM_BK, 128};
+            const cuuint32_t box[2] = {GM_BK, (cuuint32_t)(bn / 2)};
             CUresult cr = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)w16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
@@ -1257,8 +1279,8 @@ extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const 
             CBL_CUDA(cudaFuncSetAttribute(k_gemm_dense_2sm, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM));
             attr3_set[dev] = true;
         }
-        const int ntiles = cbl_ceil_div(R, GM_BN) * cbl_ceil_div(ntok, 256);
-        int nclusters = cbl_sm_count() / 2;
+        const int ntiles = cbl_ceil_div(R, bn) * ntt;
+        int nclusters = pairs;
         if (nclusters > ntiles) nclusters = ntiles;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1272,7 +1294,7 @@ extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const 
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, bias, (unsigned int*)workspace));
+        CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, bias, bn, (unsigned int*)workspace));
         return cbl_check_launch();
     }
     dim3 grid(cbl_ceil_div(ntok, GM_BM), cbl_ceil_div(R, GM_BN));
