@@ -356,7 +356,8 @@ int cbl_repack_b3(const cbl_packed* m, const int32_t* tile_rows, int32_t ntile, 
 /* Up to 4 matrices that share the input x [ntok, >= C] (row stride ldx) and its column orders (perms int32 [M, C] when
  * M > 1): ys[i][t * ldy + r] = round(row_scale[r] * sum_c W_i[r, c] x[t, c]), ntok up to cbl_gemm_b3_max_tokens.  stage: cbl_prep_x_bytes(ntok, C,
  * M) bytes, 16-byte aligned.  workspace: cbl_gemm_b3_workspace_bytes bytes (arrival counters, zero before the first call
- * and left zero, then partial sums).  Results do not depend on timing: partial sums are added in a fixed order. */
+ * and left zero, then partial sums).  Results do not depend on timing: partial sums are added in a fixed order.
+ * x == NULL: stage already holds the activations (cbl_prep_x, cbl_add_rmsnorm_stage, cbl_silu_mul_stage). */
 size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int32_t ntok);
 int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
                 int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s);
@@ -389,7 +390,7 @@ int cbl_decode_raw(const cbl_packed* m, void* out, cbl_stream s);
 int cbl_decode_raw_wide(const cbl_packed* m, void* out, int32_t C_out, cbl_stream s);
 int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok, int64_t ldx,
                    void* y, int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s);
-/* The same plus a bias [R] in y's type: y = round(round(product) + bias). */
+/* The same plus a bias [R] in y's type (or NULL): y = round(round(product) + bias).  x == NULL: stage already holds the activations. */
 int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok, int64_t ldx,
                    void* y, int ydtype, int64_t ldy, const void* bias, void* stage, void* workspace, cbl_stream s);
 
@@ -435,6 +436,13 @@ int cbl_attn_decode(const void* q, const void* kc, const void* vc, const int32_t
 
 /* out[b, i] = round(round(silu(gate_up[b, i])) * gate_up[b, I + i]); gate_up [B, ld], out [B, I] contiguous. */
 int cbl_silu_mul(const void* gate_up, int dtype, int64_t ld, int32_t B, int32_t I, void* out, cbl_stream s);
+/* cbl_add_rmsnorm and cbl_silu_mul with their result in the staging buffer (cbl_prep_x_bytes(B, columns, 1) bytes) of the product that
+ * follows instead of a vector of its own: the values rounded to `dtype`, then as cbl_prep_x would stage them. */
+int32_t cbl_add_rmsnorm_stage_max_columns(void);
+int cbl_add_rmsnorm_stage(float* h, const void* add, int64_t ld_add, const void* w, int dtype, float eps, int32_t B, int32_t H, void* stage,
+                          cbl_stream s);
+int32_t cbl_silu_mul_stage_max_columns(void);
+int cbl_silu_mul_stage(const void* gate_up, int dtype, int64_t ld, int32_t B, int32_t I, void* stage, cbl_stream s);
 
 /* Dense 16-bit output head for small batches: logits[b, v] = <W[v, :], x[b, :]>, W [V, H] and x [B, H]
  * contiguous in `dtype`, fp32 accumulation, logits in `ldtype` (CBL_F32 / F16 / BF16) with row stride ldl.

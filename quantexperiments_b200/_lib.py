@@ -133,6 +133,10 @@ SIGNATURES = {
     "cbl_attn_decode": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int32, c_int32, c_int32, c_int32, c_int32, c_float,
                                 c_void_p, c_void_p, c_int32, c_void_p]),
     "cbl_silu_mul": (c_int, [c_void_p, c_int, c_int64, c_int32, c_int32, c_void_p, c_void_p]),
+    "cbl_add_rmsnorm_stage_max_columns": (c_int32, []),
+    "cbl_add_rmsnorm_stage": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int, c_float, c_int32, c_int32, c_void_p, c_void_p]),
+    "cbl_silu_mul_stage_max_columns": (c_int32, []),
+    "cbl_silu_mul_stage": (c_int, [c_void_p, c_int, c_int64, c_int32, c_int32, c_void_p, c_void_p]),
     "cbl_head_gemv_max_batch": (c_int32, []),
     "cbl_head_gemv": (c_int, [c_void_p, c_void_p, c_int, c_int32, c_int32, c_int32, c_void_p, c_int, c_int64, c_void_p]),
     "cbl_gemv_l8_silu_mul": (c_int, [POINTER(L8), c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p]),

@@ -699,9 +699,9 @@ extern "C" size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int
 
 extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
                            int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
-    if (!mats || !x || !ys || !stage || !workspace || n < 1) return CBL_EINVAL;
+    if (!mats || !ys || !stage || !workspace || n < 1) return CBL_EINVAL;
     if (n > B3_MAX_MATS || ntok > cbl_gemm_b3_max_tokens(mats[0].copies)) return CBL_EUNSUPPORTED;
-    if (ntok < 1 || ldx < mats[0].C) return CBL_EINVAL;
+    if (ntok < 1 || (x && ldx < mats[0].C)) return CBL_EINVAL;
     if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
     if (((uintptr_t)stage % 16) || ((uintptr_t)workspace % 16)) return CBL_EINVAL;
     for (int i = 0; i < n; i++) {
@@ -715,8 +715,10 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
     int rc = b3_plan(mats, n, ntok, pl);
     if (rc) return rc;
     if (pl.U == 0) return CBL_OK;
-    rc = cbl_prep_x(x, xdtype, ntok, C, ldx, perms, M, stage, s);
-    if (rc) return rc;
+    if (x) {                                                   // x == NULL: the caller has staged the activations
+        rc = cbl_prep_x(x, xdtype, ntok, C, ldx, perms, M, stage, s);
+        if (rc) return rc;
+    }
     const int Bpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
     B3Launch P;
     P.nkb = cbl_ceil_div(C, B3_KB);

@@ -1201,18 +1201,21 @@ extern "C" int cbl_gemm_l8_2sm(const cbl_l8* m, const void* x, int xdtype, int32
 // ---- two-phase variant: host side
 extern "C" int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok,
                               int64_t ldx, void* y, int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
+    if (!x) return CBL_EINVAL;
     return cbl_gemm_dense_bias(w16, R, C, row_scale, x, xdtype, ntok, ldx, y, ydtype, ldy, nullptr, stage, workspace, s);
 }
 
 extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok,
                               int64_t ldx, void* y, int ydtype, int64_t ldy, const void* bias, void* stage, void* workspace, cbl_stream s) {
-    if (!w16 || !row_scale || !x || !y || !stage || !workspace) return CBL_EINVAL;
-    if (R <= 0 || C <= 0 || C % 8 || ntok <= 0 || ldx < C || ldy < R) return CBL_EINVAL;
+    if (!w16 || !row_scale || !y || !stage || !workspace) return CBL_EINVAL;
+    if (R <= 0 || C <= 0 || C % 8 || ntok <= 0 || (x && ldx < C) || ldy < R) return CBL_EINVAL;
     if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
     if (((uintptr_t)stage % 16) || ((uintptr_t)w16 % 16) || ((uintptr_t)workspace % 4)) return CBL_EINVAL;
     const cudaStream_t st = (cudaStream_t)s;
-    int rc = cbl_prep_x(x, xdtype, ntok, C, ldx, nullptr, 1, stage, s);
-    if (rc) return rc;
+    if (x) {                                                   // x == NULL: the caller has staged the activations
+        const int rc = cbl_prep_x(x, xdtype, ntok, C, ldx, nullptr, 1, stage, s);
+        if (rc) return rc;
+    }
     const int Mpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
     encode_tiled_fn enc = get_encode();
     if (!enc) return CBL_ECUDA;

@@ -109,9 +109,12 @@ __global__ void __launch_bounds__(512) k_add_rmsnorm(float* __restrict__ h, cons
 // The same with the row in registers between the two uses: four values per access, rows of up to 4 x 256 x ADDNORM_NV values.
 // One read and one write of the residual row instead of two reads (700 rows of 3584: 15 -> 7 us).
 constexpr int ADDNORM_NV = 8;
-template <typename T>
+// STAGE: the product that follows takes fp16 activations scaled by a power of two per row (cbl_prep_x's layout, columns padded
+// to Cpad): write those instead of x, the values rounded to T first as if x had been stored.
+template <typename T, bool STAGE>
 __global__ void __launch_bounds__(256) k_add_rmsnorm4(float* __restrict__ h, const T* __restrict__ add, int64_t ld_add,
-                                                      const T* __restrict__ w, float eps, int H, T* __restrict__ x) {
+                                                      const T* __restrict__ w, float eps, int H, T* __restrict__ x, __half* __restrict__ xp,
+                                                      int Cpad, float* __restrict__ xinv) {
     __shared__ float red[8];
     const int b = blockIdx.x, tid = threadIdx.x, n4 = H >> 2;
     uint2 wv[ADDNORM_NV];
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm4(float* __restrict__ h, con
     for (int k = 0; k < 8; k++) ss += red[k];
     const float rstd = rsqrtf(ss / (float)H + eps);
     uint2* xb = (uint2*)(x + (int64_t)b * H);
+    float mx = 0.f;
 #pragma unroll
     for (int k = 0; k < ADDNORM_NV; k++) {
         const int i = tid + 256 * k;
@@ -164,7 +168,31 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm4(float* __restrict__ h, con
         t[1] = cbl_cvt_out<T>(v[k].y * rstd * c.y);
         t[2] = cbl_cvt_out<T>(v[k].z * rstd * c.z);
         t[3] = cbl_cvt_out<T>(v[k].w * rstd * c.w);
-        xb[i] = o;
+        if (STAGE) {
+            v[k] = four(o);
+            mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[k].x), fabsf(v[k].y))), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+        } else xb[i] = o;
+    }
+    if (STAGE) {
+        mx = warp_max(mx);
+        __syncthreads();                                       // the sums of squares have been read
+        if ((tid & 31) == 0) red[tid >> 5] = mx;
+        __syncthreads();
+        mx = red[0];
+#pragma unroll
+        for (int k = 1; k < 8; k++) mx = fmaxf(mx, red[k]);
+        const int e = cbl_scale_exp(mx);
+        const float sc = ldexpf(1.f, -e);
+        if (tid == 0) xinv[b] = ldexpf(1.f, e);
+        uint2* d = (uint2*)(xp + (int64_t)b * Cpad);
+#pragma unroll
+        for (int k = 0; k < ADDNORM_NV; k++) {
+            const int i = tid + 256 * k;
+            if (i >= n4) continue;
+            const __half2 lo = __floats2half2_rn(v[k].x * sc, v[k].y * sc), hi = __floats2half2_rn(v[k].z * sc, v[k].w * sc);
+            d[i] = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+        }
+        for (int i = n4 + tid; i < Cpad / 4; i += 256) d[i] = make_uint2(0u, 0u);
     }
 }
 
@@ -211,8 +239,8 @@ __global__ void __launch_bounds__(128) k_rope_kv(const T* __restrict__ qkv, int6
     }
 }
 
-// Prompts (rows are consecutive positions of one sequence, head size 128): a block takes eight rows.  Angles are computed once
-// per row, not once per head; heads are rotated 16 bytes at a time; eight positions of a value dimension are one
+// Prompts (rows are consecutive positions of one sequence, head size 128): a block takes eight rows and a share of the
+// heads.  Angles are computed once per row and share, not once per head; heads are rotated 16 bytes at a time; eight positions of a value dimension are one
 // 16-byte store into the dimension-major cache (700 rows: 24 -> 7 us).
 constexpr int ROPE_ROWS = 8;
 template <typename T>
@@ -243,9 +271,9 @@ __global__ void __launch_bounds__(256) k_rope_prompt(const T* __restrict__ qkv, 
         }
         return p;
     };
-    const int nrow = min(ROPE_ROWS, rows - r0), heads = NH + NKV;
-    for (int k = tid; k < ROPE_ROWS * heads * 8; k += 256) {
-        const int j = k & 7, hd = (k >> 3) % heads, rr = (k >> 3) / heads, p = pos0 + r0 + rr;
+    const int nrow = min(ROPE_ROWS, rows - r0), heads = NH + NKV, ny = gridDim.y, mine = (heads - (int)blockIdx.y + ny - 1) / ny;
+    for (int k = tid; k < ROPE_ROWS * mine * 8; k += 256) {
+        const int j = k & 7, hd = blockIdx.y + (k >> 3) % mine * ny, rr = (k >> 3) / mine, p = pos0 + r0 + rr;
         if (rr >= nrow || p < 0 || p >= max_len) continue;
         const Pack a = load(r0 + rr, hd * HD + 8 * j), b = load(r0 + rr, hd * HD + HALF + 8 * j);
         Pack o1, o2;
@@ -261,7 +289,7 @@ __global__ void __launch_bounds__(256) k_rope_prompt(const T* __restrict__ qkv, 
     }
     const int p0 = pos0 + r0;
     const bool whole = nrow == ROPE_ROWS && p0 >= 0 && p0 + ROPE_ROWS <= max_len && p0 % 8 == 0 && max_len % 8 == 0;
-    for (int kv = 0; kv < NKV; kv++) {
+    for (int kv = blockIdx.y; kv < NKV; kv += ny) {
         if (tid < ROPE_ROWS * 16) {
             const int rr = tid >> 4, j = tid & 15;
             if (rr < nrow) *(uint4*)&s_v[rr][8 * j] = load(r0 + rr, (heads + kv) * HD + 8 * j).u;
@@ -497,6 +525,54 @@ __global__ void __launch_bounds__(256) k_silu_mul8(const T* __restrict__ gu, int
 #pragma unroll
     for (int e = 0; e < 8; e++) o.t[e] = cbl_cvt_out<T>(to_f(cbl_cvt_out<T>(g[e] / (1.f + __expf(-g[e])))) * u[e]);
     *(uint4*)(out + (int64_t)b * I + i) = o.v;
+}
+
+// silu * up straight into the staging buffer of the product that follows: a block per row, the row in registers between the
+// search for its largest magnitude and the conversion; rows of up to 8 x 1024 x SILU_NV values.
+constexpr int SILU_NV = 4;
+template <typename T>
+__global__ void __launch_bounds__(1024) k_silu_stage(const T* __restrict__ gu, int64_t ld, int I, __half* __restrict__ xp, int Cpad,
+                                                     float* __restrict__ xinv) {
+    pdl_enter();
+    __shared__ float red[32];
+    const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    const T* row = gu + (int64_t)b * ld;
+    union Pack { uint4 v; T t[8]; } o[SILU_NV];
+    float mx = 0.f;
+#pragma unroll
+    for (int k = 0; k < SILU_NV; k++) {
+        const int i = (tid + nt * k) * 8;
+        o[k].v = make_uint4(0, 0, 0, 0);
+        if (i < I) {
+            float g[8], u[8];
+            unpack8<T>(__ldcg((const uint4*)(row + i)), g);
+            unpack8<T>(__ldcg((const uint4*)(row + I + i)), u);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                o[k].t[e] = cbl_cvt_out<T>(to_f(cbl_cvt_out<T>(g[e] / (1.f + __expf(-g[e])))) * u[e]);
+                mx = fmaxf(mx, fabsf(to_f(o[k].t[e])));
+            }
+        }
+    }
+    mx = warp_max(mx);
+    if ((tid & 31) == 0) red[tid >> 5] = mx;
+    __syncthreads();
+    mx = 0.f;
+    for (int k = 0; k < nt / 32; k++) mx = fmaxf(mx, red[k]);
+    const int ex = cbl_scale_exp(mx);
+    const float sc = ldexpf(1.f, -ex);
+    if (tid == 0) xinv[b] = ldexpf(1.f, ex);
+#pragma unroll
+    for (int k = 0; k < SILU_NV; k++) {
+        const int i = (tid + nt * k) * 8;
+        if (i < Cpad) {
+            uint4 d;
+            __half2* hd = (__half2*)&d;
+#pragma unroll
+            for (int e = 0; e < 4; e++) hd[e] = __floats2half2_rn(to_f(o[k].t[2 * e]) * sc, to_f(o[k].t[2 * e + 1]) * sc);
+            *(uint4*)(xp + (int64_t)b * Cpad + i) = d;
+        }
+    }
 }
 
 template <typename T>
@@ -831,10 +907,24 @@ extern "C" int cbl_add_rmsnorm(float* h, const void* add, int64_t ld_add, const 
     const bool vec = H % 4 == 0 && H <= 4 * 256 * ADDNORM_NV && (uintptr_t)h % 16 == 0 && (uintptr_t)x % 8 == 0 && (uintptr_t)w % 8 == 0 &&
                      (!add || ((uintptr_t)add % 8 == 0 && ld_add % 4 == 0));
     if (vec)
-        CBL_BY_TYPE(dtype, return step_launch(k_add_rmsnorm4<T>, dim3(B), dim3(256), 0, (cudaStream_t)s, h, (const T*)add, ld_add, (const T*)w, eps,
-                                              (int)H, (T*)x));
+        CBL_BY_TYPE(dtype, return step_launch(k_add_rmsnorm4<T, false>, dim3(B), dim3(256), 0, (cudaStream_t)s, h, (const T*)add, ld_add, (const T*)w, eps,
+                                              (int)H, (T*)x, (__half*)nullptr, 0, (float*)nullptr));
     CBL_BY_TYPE(dtype, return step_launch(k_add_rmsnorm<T>, dim3(B), dim3(512), 0, (cudaStream_t)s, h, (const T*)add, ld_add, (const T*)w, eps,
                                           (int)H, (T*)x));
+}
+
+extern "C" int32_t cbl_add_rmsnorm_stage_max_columns(void) { return 4 * 256 * ADDNORM_NV; }
+
+// As cbl_add_rmsnorm, x going into the staging buffer of the product that follows (the layout of cbl_prep_x, one column order).
+extern "C" int cbl_add_rmsnorm_stage(float* h, const void* add, int64_t ld_add, const void* w, int dtype, float eps, int32_t B, int32_t H, void* stage,
+                                     cbl_stream s) {
+    if (!h || !w || !stage || !is16(dtype) || H < 1 || B < 0) return CBL_EINVAL;
+    if (H % 4 || H > 4 * 256 * ADDNORM_NV) return CBL_EUNSUPPORTED;
+    if ((uintptr_t)h % 16 || (uintptr_t)stage % 16 || (uintptr_t)w % 8 || (add && ((uintptr_t)add % 8 || ld_add % 4))) return CBL_EINVAL;
+    if (B == 0) return CBL_OK;
+    const int Cpad = (H + 511) / 512 * 512, Bpad = (B + 7) / 8 * 8;
+    CBL_BY_TYPE(dtype, return step_launch(k_add_rmsnorm4<T, true>, dim3(B), dim3(256), 0, (cudaStream_t)s, h, (const T*)add, ld_add, (const T*)w, eps,
+                                          (int)H, (T*)nullptr, (__half*)stage, Cpad, (float*)((__half*)stage + (int64_t)Bpad * Cpad)));
 }
 
 extern "C" int cbl_rope_kv(const void* qkv, int dtype, int64_t ld, const void* bias, const int32_t* pos, int32_t pos0, int32_t seq0,
@@ -846,7 +936,7 @@ extern "C" int cbl_rope_kv(const void* qkv, int dtype, int64_t ld, const void* b
     if (rows > 65535) return CBL_EUNSUPPORTED;
     if (!pos && HD == 128 && ld % 8 == 0 && (uintptr_t)qkv % 16 == 0 && (!bias || (uintptr_t)bias % 16 == 0) && (uintptr_t)q_out % 16 == 0 &&
         (uintptr_t)kc % 16 == 0 && (uintptr_t)vc % 16 == 0)
-        CBL_BY_TYPE(dtype, return step_launch(k_rope_prompt<T>, dim3(cbl_ceil_div(rows, ROPE_ROWS)), dim3(256), 0, (cudaStream_t)s, (const T*)qkv, ld,
+        CBL_BY_TYPE(dtype, return step_launch(k_rope_prompt<T>, dim3(cbl_ceil_div(rows, ROPE_ROWS), NKV < 8 ? NKV : 8), dim3(256), 0, (cudaStream_t)s, (const T*)qkv, ld,
                                               (const T*)bias, (int)pos0, (int)seq0, (int)rows, (int)NH, (int)NKV, theta, (int)max_len, (T*)q_out, (T*)kc,
                                               (T*)vc));
     CBL_BY_TYPE(dtype, return step_launch(k_rope_kv<T>, dim3(NH + NKV, rows), dim3(128), 0, (cudaStream_t)s, (const T*)qkv, ld, (const T*)bias,
@@ -907,6 +997,20 @@ extern "C" int cbl_silu_mul(const void* gate_up, int dtype, int64_t ld, int32_t 
     const int cap = cbl_ceil_div(4 * cbl_sm_count(), B);
     if (gx > cap) gx = cap < 1 ? 1 : cap;
     CBL_BY_TYPE(dtype, return step_launch(k_silu_mul<T>, dim3(gx, B), dim3(256), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (T*)out));
+}
+
+extern "C" int32_t cbl_silu_mul_stage_max_columns(void) { return 8 * 1024 * SILU_NV; }
+
+// As cbl_silu_mul, the result going into the staging buffer of the product that follows (the layout of cbl_prep_x, one column order).
+extern "C" int cbl_silu_mul_stage(const void* gate_up, int dtype, int64_t ld, int32_t B, int32_t I, void* stage, cbl_stream s) {
+    if (!gate_up || !stage || !is16(dtype) || B < 0 || I < 1) return CBL_EINVAL;
+    const int Cpad = (I + 511) / 512 * 512, Bpad = (B + 7) / 8 * 8;
+    if (I % 8 || Cpad > 8 * 1024 * SILU_NV) return CBL_EUNSUPPORTED;
+    if (ld % 8 || (uintptr_t)gate_up % 16 || (uintptr_t)stage % 16) return CBL_EINVAL;
+    if (B == 0) return CBL_OK;
+    int nt = (cbl_ceil_div(Cpad / 8, SILU_NV) + 31) / 32 * 32;
+    CBL_BY_TYPE(dtype, return step_launch(k_silu_stage<T>, dim3(B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage, Cpad,
+                                          (float*)((__half*)stage + (int64_t)Bpad * Cpad)));
 }
 
 extern "C" int32_t cbl_head_gemv_max_batch(void) { return HEAD_BMAX; }

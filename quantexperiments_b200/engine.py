@@ -136,8 +136,8 @@ class _Stage:
         self.group = stack.l8 if self.B == 1 and stack.tables else None
         self.rows = stack.b3(self.B) if self.group is None and stack.shared else None     # the weight rows as the M side, one launch
 
-    def run(self, x: torch.Tensor) -> None:
-        self.stack.run(x, self.out)
+    def run(self, x: torch.Tensor | None, staged: torch.Tensor | None = None) -> None:
+        self.stack.run(x, self.out, staged)
 
 
 class DecodeEngine:
@@ -192,10 +192,22 @@ class DecodeEngine:
                         "gu": Stack([_lin(L[n]) for n in ("gate", "up")]), "down": Stack([_lin(L["down"])])} for L in layers]
         self.stages = [{"qkv": _Stage(S["qkv"], self.yqkv), "o": _Stage(S["o"], self.yo), "gu": _Stage(S["gu"], self.ygu),
                         "down": _Stage(S["down"], self.yd)} for S in self.stacks]
+        # several sequences, one column order: add + norm and silu * up write the fp16 staging buffer of the product after them
+        self.stage_h = self.stage_i = None
+        if self._stages_inputs(B):
+            self.stage_h, self.stage_i = self._stage_buffers(B)
         self.graph = None
         self.only_linears = False
         # one token, one column order everywhere: the operator that follows a product runs on its fp32 sums (one small kernel)
         self.fused = B == 1 and all(st.group is not None for S in self.stages for st in S.values()) and H <= lib.cbl_gemv_l8_add_norm_max_rows()
+
+    def _stages_inputs(self, n: int) -> bool:
+        c = self.cfg
+        return (all(S[k].takes_staged(n) for S in self.stacks for k in ("qkv", "gu", "down")) and c.hidden % 4 == 0 and c.inter % 8 == 0 and
+                c.hidden <= lib.cbl_add_rmsnorm_stage_max_columns() and c.inter <= lib.cbl_silu_mul_stage_max_columns() - 512)
+
+    def _stage_buffers(self, n: int):
+        return tuple(torch.empty(lib.cbl_prep_x_bytes(n, k, 1), dtype=torch.uint8, device=self.dev) for k in (self.cfg.hidden, self.cfg.inter))
 
     # -- operators (thin wrappers over the C ABI; all on the current stream)
     def _embed(self, tok, rows: int, h) -> None:
@@ -206,7 +218,12 @@ class DecodeEngine:
             _lib.check("cbl_embed_rows", lib.cbl_embed_rows(self.embed.data_ptr(), _dt(self.dtype), self.vocab_rows, self.cfg.hidden, tok.data_ptr(),
                                                             rows, h.data_ptr(), _stream()))
 
-    def _addnorm(self, h, add, w, x, rows: int) -> None:
+    def _addnorm(self, h, add, w, x, rows: int, stage=None) -> None:
+        if stage is not None:
+            _lib.check("cbl_add_rmsnorm_stage", lib.cbl_add_rmsnorm_stage(h.data_ptr(), None if add is None else add.data_ptr(),
+                                                                          0 if add is None else add.stride(0), w.data_ptr(), _dt(self.dtype),
+                                                                          self.cfg.eps, rows, self.cfg.hidden, stage.data_ptr(), _stream()))
+            return
         _lib.check("cbl_add_rmsnorm", lib.cbl_add_rmsnorm(h.data_ptr(), None if add is None else add.data_ptr(),
                                                           0 if add is None else add.stride(0), w.data_ptr(), _dt(self.dtype),
                                                           self.cfg.eps, rows, self.cfg.hidden, x.data_ptr(), _stream()))
@@ -217,7 +234,11 @@ class DecodeEngine:
                                                   None if pos is None else pos.data_ptr(), pos0, seq0, rows, c.n_heads, c.n_kv, c.head_dim,
                                                   c.rope_theta, self.cache_len, qr.data_ptr(), kc.data_ptr(), vc.data_ptr(), _stream()))
 
-    def _silu(self, ygu, act, rows: int) -> None:
+    def _silu(self, ygu, act, rows: int, stage=None) -> None:
+        if stage is not None:
+            _lib.check("cbl_silu_mul_stage", lib.cbl_silu_mul_stage(ygu.data_ptr(), _dt(self.dtype), ygu.stride(0), rows, self.cfg.inter,
+                                                                    stage.data_ptr(), _stream()))
+            return
         _lib.check("cbl_silu_mul", lib.cbl_silu_mul(ygu.data_ptr(), _dt(self.dtype), ygu.stride(0), rows, self.cfg.inter, act.data_ptr(),
                                                     _stream()))
 
@@ -237,19 +258,20 @@ class DecodeEngine:
             if self.fused:
                 self._step_fused(s)
                 return
-            add = None
+            add, sh, si = None, self.stage_h, self.stage_i
+            x, act = (self.x16, self.act) if sh is None else (None, None)
             for li, (L, S) in enumerate(zip(self.layers, self.stages)):
-                self._addnorm(self.h, add, L["ln1"], self.x16, B)
-                S["qkv"].run(self.x16)
+                self._addnorm(self.h, add, L["ln1"], self.x16, B, sh)
+                S["qkv"].run(x, sh)
                 self._rope(self.yqkv, self.biases[li], self.pos, 0, 0, B, self.qr, self.kc[li], self.vc[li])
                 _lib.check("cbl_attn_decode", lib.cbl_attn_decode(self.qr.data_ptr(), self.kc[li].data_ptr(), self.vc[li].data_ptr(),
                                                                   self.pos.data_ptr(), dtc, B, c.n_heads, c.n_kv, c.head_dim, self.cache_len,
                                                                   c.head_dim ** -0.5, self.ao.data_ptr(), self.att_ws.data_ptr(), self.nsplit, s))
                 S["o"].run(self.ao)
-                self._addnorm(self.h, self.yo, L["ln2"], self.x16, B)
-                S["gu"].run(self.x16)
-                self._silu(self.ygu, self.act, B)
-                S["down"].run(self.act)
+                self._addnorm(self.h, self.yo, L["ln2"], self.x16, B, sh)
+                S["gu"].run(x, sh)
+                self._silu(self.ygu, self.act, B, si)
+                S["down"].run(act, si)
                 add = self.yd
             self._addnorm(self.h, add, self.final_norm, self.x16, B)
             self.lm_head.run(self.x16, self.logits)
@@ -301,26 +323,33 @@ class DecodeEngine:
             yqkv, qr = torch.empty(T, (NH + 2 * NKV) * HD, **a), torch.empty(T, NH * HD, **a)
             yo, ygu, act, yd = torch.empty(T, H, **a), torch.empty(T, 2 * I, **a), torch.empty(T, I, **a), torch.empty(T, H, **a)
             self._embed(ids, T, h)
-            add = None
+            add, last = None, len(self.layers) - 1
+            st = T > 1 and self._stages_inputs(T)
+            sh, si = self._stage_buffers(T) if st else (None, None)
             for li, L in enumerate(self.layers):
-                self._addnorm(h, add, L["ln1"], x, T)
-                self.stacks[li]["qkv"].run(x, yqkv)
+                # behind the last layer's attention only the last position is asked for: everything that follows runs on one row
+                n = 1 if li == last else T
+                self._addnorm(h, add, L["ln1"], x, T, sh)
+                self.stacks[li]["qkv"].run(None if st else x, yqkv, sh)
                 kc, vc = self.kc[li], self.vc[li]
                 self._rope(yqkv, self.biases[li], None, 0, seq, T, qr, kc, vc)
-                q4 = qr.view(T, NH, HD).transpose(0, 1)[None]
+                q4 = qr[T - n:].view(n, NH, HD).transpose(0, 1)[None]
                 v4 = yqkv[:, (NH + NKV) * HD:].view(T, NKV, HD).transpose(0, 1)[None]         # the values as projected (+ bias below)
                 if self.biases[li] is not None:
                     v4 = (v4 + self.biases[li][(NH + NKV) * HD:].view(1, NKV, 1, HD)).to(self.dtype)
-                ao = torch.nn.functional.scaled_dot_product_attention(q4, kc[seq, :, :T][None], v4, is_causal=True, enable_gqa=True)
-                ao = ao[0].transpose(0, 1).reshape(T, NH * HD)
+                ao = torch.nn.functional.scaled_dot_product_attention(q4, kc[seq, :, :T][None], v4, is_causal=n > 1, enable_gqa=True)
+                ao = ao[0].transpose(0, 1).reshape(n, NH * HD)
+                if n < T:
+                    h, x, yo, ygu, act, yd = h[T - 1:].clone(), x[:1], yo[:1], ygu[:1], act[:1], yd[:1]
+                    st, sh, si = False, None, None
                 self.stacks[li]["o"].run(ao, yo)
-                self._addnorm(h, yo, L["ln2"], x, T)
-                self.stacks[li]["gu"].run(x, ygu)
-                self._silu(ygu, act, T)
-                self.stacks[li]["down"].run(act, yd)
+                self._addnorm(h, yo, L["ln2"], x, n, sh)
+                self.stacks[li]["gu"].run(None if st else x, ygu, sh)
+                self._silu(ygu, act, n, si)
+                self.stacks[li]["down"].run(None if st else act, yd, si)
                 add = yd
-            hl, xl = h[T - 1:T].clone(), torch.empty(1, H, **a)
-            self._addnorm(hl, yd[T - 1:T], self.final_norm, xl, 1)
+            xl = x[:1]
+            self._addnorm(h, yd, self.final_norm, xl, 1)
             lg = self.logits[seq:seq + 1]
             self.lm_head.run(xl, lg)
             _lib.check("cbl_argmax", lib.cbl_argmax(lg.data_ptr(), _dt(lg.dtype), lg.stride(0), 1, lg.shape[1], self.tok[seq:].data_ptr(), None,

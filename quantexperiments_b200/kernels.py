@@ -445,9 +445,13 @@ class B3Group:
             cls._scratch[key] = (st, ws)
         return st, ws
 
-    def run(self, X: torch.Tensor, ys: list[torch.Tensor]) -> list[torch.Tensor]:
-        B = X.shape[0]
-        if X.dim() != 2 or X.shape[1] < self.C or (self.M == 1 and X.shape[1] != self.C) or X.stride(1) != 1 or X.device != self.device:
+    def run(self, X: torch.Tensor | None, ys: list[torch.Tensor], staged: torch.Tensor | None = None) -> list[torch.Tensor]:
+        """`staged` (X None, one column order): the activations as cbl_prep_x lays them out, written by the operator before."""
+        B = ys[0].shape[0] if X is None else X.shape[0]
+        if X is None:
+            if staged is None or self.M != 1:
+                raise ValueError("staged activations serve one column order")
+        elif X.dim() != 2 or X.shape[1] < self.C or (self.M == 1 and X.shape[1] != self.C) or X.stride(1) != 1 or X.device != self.device:
             raise ValueError("X must be [B, C] with unit column stride on the matrices' device")
         if not 1 <= B <= self.bmax:
             raise ValueError(f"batch {B} outside 1..{self.bmax}")
@@ -463,9 +467,12 @@ class B3Group:
         if need is None:
             need = self._ws_bytes[B] = (lib.cbl_prep_x_bytes(B, self.C, self.M), lib.cbl_gemm_b3_workspace_bytes(st, len(self.mats), B))
         stage, ws = self.buffers(self.device, *need)
+        if X is None:
+            stage, x = staged, (None, 0, B, 0)
+        else:
+            x = (X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1])
         with torch.cuda.device(self.device):
-            _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1], _ptr(self.perms),
-                                                      self._ys, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
+            _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), *x, _ptr(self.perms), self._ys, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
         return ys
 
     def status(self) -> None:
@@ -494,10 +501,11 @@ class DenseStack:
         self.row_scale = dms[0].row_scale if len(dms) == 1 else torch.cat([dm.row_scale for dm in dms])
         self.ld = (self.C + 7) // 8 * 8
 
-    def gemm(self, X: torch.Tensor, Y: torch.Tensor | None = None) -> torch.Tensor:
-        if X.dim() != 2 or X.shape[1] != self.C or X.stride(1) != 1 or X.device != self.device:
+    def gemm(self, X: torch.Tensor | None, Y: torch.Tensor | None = None, staged: torch.Tensor | None = None) -> torch.Tensor:
+        """`staged` (X None): the activations of Y's rows as cbl_prep_x lays them out, written by the operator before."""
+        if X is not None and (X.dim() != 2 or X.shape[1] != self.C or X.stride(1) != 1 or X.device != self.device):
             raise ValueError("X must be [T, C] with unit column stride on the matrices' device")
-        T = X.shape[0]
+        T = Y.shape[0] if X is None else X.shape[0]
         if Y is None:
             Y = torch.empty(T, self.R, dtype=X.dtype, device=self.device)
         if Y.shape != (T, self.R) or Y.stride(1) != 1:
@@ -512,18 +520,18 @@ class DenseStack:
         sc = pair[pair[2]]
         if sc is None or sc.numel() < need:
             sc = pair[pair[2]] = torch.empty(need, dtype=torch.uint8, device=self.device)
-        need = lib.cbl_gemm_stage_bytes(T, self.C) + 16
+        need = lib.cbl_gemm_stage_bytes(T if X is not None else 8, self.C) + 16
         st = DenseStack._stage.get(key)
         if st is None or st.numel() < need:
             st = DenseStack._stage[key] = torch.zeros(need, dtype=torch.uint8, device=self.device)
+        x = (None, 0, T, 0, staged.data_ptr()) if X is None else (X.data_ptr(), _dt(X.dtype), T, X.stride(0), st.data_ptr())
         with torch.cuda.device(self.device):
             s, row = _stream(), 0
             for dm in self.dms:
                 _lib.check("cbl_decode_raw", lib.cbl_decode_raw(ctypes.byref(dm.struct()), sc.data_ptr() + row * self.ld * 2, s))
                 row += dm.R
-            _lib.check("cbl_gemm_dense", lib.cbl_gemm_dense(sc.data_ptr(), self.R, self.C, self.row_scale.data_ptr(), X.data_ptr(), _dt(X.dtype),
-                                                            T, X.stride(0), Y.data_ptr(), _dt(Y.dtype), Y.stride(0), st.data_ptr(),
-                                                            st.data_ptr() + st.numel() - 16, s))
+            _lib.check("cbl_gemm_dense_bias", lib.cbl_gemm_dense_bias(sc.data_ptr(), self.R, self.C, self.row_scale.data_ptr(), *x[:4], Y.data_ptr(),
+                                                                      _dt(Y.dtype), Y.stride(0), None, x[4], st.data_ptr() + st.numel() - 16, s))
         return Y
 
     @classmethod

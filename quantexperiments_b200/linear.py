@@ -235,12 +235,18 @@ class Stack:
             for l in self.lins:
                 l.group(n)
 
-    def run(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
-        n = x.shape[0]
+    def takes_staged(self, n: int) -> bool:
+        """Whether run() accepts the n tokens' activations staged by the operator before (cbl_prep_x's layout)."""
+        return self.shared and self.lins[0].dm.M == 1 and (n > 1 or not self.tables) and (n < DENSE_MIN_TOKENS or self.dense is not None)
+
+    def run(self, x: torch.Tensor | None, y: torch.Tensor, staged: torch.Tensor | None = None) -> torch.Tensor:
+        n = y.shape[0]
         if n >= DENSE_MIN_TOKENS and self.dense is not None:
-            return self.dense.gemm(x, y)
+            return self.dense.gemm(x, y, staged)
         ys = list(y.split(self.Rs, 1))
-        if n == 1 and self.tables:
+        if x is None:
+            self.b3(n).run(None, ys, staged)
+        elif n == 1 and self.tables:
             self.l8.run(x[0], [t[0] for t in ys])
         elif self.shared and n < DENSE_MIN_TOKENS:
             self.b3(n).run(x, ys)

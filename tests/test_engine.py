@@ -581,3 +581,28 @@ def test_engine_logits_match_a_hugging_face_qwen2_with_reference_decoded_weights
     rel = float((got - want).norm() / want.norm())
     assert rel < 2e-2, rel
     assert (got.argmax(-1) == want.argmax(-1)).float().mean() >= 0.9
+
+
+@pytest.mark.parametrize("B,H", [(1, 896), (3, 3584), (9, 8192), (200, 512), (2, 20480)])
+def test_staging_operators_write_what_the_staging_pass_would(B, H):
+    """cbl_silu_mul_stage / cbl_add_rmsnorm_stage against the plain operator followed by cbl_prep_x, bit for bit."""
+    from quantexperiments_b200 import _lib as L
+    s = torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(H)
+    n = L.lib.cbl_prep_x_bytes(B, H, 1)
+    live = lambda t: torch.cat([t[:B * ((H + 511) // 512 * 1024)].view(torch.int16), t[-4 * ((B + 7) // 8 * 8):][:4 * B].view(torch.int16)])   # noqa: E731
+    for dt, dtc in ((torch.bfloat16, L.BF16), (torch.float16, L.F16)):
+        gu = (torch.randn(B, 2 * H, device="cuda", generator=g) * torch.logspace(-2, 1, B, device="cuda")[:, None]).to(dt)
+        act, a, b = torch.empty(B, H, device="cuda", dtype=dt), torch.zeros(n, device="cuda", dtype=torch.uint8), torch.zeros(n, device="cuda", dtype=torch.uint8)
+        L.check("cbl_silu_mul", L.lib.cbl_silu_mul(gu.data_ptr(), dtc, 2 * H, B, H, act.data_ptr(), s))
+        L.check("cbl_prep_x", L.lib.cbl_prep_x(act.data_ptr(), dtc, B, H, H, None, 1, a.data_ptr(), s))
+        L.check("cbl_silu_mul_stage", L.lib.cbl_silu_mul_stage(gu.data_ptr(), dtc, 2 * H, B, H, b.data_ptr(), s))
+        assert torch.equal(live(a), live(b))
+        if H > L.lib.cbl_add_rmsnorm_stage_max_columns():
+            continue
+        h = torch.randn(B, H, device="cuda", generator=g)
+        h2, w, add = h.clone(), torch.rand(H, device="cuda", generator=g).to(dt), gu[:, :H]
+        L.check("cbl_add_rmsnorm", L.lib.cbl_add_rmsnorm(h.data_ptr(), add.data_ptr(), 2 * H, w.data_ptr(), dtc, 1e-6, B, H, act.data_ptr(), s))
+        L.check("cbl_prep_x", L.lib.cbl_prep_x(act.data_ptr(), dtc, B, H, H, None, 1, a.data_ptr(), s))
+        L.check("cbl_add_rmsnorm_stage", L.lib.cbl_add_rmsnorm_stage(h2.data_ptr(), add.data_ptr(), 2 * H, w.data_ptr(), dtc, 1e-6, B, H, b.data_ptr(), s))
+        assert torch.equal(live(a), live(b)) and torch.equal(h, h2)
