@@ -530,8 +530,8 @@ __global__ void __launch_bounds__(256) k_silu_mul8(const T* __restrict__ gu, int
 // silu * up straight into the staging buffer of the product that follows: a block per row, the row in registers between the
 // search for its largest magnitude and the conversion; rows of up to 8 x 1024 x SILU_NV values.
 constexpr int SILU_NV = 4;
-template <typename T>
-__global__ void __launch_bounds__(1024) k_silu_stage(const T* __restrict__ gu, int64_t ld, int I, __half* __restrict__ xp, int Cpad,
+template <typename T, int NT, int BPS>
+__global__ void __launch_bounds__(NT, BPS) k_silu_stage(const T* __restrict__ gu, int64_t ld, int I, __half* __restrict__ xp, int Cpad,
                                                      float* __restrict__ xinv) {
     pdl_enter();
     __shared__ float red[32];
@@ -1009,7 +1009,11 @@ extern "C" int cbl_silu_mul_stage(const void* gate_up, int dtype, int64_t ld, in
     if (ld % 8 || (uintptr_t)gate_up % 16 || (uintptr_t)stage % 16) return CBL_EINVAL;
     if (B == 0) return CBL_OK;
     int nt = (cbl_ceil_div(Cpad / 8, SILU_NV) + 31) / 32 * 32;
-    CBL_BY_TYPE(dtype, return step_launch(k_silu_stage<T>, dim3(B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage, Cpad,
+    // two blocks per SM while a row's threads allow it: one block at a time leaves the memory idle between its phases
+    if (nt <= 640)
+        CBL_BY_TYPE(dtype, return step_launch(k_silu_stage<T, 640, 2>, dim3(B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage,
+                                              Cpad, (float*)((__half*)stage + (int64_t)Bpad * Cpad)));
+    CBL_BY_TYPE(dtype, return step_launch(k_silu_stage<T, 1024, 1>, dim3(B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage, Cpad,
                                           (float*)((__half*)stage + (int64_t)Bpad * Cpad)));
 }
 
