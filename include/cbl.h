@@ -102,6 +102,13 @@ int cbl_assign(const float* x, const float* wt, int64_t n, int32_t d, const void
 /* [R, n] tags (low `bits` bits of each int64) -> [R, ceil(n * bits / 32)] int32, a little-endian bit stream per row.
  * replaces shapequant/packed.py:60-77 (pack_bits). */
 int cbl_pack_tags(const int64_t* vals, int64_t R, int32_t n, int32_t bits, int32_t* words, cbl_stream s);
+/* The same; *bad (device, may be NULL) is set to 1 when a value does not fit `bits` bits. */
+int cbl_pack_tags_checked(const int64_t* vals, int64_t R, int32_t n, int32_t bits, int32_t* words, int32_t* bad, cbl_stream s);
+/* cbl_assign over the chunks of the rows of w [R, C] (row stride ld) divided by their fp16 scale [R], the last chunk of a row
+ * filled up with zeros: idx, err [R * ceil(C / 8)].  fp16 book [K, 8], K a multiple of 256.  used [K] (may be NULL): set to 1 for
+ * every codeword that was chosen.  An err of NaN where x is finite: a bounded device-side wait expired. */
+int cbl_snap_rows(const float* w, int64_t R, int32_t C, int64_t ld, const void* scale, const void* book, int32_t K, int64_t* idx, float* err,
+                  unsigned char* used, cbl_stream s);
 
 /* Unpacked tags of plane `plane` (0 or 1) as int32 [R, C/d].
  * replaces shapequant/packed.py:80-90 (unpack_bits) / :246-248 (PackedFile.local_tags). */

@@ -75,6 +75,8 @@ SIGNATURES = {
     "cbl_assign_max_codewords": (c_int, []),
     "cbl_assign": (c_int, [c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_int, c_int32, c_void_p, c_void_p, c_void_p]),
     "cbl_pack_tags": (c_int, [c_void_p, c_int64, c_int32, c_int32, c_void_p, c_void_p]),
+    "cbl_pack_tags_checked": (c_int, [c_void_p, c_int64, c_int32, c_int32, c_void_p, c_void_p, c_void_p]),
+    "cbl_snap_rows": (c_int, [c_void_p, c_int64, c_int32, c_int64, c_void_p, c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p]),
     "cbl_t16_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "cbl_repack_t16": (c_int, [POINTER(Packed), c_void_p, c_int32, c_void_p, c_void_p]),
     "cbl_prep_x_bytes": (c_size_t, [c_int32, c_int32, c_int32]),

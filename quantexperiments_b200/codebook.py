@@ -108,12 +108,13 @@ def pack_bits(vals: torch.Tensor, bits: int) -> torch.Tensor:
     if vals.device.type != "cuda":
         raise ValueError("pack_bits needs a CUDA tensor (no CPU path)")
     R, n = vals.shape
-    if vals.numel() and (int(vals.min()) < 0 or int(vals.max()) >= (1 << bits)):
-        raise ValueError(f"values out of range for {bits} bits")
     v = vals.to(torch.int64).contiguous()
     out = torch.empty(R, (n * bits + 31) // 32, dtype=torch.int32, device=vals.device)
     with torch.cuda.device(vals.device):
-        _lib.check("cbl_pack_tags", lib.cbl_pack_tags(v.data_ptr(), R, n, bits, out.data_ptr(), _stream()))
+        bad = torch.zeros(1, dtype=torch.int32, device=vals.device)
+        _lib.check("cbl_pack_tags_checked", lib.cbl_pack_tags_checked(v.data_ptr(), R, n, bits, out.data_ptr(), bad.data_ptr(), _stream()))
+    if v.numel() and int(bad):
+        raise ValueError(f"values out of range for {bits} bits")
     return out
 
 
@@ -167,9 +168,22 @@ def snap(w: torch.Tensor, codebook: torch.Tensor, *, d: int = 8, perm: torch.Ten
     if perm is not None:
         w32 = w32.index_select(1, perm.to(w32.device))
     scale16 = _fp16_row_rms(w32)
-    chunks, pad = chunk_rows(w32 / scale16.to(torch.float32)[:, None], d)
-    book16 = codebook.to(torch.float16)
-    idx, err = assign(chunks, book16, wt=_chunk_weights(tuple(w32.shape), d, scale16, perm, col_weight, row_weighted))
-    cm = CodebookMatrix(idx.view(w32.shape[0], -1), book16, scale16, pad, cols, perm)
-    stats = {"codebook_usage": torch.unique(idx).numel() / book16.shape[0], "normalized_chunk_mse": float(err.mean())}
+    book16 = codebook.to(torch.float16).contiguous()
+    rows, K = w32.shape[0], book16.shape[0]
+    used = torch.zeros(K, dtype=torch.uint8, device=w32.device)
+    if d == 8 and book16.shape[1] == 8 and K % 256 == 0 and K <= 4096 and col_weight is None and not row_weighted and w32.numel():
+        # the kernel divides by the scale, cuts the chunks and marks the words it uses
+        pad, w32 = (-cols) % d, w32 if w32.stride(1) == 1 else w32.contiguous()
+        nch = (cols + pad) // d
+        idx = torch.empty(rows * nch, dtype=torch.int64, device=w32.device)
+        err = torch.empty(rows * nch, dtype=torch.float32, device=w32.device)
+        with torch.cuda.device(w32.device):
+            _lib.check("cbl_snap_rows", lib.cbl_snap_rows(w32.data_ptr(), rows, cols, w32.stride(0), scale16.data_ptr(), book16.data_ptr(), K, idx.data_ptr(),
+                                                          err.data_ptr(), used.data_ptr(), _stream()))
+    else:
+        chunks, pad = chunk_rows(w32 / scale16.to(torch.float32)[:, None], d)
+        idx, err = assign(chunks, book16, wt=_chunk_weights(tuple(w32.shape), d, scale16, perm, col_weight, row_weighted))
+        used[idx] = 1
+    cm = CodebookMatrix(idx.view(rows, -1), book16, scale16, pad, cols, perm)
+    stats = {"codebook_usage": int(used.sum()) / K, "normalized_chunk_mse": float(err.mean())}
     return Snapped(cm, err, stats)

@@ -8,7 +8,7 @@
 //              group is evaluated once more at the end to name the first codeword that reaches the minimum.
 //              Bound by the fp32 FMA rate, not by memory: 65 kflop per 44 bytes of traffic.
 // k_pack_tags  one thread per 32-bit word of the stream.
-#include "cbl_common.cuh"
+#include "cbl_tc.cuh"
 #include <cmath>
 
 constexpr int AS_THREADS = 256, AS_GROUP = 8;
@@ -115,6 +115,394 @@ k_assign(const float* __restrict__ x, const float* __restrict__ wt, int64_t n, c
     }
 }
 
+// ------------------------------------------------------------------------------------ unweighted snap on the tensor cores
+//
+// The same minimum with the distances of a tile of 128 chunks to all codewords on tcgen05.mma, for fp16 books of a multiple
+// of 256 words.  A chunk's -2 x is split into two fp16 parts (22 bits; the book is fp16 as it is), |c|^2 into three that
+// ride along in the unused half of K = 16:
+//     A1 = [hi(-2 x) | f f f 0 0 0 0 0]   A2 = [lo(-2 x) | 0]   B = [c | hi, mid, lo of |c|^2 | 0]
+// so A1 B + A2 B = f |c|^2 - 2 x.c in fp32 (f: a power of two per chunk that keeps large chunks inside fp16; 1 otherwise).
+// Book and chunks are scaled by one more power of two when the book's largest value is not within 2 .. 64.
+// Sixteen warps read the 128 x 256 results out of tensor memory and keep the two groups of 16 codewords with the smallest
+// values per chunk; those of the best group - and of the second where it is closer than the arithmetic above can tell -
+// are then evaluated in fp32 exactly as k_assign does, in index order.
+//
+// 8.49 M chunks x 4096 words: 11.1 ms by k_assign (0.65 of the fp32 FMA rate); here 128 results per clock and SM leave the
+// tensor cores (two MMAs of 128 clocks per 128 x 256) and 64 lanes of minimum take the same time.
+constexpr int AT_TILE = 128, AT_N = 256, AT_EPI = 512, AT_THREADS = AT_EPI + 64 + 32;
+constexpr int AT_PROD_WARP = 16, AT_MMA_WARP = 18;
+constexpr int AT_A_BYTES = 4096;                 // 128 rows x 16 fp16
+constexpr int AT_BOOK = 131072;
+constexpr int AT_STAGE = 2 * AT_A_BYTES + AT_TILE * 36;         // A1 | A2 | the chunks in fp32 | the scales f
+constexpr int AT_SMEM = AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * 16 + 4 * AT_TILE * 8;
+constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
+
+__device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < AT_WAIT_LIMIT; i++) {
+        uint32_t ok;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void at_umma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+// K-major without swizzle, K = 16: core matrices of 8 rows x 16 bytes; the two of a row group are 128 bytes apart (leading
+// byte offset), row groups 256 (stride byte offset).
+__device__ __forceinline__ uint64_t at_desc(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)(128 >> 4) << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46;
+}
+__device__ __forceinline__ uint32_t at_row(int r) { return (uint32_t)((r >> 3) * 256 + (r & 7) * 16); }      // first half; the second 128 bytes on
+__device__ __forceinline__ void at_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+}
+
+// Waits for the loads issued so far; the values cannot be used ahead of it.
+__device__ __forceinline__ void at_landed(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), 
+                   "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+                 :
+                 : "memory");
+}
+
+// Where the chunks come from: an array of them, or rows of a matrix divided by their fp16 scale (zero columns appended).
+struct AtSource {
+    const float* x;
+    const __half* scale;                         // NULL: x is [n][8]
+    int C, nch;                                  // columns and chunks of a row
+    int64_t ld;
+};
+__device__ __forceinline__ void at_chunk(const AtSource& s, int64_t ci, float (&v)[8]) {
+    if (!s.scale) {
+        const float4 lo = __ldg((const float4*)s.x + 2 * ci), hi = __ldg((const float4*)s.x + 2 * ci + 1);
+        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+        return;
+    }
+    const int64_t r = ci / s.nch;
+    const int c = (int)(ci - r * s.nch) * 8;
+    const float* p = s.x + r * s.ld + c;
+    const float sc = __half2float(s.scale[r]);
+    if (c + 8 <= s.C && ((uintptr_t)p & 15) == 0) {
+        const float4 lo = __ldg((const float4*)p), hi = __ldg((const float4*)p + 1);
+        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = c + i < s.C ? __ldg(p + i) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = __fdiv_rn(v[i], sc);
+}
+
+struct AtPart { float best; int bg; float second; int sg; };
+
+__global__ void __launch_bounds__(AT_THREADS, 1)
+k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int64_t* __restrict__ idx, float* __restrict__ err,
+            unsigned char* __restrict__ used) {
+    extern __shared__ __align__(1024) unsigned char at_smem[];
+    __shared__ __align__(8) unsigned long long s_bar[8];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort;
+    __shared__ unsigned int s_max;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
+    const uint32_t sb = cbl_smem_u32(at_smem), bar0 = cbl_smem_u32(s_bar);
+    auto full_a = [&](int s) { return bar0 + 8u * s; };
+    auto empty_a = [&](int s) { return bar0 + 16u + 8u * s; };
+    auto acc_full = [&](int b) { return bar0 + 32u + 8u * b; };
+    auto acc_empty = [&](int b) { return bar0 + 48u + 8u * b; };
+    AtPart* s_part = (AtPart*)(at_smem + AT_BOOK + 2 * AT_STAGE);
+    float2* s_ex = (float2*)(at_smem + AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * 16);
+    const int64_t ntile = (n + AT_TILE - 1) / AT_TILE;
+    const int nstep = K / AT_N;
+    if (tid == 0) {
+        s_abort = 0;
+        s_max = 0u;
+        for (int s = 0; s < 2; s++) {
+            mbar_init(full_a(s), 2);
+            mbar_init(empty_a(s), 1 + 4);                      // the MMAs, and the epilogue's last look at the fp32 chunks
+            mbar_init(acc_full(s), 1);
+            mbar_init(acc_empty(s), 8);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == AT_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cbl_smem_u32(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    __syncthreads();
+    {
+        float mx = 0.f;
+        for (int k = tid; k < K * 4; k += AT_THREADS) {
+            const uint32_t w = __ldg((const uint32_t*)book + k) & 0x7FFF7FFFu;
+            const float2 f = __half22float2(*(const __half2*)&w);
+            mx = fmaxf(mx, fmaxf(f.x, f.y));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) atomicMax(&s_max, __float_as_uint(mx));
+    }
+    __syncthreads();
+    const float top = __uint_as_float(s_max);
+    const int q2 = top > 0.f && top < 3.0e38f && (top < 2.f || top >= 64.f) ? (top < 2.f ? 1 : 5) - ilogbf(top) : 0;
+    const float bs = ldexpf(1.f, q2);                          // scale of book and chunks
+    for (int k = tid; k < K; k += AT_THREADS) {
+        const uint4 w = __ldg((const uint4*)book + k);
+        const __half2* h = (const __half2*)&w;
+        uint4 scaled;
+        __half2* g = (__half2*)&scaled;
+        float sq = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 f = __half22float2(h[i]);
+            g[i] = __floats2half2_rn(f.x * bs, f.y * bs);
+            sq += f.x * f.x;
+            sq += f.y * f.y;
+        }
+        sq = sq * bs * bs;
+        __align__(16) __half part[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) part[i] = __float2half_rn(0.f);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            part[i] = __float2half_rn(sq);
+            sq -= __half2float(part[i]);
+        }
+        unsigned char* row = at_smem + at_row(k);
+        *(uint4*)row = scaled;
+        *(uint4*)(row + 128) = *(const uint4*)part;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    // A wait that expires is remembered (the errors of the block become NaN); the roles keep their step (they meet at named barriers).
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (!at_wait(bar, parity)) s_abort = 1;
+        __syncwarp();
+    };
+
+    if (warp == AT_MMA_WARP) {
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(AT_N >> 3) << 17) | ((uint32_t)(AT_TILE >> 4) << 24);
+        int it = 0;
+        uint32_t use = 0;                                      // uses of the two accumulators so far
+        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++) {
+            const int ab = it & 1;
+            wait(full_a(ab), (it >> 1) & 1);
+            const uint64_t a1 = at_desc(sb + AT_BOOK + ab * AT_STAGE), a2 = at_desc(sb + AT_BOOK + ab * AT_STAGE + AT_A_BYTES);
+            for (int j = 0; j < nstep; j++, use++) {
+                const int b = use & 1;
+                wait(acc_empty(b), ((use >> 1) & 1) ^ 1);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t bd = at_desc(sb + (uint32_t)j * (AT_N * 32));
+                if (elect_one()) {
+                    at_umma(tmem + b * AT_N, a1, bd, idesc, 0u);
+                    at_umma(tmem + b * AT_N, a2, bd, idesc, 1u);
+                    umma_commit(acc_full(b));
+                    if (j == nstep - 1) umma_commit(empty_a(ab));
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp >= AT_PROD_WARP) {
+        // ---------------- producer: two chunks of the tile per thread
+        int it = 0;
+        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++) {
+            const int ab = it & 1;
+            float v[2][8];
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int64_t ci = t * AT_TILE + c * 64 + tid - AT_EPI;
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[c][i] = 0.f;
+                if (ci < n) at_chunk(src, ci, v[c]);
+            }
+            wait(empty_a(ab), ((it >> 1) & 1) ^ 1);
+            unsigned char* st = at_smem + AT_BOOK + ab * AT_STAGE;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int r = c * 64 + tid - AT_EPI;
+                float mx = 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[c][i]));
+                mx *= bs;
+                const int e = mx > 8192.f && mx < 3.0e38f ? ilogbf(mx) - 12 : 0;      // |2 x| f < 2^14 (f only shrinks)
+                const float f = ldexpf(1.f, -e), fs = -2.0f * f * bs;
+                __align__(16) __half hi[8], lo[8], ff[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float a = fs * v[c][i];
+                    hi[i] = __float2half_rn(a);
+                    lo[i] = __float2half_rn(a - __half2float(hi[i]));
+                    ff[i] = __float2half_rn(i < 3 ? f : 0.f);
+                }
+                const uint32_t o = at_row(r);
+                *(uint4*)(st + o) = *(const uint4*)hi;
+                *(uint4*)(st + o + 128) = *(const uint4*)ff;
+                *(uint4*)(st + AT_A_BYTES + o) = *(const uint4*)lo;
+                *(uint4*)(st + AT_A_BYTES + o + 128) = make_uint4(0, 0, 0, 0);
+                float4* xs = (float4*)(st + 2 * AT_A_BYTES) + r;       // [2][128]: the two halves of the chunks
+                xs[0] = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+                xs[AT_TILE] = make_float4(v[c][4], v[c][5], v[c][6], v[c][7]);
+                ((float*)(st + 2 * AT_A_BYTES + AT_TILE * 32))[r] = f;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full_a(ab));
+        }
+    } else {
+        // ---------------- epilogue: warpgroup w reads half w & 1 of accumulator w >> 1; a thread's lane is a chunk of the tile
+        const int w = warp >> 2, row = (warp & 3) * 32 + lane, b = w >> 1;
+        const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(b * AT_N + (w & 1) * 128);
+        uint32_t use = b;                                      // accumulator uses are numbered over all tiles; this warpgroup takes every other
+        int it = 0;
+        uint32_t base = 0;
+        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++, base += nstep) {
+            float best = INFINITY, second = INFINITY;
+            int bg = 0, sg = 0;
+            for (; use < base + nstep; use += 2) {
+                const int j = (int)(use - base), g0 = j * 16 + (w & 1) * 8;
+                wait(acc_full(b), (use >> 1) & 1);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t va[32], vb[32];
+                auto look = [&](const uint32_t (&v)[32], int g) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        float m = as_min3(__uint_as_float(v[16 * h]), __uint_as_float(v[16 * h + 1]), __uint_as_float(v[16 * h + 2]));
+#pragma unroll
+                        for (int q = 3; q < 15; q += 2) m = as_min3(m, __uint_as_float(v[16 * h + q]), __uint_as_float(v[16 * h + q + 1]));
+                        m = fminf(m, __uint_as_float(v[16 * h + 15]));
+                        if (m < second) {
+                            const bool top = m < best;
+                            second = top ? best : m;
+                            sg = top ? bg : g + h;
+                            best = top ? m : best;
+                            bg = top ? g + h : bg;
+                        }
+                    }
+                };
+                at_ld32(ta, va);
+                at_landed(va);
+                at_ld32(ta + 32, vb);
+                look(va, g0);
+                at_landed(vb);
+                at_ld32(ta + 64, va);
+                look(vb, g0 + 2);
+                at_landed(va);
+                at_ld32(ta + 96, vb);
+                look(va, g0 + 4);
+                at_landed(vb);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(b));
+                look(vb, g0 + 6);
+            }
+            AtPart mine = {best, bg, second, sg};
+            s_part[w * AT_TILE + row] = mine;
+            asm volatile("bar.sync 1, %0;" ::"n"(AT_EPI) : "memory");
+            // all four warpgroups know the two best groups of their chunk; each evaluates a quarter of a group's words
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const AtPart p = s_part[q * AT_TILE + row];
+                if (q == 0) { best = p.best; bg = p.bg; second = p.second; sg = p.sg; continue; }
+                auto add = [&](float v, int g) {
+                    if (v < best || (v == best && g < bg)) { second = best; sg = bg; best = v; bg = g; }
+                    else if (v < second || (v == second && g < sg)) { second = v; sg = g; }
+                };
+                add(p.best, p.bg);
+                add(p.second, p.sg);
+            }
+            const unsigned char* st = at_smem + AT_BOOK + (it & 1) * AT_STAGE;
+            const float4 x0 = ((const float4*)(st + 2 * AT_A_BYTES))[row], x1 = ((const float4*)(st + 2 * AT_A_BYTES))[AT_TILE + row];
+            const float f = ((const float*)(st + 2 * AT_A_BYTES + AT_TILE * 32))[row];
+            const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            float xx = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) xx += xv[i] * xv[i];
+            float bd = INFINITY;
+            int bi = 0;
+            const float ibs = ldexpf(1.f, -q2);
+            auto exact = [&](int g) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int k = g * 16 + w * 4 + q;
+                    // (a book that was scaled down may have lost bits in shared memory)
+                    const uint4 cw = q2 >= 0 ? *(const uint4*)(at_smem + at_row(k)) : __ldg((const uint4*)book + k);
+                    const __half2* h = (const __half2*)&cw;
+                    float c[8], d = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float2 p = __half22float2(h[i]);
+                        c[2 * i] = q2 > 0 ? p.x * ibs : p.x;
+                        c[2 * i + 1] = q2 > 0 ? p.y * ibs : p.y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++) d += c[i] * c[i];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) d = fmaf(-2.0f * xv[i], c[i], d);
+                    if (d < bd || (d == bd && k < bi)) { bd = d; bi = k; }
+                }
+            };
+            exact(bg);
+            // what the split operands and the accumulation can be off by, several times over
+            if ((second - best) <= 1e-5f * f * (bs * bs) * (fabsf(bd) + xx)) exact(sg);
+            s_ex[w * AT_TILE + row] = make_float2(bd, __int_as_float(bi));
+            asm volatile("bar.sync 1, %0;" ::"n"(AT_EPI) : "memory");
+            if (w == 0) {
+#pragma unroll
+                for (int q = 1; q < 4; q++) {
+                    const float2 p = s_ex[q * AT_TILE + row];
+                    const int k = __float_as_int(p.y);
+                    if (p.x < bd || (p.x == bd && k < bi)) { bd = p.x; bi = k; }
+                }
+                const int64_t ci = t * AT_TILE + row;
+                if (ci < n) {
+                    idx[ci] = bi;
+                    err[ci] = s_abort ? __int_as_float(0x7fc00000) : fmaxf(bd + xx, 0.f);      // an expired wait shows as NaN
+                    if (used) used[bi] = 1;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty_a(it & 1));
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == AT_MMA_WARP) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+static int launch_assign_tc(const AtSource& src, int64_t n, const void* book, int K, int64_t* idx, float* err, unsigned char* used, cudaStream_t st) {
+    static bool attr_set[64] = {};
+    int dev = 0;
+    CBL_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        CBL_CUDA(cudaFuncSetAttribute(k_assign_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM));
+        attr_set[dev] = true;
+    }
+    const int64_t tiles = (n + AT_TILE - 1) / AT_TILE;
+    const int grid = (int)(tiles < cbl_sm_count() ? tiles : cbl_sm_count());
+    k_assign_tc<<<grid, AT_THREADS, AT_SMEM, st>>>(src, n, (const __half*)book, K, idx, err, used);
+    return cbl_check_launch();
+}
+
 extern "C" int cbl_assign_max_codewords() { return 4096; }
 
 extern "C" int cbl_assign(const float* x, const float* wt, int64_t n, int32_t d, const void* book, int bdtype, int32_t K, int64_t* idx,
@@ -124,6 +512,9 @@ extern "C" int cbl_assign(const float* x, const float* wt, int64_t n, int32_t d,
     if (d != 8 || K > 4096) return CBL_EUNSUPPORTED;
     if (((uintptr_t)x % 16) || (wt && ((uintptr_t)wt % 16))) return CBL_EINVAL;
     if (n == 0) return CBL_OK;
+    // fp16 books of whole MMA tiles, unweighted, at least a few tiles of chunks: the tensor cores find the candidates
+    if (!wt && bdtype == CBL_F16 && K % AT_N == 0 && (uintptr_t)book % 16 == 0 && n >= 4 * AT_TILE)
+        return launch_assign_tc(AtSource{x, nullptr, 0, 0, 0}, n, book, K, idx, err, nullptr, (cudaStream_t)s);
     const int Kpad = (K + AS_GROUP - 1) / AS_GROUP * AS_GROUP;
     const size_t smem = (size_t)Kpad * 36;
     static bool attr_set[64][2] = {};
@@ -144,8 +535,19 @@ extern "C" int cbl_assign(const float* x, const float* wt, int64_t n, int32_t d,
     return cbl_check_launch();
 }
 
+// The chunks of w / scale: rows of a matrix divided by their fp16 scale, cut into chunks of 8, zeros appended to the last.
+extern "C" int cbl_snap_rows(const float* w, int64_t R, int32_t C, int64_t ld, const void* scale, const void* book, int32_t K, int64_t* idx, float* err,
+                             unsigned char* used, cbl_stream s) {
+    if (!w || !scale || !book || !idx || !err || R < 0 || C < 1 || ld < C) return CBL_EINVAL;
+    if (K < AT_N || K > 4096 || K % AT_N || (uintptr_t)book % 16) return CBL_EUNSUPPORTED;
+    if (R == 0) return CBL_OK;
+    const int nch = cbl_ceil_div(C, 8);
+    return launch_assign_tc(AtSource{w, (const __half*)scale, C, nch, ld}, R * nch, book, K, idx, err, used, (cudaStream_t)s);
+}
+
 // ------------------------------------------------------------------------------------ bit packing
-__global__ void __launch_bounds__(256) k_pack_tags(const int64_t* __restrict__ vals, int64_t R, int n, int bits, int W, int32_t* __restrict__ words) {
+__global__ void __launch_bounds__(256) k_pack_tags(const int64_t* __restrict__ vals, int64_t R, int n, int bits, int W, int32_t* __restrict__ words,
+                                                   int* __restrict__ bad) {
     const int64_t gi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= R * W) return;
     const int64_t r = gi / W;
@@ -154,7 +556,8 @@ __global__ void __launch_bounds__(256) k_pack_tags(const int64_t* __restrict__ v
     const unsigned long long mask = (1ull << bits) - 1ull;
     unsigned int out = 0;
     for (int t = (int)(b0 / bits); t < n && (int64_t)t * bits < b0 + 32; t++) {
-        const unsigned long long v = (unsigned long long)vals[r * n + t] & mask;
+        const unsigned long long full = (unsigned long long)vals[r * n + t], v = full & mask;
+        if (bad && full != v) *bad = 1;
         const int64_t sh = (int64_t)t * bits - b0;          // position of the tag's bit 0 relative to the word
         out |= sh >= 0 ? (unsigned int)(v << sh) : (unsigned int)(v >> (-sh));
     }
@@ -162,10 +565,14 @@ __global__ void __launch_bounds__(256) k_pack_tags(const int64_t* __restrict__ v
 }
 
 extern "C" int cbl_pack_tags(const int64_t* vals, int64_t R, int32_t n, int32_t bits, int32_t* words, cbl_stream s) {
+    return cbl_pack_tags_checked(vals, R, n, bits, words, nullptr, s);
+}
+
+extern "C" int cbl_pack_tags_checked(const int64_t* vals, int64_t R, int32_t n, int32_t bits, int32_t* words, int32_t* bad, cbl_stream s) {
     if (!vals || !words || R < 0 || n < 1 || bits < 1 || bits > 16) return CBL_EINVAL;
     const int W = (int)(((int64_t)n * bits + 31) / 32);
     const int64_t total = R * W;
     if (total == 0) return CBL_OK;
-    k_pack_tags<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)s>>>(vals, R, n, bits, W, words);
+    k_pack_tags<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)s>>>(vals, R, n, bits, W, words, bad);
     return cbl_check_launch();
 }

@@ -147,3 +147,40 @@ def test_codebook_matrix_decode_with_padding_and_permutation_matches_the_referen
     small = cb.CodebookMatrix(cm.idx % 48, cm.codebook[:48], cm.row_scale, pad, cols, None)
     ref = orc.codebook_decode((z["idx"] % 48), z["codebook"][:48], z["row_scale"], pad, cols, None)
     assert np.array_equal(cb.decode(small).cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("K", [256, 4096])
+@pytest.mark.parametrize("scale_x,scale_c", [(1.0, 1.0), (1e-4, 1e-4), (300.0, 200.0), (1e4, 1.0), (1.0, 1e-3)])
+def test_tensor_core_assign_finds_the_exact_minimum(K, scale_x, scale_c):
+    """The tensor-core path (fp16 book of whole MMA tiles): chunks and books of very different sizes, ragged chunk counts, a tile's
+    edges; every index within rounding of the float64 minimum and the error as the scalar kernel computes it."""
+    from quantexperiments_b200 import codebook as cb
+    g = torch.Generator().manual_seed(K)
+    book = (torch.randn(K, 8, generator=g) * scale_c).half()
+    for n in (512, 513, 20001):
+        x = torch.randn(n, 8, generator=g) * scale_x
+        x[5] = 0.0
+        x[6] = book[K - 1].float()
+        idx, err = cb.assign(x.cuda(), book.cuda())
+        d = ((x.double()[:, None, :] - book.double()[None, :, :]) ** 2).sum(-1) if n < 1000 else None
+        xi, size = x.double(), (x.double() ** 2).sum(1)
+        got = ((xi - book.double()[idx.cpu()]) ** 2).sum(1)
+        best = d.min(1).values if d is not None else torch.cat([((c[:, None] - book.double()[None]) ** 2).sum(-1).min(1).values for c in xi.split(2000)])
+        tol = 4e-6 * (size + got) + 1e-30
+        assert ((got - best) <= tol).all()
+        assert ((err.cpu().double() - got).abs() <= tol).all()
+        assert int(idx[6]) == K - 1 or torch.equal(book[int(idx[6])], book[K - 1])
+
+
+def test_snap_rows_equals_snap_by_chunks():
+    """snap() of a plain matrix (division and chunking inside the kernel, ragged columns) against assign() of the chunks."""
+    from quantexperiments_b200 import codebook as cb
+    g = torch.Generator(device="cuda").manual_seed(4)
+    book = torch.randn(4096, 8, device="cuda", generator=g).half()
+    for R, C in ((37, 1001), (256, 512), (130, 8)):
+        w = torch.randn(R, C, device="cuda", generator=g) * 0.02
+        r = cb.snap(w, book)
+        chunks, pad = cb.chunk_rows(w / r["row_scale"].float()[:, None], 8)
+        idx, err = cb.assign(chunks, book)
+        assert torch.equal(r["idx"].reshape(-1), idx) and torch.equal(r.err, err) and r["pad"] == pad
+        assert r.stats["codebook_usage"] == idx.unique().numel() / 4096
