@@ -38,6 +38,11 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -527,23 +532,24 @@ __global__ void __launch_bounds__(256) k_silu_mul8(const T* __restrict__ gu, int
     *(uint4*)(out + (int64_t)b * I + i) = o.v;
 }
 
-// silu * up straight into the staging buffer of the product that follows: a block per row, the row in registers between the
-// search for its largest magnitude and the conversion; rows of up to 8 x 1024 x SILU_NV values.
+// silu * up straight into the staging buffer of the product that follows: the blocks of a cluster share a row, which stays in
+// registers between the search for its largest magnitude and the conversion; up to 8 x 1024 x SILU_NV values per block.
 constexpr int SILU_NV = 4;
 template <typename T, int NT, int BPS>
 __global__ void __launch_bounds__(NT, BPS) k_silu_stage(const T* __restrict__ gu, int64_t ld, int I, __half* __restrict__ xp, int Cpad,
-                                                     float* __restrict__ xinv) {
+                                                        float* __restrict__ xinv) {
     pdl_enter();
     __shared__ float red[32];
-    const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    __shared__ float s_mx;
+    const int b = blockIdx.y, rank = blockIdx.x, cs = gridDim.x, tid = threadIdx.x, nt = blockDim.x, per = Cpad / 8 / cs;
     const T* row = gu + (int64_t)b * ld;
     union Pack { uint4 v; T t[8]; } o[SILU_NV];
     float mx = 0.f;
 #pragma unroll
     for (int k = 0; k < SILU_NV; k++) {
-        const int i = (tid + nt * k) * 8;
+        const int c = tid + nt * k, i = (rank * per + c) * 8;
         o[k].v = make_uint4(0, 0, 0, 0);
-        if (i < I) {
+        if (c < per && i < I) {
             float g[8], u[8];
             unpack8<T>(__ldcg((const uint4*)(row + i)), g);
             unpack8<T>(__ldcg((const uint4*)(row + I + i)), u);
@@ -559,20 +565,32 @@ __global__ void __launch_bounds__(NT, BPS) k_silu_stage(const T* __restrict__ gu
     __syncthreads();
     mx = 0.f;
     for (int k = 0; k < nt / 32; k++) mx = fmaxf(mx, red[k]);
+    if (cs > 1) {
+        if (tid == 0) s_mx = mx;
+        cluster_sync_all();
+        for (int r = 0; r < cs; r++) {
+            uint32_t a;
+            float v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(cbl_smem_u32(&s_mx)), "r"(r));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+            mx = fmaxf(mx, v);
+        }
+    }
     const int ex = cbl_scale_exp(mx);
     const float sc = ldexpf(1.f, -ex);
-    if (tid == 0) xinv[b] = ldexpf(1.f, ex);
+    if (tid == 0 && rank == 0) xinv[b] = ldexpf(1.f, ex);
 #pragma unroll
     for (int k = 0; k < SILU_NV; k++) {
-        const int i = (tid + nt * k) * 8;
-        if (i < Cpad) {
+        const int c = tid + nt * k;
+        if (c < per) {
             uint4 d;
             __half2* hd = (__half2*)&d;
 #pragma unroll
             for (int e = 0; e < 4; e++) hd[e] = __floats2half2_rn(to_f(o[k].t[2 * e]) * sc, to_f(o[k].t[2 * e + 1]) * sc);
-            *(uint4*)(xp + (int64_t)b * Cpad + i) = d;
+            *(uint4*)(xp + (int64_t)b * Cpad + (rank * per + c) * 8) = d;
         }
     }
+    if (cs > 1) cluster_sync_all();                              // no block leaves while another may still read its maximum
 }
 
 template <typename T>
@@ -819,10 +837,6 @@ __global__ void __launch_bounds__(256, 3) k_head_mma(const T* __restrict__ W, co
 // thread blocks per row: every block reduces its share, block 0 collects the others' results through
 // distributed shared memory.
 constexpr int ARGMAX_CTAS = 8;
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __global__ void __launch_bounds__(1024) k_argmax(const void* __restrict__ logits, int ldtype, int64_t ldl, int V, int64_t* __restrict__ tok,
                                                  int32_t* __restrict__ pos) {
     pdl_enter();
@@ -1008,13 +1022,21 @@ extern "C" int cbl_silu_mul_stage(const void* gate_up, int dtype, int64_t ld, in
     if (I % 8 || Cpad > 8 * 1024 * SILU_NV) return CBL_EUNSUPPORTED;
     if (ld % 8 || (uintptr_t)gate_up % 16 || (uintptr_t)stage % 16) return CBL_EINVAL;
     if (B == 0) return CBL_OK;
-    int nt = (cbl_ceil_div(Cpad / 8, SILU_NV) + 31) / 32 * 32;
-    // two blocks per SM while a row's threads allow it: one block at a time leaves the memory idle between its phases
+    if (B > 65535) return CBL_EUNSUPPORTED;
+    // few rows: eight blocks share one (32 rows of 18944: 6.2 us, 8.2 with a block per row); many: two blocks per SM while a
+    // row's threads allow it (one block at a time leaves the memory idle between its phases)
+    float* xinv = (float*)((__half*)stage + (int64_t)Bpad * Cpad);
+    if (B <= 128) {
+        const int nt = (cbl_ceil_div(Cpad / 64, 2) + 31) / 32 * 32;
+        CBL_BY_TYPE(dtype, return (step_launch<8>(k_silu_stage<T, 640, 2>, dim3(8, B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I,
+                                                  (__half*)stage, Cpad, xinv)));
+    }
+    const int nt = (cbl_ceil_div(Cpad / 8, SILU_NV) + 31) / 32 * 32;
     if (nt <= 640)
-        CBL_BY_TYPE(dtype, return step_launch(k_silu_stage<T, 640, 2>, dim3(B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage,
-                                              Cpad, (float*)((__half*)stage + (int64_t)Bpad * Cpad)));
-    CBL_BY_TYPE(dtype, return step_launch(k_silu_stage<T, 1024, 1>, dim3(B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage, Cpad,
-                                          (float*)((__half*)stage + (int64_t)Bpad * Cpad)));
+        CBL_BY_TYPE(dtype, return (step_launch(k_silu_stage<T, 640, 2>, dim3(1, B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage,
+                                               Cpad, xinv)));
+    CBL_BY_TYPE(dtype, return (step_launch(k_silu_stage<T, 1024, 1>, dim3(1, B), dim3(nt), 0, (cudaStream_t)s, (const T*)gate_up, ld, (int)I, (__half*)stage,
+                                           Cpad, xinv)));
 }
 
 extern "C" int32_t cbl_head_gemv_max_batch(void) { return HEAD_BMAX; }
