@@ -33,16 +33,12 @@
 
 constexpr int L8_NT = 512;                       // threads per block; a thread handles 4 consecutive rows per ring stage
 constexpr int L8_NWARP = L8_NT / 32;
-constexpr int L8_THREADS = L8_NT;                // the last warp to read a ring stage refills it
 constexpr int L8_RPT = 8;                        // rows per thread: a block covers at most 4096 rows
 constexpr int L8_STEP_ROWS = 4 * L8_NT;           // 2048 rows per step of the block
-constexpr int L8_STAGE_ROWS = L8_STEP_ROWS / 2;   // a ring stage holds half a step: the rows of 8 warps
-constexpr int L8_STAGE_WARPS = L8_NWARP / 2;
-constexpr int L8_STAGE_BYTES = 3 * L8_STAGE_ROWS * 4;   // three tag planes
-constexpr int L8_MAX_STAGES = 8;
-constexpr int L8_DYN_SMEM = 231424;              // all of an SM's shared memory but 1 KB for the static part
-constexpr int L8_ACC_BYTES = L8_NT * L8_RPT * 4;  // fp32 row sums of a block between tiles
-constexpr uint32_t L8_WAIT_LIMIT = 1u << 20;     // mbarrier polls before a wait gives up
+constexpr int L8_TABLE_BYTES = 65536;            // table of one tile: 4096 entries x 8 columns x 2 bytes
+constexpr int L8_XSLOTS = 32;                    // tiles whose scaled activations are staged
+constexpr int L8_DYN_SMEM = 2 * L8_TABLE_BYTES + L8_XSLOTS * 128;
+constexpr int L8_AHEAD = 4;                      // tiles of a block whose tags are sent to L2 before the predecessor is waited for
 constexpr int L8_MAX_GROUP = 4;
 constexpr int L8_MAX_BLOCKS = 160;
 constexpr int L8_MAX_ORDERS = 16;
@@ -61,32 +57,10 @@ extern "C" size_t cbl_gemv_l8_workspace_bytes(int32_t R) {
     return L8_PART_BYTES + L8_CTL_WORDS * 4 + l8_rows_max(R) * 4;
 }
 
-__device__ __forceinline__ void l8_mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void l8_mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void l8_bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
-                 "r"(bytes), "r"(bar)
-                 : "memory");
-}
-// Bounded wait for a phase of an mbarrier; false when the limit ran out.
-__device__ __forceinline__ bool l8_mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < L8_WAIT_LIMIT; i++) {
-        uint32_t ok;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ uint32_t l8_lds32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+// 16 bytes of tags: read once per call, so they need not stay in L1.
+__device__ __forceinline__ uint4 l8_ldg128(const uint32_t* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ void l8_sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
@@ -97,26 +71,13 @@ __device__ __forceinline__ void l8_mma1688(float (&c)[4], uint32_t a0, uint32_t 
         : "r"(a0), "r"(a1), "r"(b0), "f"(0.0f));
 }
 
-// One signed 16-bit table entry (sign-extended) from a shared-memory address.
-__device__ __forceinline__ int l8_entry(uint32_t addr) {
-    int v;
-    asm volatile("ld.shared.s16 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-
 // Sum of a row's 8 table entries of one tile (exact: the entries are 16-bit integers).  (w0, w1, w2) is the row's
-// 96-bit stream of 8 tags, slot s at bit 12 s; col[s] = table base | 2 * column of slot s for this lane.  Entry
-// address = base + tag * 16 + column * 2: the base is 64 KB aligned, so the three fields are merged with one logic
-// operation per tag.
-__device__ __forceinline__ int l8_row8(uint32_t w0, uint32_t w1, uint32_t w2, const uint32_t (&col)[8]) {
-    const int e0 = l8_entry(((w0 << 4) & 0xFFF0u) | col[0]);
-    const int e1 = l8_entry(((w0 >> 8) & 0xFFF0u) | col[1]);
-    const int e2 = l8_entry((__funnelshift_r(w0, w1, 20) & 0xFFF0u) | col[2]);
-    const int e3 = l8_entry((w1 & 0xFFF0u) | col[3]);
-    const int e4 = l8_entry(((w1 >> 12) & 0xFFF0u) | col[4]);
-    const int e5 = l8_entry((__funnelshift_r(w1, w2, 24) & 0xFFF0u) | col[5]);
-    const int e6 = l8_entry(((w2 >> 4) & 0xFFF0u) | col[6]);
-    const int e7 = l8_entry(((w2 >> 16) & 0xFFF0u) | col[7]);
+// 96-bit stream of 8 tags, slot s at bit 12 s; col[s] = table | 2 * column of slot s for this lane.  An entry stands at
+// table + tag * 16 + column * 2: the three fields are merged with one logic operation per tag.
+__device__ __forceinline__ int l8_row8(const unsigned char* tables, uint32_t w0, uint32_t w1, uint32_t w2, const uint32_t (&col)[8]) {
+    auto entry = [&](uint32_t tag16, uint32_t c) { return (int)*(const short*)(tables + ((tag16 & 0xFFF0u) | c)); };
+    const int e0 = entry(w0 << 4, col[0]), e1 = entry(w0 >> 8, col[1]), e2 = entry(__funnelshift_r(w0, w1, 20), col[2]), e3 = entry(w1, col[3]);
+    const int e4 = entry(w1 >> 12, col[4]), e5 = entry(__funnelshift_r(w1, w2, 24), col[5]), e6 = entry(w2 >> 4, col[6]), e7 = entry(w2 >> 16, col[7]);
     return ((e0 + e1) + (e2 + e3)) + ((e4 + e5) + (e6 + e7));
 }
 
@@ -159,12 +120,11 @@ struct L8Plan {
 // Barrier among the block's 512 threads.
 __device__ __forceinline__ void l8_sync_block() { asm volatile("bar.sync 1, %0;" ::"n"(L8_NT) : "memory"); }
 
-__global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant__ L8Launch P, const __grid_constant__ L8Plan plan,
-                                                           const void* __restrict__ x, int xdtype) {
-    extern __shared__ __align__(128) unsigned char l8_smem[];
-    __shared__ __align__(8) unsigned long long s_bar[L8_MAX_STAGES];       // full[stage]: the stage's tags have landed
-    __shared__ int s_abort;
-    __shared__ unsigned int s_readers[L8_MAX_STAGES];   // warps that have read the stage's current contents
+__global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8Launch P, const __grid_constant__ L8Plan plan,
+                                                      const void* __restrict__ x, int xdtype) {
+    extern __shared__ __align__(128) unsigned char l8_smem[];              // two 64 KB tables | scaled activations of 32 tiles
+    __shared__ float s_inv[L8_XSLOTS];                                      // factor that undoes a tile's scale
+    __shared__ float s_sum[L8_NT];                                          // sums of the groups of splits (output phase)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     if ((int)blockIdx.x >= plan.nblocks) return;
@@ -174,94 +134,80 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
     const cbl_l8& mm = P.m[mi];
     // Programmatic dependent launch: this kernel waits for its predecessor only where it first touches data that
     // depends on it (x, the work space, y), and lets its successor in when its own lookups are done (below).
-
-    // ---- shared memory: two 64 KB tables on a 64 KB boundary; below and above them the fp32 row sums of the
-    // block (16 KB) and the ring stages
-    const uint32_t base = cbl_smem_u32(l8_smem), end = base + (uint32_t)L8_DYN_SMEM;
-    const uint32_t tbl0 = (base + 65535u) & ~65535u;
-    const uint32_t hi0 = tbl0 + 131072u;
-    uint32_t lo0 = (base + 127u) & ~127u, hi1 = hi0, sacc;
-    if (end >= hi0 + L8_ACC_BYTES) { sacc = hi0; hi1 += L8_ACC_BYTES; } else { sacc = lo0; lo0 += L8_ACC_BYTES; }
-    const int n_lo = tbl0 > lo0 ? (int)((tbl0 - lo0) / L8_STAGE_BYTES) : 0;
-    const int n_hi = end > hi1 ? (int)((end - hi1) / L8_STAGE_BYTES) : 0;
-    const int S = min(L8_MAX_STAGES, n_lo + n_hi);
-    if (hi1 > end || S < 2) {                          // cannot happen with the launch configuration of this file
-        if (tid == 0) atomicExch(P.status, 2u);
-        return;
-    }
-    auto stage_addr = [&](int s) { return s < n_lo ? lo0 + (uint32_t)s * L8_STAGE_BYTES : hi1 + (uint32_t)(s - n_lo) * L8_STAGE_BYTES; };
-    const uint32_t bar0 = cbl_smem_u32(s_bar);
-
     const int nrow_it = (nrows + L8_STEP_ROWS - 1) / L8_STEP_ROWS;     // <= 2
     const int ntl = tile_hi - tile_lo;
-    const int nit = ntl * nrow_it;                     // iterations of this block: (tile, row step), tile-major; two ring stages each
-    if (tid < S) {
-        l8_mbar_init(bar0 + 8 * tid, 1);                             // full: the issuing lane's arrive + the bytes of three copies
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (tid == 0) s_abort = 0;
-    if (tid < L8_MAX_STAGES) s_readers[tid] = 0u;
-    __syncthreads();
+    const int nit = ntl * nrow_it;                     // iterations of this block: (tile, row step), tile-major
 
-    // ---- tag ring.  Stage n (half n & 1 of iteration n / 2) lives in ring slot n mod S.  Nobody is the producer: the
-    // warp that is the LAST of a stage's 8 readers issues the copies of stage n + S into the slot (lanes 0..2 the three
-    // tag planes, lane 0 announces the bytes), without waiting for anything.  Weights do not depend on the previous
-    // kernel: warp 0 fills the ring before the wait below.
-    auto issue = [&](int n) {                           // whole warp; stage n -> slot n mod S
-        const int i = n >> 1, ti = i / nrow_it, k = i - ti * nrow_it;
-        const int r0 = k * L8_STEP_ROWS + (n & 1) * L8_STAGE_ROWS;
-        const int cnt = max(0, min(L8_STAGE_ROWS, nrows - r0));
-        const int slot = n % S;
-        const uint32_t bar = bar0 + 8 * slot;
-        if (lane == 0) {
-            if (cnt > 0) l8_mbar_expect_tx(bar, 12u * (uint32_t)cnt);
-            else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");      // an empty half completes at once
+    // ---- tags: 16 bytes per plane and step of this thread's four rows, asked for two iterations ahead.  Weights do not
+    // depend on the previous kernel: the first two iterations are requested here, what follows is sent on its way to L2.
+    const uint32_t* tags = (const uint32_t*)mm.words + (int64_t)tile_lo * 3 * mm.Rpad + row_lo + 4 * tid;
+    const int64_t plane = mm.Rpad;
+    auto fetch = [&](uint4 (&w)[3], int it) {
+        const int ti = nrow_it == 2 ? it >> 1 : it, r0 = (it - ti * nrow_it) * L8_STEP_ROWS;
+        if (it < nit && r0 + 4 * tid < nrows) {
+            const uint32_t* p = tags + (int64_t)ti * 3 * plane + r0;
+            w[0] = l8_ldg128(p);
+            w[1] = l8_ldg128(p + plane);
+            w[2] = l8_ldg128(p + 2 * plane);
         }
-        __syncwarp();
-        if (lane < 3 && cnt > 0)
-            l8_bulk_g2s(stage_addr(slot) + lane * (L8_STAGE_ROWS * 4),
-                        (const uint32_t*)mm.words + ((int64_t)(tile_lo + ti) * 3 + lane) * mm.Rpad + row_lo + r0, 4u * (uint32_t)cnt, bar);
     };
-    if (warp == 0)
-        for (int n = 0; n < S && n < 2 * nit; n++) issue(n);
+    uint4 wa[3], wb[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) wa[i] = wb[i] = make_uint4(0, 0, 0, 0);
+    fetch(wa, 0);
+    fetch(wb, 1);
+    if (tid < 3 * (L8_AHEAD < ntl ? L8_AHEAD : ntl))
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const uint32_t*)mm.words + ((int64_t)tile_lo * 3 + tid) * plane + row_lo),
+                     "r"(4 * nrows)
+                     : "memory");
 
     // ---- tables.  The book's mma A fragments stay in registers for all tiles of a book (one 16-byte load per two
     // 16-codeword blocks); everything that does not depend on the previous kernel is requested before the wait.
     const int ntile1 = mm.ntile / mm.books;
     uint4 af[8];
-    int cur_book = -1, jx = 0;
     auto set_book = [&](int book) {
         const uint4* fr = (const uint4*)(book ? mm.frag2 : mm.frag);
 #pragma unroll
         for (int i = 0; i < 8; i++) af[i] = __ldg(fr + (warp + i * L8_NWARP) * 32 + lane);
-        // |<codeword, x_chunk>| <= norm * |x_chunk| < 2^(jx + 1) * 2^(13 - jx) = 2^14: every entry fits 16 bits with room to spare
-        jx = book ? mm.book_exp2 : mm.book_exp;
-        cur_book = book;
     };
-    set_book(tile_lo / ntile1);
+    // The values pass through an empty asm, so that the compiler keeps them in registers: left alone it loads them again,
+    // from L2, inside every build.
+    auto pin_book = [&]() {
+#pragma unroll
+        for (int i = 0; i < 8; i++) asm volatile("" : "+r"(af[i].x), "+r"(af[i].y), "+r"(af[i].z), "+r"(af[i].w));
+    };
+    int cur_book = tile_lo >= ntile1;
+    set_book(cur_book);
 
-    asm volatile("griddepcontrol.wait;" ::: "memory");              // x, accumulators and outputs belong to earlier kernels until here
-    float* fsum = P.fsum[mi];
-    if (P.calls && fsum) fsum += (int64_t)((__ldcg(P.calls) + 1u) & 1u) * P.fsum_stride;
-
+    // ---- activations of a tile: lane (g, t) holds elements 2 lane, 2 lane + 1, the B fragment of the build (k = 2t, 2t + 1 of
+    // chunk column g).  Where they stand comes from the column order; the bits are converted only where they are used, so that
+    // the loads of several tiles are in flight together.
     const int32_t* perm = mm.perms ? mm.perms + (int64_t)order * mm.C : nullptr;
-    auto load_x = [&](int tile, float& xa, float& xb) {
-        const int ctile = tile % ntile1, c0 = ctile * 64 + 2 * lane;
-        xa = xb = 0.f;
-        if (c0 < mm.C) {
-            xa = cbl_load_in(x, xdtype, perm ? perm[c0] : c0);
-            xb = cbl_load_in(x, xdtype, perm ? perm[c0 + 1] : c0 + 1);
-        }
+    auto x_place = [&](int tile) {                      // -1: past the last column
+        const int c0 = (tile >= ntile1 ? tile - ntile1 : tile) * 64 + 2 * lane;
+        if (c0 >= mm.C) return make_int2(-1, -1);
+        return perm ? make_int2(__ldg(perm + c0), __ldg(perm + c0 + 1)) : make_int2(c0, c0 + 1);
     };
-    float xa, xb;
-    load_x(tile_lo, xa, xb);
-
-    // ---- table build: 16 codeword blocks per warp; the tile's 64 activations are this warp's B fragment
-    // (lane (g, t) holds k = 2t, 2t+1 of chunk column g = elements 2 lane, 2 lane + 1 of the tile).  The activations
-    // are scaled by a power of two that brings the largest Euclidean norm of the tile's 8 chunks below
+    auto x_bits = [&](int2 at) {
+        uint2 v = make_uint2(0u, 0u);
+        if (at.x >= 0) {
+            if (xdtype == CBL_F32) v = make_uint2(((const uint32_t*)x)[at.x], ((const uint32_t*)x)[at.y]);
+            else v = make_uint2(((const unsigned short*)x)[at.x], ((const unsigned short*)x)[at.y]);
+        }
+        return v;
+    };
+    auto x_val = [&](uint32_t v) {
+        if (xdtype == CBL_BF16) return __uint_as_float(v << 16);
+        if (xdtype == CBL_F16) return __half2float(__ushort_as_half((unsigned short)v));
+        return __uint_as_float(v);
+    };
+    // The activations are scaled by a power of two that brings the largest Euclidean norm of the tile's 8 chunks below
     // 2^13 * 2^-jx: the products then stay below 2^14 in magnitude whatever the inputs (Cauchy-Schwarz) and
-    // are stored as rounded 16-bit integers; the returned factor undoes the scale on the integer sum of a row.
-    auto build = [&](uint32_t tbl, float va, float vb) -> float {
+    // are stored as rounded 16-bit integers; `inv` undoes the scale on the integer sum of a row.
+    auto scaled = [&](uint2 v, int tile, float& inv) -> uint32_t {
+        // |<codeword, x_chunk>| <= norm * |x_chunk| < 2^(jx + 1) * 2^(13 - jx) = 2^14: every entry fits 16 bits with room to spare
+        const int jx = tile >= ntile1 ? mm.book_exp2 : mm.book_exp;
+        const float va = x_val(v.x), vb = x_val(v.y);
         float me = fmaxf(fabsf(va), fabsf(vb));          // largest element of the tile: a first scale, so that squares cannot overflow
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) me = fmaxf(me, __shfl_xor_sync(0xffffffffu, me, o));
@@ -279,9 +225,33 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
         // a NaN or infinity among the tile's activations must reach every output, as it would in a matrix product
         const bool nonfinite = __any_sync(0xffffffffu, !(fabsf(va) <= 3.0e38f) || !(fabsf(vb) <= 3.0e38f));
         const float sc = l8_pow2(-k);
+        inv = nonfinite ? __int_as_float(0x7fc00000) : l8_pow2(k);
         const __half2 xh = __floats2half2_rn(va * sc, vb * sc);
-        const uint32_t b0 = *(const uint32_t*)&xh;
-        const uint32_t a0 = tbl + (uint32_t)g * 16u + (uint32_t)t * 4u + (uint32_t)warp * 512u;
+        return *(const uint32_t*)&xh;
+    };
+    // Every warp needs every tile's fragment, but the loads and the reductions behind one are a long chain: each warp
+    // prepares one tile of the next 16 ahead of time, and a build reads the result from shared memory.
+    uint32_t* s_x = (uint32_t*)(l8_smem + 2 * L8_TABLE_BYTES);
+    auto stage_x = [&](uint2 v, int j) {                // tile j of this block -> slot j mod L8_XSLOTS
+        float inv;
+        const uint32_t b = scaled(v, tile_lo + j, inv);
+        s_x[(j & (L8_XSLOTS - 1)) * 32 + lane] = b;
+        if (lane == 0) s_inv[j & (L8_XSLOTS - 1)] = inv;
+    };
+    const int2 at0 = x_place(tile_lo);
+    const bool own = 1 + warp < ntl;
+    const int2 at1 = own ? x_place(tile_lo + 1 + warp) : make_int2(-1, -1);
+
+    asm volatile("griddepcontrol.wait;" ::: "memory");              // x, accumulators and outputs belong to earlier kernels until here
+    const uint2 x0 = x_bits(at0);
+    uint2 xn = x_bits(at1);
+    float* fsum = P.fsum[mi];
+    if (P.calls && fsum) fsum += (int64_t)((__ldcg(P.calls) + 1u) & 1u) * P.fsum_stride;
+    pin_book();
+
+    // ---- table build: 16 codeword blocks per warp against the tile's 64 activations
+    auto build = [&](uint32_t tbl, uint32_t b0) {
+        const uint32_t a0 = cbl_smem_u32(l8_smem) + tbl + (uint32_t)g * 16u + (uint32_t)t * 4u + (uint32_t)warp * 512u;
         // four products in flight at a time (their latencies overlap), then the eight stores of the group
 #pragma unroll
         for (int i = 0; i < 8; i += 2) {
@@ -300,108 +270,66 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
                 l8_sts32(a + 128u, hi);
             }
         }
-        return nonfinite ? __int_as_float(0x7fc00000) : l8_pow2(k);
     };
-
-    uint32_t col[8];
+    float inv_cur, inv_nxt = 0.f;
+    build(0u, scaled(x0, tile_lo, inv_cur));
+    if (own) stage_x(xn, 1 + warp);
+    uint32_t col[8];                                    // table (bit 16) | 2 * column of slot s for this lane
 #pragma unroll
-    for (int s = 0; s < 8; s++) col[s] = tbl0 | (uint32_t)(((s + lane) & 7) << 1);
-
-    float inv_cur = build(tbl0, xa, xb), inv_nxt = 0.f;
-    if (ntl > 1) load_x(tile_lo + 1, xa, xb);
-
+    for (int s = 0; s < 8; s++) col[s] = (uint32_t)(((s + lane) & 7) << 1);
     l8_sync_block();                                // the first table is complete
 
-    // ---- main loop over the ring iterations.  Warps run through the ring on their own; the tags of iteration i + 1
-    // are fetched from the ring before the lookups of iteration i; a row's fp32 sum lives in shared memory between
-    // tiles (each row belongs to one thread).  After a wait has expired the loop only keeps its shape (it contains
-    // barriers) and does no more work.
-    const int half = warp / L8_STAGE_WARPS, tih = tid - half * (L8_NT / 2);    // this thread's half step and index in it
-    int cstage = half, kf = 0, cn = half;              // ring slot, row step and stage number of the next fetch
-    uint32_t cphase = 0;
-    bool dead = false;
-    uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0, w2 = w0;
-    auto fetch = [&]() {                                // tags of the next ring iteration (row step kf) -> w0..w2
-        if (!dead && !l8_mbar_wait(bar0 + 8 * cstage, cphase)) { s_abort = 1; dead = true; }
-        w0 = w1 = w2 = make_uint4(0, 0, 0, 0);
-        if (!dead && kf * L8_STEP_ROWS + 4 * tid < nrows) {
-            const uint32_t a = stage_addr(cstage) + (uint32_t)tih * 16u;
-            w0 = cbl_lds128(a);
-            w1 = cbl_lds128(a + L8_STAGE_ROWS * 4);
-            w2 = cbl_lds128(a + 2 * L8_STAGE_ROWS * 4);
-        }
-        __syncwarp();
-        // the last of the stage's readers refills its slot with the stage S further on
-        unsigned int last = 0;
-        if (lane == 0 && atomicAdd(&s_readers[cstage], 1u) == L8_STAGE_WARPS - 1) {
-            atomicExch(&s_readers[cstage], 0u);
-            last = 1;
-        }
-        if (__shfl_sync(0xffffffffu, last, 0) && cn + S < 2 * nit && !dead) issue(cn + S);
-        cn += 2;
-        cstage += 2;
-        if (cstage >= S) { cstage -= S; cphase ^= 1u; }
-        if (++kf == nrow_it) kf = 0;
-    };
-    fetch();
+    // ---- main loop.  The next tile's table goes into the other buffer while this tile is looked up: one half of the warps
+    // builds its share before its lookups of the tile, the other half after them, so that at any time some warps keep the
+    // shared-memory pipe busy with lookups while others run the tensor-core products of the build.
+    const int half = warp / (L8_NWARP / 2);
     float acc[2][4];                                    // this thread's 4 rows of row step 0 and of row step 1
 #pragma unroll
     for (int u = 0; u < 4; u++) acc[0][u] = acc[1][u] = 0.f;
     int k = 0, ti = 0;
-    for (int it = 0; it < nit; it++) {
-        // The next tile's table goes into the other buffer while this tile is looked up: one half of the warps builds
-        // its share before its lookups of the tile, the other half after them, so that at any time some warps keep the
-        // shared-memory pipe busy with lookups while others run the tensor-core products of the build.
-        const bool build_now = ti + 1 < ntl && (half == 0 ? k == 0 : k == nrow_it - 1);
-        if (build_now && half == 0) {
-            const int nb = (tile_lo + ti + 1) / ntile1;
-            if (nb != cur_book) set_book(nb);
-            inv_nxt = build(tbl0 + (uint32_t)(((ti + 1) & 1) << 16), xa, xb);
-            if (ti + 2 < ntl) load_x(tile_lo + ti + 2, xa, xb);
+    auto build_next = [&]() {                           // this warp's share of tile ti + 1
+        const int j = ti + 1, nb = tile_lo + j >= ntile1;
+        if (nb != cur_book) {
+            set_book(nb);
+            cur_book = nb;
         }
-        const uint4 c0 = w0, c1 = w1, c2 = w2;
-        dead = dead || *(volatile int*)&s_abort != 0;
-        const bool act = !dead && k * L8_STEP_ROWS + 4 * tid < nrows;
-        if (it + 1 < nit) fetch();
-        if (act) {
-            const float r0 = (float)l8_row8(c0.x, c1.x, c2.x, col) * inv_cur, r1 = (float)l8_row8(c0.y, c1.y, c2.y, col) * inv_cur;
-            const float r2 = (float)l8_row8(c0.z, c1.z, c2.z, col) * inv_cur, r3 = (float)l8_row8(c0.w, c1.w, c2.w, col) * inv_cur;
+        pin_book();
+        inv_nxt = s_inv[j & (L8_XSLOTS - 1)];
+        build((uint32_t)(j & 1) * L8_TABLE_BYTES, s_x[(j & (L8_XSLOTS - 1)) * 32 + lane]);
+    };
+    auto step = [&](uint4 (&w)[3], int it) {
+        const bool build_now = ti + 1 < ntl && (half == 0 ? k == 0 : k == nrow_it - 1);
+        if (build_now && half == 0) build_next();
+        const uint4 c0 = w[0], c1 = w[1], c2 = w[2];
+        fetch(w, it + 2);
+        if (k * L8_STEP_ROWS + 4 * tid < nrows) {
+            const float r0 = (float)l8_row8(l8_smem, c0.x, c1.x, c2.x, col) * inv_cur, r1 = (float)l8_row8(l8_smem, c0.y, c1.y, c2.y, col) * inv_cur;
+            const float r2 = (float)l8_row8(l8_smem, c0.z, c1.z, c2.z, col) * inv_cur, r3 = (float)l8_row8(l8_smem, c0.w, c1.w, c2.w, col) * inv_cur;
             if (k == 0) { acc[0][0] += r0; acc[0][1] += r1; acc[0][2] += r2; acc[0][3] += r3; }
             else { acc[1][0] += r0; acc[1][1] += r1; acc[1][2] += r2; acc[1][3] += r3; }
         }
-        if (build_now && half == 1) {
-            const int nb = (tile_lo + ti + 1) / ntile1;
-            if (nb != cur_book) set_book(nb);
-            inv_nxt = build(tbl0 + (uint32_t)(((ti + 1) & 1) << 16), xa, xb);
-            if (ti + 2 < ntl) load_x(tile_lo + ti + 2, xa, xb);
-        }
+        if (build_now && half == 1) build_next();
         if (++k == nrow_it) {
+            // the activations of the 16 tiles after the staged ones: asked for one tile before they are prepared, prepared
+            // one tile before the first of them is read (the slots written are not the one read meanwhile)
+            if ((ti & 15) == 14 && ti + 3 + warp < ntl) xn = x_bits(x_place(tile_lo + ti + 3 + warp));
+            if ((ti & 15) == 15 && ti + 2 + warp < ntl) stage_x(xn, ti + 2 + warp);
             k = 0;
             ti++;
-            const uint32_t tn = tbl0 + (uint32_t)((ti & 1) << 16);
 #pragma unroll
-            for (int s = 0; s < 8; s++) col[s] = (col[s] & 0xFFFFu) | tn;
+            for (int s = 0; s < 8; s++) col[s] ^= L8_TABLE_BYTES;
             inv_cur = inv_nxt;
             l8_sync_block();                        // next table complete; every reader of this one is done
         }
+    };
+    for (int it = 0; it < nit; it += 2) {
+        step(wa, it);
+        if (it + 1 < nit) step(wb, it + 1);
     }
-    // The next kernel of the stream may become resident from here on.  (Not earlier: a block of this kernel fills its
-    // SM, so an early successor would be packed onto the few SMs this launch leaves free instead of spreading
+    // The next kernel of the stream may become resident from here on.  (Not earlier: a block of this kernel takes more than
+    // half of its SM, so an early successor would be packed onto the few SMs this launch leaves free instead of spreading
     // over the SMs as they empty.)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // the row sums go to shared memory, indexed by row of the block, for the output phase
-#pragma unroll
-    for (int kk = 0; kk < 2; kk++)
-        if (kk * L8_STEP_ROWS + 4 * tid < nrows)
-            asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(sacc + (uint32_t)(kk * L8_STEP_ROWS + 4 * tid) * 4u), "f"(acc[kk][0]),
-                         "f"(acc[kk][1]), "f"(acc[kk][2]), "f"(acc[kk][3])
-                         : "memory");
-    l8_sync_block();
-    if (*(volatile int*)&s_abort) {
-        // a staged copy never completed: report and leave (the waits that gave up were bounded)
-        if (tid == 0) atomicExch(P.status, 1u);
-        return;
-    }
 
     // ---- row sums -> outputs
     const int32_t* rix = mm.row_index;
@@ -422,23 +350,27 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
         if (P.mode == 0) put(r, v * __half2float(((const __half*)mm.row_scale)[r]));
         else fsum[r] = v;
     };
-    const int n512 = (nrows + L8_NT - 1) / L8_NT;
     if (splits <= 1) {
-        for (int j = 0; j < n512; j++) {
-            const int q = j * L8_NT + tid;
-            if (q >= nrows) break;
-            const int r = source_row(row_lo + q);
-            if (r >= 0) emit(r, __uint_as_float(l8_lds32(sacc + (uint32_t)q * 4u)));
-        }
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int q = kk * L8_STEP_ROWS + 4 * tid + u;
+                const int r = q < nrows ? source_row(row_lo + q) : -1;
+                if (r >= 0) emit(r, acc[kk][u]);
+            }
         return;
     }
-    // this block's partial sums -> its slot, each with its valid flag
+    // this block's partial sums -> its slot, each with its valid flag (16 bytes per store, indivisible by 8-byte words)
     unsigned long long* slot = P.partial + (size_t)blockIdx.x * L8_SLOT_ROWS;
-    for (int j = 0; j < n512; j++) {
-        const int q = j * L8_NT + tid;
-        if (q < nrows) __stcg(slot + q, (1ull << 32) | (unsigned long long)l8_lds32(sacc + (uint32_t)q * 4u));
-    }
-    l8_sync_block();                                // the row sums in shared memory have been read: the space is staging now
+#pragma unroll
+    for (int kk = 0; kk < 2; kk++)
+        if (kk * L8_STEP_ROWS + 4 * tid < nrows) {
+            unsigned long long* w = slot + kk * L8_STEP_ROWS + 4 * tid;
+#pragma unroll
+            for (int u = 0; u < 4; u += 2)
+                __stcg((uint4*)(w + u), make_uint4(__float_as_uint(acc[kk][u]), 1u, __float_as_uint(acc[kk][u + 1]), 1u));
+        }
     // every block sums its share of the part's rows over the splits: thread (row, group) adds the splits
     // group, group + G, ... in order, the groups are added in order through shared memory
     const int s_me = (int)blockIdx.x - first;
@@ -488,11 +420,11 @@ __global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant
         }
         if (G > 1) {
             l8_sync_block();                        // previous readers of the staging rows
-            if (grp < G) l8_sts32(sacc + (uint32_t)(grp * nqq + r) * 4u, __float_as_uint(sum));
+            if (grp < G) s_sum[grp * nqq + r] = sum;
             l8_sync_block();
             if (grp == 0) {
                 sum = 0.f;
-                for (int gq = 0; gq < G; gq++) sum += __uint_as_float(l8_lds32(sacc + (uint32_t)(gq * nqq + r) * 4u));
+                for (int gq = 0; gq < G; gq++) sum += s_sum[gq * nqq + r];
             }
         }
         if (grp == 0 && rr >= 0 && !late) {
@@ -787,7 +719,7 @@ static int launch_l8(L8Launch& P, const void* x, int xdtype, cudaStream_t st, in
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(plan.nblocks);
-    cfg.blockDim = dim3(L8_THREADS);
+    cfg.blockDim = dim3(L8_NT);
     cfg.dynamicSmemBytes = L8_DYN_SMEM;
     CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_l8, P, plan, x, xdtype));
     return cbl_check_launch();
