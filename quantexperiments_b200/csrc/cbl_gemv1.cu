@@ -5,11 +5,10 @@
 // once, as 16-bit integers with a power-of-two scale per tile (the scale comes from a Cauchy-Schwarz bound, so no
 // entry can saturate), into 64 KB of shared memory; after that every weight chunk (8 weights, 12 bits in HBM)
 // costs ONE 2-byte shared-memory read and half an integer add (three-input adds; a row's 8 entries sum exactly).  Two tables
-// alternate: while the block looks tile t up, its warps build tile t + 1, so only a block's first build
-// is exposed.  The tags of the block's rows stream through a ring of shared-memory stages filled by bulk
-// copies (cp.async.bulk + mbarrier, 8 stages = 96 KB in flight, started before the kernel waits for its
-// predecessor); nobody is the producer: the last warp to read a stage issues the copies that refill it.  A block owns a rectangle (rows x tiles) of one matrix; a thread owns up to 8 rows
-// of it and keeps their fp32 sums in registers over all the block's tiles.
+// alternate: while 16 warps look tile t up, 8 others build tile t + 1, so that only a block's first build (by the 16) is
+// exposed.  A block owns a rectangle (rows x tiles) of one matrix; a looking thread owns up to 8 rows of it, reads their
+// tags straight into registers two steps ahead (the first tiles are sent to L2 before the kernel waits for its
+// predecessor) and keeps their fp32 sums in registers over all the block's tiles.
 //
 // Row sums of blocks that share rows (different tile ranges) meet without atomics, fences or counters, and in a
 // FIXED order, so two runs agree bit for bit: every block stores its fp32 partial sums into its own slot of the
@@ -20,11 +19,18 @@
 // trips after the last lookup.  (All blocks of a launch are resident at once - one block per SM, at most as many
 // blocks as SMs - so the poll cannot starve the block it waits for.)
 //
-// Shared-memory gathers bound this kernel, not HBM: a warp's 32 random 2-byte reads take as many cycles
-// as the most loaded bank has requests, 3.3 on average.  Per lane the column it reads rotates with the lane
-// index ((slot + row position / 4) mod 8; the tags are stored in that rotated order), which keeps same-column lanes from
-// piling on the few banks one column's entries occupy.  A thread takes 4 consecutive rows per step (one 16-byte
-// read per tag plane, 32 independent table reads in flight): the loop is bound by latency, not by issue slots.
+// Shared-memory gathers bound the loop, not HBM: a warp's 32 random 2-byte reads take as many cycles as the most
+// loaded bank has requests, 3.3 on average: 1690 clocks per 2048 rows and tile, 690 without conflicts.  Per lane the
+// column it reads rotates with the lane index ((slot + row position / 4) mod 8; the tags are stored in that rotated order),
+// which keeps same-column lanes from piling on the few banks one column's entries occupy.  A thread takes 4 consecutive rows
+// per step (one 16-byte read per tag plane, 32 independent table reads in flight).  A build takes about 1450 clocks beside
+// the lookups (256 products of 2.5 clocks at best, 512 clocks of stores), which is what bounds blocks of fewer than 1700 rows.
+//
+// Measured (activations and result in global memory, one launch after the other): 18944 x 3584 10.5 us, the gate|up pair
+// 15.6, 3584 x 18944 11.3, 512 x 3584 4.8, 27648 x 5120 with two books and 16 column orders 34.4.  With a ring of bulk copies
+// for the tags and every warp both building and looking up, the book's fragments loaded again in every build, those were
+// 13.3, 21.1, 13.1, 6.0 and 58.8; without the separate builders 11.6, 16.4, 11.8, 4.8 and 36.1.  Four builders
+// take 10.4 us for the first but 43.5 for the last.
 #include <map>
 #include <mutex>
 #include <vector>
@@ -33,12 +39,19 @@
 
 constexpr int L8_NT = 512;                       // threads per block; a thread handles 4 consecutive rows per ring stage
 constexpr int L8_NWARP = L8_NT / 32;
+constexpr int L8_BUILDERS = 8;                   // warps that build the tables after the first
+constexpr int L8_FRAGS = 128 / L8_BUILDERS;      // pairs of 16 codewords that one of them holds
+constexpr int L8_THREADS = L8_NT + 32 * L8_BUILDERS;
+constexpr int L8_REGS_LAUNCH = 80, L8_REGS_LOOK = 72, L8_REGS_BUILD = 96;   // registers per thread: at launch, and as the roles share them
+static_assert(L8_THREADS * L8_REGS_LAUNCH >= L8_NT * L8_REGS_LOOK + 32 * L8_BUILDERS * L8_REGS_BUILD, "registers of the block");
+constexpr int L8_PIPE = 2;                       // pairs of 16 codewords whose products a builder has in flight
 constexpr int L8_RPT = 8;                        // rows per thread: a block covers at most 4096 rows
 constexpr int L8_STEP_ROWS = 4 * L8_NT;           // 2048 rows per step of the block
 constexpr int L8_TABLE_BYTES = 65536;            // table of one tile: 4096 entries x 8 columns x 2 bytes
-constexpr int L8_XSLOTS = 32;                    // tiles whose scaled activations are staged
+constexpr int L8_XSLOTS = 2 * L8_BUILDERS;       // tiles whose scaled activations are staged
 constexpr int L8_DYN_SMEM = 2 * L8_TABLE_BYTES + L8_XSLOTS * 128;
 constexpr int L8_AHEAD = 4;                      // tiles of a block whose tags are sent to L2 before the predecessor is waited for
+constexpr int L8_MEET = 10;                      // partial sums of a row that one thread has in flight
 constexpr int L8_MAX_GROUP = 4;
 constexpr int L8_MAX_BLOCKS = 160;
 constexpr int L8_MAX_ORDERS = 16;
@@ -117,15 +130,19 @@ struct L8Plan {
                              // w = tile_lo | tile_hi << 16; the blocks of a part are consecutive, in split order
 };
 
-// Barrier among the block's 512 threads.
+// Named barriers of a block: 1 = the 512 looking threads, 2 = the builders, 3 and 4 = table 0, 1 is complete (builders arrive,
+// the others wait), 5 and 6 = table 0, 1 has been read (the other way round).
+__device__ __forceinline__ void l8_bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(L8_THREADS) : "memory"); }
+__device__ __forceinline__ void l8_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(L8_THREADS) : "memory"); }
 __device__ __forceinline__ void l8_sync_block() { asm volatile("bar.sync 1, %0;" ::"n"(L8_NT) : "memory"); }
 
-__global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8Launch P, const __grid_constant__ L8Plan plan,
-                                                      const void* __restrict__ x, int xdtype) {
-    extern __shared__ __align__(128) unsigned char l8_smem[];              // two 64 KB tables | scaled activations of 32 tiles
+__global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant__ L8Launch P, const __grid_constant__ L8Plan plan,
+                                                           const void* __restrict__ x, int xdtype) {
+    extern __shared__ __align__(128) unsigned char l8_smem[];              // two 64 KB tables | scaled activations of the builders' next tiles
     __shared__ float s_inv[L8_XSLOTS];                                      // factor that undoes a tile's scale
+    __shared__ float s_tinv[2];                                             // the same, of the tile in a table
     __shared__ float s_sum[L8_NT];                                          // sums of the groups of splits (output phase)
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int g = lane >> 2, t = lane & 3;
     if ((int)blockIdx.x >= plan.nblocks) return;
     const int4 d = plan.r[blockIdx.x];
@@ -138,46 +155,8 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
     const int ntl = tile_hi - tile_lo;
     const int nit = ntl * nrow_it;                     // iterations of this block: (tile, row step), tile-major
 
-    // ---- tags: 16 bytes per plane and step of this thread's four rows, asked for two iterations ahead.  Weights do not
-    // depend on the previous kernel: the first two iterations are requested here, what follows is sent on its way to L2.
-    const uint32_t* tags = (const uint32_t*)mm.words + (int64_t)tile_lo * 3 * mm.Rpad + row_lo + 4 * tid;
-    const int64_t plane = mm.Rpad;
-    auto fetch = [&](uint4 (&w)[3], int it) {
-        const int ti = nrow_it == 2 ? it >> 1 : it, r0 = (it - ti * nrow_it) * L8_STEP_ROWS;
-        if (it < nit && r0 + 4 * tid < nrows) {
-            const uint32_t* p = tags + (int64_t)ti * 3 * plane + r0;
-            w[0] = l8_ldg128(p);
-            w[1] = l8_ldg128(p + plane);
-            w[2] = l8_ldg128(p + 2 * plane);
-        }
-    };
-    uint4 wa[3], wb[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) wa[i] = wb[i] = make_uint4(0, 0, 0, 0);
-    fetch(wa, 0);
-    fetch(wb, 1);
-    if (tid < 3 * (L8_AHEAD < ntl ? L8_AHEAD : ntl))
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const uint32_t*)mm.words + ((int64_t)tile_lo * 3 + tid) * plane + row_lo),
-                     "r"(4 * nrows)
-                     : "memory");
-
-    // ---- tables.  The book's mma A fragments stay in registers for all tiles of a book (one 16-byte load per two
-    // 16-codeword blocks); everything that does not depend on the previous kernel is requested before the wait.
     const int ntile1 = mm.ntile / mm.books;
-    uint4 af[8];
-    auto set_book = [&](int book) {
-        const uint4* fr = (const uint4*)(book ? mm.frag2 : mm.frag);
-#pragma unroll
-        for (int i = 0; i < 8; i++) af[i] = __ldg(fr + (warp + i * L8_NWARP) * 32 + lane);
-    };
-    // The values pass through an empty asm, so that the compiler keeps them in registers: left alone it loads them again,
-    // from L2, inside every build.
-    auto pin_book = [&]() {
-#pragma unroll
-        for (int i = 0; i < 8; i++) asm volatile("" : "+r"(af[i].x), "+r"(af[i].y), "+r"(af[i].z), "+r"(af[i].w));
-    };
-    int cur_book = tile_lo >= ntile1;
-    set_book(cur_book);
+    const int64_t plane = mm.Rpad;
 
     // ---- activations of a tile: lane (g, t) holds elements 2 lane, 2 lane + 1, the B fragment of the build (k = 2t, 2t + 1 of
     // chunk column g).  Where they stand comes from the column order; the bits are converted only where they are used, so that
@@ -229,77 +208,132 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
         const __half2 xh = __floats2half2_rn(va * sc, vb * sc);
         return *(const uint32_t*)&xh;
     };
-    // Every warp needs every tile's fragment, but the loads and the reductions behind one are a long chain: each warp
-    // prepares one tile of the next 16 ahead of time, and a build reads the result from shared memory.
-    uint32_t* s_x = (uint32_t*)(l8_smem + 2 * L8_TABLE_BYTES);
-    auto stage_x = [&](uint2 v, int j) {                // tile j of this block -> slot j mod L8_XSLOTS
-        float inv;
-        const uint32_t b = scaled(v, tile_lo + j, inv);
-        s_x[(j & (L8_XSLOTS - 1)) * 32 + lane] = b;
-        if (lane == 0) s_inv[j & (L8_XSLOTS - 1)] = inv;
+    // products of 32 codewords (two blocks of 16) with a tile's activations, and their way into the table as integers
+    auto mul = [&](float (&c)[2][4], const uint4& f, uint32_t b0) {
+        l8_mma1688(c[0], f.x, f.y, b0);
+        l8_mma1688(c[1], f.z, f.w, b0);
     };
-    const int2 at0 = x_place(tile_lo);
-    const bool own = 1 + warp < ntl;
-    const int2 at1 = own ? x_place(tile_lo + 1 + warp) : make_int2(-1, -1);
-
-    asm volatile("griddepcontrol.wait;" ::: "memory");              // x, accumulators and outputs belong to earlier kernels until here
-    const uint2 x0 = x_bits(at0);
-    uint2 xn = x_bits(at1);
-    float* fsum = P.fsum[mi];
-    if (P.calls && fsum) fsum += (int64_t)((__ldcg(P.calls) + 1u) & 1u) * P.fsum_stride;
-    pin_book();
-
-    // ---- table build: 16 codeword blocks per warp against the tile's 64 activations
-    auto build = [&](uint32_t tbl, uint32_t b0) {
-        const uint32_t a0 = cbl_smem_u32(l8_smem) + tbl + (uint32_t)g * 16u + (uint32_t)t * 4u + (uint32_t)warp * 512u;
-        // four products in flight at a time (their latencies overlap), then the eight stores of the group
+    auto put_table = [&](const float (&c)[2][4], uint32_t a) {
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            float c[4][4];
-            l8_mma1688(c[0], af[i].x, af[i].y, b0);
-            l8_mma1688(c[1], af[i].z, af[i].w, b0);
-            l8_mma1688(c[2], af[i + 1].x, af[i + 1].y, b0);
-            l8_mma1688(c[3], af[i + 1].z, af[i + 1].w, b0);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                // round to integer by adding 1.5 * 2^23: the low 16 bits of the sum's pattern are the two's-complement value
-                const uint32_t lo = __byte_perm(__float_as_uint(c[q][0] + 12582912.f), __float_as_uint(c[q][1] + 12582912.f), 0x5410);
-                const uint32_t hi = __byte_perm(__float_as_uint(c[q][2] + 12582912.f), __float_as_uint(c[q][3] + 12582912.f), 0x5410);
-                const uint32_t a = a0 + (uint32_t)((i + (q >> 1)) * L8_NWARP * 512 + (q & 1) * 256);   // codeword block ((warp + 16 i') * 2 + h) * 16
-                l8_sts32(a, lo);
-                l8_sts32(a + 128u, hi);
-            }
+        for (int q = 0; q < 2; q++) {
+            // round to integer by adding 1.5 * 2^23: the low 16 bits of the sum's pattern are the two's-complement value
+            const uint32_t lo = __byte_perm(__float_as_uint(c[q][0] + 12582912.f), __float_as_uint(c[q][1] + 12582912.f), 0x5410);
+            const uint32_t hi = __byte_perm(__float_as_uint(c[q][2] + 12582912.f), __float_as_uint(c[q][3] + 12582912.f), 0x5410);
+            l8_sts32(a + (uint32_t)q * 256u, lo);
+            l8_sts32(a + (uint32_t)q * 256u + 128u, hi);
         }
     };
-    float inv_cur, inv_nxt = 0.f;
-    build(0u, scaled(x0, tile_lo, inv_cur));
-    if (own) stage_x(xn, 1 + warp);
+    const uint32_t sbase = cbl_smem_u32(l8_smem) + (uint32_t)g * 16u + (uint32_t)t * 4u;
+
+    if (warp >= L8_NWARP) {
+        // ======== builders: the tables of the tiles after the first, each while the one before it is looked up.  A warp's share of
+        // the book stays in registers; its products are issued L8_PIPE pairs ahead of the stores, since one takes 47 clocks.
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L8_REGS_BUILD));
+        const int bw = warp - L8_NWARP;
+        uint32_t* s_x = (uint32_t*)(l8_smem + 2 * L8_TABLE_BYTES);
+        uint4 af[L8_FRAGS];
+        auto set_book = [&](int book) {
+            const uint4* fr = (const uint4*)(book ? mm.frag2 : mm.frag);
+#pragma unroll
+            for (int i = 0; i < L8_FRAGS; i++) af[i] = __ldg(fr + (bw + i * L8_BUILDERS) * 32 + lane);
+        };
+        int cur_book = tile_lo + 1 >= ntile1;
+        if (ntl > 1) set_book(cur_book);
+        const int2 at = 1 + bw < ntl ? x_place(tile_lo + 1 + bw) : make_int2(-1, -1);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint2 xn = x_bits(at);
+        for (int j = 1; j < ntl; j++) {
+            if (((j - 1) & (L8_BUILDERS - 1)) == 0) {
+                // the loads and the reductions behind a tile's activations are a long chain: each warp prepares one of the next
+                // L8_BUILDERS tiles, and asks for the one after it
+                if (j + bw < ntl) {
+                    float inv;
+                    const int slot = (j + bw) & (L8_XSLOTS - 1);
+                    s_x[slot * 32 + lane] = scaled(xn, tile_lo + j + bw, inv);
+                    if (lane == 0) s_inv[slot] = inv;
+                }
+                if (j + L8_BUILDERS + bw < ntl) xn = x_bits(x_place(tile_lo + j + L8_BUILDERS + bw));
+                asm volatile("bar.sync 2, %0;" ::"n"(32 * L8_BUILDERS) : "memory");
+            }
+            const int nb = tile_lo + j >= ntile1;
+            if (nb != cur_book) {
+                set_book(nb);
+                cur_book = nb;
+            }
+            // the values pass through an empty asm, so that the compiler keeps them in registers: left alone it loads them again,
+            // from L2, inside every build
+#pragma unroll
+            for (int i = 0; i < L8_FRAGS; i++) asm volatile("" : "+r"(af[i].x), "+r"(af[i].y), "+r"(af[i].z), "+r"(af[i].w));
+            const uint32_t b0 = s_x[(j & (L8_XSLOTS - 1)) * 32 + lane];
+            float c[L8_PIPE][2][4];
+#pragma unroll
+            for (int i = 0; i < L8_PIPE; i++) mul(c[i], af[i], b0);
+            if (j >= 2) l8_bar_sync(5 + (j & 1));
+            if (bw == 0 && lane == 0) s_tinv[j & 1] = s_inv[j & (L8_XSLOTS - 1)];
+            const uint32_t a = sbase + (uint32_t)(j & 1) * L8_TABLE_BYTES + (uint32_t)bw * 512u;
+#pragma unroll
+            for (int i = 0; i < L8_FRAGS; i++) {
+                put_table(c[i % L8_PIPE], a + (uint32_t)(i * L8_BUILDERS) * 512u);
+                if (i + L8_PIPE < L8_FRAGS) mul(c[i % L8_PIPE], af[i + L8_PIPE], b0);
+            }
+            l8_bar_arrive(3 + (j & 1));
+        }
+        return;
+    }
+
+    // ======== lookups
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L8_REGS_LOOK));
+    // tags: 16 bytes per plane and step of this thread's four rows, asked for two iterations ahead.  Weights do not
+    // depend on the previous kernel: the first tiles' are sent on their way to L2 before it is waited for.
+    const uint32_t* tags = (const uint32_t*)mm.words + (int64_t)tile_lo * 3 * mm.Rpad + row_lo + 4 * tid;
+    auto fetch = [&](uint4 (&w)[3], int it) {
+        const int ti = nrow_it == 2 ? it >> 1 : it, r0 = (it - ti * nrow_it) * L8_STEP_ROWS;
+        if (it < nit && r0 + 4 * tid < nrows) {
+            const uint32_t* p = tags + (int64_t)ti * 3 * plane + r0;
+            w[0] = l8_ldg128(p);
+            w[1] = l8_ldg128(p + plane);
+            w[2] = l8_ldg128(p + 2 * plane);
+        }
+    };
+    if (tid < 3 * (L8_AHEAD < ntl ? L8_AHEAD : ntl))
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const uint32_t*)mm.words + ((int64_t)tile_lo * 3 + tid) * plane + row_lo),
+                     "r"(4 * nrows)
+                     : "memory");
+    float inv_cur;
+    uint4 wa[3], wb[3];
+    {
+        // the first table, by all these warps: nothing can be looked up before it is there
+        uint4 af[8];
+        const uint4* fr = (const uint4*)(tile_lo >= ntile1 ? mm.frag2 : mm.frag);
+#pragma unroll
+        for (int i = 0; i < 8; i++) af[i] = __ldg(fr + (warp + i * L8_NWARP) * 32 + lane);
+        const int2 at = x_place(tile_lo);
+        asm volatile("griddepcontrol.wait;" ::: "memory");          // x, accumulators and outputs belong to earlier kernels until here
+        const uint2 xv = x_bits(at);
+#pragma unroll
+        for (int i = 0; i < 3; i++) wa[i] = wb[i] = make_uint4(0, 0, 0, 0);
+        fetch(wa, 0);
+        const uint32_t b0 = scaled(xv, tile_lo, inv_cur);
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            float c[2][2][4];
+            mul(c[0], af[i], b0);
+            mul(c[1], af[i + 1], b0);
+            put_table(c[0], sbase + (uint32_t)(warp + i * L8_NWARP) * 512u);
+            put_table(c[1], sbase + (uint32_t)(warp + (i + 1) * L8_NWARP) * 512u);
+        }
+        fetch(wb, 1);
+    }
     uint32_t col[8];                                    // table (bit 16) | 2 * column of slot s for this lane
 #pragma unroll
     for (int s = 0; s < 8; s++) col[s] = (uint32_t)(((s + lane) & 7) << 1);
     l8_sync_block();                                // the first table is complete
 
-    // ---- main loop.  The next tile's table goes into the other buffer while this tile is looked up: one half of the warps
-    // builds its share before its lookups of the tile, the other half after them, so that at any time some warps keep the
-    // shared-memory pipe busy with lookups while others run the tensor-core products of the build.
-    const int half = warp / (L8_NWARP / 2);
     float acc[2][4];                                    // this thread's 4 rows of row step 0 and of row step 1
 #pragma unroll
     for (int u = 0; u < 4; u++) acc[0][u] = acc[1][u] = 0.f;
     int k = 0, ti = 0;
-    auto build_next = [&]() {                           // this warp's share of tile ti + 1
-        const int j = ti + 1, nb = tile_lo + j >= ntile1;
-        if (nb != cur_book) {
-            set_book(nb);
-            cur_book = nb;
-        }
-        pin_book();
-        inv_nxt = s_inv[j & (L8_XSLOTS - 1)];
-        build((uint32_t)(j & 1) * L8_TABLE_BYTES, s_x[(j & (L8_XSLOTS - 1)) * 32 + lane]);
-    };
     auto step = [&](uint4 (&w)[3], int it) {
-        const bool build_now = ti + 1 < ntl && (half == 0 ? k == 0 : k == nrow_it - 1);
-        if (build_now && half == 0) build_next();
         const uint4 c0 = w[0], c1 = w[1], c2 = w[2];
         fetch(w, it + 2);
         if (k * L8_STEP_ROWS + 4 * tid < nrows) {
@@ -308,18 +342,15 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
             if (k == 0) { acc[0][0] += r0; acc[0][1] += r1; acc[0][2] += r2; acc[0][3] += r3; }
             else { acc[1][0] += r0; acc[1][1] += r1; acc[1][2] += r2; acc[1][3] += r3; }
         }
-        if (build_now && half == 1) build_next();
         if (++k == nrow_it) {
-            // the activations of the 16 tiles after the staged ones: asked for one tile before they are prepared, prepared
-            // one tile before the first of them is read (the slots written are not the one read meanwhile)
-            if ((ti & 15) == 14 && ti + 3 + warp < ntl) xn = x_bits(x_place(tile_lo + ti + 3 + warp));
-            if ((ti & 15) == 15 && ti + 2 + warp < ntl) stage_x(xn, ti + 2 + warp);
             k = 0;
-            ti++;
+            if (ti + 2 < ntl) l8_bar_arrive(5 + (ti & 1));
+            if (++ti < ntl) {
 #pragma unroll
-            for (int s = 0; s < 8; s++) col[s] ^= L8_TABLE_BYTES;
-            inv_cur = inv_nxt;
-            l8_sync_block();                        // next table complete; every reader of this one is done
+                for (int s = 0; s < 8; s++) col[s] ^= L8_TABLE_BYTES;
+                l8_bar_sync(3 + (ti & 1));
+                inv_cur = s_tinv[ti & 1];
+            }
         }
     };
     for (int it = 0; it < nit; it += 2) {
@@ -332,6 +363,8 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---- row sums -> outputs
+    float* fsum = P.fsum[mi];
+    if (P.calls && fsum) fsum += (int64_t)((__ldcg(P.calls) + 1u) & 1u) * P.fsum_stride;
     const int32_t* rix = mm.row_index;
     auto source_row = [&](int p) {                      // source row of row position p, -1 for padding
         const int r = rix ? rix[p] : p;
@@ -374,7 +407,7 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
     // every block sums its share of the part's rows over the splits: thread (row, group) adds the splits
     // group, group + G, ... in order, the groups are added in order through shared memory
     const int s_me = (int)blockIdx.x - first;
-    const int q_lo = (int)((int64_t)nrows * s_me / splits), q_hi = (int)((int64_t)nrows * (s_me + 1) / splits);
+    const int q_lo = nrows * s_me / splits, q_hi = nrows * (s_me + 1) / splits;
     const int nq = q_hi - q_lo;
     unsigned long long* slots = P.partial + (size_t)first * L8_SLOT_ROWS;
     bool late = false;
@@ -393,19 +426,19 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
         float sum = 0.f;
         if (grp < G) {
             unsigned long long* src = slots + q_lo + q0 + r;
-            for (int j0 = grp; j0 < splits; j0 += 8 * G) {
-                float v[8];
+            for (int j0 = grp; j0 < splits; j0 += L8_MEET * G) {
+                float v[L8_MEET];
                 uint32_t need = 0;
 #pragma unroll
-                for (int u = 0; u < 8; u++)
+                for (int u = 0; u < L8_MEET; u++)
                     if (j0 + u * G < splits) need |= 1u << u;
                 for (uint32_t poll = 0; need && poll < L8_MEET_LIMIT; poll++) {
-                    unsigned long long w[8];
+                    unsigned long long w[L8_MEET];
 #pragma unroll
-                    for (int u = 0; u < 8; u++)
+                    for (int u = 0; u < L8_MEET; u++)
                         if (need >> u & 1u) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w[u]) : "l"(src + (size_t)(j0 + u * G) * L8_SLOT_ROWS) : "memory");
 #pragma unroll
-                    for (int u = 0; u < 8; u++)
+                    for (int u = 0; u < L8_MEET; u++)
                         if ((need >> u & 1u) && (w[u] >> 32)) {
                             v[u] = __uint_as_float((uint32_t)w[u]);
                             need &= ~(1u << u);
@@ -414,7 +447,7 @@ __global__ void __launch_bounds__(L8_NT, 1) k_gemv_l8(const __grid_constant__ L8
                 }
                 if (need) late = true;
 #pragma unroll
-                for (int u = 0; u < 8; u++)
+                for (int u = 0; u < L8_MEET; u++)
                     if (j0 + u * G < splits) sum += v[u];
             }
         }
@@ -697,6 +730,10 @@ static int launch_l8(L8Launch& P, const void* x, int xdtype, cudaStream_t st, in
         std::lock_guard<std::mutex> lock(mu);
         if (!attr_set[dev]) {
             CBL_CUDA(cudaFuncSetAttribute(k_gemv_l8, cudaFuncAttributeMaxDynamicSharedMemorySize, L8_DYN_SMEM));
+            // the roles' registers come out of what the block is launched with: a build with fewer would wait for ever
+            cudaFuncAttributes fa;
+            CBL_CUDA(cudaFuncGetAttributes(&fa, k_gemv_l8));
+            if (fa.numRegs != L8_REGS_LAUNCH) return CBL_EUNSUPPORTED;
             attr_set[dev] = true;
         }
         auto it = cache.find(key);
@@ -719,7 +756,7 @@ static int launch_l8(L8Launch& P, const void* x, int xdtype, cudaStream_t st, in
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(plan.nblocks);
-    cfg.blockDim = dim3(L8_NT);
+    cfg.blockDim = dim3(L8_THREADS);
     cfg.dynamicSmemBytes = L8_DYN_SMEM;
     CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_l8, P, plan, x, xdtype));
     return cbl_check_launch();
