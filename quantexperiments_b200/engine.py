@@ -199,7 +199,10 @@ class DecodeEngine:
         self.graph = None
         self.only_linears = False
         # one token, one column order everywhere: the operator that follows a product runs on its fp32 sums (one small kernel)
-        self.fused = B == 1 and all(st.group is not None for S in self.stages for st in S.values()) and H <= lib.cbl_gemv_l8_add_norm_max_rows()
+        tables = B == 1 and all(st.group is not None for S in self.stages for st in S.values()) and H <= lib.cbl_gemv_l8_add_norm_max_rows()
+        plain = all(m.dm.M == 1 for S in self.stages for st in S.values() for m in st.stack.lins)
+        # the fused step, for matrices of one column order and of several (whose products read the same vectors)
+        self.fused, self.fused_orders = tables and plain, tables and not plain
 
     def _stages_inputs(self, n: int) -> bool:
         c = self.cfg
@@ -255,7 +258,7 @@ class DecodeEngine:
                 return
             s = _stream()
             self._embed(self.tok, B, self.h)
-            if self.fused:
+            if self.fused or self.fused_orders:
                 self._step_fused(s)
                 return
             add, sh, si = None, self.stage_h, self.stage_i

@@ -22,19 +22,30 @@ import torch
 from . import _cblhost, _lib
 from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix
 
-# One token, one column order: activation-side tables (L8Matrix) at every number of rows (64 x 3584: 5.8 us against 8.4 by
-# codeword gathers, 4096 x 3584: 6.8 against 10.1, 18944 x 3584: 13.2 against 14.5).  With several column orders every order
-# needs its own tables; those matrices gather codewords (B3Matrix) at every token count (5120 x 5120, 16 orders, two
-# books: 24 us against 47; 27648 x 5120: 55 against 59).  The rows per order from which the tables would still do are
-# what RowParallelLinear.attach() asks for.
-L8_MIN_ROWS = 1
-L8_MIN_ROWS_PER_ORDER = 1536
+# One token: activation-side tables (L8Matrix) at every number of rows with one column order (64 x 3584: 4.8 us against 8.4
+# by codeword gathers, 4096 x 3584: 6.6 against 10.1, 18944 x 3584: 10.5 against 14.5).  With several column orders
+# every order needs tables of its own, about 1 us each, L8_SMS of them at a time: they pay while a table serves enough rows.
+# Measured against the gathers, us: 512 x 3584 in 4 orders 6.1 / 12.7; 27648 x 5120, two books, 16 orders (17 tables per SM,
+# 1728 rows each) 34.4 / 54.6; 3584 x 18944 in 16 orders (32, 224 rows) 35.4 / 40.2; q|k|v of 3584, 16 orders (18, 96) 21.9 / 15.2;
+# 512 x 18944 in 16 orders (32, 32) 35.1 / 24.4; 8000 x 18944, two books, 16 orders (64, 500) 72.5 / 64.1.  Up to ten
+# tables per SM win at any number of rows; above, 16 rows per table and further table put all of these on the right side
+# or within 5 us of it.
+L8_SMS = 148
 # Tokens up to which the book lies three times in shared memory (the activations of more tokens need the room: two copies).
 B3_MAX_3COPIES = 16
 # Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM.
 DENSE_MIN_TOKENS = 129
 # counts loader.pool_layouts() calls: native plans made before one hold old addresses
 pool_epoch = 0
+
+
+def tables_pay(lins: list) -> bool:
+    """Whether one token of linears that read the same activations runs on the table-lookup kernel."""
+    orders = sum(l.dm.M for l in lins)
+    if all(l.dm.M == 1 for l in lins):
+        return True
+    builds = sum(l.dm.M * l.dm.books * -(-l.dm.nch // 8) for l in lins) / L8_SMS
+    return max(l.dm.M for l in lins) <= L8Matrix.MAX_ORDERS and orders <= L8_SMS and sum(l.R for l in lins) >= 16 * orders * (builds - 10)
 
 
 class PackedLinear(torch.nn.Module):
@@ -114,7 +125,7 @@ class PackedLinear(torch.nn.Module):
         self._host_bias = self.bias
         self._host = _cblhost.plan(dm.device.index, self.in_features, self.C, dm.M, [self.R], 0 if dm.perms is None else dm.perms.data_ptr(),
                                    DENSE_MIN_TOKENS, self.bias)
-        if self._l8 is not None and self.use_l8() and dm.M == 1:
+        if self._l8 is not None and self.use_l8():
             _cblhost.set(self._host, "l8", bytes(self._l8.struct()))
         for g in self._b3.values():
             _cblhost.set(self._host, "b3", bytes(g.mats[0].struct()))
@@ -123,11 +134,7 @@ class PackedLinear(torch.nn.Module):
 
     def use_l8(self) -> bool:
         """One token runs on the table-lookup kernel (any number of column orders up to its limit)."""
-        if not self.dm.fast:
-            return False
-        if self.dm.M == 1:
-            return self.R >= L8_MIN_ROWS
-        return self.dm.M <= L8Matrix.MAX_ORDERS and self.R >= L8_MIN_ROWS_PER_ORDER * self.dm.M
+        return self.dm.fast and not self.wide and tables_pay([self])
 
     def gemv(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x [C] (fp16 / bf16 / fp32, contiguous) -> y [R] in x's dtype (or `out`'s)."""
@@ -135,7 +142,7 @@ class PackedLinear(torch.nn.Module):
             y = out if out is not None else torch.empty(self.R, dtype=x.dtype, device=x.device)
             self.dm.gemv_generic(x.reshape(1, -1), y.reshape(1, -1))
             return y
-        if self.dm.M == 1 and self.use_l8():
+        if self.use_l8():
             return self.l8.run(x, out)
         y = out if out is not None else torch.empty(self.R, dtype=x.dtype, device=x.device)
         self.group(1).run(x.reshape(1, -1), [y.reshape(1, -1)])
@@ -156,7 +163,7 @@ class PackedLinear(torch.nn.Module):
             self.dm.gemv_generic(x2 if x2.stride(1) == 1 else x2.contiguous(), y)
             return y
         x2 = x2 if x2.stride(1) == 1 else x2.contiguous()
-        if n == 1 and self.dm.M == 1 and self.use_l8() and y.is_contiguous():
+        if n == 1 and self.use_l8() and y.is_contiguous():
             self.l8.run(x2[0], y[0])
         elif n < DENSE_MIN_TOKENS:
             self.group(n).run(x2, [y])
@@ -196,7 +203,7 @@ class Stack:
         p0 = lins[0].dm.perms
         self.shared = len(lins) <= B3Group.MAX and all(l.dm.fast and l.dm.M == lins[0].dm.M and (l.dm.perms is p0 or (
             p0 is not None and l.dm.perms is not None and torch.equal(l.dm.perms, p0))) for l in lins)
-        self.tables = all(l.dm.fast and l.dm.M == 1 for l in lins) and len(lins) <= L8Group.MAX
+        self.tables = all(l.dm.fast and not l.wide for l in lins) and len(lins) <= L8Group.MAX and tables_pay(lins)
         self.fast = all(l.dm.fast for l in lins)
         self.dense = DenseStack([l.dm for l in lins]) if self.fast and len({l.C for l in lins}) == 1 and not any(l.wide for l in lins) else None
         self._l8 = None

@@ -223,7 +223,7 @@ class RowParallelLinear:
             self.fused = PeerReduceGemv(self.l8_multi, arena)
             return
         if not self.lin.use_l8():
-            raise ValueError("the fused path runs matrices with at least 2048 rows")
+            raise ValueError("the fused path runs matrices in the table-lookup layout")
         self.fused = PeerReduceGemv(self.lin.l8, arena)
 
     def forward_fused(self, x: torch.Tensor, y: torch.Tensor | None = None) -> torch.Tensor:

@@ -254,6 +254,19 @@ def test_batch1_product_with_column_orders_matches_fp32_matmul(R, C, books, M):
     assert int(_l8_counters(l8_workspace(dm.device, R)).count_nonzero()) == 0
 
 
+@pytest.mark.parametrize("n,R,C,books", [(4, 100, 1088, 1), (4, 70, 2312, 2), (2, 66500, 136, 2)])
+def test_batch1_product_with_many_tiles_per_block(n, R, C, books):
+    """64 segments leave two blocks to each: 9 and 37 tiles per block, over the change of the book; two steps of rows per tile."""
+    from quantexperiments_b200.kernels import L8Group, L8Matrix
+    M = 16 if R < 1000 else 1
+    ms = [orc.synth_matrix(R, C, seed=R + C + i, books=books, M=M) for i in range(n)]
+    grp = L8Group([L8Matrix(_dm(m)) for m in ms])
+    x = torch.randn(C, generator=torch.Generator().manual_seed(C)).bfloat16()
+    ys = grp.run(x.cuda(), [torch.full((R,), float("nan"), device="cuda") for _ in ms])
+    for m, y in zip(ms, ys):
+        assert orc.max_rel_err(y.cpu().numpy(), orc.linear_ref(x.float().numpy()[None], orc.synth_decode(m))[0]) < TOL
+
+
 def test_batch1_product_is_bit_reproducible_and_flags_non_finite_inputs():
     """Blocks that share rows meet in integer accumulators, so the arrival order cannot change a bit: repeated
     calls and graph replays return identical outputs (the reference tests its ticket-ordered split-K the same way,
