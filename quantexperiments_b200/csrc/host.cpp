@@ -15,7 +15,10 @@
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/library.h>
 
 #include <map>
 #include <mutex>
@@ -273,14 +276,92 @@ PyObject* py_status(PyObject*, PyObject* args) {
     return PyLong_FromLong(bad);
 }
 
+// decode(packed descriptor, device, type code, first row, end row) -> dense [rows, C]
+PyObject* py_decode(PyObject*, PyObject* args) {
+    Py_buffer buf;
+    int device, dt, r0, r1;
+    if (!PyArg_ParseTuple(args, "y*iiii", &buf, &device, &dt, &r0, &r1)) return nullptr;
+    cbl_packed m;
+    const bool ok = buf.len == (Py_ssize_t)sizeof(m) && (dt == CBL_F32 || dt == CBL_F16 || dt == CBL_BF16);
+    if (ok) memcpy((void*)&m, buf.buf, sizeof(m));
+    PyBuffer_Release(&buf);
+    if (!ok) { PyErr_SetString(PyExc_ValueError, "wrong descriptor size or type"); return nullptr; }
+    try {
+        const at::Device dev(at::kCUDA, (c10::DeviceIndex)device);
+        const c10::cuda::OptionalCUDAGuard guard(dev);
+        const int64_t shape[2] = {r1 - r0, m.C};
+        at::Tensor y = at::detail::empty_cuda(c10::IntArrayRef(shape, 2), dt == CBL_F32 ? at::kFloat : dt == CBL_F16 ? at::kHalf : at::kBFloat16, dev, std::nullopt);
+        const int rc = cbl_dequant(&m, y.mutable_data_ptr(), dt, m.C, r0, r1, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream());
+        if (rc) return fail("cbl_dequant", rc);
+        return THPVariable_Wrap(std::move(y));
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+// ---- the torch operator shapequant::linear(x, handle): calls what set_linear() was given, a Python function of the same arguments
+PyObject* g_linear = nullptr;
+
+at::Tensor linear_op(const at::Tensor& x, int64_t handle) {
+    const PyGILState_STATE gil = PyGILState_Ensure();
+    PyObject* args[2] = {THPVariable_Wrap(x), PyLong_FromLongLong(handle)};
+    PyObject* y = g_linear && args[0] && args[1] ? PyObject_Vectorcall(g_linear, args, 2, nullptr) : nullptr;
+    Py_XDECREF(args[0]);
+    Py_XDECREF(args[1]);
+    at::Tensor out;
+    if (y && THPVariable_Check(y)) out = THPVariable_Unpack(y);
+    Py_XDECREF(y);
+    if (!out.defined()) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "shapequant::linear has no implementation or returned no tensor");
+        python_error e;
+        e.persist();
+        PyGILState_Release(gil);
+        throw e;
+    }
+    PyGILState_Release(gil);
+    return out;
+}
+
+// The operator is for inference: its result takes part in autograd, and a backward pass through it is an error.
+struct NoBackward : torch::autograd::Function<NoBackward> {
+    static at::Tensor forward(torch::autograd::AutogradContext*, const at::Tensor& x, int64_t handle) {
+        const at::AutoDispatchBelowADInplaceOrView guard;
+        return linear_op(x, handle);
+    }
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext*, const torch::autograd::variable_list&) {
+        TORCH_CHECK_NOT_IMPLEMENTED(false, "shapequant::linear has no backward");
+    }
+};
+
+at::Tensor linear_autograd(const at::Tensor& x, int64_t handle) {
+    if (x.requires_grad() && at::GradMode::is_enabled()) return NoBackward::apply(x, handle);
+    static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("shapequant::linear", "").typed<at::Tensor(const at::Tensor&, int64_t)>();
+    const at::AutoDispatchBelowADInplaceOrView guard;
+    return op.call(x, handle);
+}
+
+PyObject* py_set_linear(PyObject*, PyObject* fn) {
+    Py_INCREF(fn);
+    Py_XDECREF(g_linear);
+    g_linear = fn;
+    Py_RETURN_NONE;
+}
+
 PyMethodDef methods[] = {
     {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "forward(plan, x) -> y or None"},
     {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias)"},
     {"set", py_set, METH_VARARGS, "set(plan, kind, descriptors, row_scale=0)"},
+    {"decode", py_decode, METH_VARARGS, "decode(packed, device, dtype, first row, end row) -> dense rows"},
+    {"set_linear", py_set_linear, METH_O, "set_linear(fn): what shapequant::linear(x, handle) runs"},
     {"status", py_status, METH_VARARGS, "status(device) -> bits"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_cblhost", "native call path of the packed linears", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
+
+TORCH_LIBRARY_FRAGMENT(shapequant, m) { m.def("linear(Tensor x, int handle) -> Tensor", {at::Tag::pt2_compliant_tag}); }
+TORCH_LIBRARY_IMPL(shapequant, CompositeExplicitAutograd, m) { m.impl("linear", linear_op); }
+TORCH_LIBRARY_IMPL(shapequant, Autograd, m) { m.impl("linear", linear_autograd); }
 
 PyMODINIT_FUNC PyInit__cblhost(void) { return PyModule_Create(&module_def); }

@@ -16,7 +16,7 @@ import math
 import numpy as np
 import torch
 
-from . import _lib
+from . import _cblhost, _lib
 from ._lib import lib
 
 _DT = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
@@ -78,6 +78,7 @@ class DeviceMatrix:
         # A column shard (tensor parallelism) of a matrix with several column orders keeps orders that name positions
         # of the FULL activation vector: x_cols is that vector's length (None: the activations are C long).
         self.x_cols = None if x_cols is None or int(x_cols) == self.C else int(x_cols)
+        self._native = None                     # (addresses, descriptor bytes) of the native decode
         if self.x_cols is not None and (self.M == 1 or self.x_cols < self.C):
             raise ValueError("x_cols (wider activations than columns) needs several column orders and x_cols >= C")
 
@@ -109,6 +110,11 @@ class DeviceMatrix:
         r0, r1 = rows if rows is not None else (0, self.R)
         n = (r1 - r0) * self.C
         if out is None:
+            key = (self.tags.data_ptr(), self.table.data_ptr(), self.row_scale.data_ptr())
+            if self._native is None or self._native[0] != key:
+                self._native = (key, bytes(self.struct()))
+            if 0 <= r0 <= r1 <= self.R and dtype in _DT:
+                return _cblhost.decode(self._native[1], self.device.index, _DT[dtype], r0, r1)
             res = torch.empty(r1 - r0, self.C, dtype=dtype, device=self.device)
         else:
             if out.numel() < n or not out.is_contiguous() or out.device != self.device:

@@ -122,11 +122,15 @@ def register(ps) -> int:
     return len(_REGISTRY) - 1
 
 
-@torch.library.custom_op("shapequant::linear", mutates_args=())
+# The operator is defined in csrc/host.cpp: the dispatcher reaches this function in about 2 us, through a torch.library.custom_op
+# in 14.
+_cblhost.set_linear(lambda x, handle: _REGISTRY[handle].forward(x))
+
+
 def linear_op(x: torch.Tensor, handle: int) -> torch.Tensor:
-    return _REGISTRY[handle].forward(x)
+    return torch.ops.shapequant.linear(x, handle)
 
 
-@linear_op.register_fake
+@torch.library.register_fake("shapequant::linear")
 def _(x: torch.Tensor, handle: int) -> torch.Tensor:
     return x.new_empty(*x.shape[:-1], _REGISTRY[handle].R)
