@@ -276,6 +276,24 @@ PyObject* py_status(PyObject*, PyObject* args) {
     return PyLong_FromLong(bad);
 }
 
+// stream(): torch's current stream on the current device; device(): that device
+PyObject* py_stream(PyObject*, PyObject*) {
+    try {
+        return PyLong_FromUnsignedLongLong((unsigned long long)c10::cuda::getCurrentCUDAStream().stream());
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+PyObject* py_device(PyObject*, PyObject*) {
+    try {
+        return PyLong_FromLong(c10::cuda::current_device());
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
 // decode(packed descriptor, device, type code, first row, end row) -> dense [rows, C]
 PyObject* py_decode(PyObject*, PyObject* args) {
     Py_buffer buf;
@@ -352,6 +370,8 @@ PyMethodDef methods[] = {
     {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "forward(plan, x) -> y or None"},
     {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias)"},
     {"set", py_set, METH_VARARGS, "set(plan, kind, descriptors, row_scale=0)"},
+    {"stream", py_stream, METH_NOARGS, "stream(): torch's current stream of the current device"},
+    {"device", py_device, METH_NOARGS, "device(): the current device"},
     {"decode", py_decode, METH_VARARGS, "decode(packed, device, dtype, first row, end row) -> dense rows"},
     {"set_linear", py_set_linear, METH_O, "set_linear(fn): what shapequant::linear(x, handle) runs"},
     {"status", py_status, METH_VARARGS, "status(device) -> bits"},

@@ -25,7 +25,7 @@ import torch
 from . import _lib
 from ._lib import lib
 from .kernels import DenseStack, _dt, _stream
-from .linear import PackedLinear, RunsLin, Stack
+from .linear import DENSE_MIN_TOKENS, PackedLinear, RunsLin, Stack
 
 NAMES = ("q", "k", "v", "o", "gate", "up", "down")
 
@@ -140,6 +140,40 @@ class _Stage:
         self.stack.run(x, self.out, staged)
 
 
+class _Ahead:
+    """The products of a prompt with their weights decoded on a second stream, one product ahead: the decode of product k + 1
+    starts when product k - 1 has left the scratch buffer, and runs beside whatever stands between the two products."""
+
+    def __init__(self, products: list, side: torch.cuda.Stream, scratch: list):
+        """`scratch`: two buffers (or None) of the caller's, taken in turn; grown here to what the products need."""
+        self.products, self.side, self.scratch, self.k, self.done = products, side, scratch, 0, None
+        dev = products[0].device
+        self.main = torch.cuda.current_stream(dev)
+        for i in range(2):
+            need = max((p.scratch_bytes() for p in products[i::2]), default=0)
+            if need and (scratch[i] is None or scratch[i].numel() < need):
+                scratch[i] = torch.empty(need, dtype=torch.uint8, device=dev)
+        side.wait_stream(self.main)                  # the buffers' earlier users
+        self.ready = self._decode(0)
+
+    def _decode(self, k: int):
+        with torch.cuda.stream(self.side):
+            self.products[k].decode(self.scratch[k & 1])
+            return self.side.record_event()
+
+    def run(self, x: torch.Tensor | None, y: torch.Tensor, staged: torch.Tensor | None = None) -> None:
+        """The next product of the list."""
+        k, ready = self.k, self.ready
+        if k + 1 < len(self.products):
+            if self.done is not None:
+                self.side.wait_event(self.done)
+            self.ready = self._decode(k + 1)
+        self.main.wait_event(ready)
+        self.products[k].gemm(x, y, staged, self.scratch[k & 1])
+        self.done = self.main.record_event()
+        self.k = k + 1
+
+
 class DecodeEngine:
     """layers: list of dicts with ln1, ln2 (16-bit [hidden]), q, k, v, o, gate, up, down (PackedLinear or
     RunsLin), bq, bk, bv (16-bit bias or None). B sequences advance together, each with its own cache and
@@ -197,6 +231,7 @@ class DecodeEngine:
         if self._stages_inputs(B):
             self.stage_h, self.stage_i = self._stage_buffers(B)
         self.graph = None
+        self._side, self._scratch = None, [None, None]      # second stream and decoded weights of prefill()
         self.only_linears = False
         # one token, one column order everywhere: the operator that follows a product runs on its fp32 sums (one small kernel)
         tables = B == 1 and all(st.group is not None for S in self.stages for st in S.values()) and H <= lib.cbl_gemv_l8_add_norm_max_rows()
@@ -329,11 +364,19 @@ class DecodeEngine:
             add, last = None, len(self.layers) - 1
             st = T > 1 and self._stages_inputs(T)
             sh, si = self._stage_buffers(T) if st else (None, None)
+            ahead = None
+            if T >= DENSE_MIN_TOKENS and all(S[k].dense is not None for S in self.stacks for k in S):
+                if self._side is None:
+                    self._side = torch.cuda.Stream(device=self.dev)
+                names = ("qkv", "o", "gu", "down")
+                ahead = _Ahead([S[k].dense for S in self.stacks for k in names][:4 * last + 1], self._side, self._scratch)
             for li, L in enumerate(self.layers):
                 # behind the last layer's attention only the last position is asked for: everything that follows runs on one row
                 n = 1 if li == last else T
                 self._addnorm(h, add, L["ln1"], x, T, sh)
-                self.stacks[li]["qkv"].run(None if st else x, yqkv, sh)
+                (ahead or self.stacks[li]["qkv"]).run(None if st else x, yqkv, sh)
+                if li == last:
+                    ahead = None
                 kc, vc = self.kc[li], self.vc[li]
                 self._rope(yqkv, self.biases[li], None, 0, seq, T, qr, kc, vc)
                 q4 = qr[T - n:].view(n, NH, HD).transpose(0, 1)[None]
@@ -345,11 +388,11 @@ class DecodeEngine:
                 if n < T:
                     h, x, yo, ygu, act, yd = h[T - 1:].clone(), x[:1], yo[:1], ygu[:1], act[:1], yd[:1]
                     st, sh, si = False, None, None
-                self.stacks[li]["o"].run(ao, yo)
+                (ahead or self.stacks[li]["o"]).run(ao, yo)
                 self._addnorm(h, yo, L["ln2"], x, n, sh)
-                self.stacks[li]["gu"].run(None if st else x, ygu, sh)
+                (ahead or self.stacks[li]["gu"]).run(None if st else x, ygu, sh)
                 self._silu(ygu, act, n, si)
-                self.stacks[li]["down"].run(None if st else act, yd, si)
+                (ahead or self.stacks[li]["down"]).run(None if st else act, yd, si)
                 add = yd
             xl = x[:1]
             self._addnorm(h, yd, self.final_norm, xl, 1)
@@ -357,7 +400,7 @@ class DecodeEngine:
             self.lm_head.run(xl, lg)
             _lib.check("cbl_argmax", lib.cbl_argmax(lg.data_ptr(), _dt(lg.dtype), lg.stride(0), 1, lg.shape[1], self.tok[seq:].data_ptr(), None,
                                                     _stream()))
-            self.pos[seq] = T
+            self.pos[seq:seq + 1].fill_(T)          # (an item assignment would copy from the host and wait)
         return lg[0].clone()
 
     def reset(self, tok=0) -> None:

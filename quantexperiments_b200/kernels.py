@@ -10,6 +10,7 @@ calls allocate nothing (CUDA-graph capturable)."""
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 
@@ -26,8 +27,13 @@ def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_stream = _cblhost.stream               # torch's current stream (torch.cuda.current_stream() costs some microseconds of Python)
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """Makes `device` current; costs next to nothing where it is."""
+    return _HERE if _cblhost.device() == device.index else torch.cuda.device(device)
 
 
 def _dt(t: torch.dtype) -> int:
@@ -78,7 +84,7 @@ class DeviceMatrix:
         # A column shard (tensor parallelism) of a matrix with several column orders keeps orders that name positions
         # of the FULL activation vector: x_cols is that vector's length (None: the activations are C long).
         self.x_cols = None if x_cols is None or int(x_cols) == self.C else int(x_cols)
-        self._native = None                     # (addresses, descriptor bytes) of the native decode
+        self._packed = None                     # (addresses, descriptor)
         if self.x_cols is not None and (self.M == 1 or self.x_cols < self.C):
             raise ValueError("x_cols (wider activations than columns) needs several column orders and x_cols >= C")
 
@@ -90,6 +96,12 @@ class DeviceMatrix:
                    torch.ones(words.shape[0], dtype=torch.float16, device=dev), K=1 << bits, d=1, C=n, device=dev)
 
     def struct(self) -> _lib.Packed:
+        key = (self.tags.data_ptr(), self.table.data_ptr(), self.row_scale.data_ptr())
+        if self._packed is None or self._packed[0] != key:
+            self._packed = (key, self._make_struct())
+        return self._packed[1]
+
+    def _make_struct(self) -> _lib.Packed:
         return _lib.Packed(self.R, self.C, self.d, self.bits, self.G, self.M, self.books, self.W, _ptr(self.tags),
                            _ptr(self.tags2), _ptr(self.table), _ptr(self.table2), _ptr(self.row_scale),
                            _ptr(self.row_book), _ptr(self.row_mask), _ptr(self.perms))
@@ -110,17 +122,14 @@ class DeviceMatrix:
         r0, r1 = rows if rows is not None else (0, self.R)
         n = (r1 - r0) * self.C
         if out is None:
-            key = (self.tags.data_ptr(), self.table.data_ptr(), self.row_scale.data_ptr())
-            if self._native is None or self._native[0] != key:
-                self._native = (key, bytes(self.struct()))
             if 0 <= r0 <= r1 <= self.R and dtype in _DT:
-                return _cblhost.decode(self._native[1], self.device.index, _DT[dtype], r0, r1)
+                return _cblhost.decode(self.struct(), self.device.index, _DT[dtype], r0, r1)
             res = torch.empty(r1 - r0, self.C, dtype=dtype, device=self.device)
         else:
             if out.numel() < n or not out.is_contiguous() or out.device != self.device:
                 raise ValueError("out must be a contiguous buffer on the matrix's device with room for the rows")
             res = out.view(-1)[:n].view(r1 - r0, self.C)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_dequant", lib.cbl_dequant(ctypes.byref(self.struct()), res.data_ptr(), _dt(res.dtype),
                                                       self.C, r0, r1, _stream()))
         return res
@@ -153,7 +162,7 @@ class DeviceMatrix:
         st = DenseStack._stage.get(key)
         if st is None or st.numel() < nst:
             st = DenseStack._stage[key] = torch.zeros(nst, dtype=torch.uint8, device=self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             s = _stream()
             _lib.check("cbl_decode_raw_wide", lib.cbl_decode_raw_wide(ctypes.byref(self.struct()), sc.data_ptr(), Cx, s))
             _lib.check("cbl_gemm_dense", lib.cbl_gemm_dense(sc.data_ptr(), self.R, Cx, self.row_scale.data_ptr(), X.data_ptr(), _dt(X.dtype), T,
@@ -179,14 +188,14 @@ class DeviceMatrix:
             Y = torch.empty(T, self.R, dtype=X.dtype, device=self.device)
         if Y.shape != (T, self.R) or Y.stride(1) != 1:
             raise ValueError("Y must be [T, R] with unit column stride")
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_generic", lib.cbl_gemv_generic(ctypes.byref(self.struct()), X.data_ptr(), _dt(X.dtype), T, X.stride(0) if T > 1 else width,
                                                                 Y.data_ptr(), _dt(Y.dtype), Y.stride(0) if T > 1 else self.R, _stream()))
         return Y
 
     def unpack(self, plane: int = 0) -> torch.Tensor:
         out = torch.empty(self.R, self.nch, dtype=torch.int32, device=self.device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_unpack_tags", lib.cbl_unpack_tags(ctypes.byref(self.struct()), plane, out.data_ptr(), _stream()))
         return out
 
@@ -277,7 +286,7 @@ class T16Matrix:
             raise ValueError("Y must be [B, R] with unit column stride")
         ldy = Y.stride(0) if Y.dim() == 2 else self.R
         xp = self.xp_buffer(B)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             s = _stream()
             _lib.check("cbl_prep_x", lib.cbl_prep_x(X.data_ptr(), _dt(X.dtype), B, self.C, X.stride(0), _ptr(self.dm.perms), self.M,
                                                     xp.data_ptr(), s))
@@ -289,14 +298,14 @@ class T16Matrix:
         """Stage a batch of activations once for several matrices that share it and its column orders
         (q|k|v, gate|up): returns the staging buffer to pass to run_prepped()."""
         xp = self.xp_buffer(B)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_prep_x", lib.cbl_prep_x(X.data_ptr(), _dt(X.dtype), B, self.C, X.stride(0), _ptr(self.dm.perms), self.M,
                                                     xp.data_ptr(), _stream()))
         return xp
 
     def run_prepped(self, xp: torch.Tensor, Y: torch.Tensor, B: int) -> torch.Tensor:
         """The product alone, on activations staged by prep() of a matrix with the same input size and column orders."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_t16", lib.cbl_gemv_t16(ctypes.byref(self.struct()), xp.data_ptr(), B, Y.data_ptr(), _dt(Y.dtype),
                                                         Y.stride(0) if Y.dim() == 2 else self.R, _stream()))
         return Y
@@ -339,14 +348,14 @@ class X16Matrix:
     def prep(self, X: torch.Tensor, B: int) -> torch.Tensor:
         """Stage a batch once for several matrices with the same input size (q|k|v, gate|up)."""
         xp = self.xp_buffer(B)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_prep_x", lib.cbl_prep_x(X.data_ptr(), _dt(X.dtype), B, self.C, X.stride(0), None, 1, xp.data_ptr(), _stream()))
         return xp
 
     def run_prepped(self, xp: torch.Tensor, Y: torch.Tensor, B: int) -> torch.Tensor:
         if B < 1 or B > self.BMAX:
             raise ValueError(f"batch {B} outside 1..{self.BMAX}")
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_x16", lib.cbl_gemv_x16(ctypes.byref(self.struct()), xp.data_ptr(), B, Y.data_ptr(), _dt(Y.dtype),
                                                         Y.stride(0) if Y.dim() == 2 else self.R, self.ws.data_ptr(), _stream()))
         return Y
@@ -477,7 +486,7 @@ class B3Group:
             stage, x = staged, (None, 0, B, 0)
         else:
             x = (X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1])
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), *x, _ptr(self.perms), self._ys, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
         return ys
 
@@ -507,8 +516,21 @@ class DenseStack:
         self.row_scale = dms[0].row_scale if len(dms) == 1 else torch.cat([dm.row_scale for dm in dms])
         self.ld = (self.C + 7) // 8 * 8
 
-    def gemm(self, X: torch.Tensor | None, Y: torch.Tensor | None = None, staged: torch.Tensor | None = None) -> torch.Tensor:
-        """`staged` (X None): the activations of Y's rows as cbl_prep_x lays them out, written by the operator before."""
+    def scratch_bytes(self) -> int:
+        return lib.cbl_dense_scratch_bytes(self.R, self.C)
+
+    def decode(self, sc: torch.Tensor) -> None:
+        """The matrices' codewords, rows stacked in order, into a scratch buffer."""
+        with _on(self.device):
+            s, row = _stream(), 0
+            for dm in self.dms:
+                _lib.check("cbl_decode_raw", lib.cbl_decode_raw(ctypes.byref(dm.struct()), sc.data_ptr() + row * self.ld * 2, s))
+                row += dm.R
+
+    def gemm(self, X: torch.Tensor | None, Y: torch.Tensor | None = None, staged: torch.Tensor | None = None,
+             decoded: torch.Tensor | None = None) -> torch.Tensor:
+        """`staged` (X None): the activations of Y's rows as cbl_prep_x lays them out, written by the operator before.
+        `decoded`: the scratch buffer that decode() has filled (None: decode now)."""
         if X is not None and (X.dim() != 2 or X.shape[1] != self.C or X.stride(1) != 1 or X.device != self.device):
             raise ValueError("X must be [T, C] with unit column stride on the matrices' device")
         T = Y.shape[0] if X is None else X.shape[0]
@@ -519,25 +541,24 @@ class DenseStack:
         if T == 0 or self.R == 0:
             return Y
         key = (self.device.index, _stream())
-        need = lib.cbl_dense_scratch_bytes(self.R, self.C)
-        # two scratch buffers alternate: the decode of this stack may run beside the GEMM of the previous one
-        pair = DenseStack._scratch.setdefault(key, [None, None, 0])
-        pair[2] ^= 1
-        sc = pair[pair[2]]
-        if sc is None or sc.numel() < need:
-            sc = pair[pair[2]] = torch.empty(need, dtype=torch.uint8, device=self.device)
+        sc = decoded
+        if sc is None:
+            need = self.scratch_bytes()
+            # two scratch buffers alternate: the decode of this stack may run beside the GEMM of the previous one
+            pair = DenseStack._scratch.setdefault(key, [None, None, 0])
+            pair[2] ^= 1
+            sc = pair[pair[2]]
+            if sc is None or sc.numel() < need:
+                sc = pair[pair[2]] = torch.empty(need, dtype=torch.uint8, device=self.device)
+            self.decode(sc)
         need = lib.cbl_gemm_stage_bytes(T if X is not None else 8, self.C) + 16
         st = DenseStack._stage.get(key)
         if st is None or st.numel() < need:
             st = DenseStack._stage[key] = torch.zeros(need, dtype=torch.uint8, device=self.device)
         x = (None, 0, T, 0, staged.data_ptr()) if X is None else (X.data_ptr(), _dt(X.dtype), T, X.stride(0), st.data_ptr())
-        with torch.cuda.device(self.device):
-            s, row = _stream(), 0
-            for dm in self.dms:
-                _lib.check("cbl_decode_raw", lib.cbl_decode_raw(ctypes.byref(dm.struct()), sc.data_ptr() + row * self.ld * 2, s))
-                row += dm.R
+        with _on(self.device):
             _lib.check("cbl_gemm_dense_bias", lib.cbl_gemm_dense_bias(sc.data_ptr(), self.R, self.C, self.row_scale.data_ptr(), *x[:4], Y.data_ptr(),
-                                                                      _dt(Y.dtype), Y.stride(0), None, x[4], st.data_ptr() + st.numel() - 16, s))
+                                                                      _dt(Y.dtype), Y.stride(0), None, x[4], st.data_ptr() + st.numel() - 16, _stream()))
         return Y
 
     @classmethod
@@ -662,14 +683,14 @@ class L8Matrix:
         x, yv = x.reshape(-1), y.reshape(-1)
         if x.numel() != self.C or not x.is_contiguous() or yv.numel() != self.R or not yv.is_contiguous():
             raise ValueError("x must be a contiguous [C] vector and y a contiguous [R] vector")
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_l8_static", lib.cbl_gemv_l8_static(ctypes.byref(self.struct()), x.data_ptr(), _dt(x.dtype),
                                                                     yv.data_ptr(), _dt(y.dtype), _stream()))
         return y
 
     def static_status(self) -> None:
         """Synchronises and raises CblError if a run_static() product gave up on a bounded device-side wait."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_l8_static_status", lib.cbl_gemv_l8_static_status(_stream()))
 
     _stage: dict = {}
@@ -695,7 +716,7 @@ class L8Matrix:
         if st is None or st.numel() < need:
             st = L8Matrix._stage[key] = torch.empty(need, dtype=torch.uint8, device=self.device)
         ws = l8_workspace(self.device, self.R)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             fn = lib.cbl_gemm_l8_2sm if two_sm else lib.cbl_gemm_l8
             _lib.check("cbl_gemm_l8", fn(ctypes.byref(self.struct_c()), X.data_ptr(), _dt(X.dtype), T, X.stride(0), Y.data_ptr(),
                                          _dt(Y.dtype), Y.stride(0), st.data_ptr(), ws.data_ptr() + ws.numel() - 16, _stream()))
@@ -704,7 +725,7 @@ class L8Matrix:
     def status(self, workspace: torch.Tensor | None = None) -> None:
         """Synchronises and raises CblError if a bounded device-side wait of an earlier run() expired."""
         ws = workspace if workspace is not None else l8_workspace(self.device, self.R)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_l8_status", lib.cbl_gemv_l8_status(ws.data_ptr(), self.R, _stream()))
 
     def run(self, x: torch.Tensor, y: torch.Tensor | None = None, workspace: torch.Tensor | None = None, wide: bool = False) -> torch.Tensor:
@@ -721,7 +742,7 @@ class L8Matrix:
         if yv.numel() != self.R or not yv.is_contiguous():
             raise ValueError("y must be a contiguous [R] vector")
         ws = workspace if workspace is not None else l8_workspace(self.device, self.R)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_l8", lib.cbl_gemv_l8(ctypes.byref(self.struct()), x.data_ptr(), _dt(x.dtype), yv.data_ptr(),
                                                       _dt(y.dtype), ws.data_ptr(), _stream()))
         return y
@@ -787,7 +808,7 @@ class L8Group:
             st = self._rows_stage[key] = torch.empty(lib.cbl_gemm_stage_bytes(lib.cbl_gemm_rows_max_tokens(), self.C), dtype=torch.uint8,
                                                      device=self.device)
         ws = l8_workspace(self.device, 0, self.rows_ws_bytes)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemm_rows_multi", lib.cbl_gemm_rows_multi(self._structs_c, len(self.mats), X.data_ptr(), _dt(X.dtype), B, X.stride(0),
                                                                       self._ys, _dt(ys[0].dtype), ldy, st.data_ptr(), ws.data_ptr(), _stream()))
         return ys
@@ -804,7 +825,7 @@ class L8Group:
                 raise ValueError("outputs must be contiguous [R_i] vectors of one dtype")
             self._ys[i] = y.data_ptr()
         ws = l8_workspace(self.device, 0, self.ws_bytes)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             _lib.check("cbl_gemv_l8_multi", lib.cbl_gemv_l8_multi(self._structs, len(self.mats), x.data_ptr(), _dt(x.dtype), self._ys,
                                                                   _dt(dt), ws.data_ptr(), _stream()))
         return ys
