@@ -528,6 +528,26 @@ def test_engine_with_the_8bit_head_and_the_4bit_embedding():
     assert eng.weight_bytes() < random_engine(_small_cfg(), seed=6).weight_bytes()
 
 
+@pytest.mark.parametrize("n,M", [(129, 1), (257, 4)])
+def test_prompt_with_weights_decoded_ahead_matches_the_steps(n, M):
+    """Prompts of the two-phase path, whose decodes run on a second stream; several in a row share the scratch buffers."""
+    from quantexperiments_b200.engine import random_engine
+    eng = random_engine(_small_cfg(max_len=260), seed=4 + M, M=M)
+    prompt = torch.randint(0, 1000, (n,), generator=torch.Generator().manual_seed(n)).tolist()
+    eng.reset(prompt[0])
+    for t in prompt:
+        eng.tok.fill_(t)
+        eng.step()
+    ref = eng.logits[0].clone()
+    got = []
+    for ids in (prompt, prompt[::-1], prompt):
+        eng.reset(0)
+        got.append(eng.prefill(ids))
+    assert (got[0] - ref).abs().max() / ref.abs().max() <= 2e-2
+    assert torch.equal(got[0], got[2]) and not torch.equal(got[0], got[1])
+    eng.check()
+
+
 def test_engine_rejects_unsupported_shapes():
     from quantexperiments_b200.engine import Cfg, random_engine
     with pytest.raises(ValueError):
