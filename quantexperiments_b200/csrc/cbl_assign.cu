@@ -127,8 +127,8 @@ k_assign(const float* __restrict__ x, const float* __restrict__ wt, int64_t n, c
 // values per chunk; those of the best group - and of the second where it is closer than the arithmetic above can tell -
 // are then evaluated in fp32 exactly as k_assign does, in index order.
 //
-// 8.49 M chunks x 4096 words: 11.1 ms by k_assign (0.65 of the fp32 FMA rate); here 128 results per clock and SM leave the
-// tensor cores (two MMAs of 128 clocks per 128 x 256) and 64 lanes of minimum take the same time.
+// 8.49 M chunks x 4096 words: 11.1 ms by k_assign (0.65 of the fp32 FMA rate), 3.6 ms here.  The epilogue bounds it: three-input
+// minima issue at half rate; with the comparison left out it takes 2.5 ms, with the products left out the same 3.6.
 constexpr int AT_TILE = 128, AT_N = 256, AT_EPI = 512, AT_THREADS = AT_EPI + 64 + 32;
 constexpr int AT_PROD_WARP = 16, AT_MMA_WARP = 18;
 constexpr int AT_A_BYTES = 4096;                 // 128 rows x 16 fp16

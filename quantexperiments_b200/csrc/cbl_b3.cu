@@ -1,4 +1,4 @@
-// Products of 1..64 tokens straight from the packed tags (d = 8, 12-bit tags, 4096-entry fp16 books, one or two summed
+// Products of 1..128 tokens straight from the packed tags (d = 8, 12-bit tags, 4096-entry fp16 books, one or two summed
 // books, any number of column orders) with the weight rows as the M side of tcgen05.mma.
 //
 // A decode thread owns a weight row.  Per k-block (64 columns = 8 chunks) it gathers the row's eight 16-byte codewords
