@@ -38,6 +38,7 @@ constexpr int B3_MAX_RX = 8, B3_MAX_ST = 3;
 constexpr int B3_MAX_MATS = 4, B3_MAX_SEGS = 2 * B3_MAX_MATS;
 constexpr int B3_MAX_TILES = 16320;              // output tiles of a launch: one arrival counter each
 constexpr int B3_CTL_WORDS = 16384;              // status word at 0, counters from 64
+constexpr int B3_MAX_BLOCKS = 160;
 constexpr int B3_MAX_PIECES = 128;               // pieces of a block
 constexpr uint32_t B3_WAIT_LIMIT = 1u << 18;
 
@@ -64,6 +65,8 @@ struct B3Launch {
     unsigned int* status;
     B3Seg seg[B3_MAX_SEGS];
     B3Mat mat[B3_MAX_MATS];
+    int first[B3_MAX_BLOCKS + 1];                // first unit of every block (and the end), and the segment that it lies in: worked
+    unsigned char seg0[B3_MAX_BLOCKS];           // out by the host, so that a block asks for its book and tags at once
 };
 
 __device__ __forceinline__ bool b3_test(uint32_t bar, uint32_t parity) {
@@ -129,7 +132,7 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     const int cta = (int)blockIdx.x;
     const int nkb = P.nkb;
-    auto start = [&](int c) { return P.ks > 0 ? c / P.ks * nkb + c % P.ks * nkb / P.ks : P.q * c + min(c, P.rem); };      // first unit of block c
+    auto start = [&](int c) { return P.first[c]; };            // first unit of block c
     auto owner = [&](int u) {                                  // block that has unit u
         if (P.ks > 0) return u / nkb * P.ks + ((u % nkb + 1) * P.ks - 1) / nkb;
         const int big = P.rem * (P.q + 1);
@@ -186,7 +189,7 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         q0 = tags(rj); q1 = tags(rj + 4); q2 = tags(rj + 8); q3 = tags(rj + 12);
     };
     if (warp < B3_DEC_WARPS) {
-        const B3Seg& sg = P.seg[seg_of(u0 / nkb)];
+        const B3Seg& sg = P.seg[P.seg0[cta]];
         begin_run(sg, u0);
         load_book(sg.table);
     }
@@ -777,6 +780,13 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
             sg.gi0 = gi; sg.gi1 = gi + m.ntile; sg.mi = i;
             gi += m.ntile;
         }
+    }
+    if (pl.G > B3_MAX_BLOCKS) return CBL_EUNSUPPORTED;
+    for (int c = 0, sg = 0; c <= pl.G; c++) {
+        const int u = pl.ks > 0 ? c / pl.ks * P.nkb + c % pl.ks * P.nkb / pl.ks : P.q * c + (c < P.rem ? c : P.rem);
+        P.first[c] = u;
+        while (sg + 1 < P.nseg && u >= P.seg[sg].gi1 * P.nkb) sg++;
+        if (c < pl.G) P.seg0[c] = (unsigned char)sg;
     }
     encode_tiled_fn enc = get_encode();
     if (!enc) return CBL_ECUDA;
