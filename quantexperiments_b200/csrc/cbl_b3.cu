@@ -782,11 +782,17 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
         }
     }
     if (pl.G > B3_MAX_BLOCKS) return CBL_EUNSUPPORTED;
-    for (int c = 0, sg = 0; c <= pl.G; c++) {
-        const int u = pl.ks > 0 ? c / pl.ks * P.nkb + c % pl.ks * P.nkb / pl.ks : P.q * c + (c < P.rem ? c : P.rem);
+    // block c of a tile's ks starts at its k-block floor(c nkb / ks); without ks, blocks 0 .. rem - 1 have one unit more than the rest
+    const int bq = pl.ks > 0 ? P.nkb / pl.ks : P.q, br = pl.ks > 0 ? P.nkb % pl.ks : 0;
+    for (int c = 0, sg = 0, u = 0, r = 0, j = 0; c <= pl.G; c++) {
         P.first[c] = u;
         while (sg + 1 < P.nseg && u >= P.seg[sg].gi1 * P.nkb) sg++;
         if (c < pl.G) P.seg0[c] = (unsigned char)sg;
+        u += bq;
+        if (pl.ks > 0) {
+            if ((r += br) >= pl.ks) { r -= pl.ks; u++; }
+            if (++j == pl.ks) j = r = 0;
+        } else if (c < P.rem) u++;
     }
     encode_tiled_fn enc = get_encode();
     if (!enc) return CBL_ECUDA;
