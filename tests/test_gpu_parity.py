@@ -254,6 +254,20 @@ def test_batch1_product_with_column_orders_matches_fp32_matmul(R, C, books, M):
     assert int(_l8_counters(l8_workspace(dm.device, R)).count_nonzero()) == 0
 
 
+@pytest.mark.parametrize("R,C,books,M,tables", [(64, 1024, 2, 4, True), (64, 18944, 1, 16, False), (6000, 18944, 1, 16, True), (200, 6144, 2, 16, False)])
+def test_one_token_with_column_orders_on_both_sides_of_the_dispatch(R, C, books, M, tables):
+    from quantexperiments_b200.linear import PackedLinear
+    m = orc.synth_matrix(R, C, seed=R + C + M, books=books, M=M)
+    t = lambda a: torch.as_tensor(a).cuda()
+    more = dict(words2=t(m["words"][1]), table2=t(m["table"][1])) if books == 2 else {}
+    lin = PackedLinear(t(m["words"][0]), t(m["table"][0]), t(m["row_scale"]), None, t(m["row_mask"]), t(m["perms"]), 4096, 8, **more)
+    assert lin.use_l8() == tables
+    x = torch.randn(1, C, generator=torch.Generator().manual_seed(R)).bfloat16()
+    yref = orc.linear_ref(x.float().numpy(), orc.synth_decode(m))
+    for _ in range(2):                                       # the second call takes the native path
+        assert orc.max_rel_err(lin(x.cuda()).float().cpu().numpy(), yref) < _out_tol(torch.bfloat16)
+
+
 @pytest.mark.parametrize("n,R,C,books", [(4, 100, 1088, 1), (4, 70, 2312, 2), (2, 66500, 136, 2)])
 def test_batch1_product_with_many_tiles_per_block(n, R, C, books):
     """64 segments leave two blocks to each: 9 and 37 tiles per block, over the change of the book; two steps of rows per tile."""
