@@ -172,13 +172,16 @@ def snap(w: torch.Tensor, codebook: torch.Tensor, *, d: int = 8, perm: torch.Ten
     rows, K = w32.shape[0], book16.shape[0]
     used = torch.zeros(K, dtype=torch.uint8, device=w32.device)
     if d == 8 and book16.shape[1] == 8 and K % 256 == 0 and K <= 4096 and col_weight is None and not row_weighted and w32.numel():
-        # the kernel divides by the scale, cuts the chunks and marks the words it uses
-        pad, w32 = (-cols) % d, w32 if w32.stride(1) == 1 else w32.contiguous()
+        # the kernel divides by the scale, cuts the chunks and marks the words it uses; it reads rows that lie apart in memory, so
+        # expanded or overlapping ones are copied (of a single row the stride says nothing)
+        pad, ld = (-cols) % d, w32.stride(0) if rows > 1 else cols
+        if (w32.stride(1) != 1 and cols > 1) or ld < cols:
+            w32, ld = w32.contiguous(), cols
         nch = (cols + pad) // d
         idx = torch.empty(rows * nch, dtype=torch.int64, device=w32.device)
         err = torch.empty(rows * nch, dtype=torch.float32, device=w32.device)
         with torch.cuda.device(w32.device):
-            _lib.check("cbl_snap_rows", lib.cbl_snap_rows(w32.data_ptr(), rows, cols, w32.stride(0), scale16.data_ptr(), book16.data_ptr(), K, idx.data_ptr(),
+            _lib.check("cbl_snap_rows", lib.cbl_snap_rows(w32.data_ptr(), rows, cols, ld, scale16.data_ptr(), book16.data_ptr(), K, idx.data_ptr(),
                                                           err.data_ptr(), used.data_ptr(), _stream()))
     else:
         chunks, pad = chunk_rows(w32 / scale16.to(torch.float32)[:, None], d)

@@ -184,3 +184,17 @@ def test_snap_rows_equals_snap_by_chunks():
         idx, err = cb.assign(chunks, book)
         assert torch.equal(r["idx"].reshape(-1), idx) and torch.equal(r.err, err) and r["pad"] == pad
         assert r.stats["codebook_usage"] == idx.unique().numel() / 4096
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_snap_of_strided_rows(weighted):
+    """Rows that overlap or repeat in memory (expanded rows, one short-strided row), every other row, every other column."""
+    from quantexperiments_b200 import codebook as cb
+    g = torch.Generator(device="cuda").manual_seed(9)
+    book = torch.randn(4096, 8, device="cuda", generator=g).half()
+    base = torch.randn(6, 40, device="cuda", generator=g)
+    line = torch.randn(64, 1, device="cuda", generator=g)
+    for w in (base[:1].expand(5, 40), line.t(), base[::2], base[:, ::2], base.t(), base.reshape(-1).as_strided((9, 40), (8, 1)), line):
+        cw = torch.rand(w.shape[1], device="cuda", generator=g) + 0.5 if weighted else None
+        got, want = cb.snap(w, book, col_weight=cw), cb.snap(w.clone(memory_format=torch.contiguous_format), book, col_weight=cw)
+        assert torch.equal(got["idx"], want["idx"]) and torch.equal(got["row_scale"], want["row_scale"]) and torch.equal(got.err, want.err)
