@@ -288,7 +288,7 @@ class RunsLin:
     def __init__(self, lin: PackedLinear):
         self.lin, self.R, self.C = lin, lin.R, lin.C
         self.perms = lin.dm.perms
-        if lin.dm.M == 1 and lin.use_l8():
+        if lin.use_l8():
             lin.l8          # build the layouts now, not inside a captured region
         else:
             lin.group(1)

@@ -201,6 +201,15 @@ def test_small_batch_product_is_deterministic_and_survives_outliers():
 
 
 # ------------------------------------------------------------------------------------------ batch-1 product
+def _linear(m, bias=None):
+    """A synthetic matrix as a PackedLinear."""
+    from quantexperiments_b200.linear import PackedLinear
+    t = lambda a: torch.as_tensor(a).cuda()
+    more = dict(words2=t(m["words"][1]), table2=t(m["table"][1])) if m["books"] == 2 else {}
+    mask, perms = (None, torch.arange(m["C"])[None].cuda()) if m["M"] == 1 else (t(m["row_mask"]), t(m["perms"]))
+    return PackedLinear(t(m["words"][0]), t(m["table"][0]), t(m["row_scale"]), None, mask, perms, 4096, 8, bias=bias, **more)
+
+
 @pytest.mark.parametrize("R,C,books", [(4864, 896, 1), (3584, 3584, 1), (2051, 1024, 1), (512, 3584, 1), (2304, 1000 * 8, 2),
                                         (4, 64, 1), (1030, 72, 2)])
 def test_batch1_product_matches_fp32_matmul(R, C, books):
@@ -266,6 +275,25 @@ def test_one_token_with_column_orders_on_both_sides_of_the_dispatch(R, C, books,
     yref = orc.linear_ref(x.float().numpy(), orc.synth_decode(m))
     for _ in range(2):                                       # the second call takes the native path
         assert orc.max_rel_err(lin(x.cuda()).float().cpu().numpy(), yref) < _out_tol(torch.bfloat16)
+
+
+def test_runs_lin_of_several_column_orders_is_ready_for_capture():
+    """RunsLin builds the layout that its one-token run reads in its constructor, not inside a captured region."""
+    from quantexperiments_b200.linear import RunsLin
+    m = orc.synth_matrix(3072, 256, seed=12, M=2)
+    lin = _linear(m)
+    rl = RunsLin(lin)
+    assert lin.use_l8() and lin._l8 is not None
+    x = torch.randn(256, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    y = torch.zeros(3072, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        rl.run(x, y)
+    g.replay()
+    torch.cuda.synchronize()
+    assert orc.max_rel_err(y.cpu().numpy()[None], orc.linear_ref(x.float().cpu().numpy()[None], orc.synth_decode(m))) < TOL
 
 
 @pytest.mark.parametrize("n,R,C,books", [(4, 100, 1088, 1), (4, 70, 2312, 2), (2, 66500, 136, 2)])
