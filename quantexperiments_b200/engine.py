@@ -222,8 +222,8 @@ class DecodeEngine:
             else:
                 sizes = (NH * HD, NKV * HD, NKV * HD)
                 self.biases.append(torch.cat([b.to(**a) if b is not None else torch.zeros(n, **a) for b, n in zip(bs, sizes)]))
-        self.stacks = [{"qkv": Stack([_lin(L[n]) for n in ("q", "k", "v")]), "o": Stack([_lin(L["o"])]),
-                        "gu": Stack([_lin(L[n]) for n in ("gate", "up")]), "down": Stack([_lin(L["down"])])} for L in layers]
+        pieces = {"qkv": ("q", "k", "v"), "o": ("o",), "gu": ("gate", "up"), "down": ("down",)}
+        self.stacks = [{k: Stack([_lin(L[n]) for n in names], step=True) for k, names in pieces.items()} for L in layers]
         self.stages = [{"qkv": _Stage(S["qkv"], self.yqkv), "o": _Stage(S["o"], self.yo), "gu": _Stage(S["gu"], self.ygu),
                         "down": _Stage(S["down"], self.yd)} for S in self.stacks]
         # several sequences, one column order: add + norm and silu * up write the fp16 staging buffer of the product after them
@@ -234,10 +234,7 @@ class DecodeEngine:
         self._side, self._scratch = None, [None, None]      # second stream and decoded weights of prefill()
         self.only_linears = False
         # one token, one column order everywhere: the operator that follows a product runs on its fp32 sums (one small kernel)
-        tables = B == 1 and all(st.group is not None for S in self.stages for st in S.values()) and H <= lib.cbl_gemv_l8_add_norm_max_rows()
-        plain = all(m.dm.M == 1 for S in self.stages for st in S.values() for m in st.stack.lins)
-        # the fused step, for matrices of one column order and of several (whose products read the same vectors)
-        self.fused, self.fused_orders = tables and plain, tables and not plain
+        self.fused = B == 1 and all(st.group is not None for S in self.stages for st in S.values()) and H <= lib.cbl_gemv_l8_add_norm_max_rows()
 
     def _stages_inputs(self, n: int) -> bool:
         c = self.cfg
@@ -293,7 +290,7 @@ class DecodeEngine:
                 return
             s = _stream()
             self._embed(self.tok, B, self.h)
-            if self.fused or self.fused_orders:
+            if self.fused:
                 self._step_fused(s)
                 return
             add, sh, si = None, self.stage_h, self.stage_i

@@ -22,30 +22,20 @@ import torch
 from . import _cblhost, _lib
 from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix
 
-# One token: activation-side tables (L8Matrix) at every number of rows with one column order (64 x 3584: 4.8 us against 8.4
-# by codeword gathers, 4096 x 3584: 6.6 against 10.1, 18944 x 3584: 10.5 against 14.5).  With several column orders
-# every order needs tables of its own, about 1 us each, L8_SMS of them at a time: they pay while a table serves enough rows.
-# Measured against the gathers, us: 512 x 3584 in 4 orders 6.1 / 12.7; 27648 x 5120, two books, 16 orders (17 tables per SM,
-# 1728 rows each) 34.4 / 54.6; 3584 x 18944 in 16 orders (32, 224 rows) 35.4 / 40.2; q|k|v of 3584, 16 orders (18, 96) 21.9 / 15.2;
-# 512 x 18944 in 16 orders (32, 32) 35.1 / 24.4; 8000 x 18944, two books, 16 orders (64, 500) 72.5 / 64.1.  Up to ten
-# tables per SM win at any number of rows; above, 16 rows per table and further table put all of these on the right side
-# or within 5 us of it.
-L8_SMS = 148
+# Rows from which one token runs on activation-side tables (L8Matrix) instead of codeword gathers (B3Matrix); of a matrix with
+# several column orders, rows per order: every order needs tables of its own, and a build costs as much as the lookups of some
+# 1300 rows.  The tables hold 16-bit integers (results off by about 1e-4), the gathers sum fp16 products in fp32 (3e-7).  Above the
+# line the tables serve (2048 x 3584: 5.5 us against 9.0 by gathers; 27648 x 5120, two books, 16 orders: 34.1 against 50.8); below
+# it they would be faster as well (512 x 3584: 4.6 against 7.6; 3584 x 3584 in 16 orders: 10.2 against 13.6), but a small
+# matrix gains three to six microseconds at most and keeps its exact sums.
+L8_MIN_ROWS = 2048
+L8_MIN_ROWS_PER_ORDER = 1536
 # Tokens up to which the book lies three times in shared memory (the activations of more tokens need the room: two copies).
 B3_MAX_3COPIES = 16
 # Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM.
 DENSE_MIN_TOKENS = 129
 # counts loader.pool_layouts() calls: native plans made before one hold old addresses
 pool_epoch = 0
-
-
-def tables_pay(lins: list) -> bool:
-    """Whether one token of linears that read the same activations runs on the table-lookup kernel."""
-    orders = sum(l.dm.M for l in lins)
-    if all(l.dm.M == 1 for l in lins):
-        return True
-    builds = sum(l.dm.M * l.dm.books * -(-l.dm.nch // 8) for l in lins) / L8_SMS
-    return max(l.dm.M for l in lins) <= L8Matrix.MAX_ORDERS and orders <= L8_SMS and sum(l.R for l in lins) >= 16 * orders * (builds - 10)
 
 
 class PackedLinear(torch.nn.Module):
@@ -134,7 +124,8 @@ class PackedLinear(torch.nn.Module):
 
     def use_l8(self) -> bool:
         """One token runs on the table-lookup kernel (any number of column orders up to its limit)."""
-        return self.dm.fast and not self.wide and tables_pay([self])
+        least = L8_MIN_ROWS if self.dm.M == 1 else L8_MIN_ROWS_PER_ORDER * self.dm.M
+        return self.dm.fast and not self.wide and self.dm.M <= L8Matrix.MAX_ORDERS and self.R >= least
 
     def gemv(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x [C] (fp16 / bf16 / fp32, contiguous) -> y [R] in x's dtype (or `out`'s)."""
@@ -191,11 +182,13 @@ class PackedLinear(torch.nn.Module):
 
 class Stack:
     """Linears that read the same activations (q|k|v, gate|up): run(x [n, C], y [n, sum R]) writes their outputs side by side.
-    One token: one table-lookup launch; up to 128 tokens: one codeword-gather launch where the pieces share their column
-    orders, else one per piece; more: every piece decoded once, one GEMM over the stacked rows.  Layouts are built on first
-    use of their token counts (or by prepare(), which a caller runs before it captures a graph)."""
+    One token: one table-lookup launch where the rows fill tables, else, and up to 128 tokens: one codeword-gather launch where
+    the pieces share their column orders, else one per piece; more: every piece decoded once, one GEMM over the stacked rows.
+    Layouts are built on first use of their token counts (or by prepare(), which a caller runs before it captures a graph).
+    step: the stack of a decode step, whose one-token form is the launch with the step's operators behind it (one column order,
+    tables whatever the rows)."""
 
-    def __init__(self, lins: list):
+    def __init__(self, lins: list, step: bool = False):
         from .kernels import DenseStack, L8Group
         self.lins, self.C, self.device = lins, lins[0].C, lins[0].dm.device
         self.Rs = [l.R for l in lins]
@@ -203,7 +196,12 @@ class Stack:
         p0 = lins[0].dm.perms
         self.shared = len(lins) <= B3Group.MAX and all(l.dm.fast and l.dm.M == lins[0].dm.M and (l.dm.perms is p0 or (
             p0 is not None and l.dm.perms is not None and torch.equal(l.dm.perms, p0))) for l in lins)
-        self.tables = all(l.dm.fast and not l.wide for l in lins) and len(lins) <= L8Group.MAX and tables_pay(lins)
+        plain = all(l.dm.fast and not l.wide and l.dm.M == 1 for l in lins)
+        if step:
+            self.tables = plain and len({l.dm.books for l in lins}) == 1
+        else:
+            self.tables = plain and self.R >= L8_MIN_ROWS or all(l.use_l8() for l in lins)
+        self.tables = self.tables and len(lins) <= L8Group.MAX
         self.fast = all(l.dm.fast for l in lins)
         self.dense = DenseStack([l.dm for l in lins]) if self.fast and len({l.C for l in lins}) == 1 and not any(l.wide for l in lins) else None
         self._l8 = None
@@ -288,10 +286,14 @@ class RunsLin:
     def __init__(self, lin: PackedLinear):
         self.lin, self.R, self.C = lin, lin.R, lin.C
         self.perms = lin.dm.perms
-        if lin.use_l8():
-            lin.l8          # build the layouts now, not inside a captured region
-        else:
+        # build the layouts now, not inside a captured region (fused epilogues take the tables whatever the rows)
+        if lin.use_l8() or self._epilogues():
+            lin.l8
+        if not lin.use_l8():
             lin.group(1)
+
+    def _epilogues(self) -> bool:
+        return self.lin.dm.fast and not self.lin.wide and self.lin.dm.M == 1
 
     def run(self, x: torch.Tensor, y: torch.Tensor, epi: dict | None = None):
         """y = W . x.  `epi` asks for the operator that follows the product in a decode step to run with it, as the
@@ -312,7 +314,7 @@ class RunsLin:
         from .kernels import L8Group, _dt, _stream, l8_workspace
         if epi.get("perms") is not None:
             raise ValueError("epi['perms']: permuted copies of the output are not produced here (the next product applies its column orders itself)")
-        if not self.lin.use_l8() or self.lin.dm.M != 1 or x.numel() != self.C:
+        if not self._epilogues() or x.numel() != self.C:
             raise ValueError("fused epilogues run one token through the table-lookup kernel (one column order)")
         mode, out = epi.get("mode"), epi["out"]
         xv = x.reshape(-1)

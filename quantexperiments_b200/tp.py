@@ -222,7 +222,7 @@ class RowParallelLinear:
                 raise ValueError("the fused path runs matrices with at most 16 column orders")
             self.fused = PeerReduceGemv(self.l8_multi, arena)
             return
-        if not self.lin.use_l8():
+        if not self.lin.dm.fast:
             raise ValueError("the fused path runs matrices in the table-lookup layout")
         self.fused = PeerReduceGemv(self.lin.l8, arena)
 

@@ -548,6 +548,13 @@ def test_prompt_with_weights_decoded_ahead_matches_the_steps(n, M):
     eng.check()
 
 
+def test_steps_of_matrices_with_column_orders_use_no_tables():
+    """Engines of such matrices gather codewords at one token: their orders share no tables of 16-bit entries."""
+    from quantexperiments_b200.engine import random_engine
+    eng = random_engine(_small_cfg(), seed=2, M=2)
+    assert not eng.fused and all(st.group is None and not st.stack.tables for S in eng.stages for st in S.values())
+
+
 def test_engine_rejects_unsupported_shapes():
     from quantexperiments_b200.engine import Cfg, random_engine
     with pytest.raises(ValueError):

@@ -263,18 +263,33 @@ def test_batch1_product_with_column_orders_matches_fp32_matmul(R, C, books, M):
     assert int(_l8_counters(l8_workspace(dm.device, R)).count_nonzero()) == 0
 
 
-@pytest.mark.parametrize("R,C,books,M,tables", [(64, 1024, 2, 4, True), (64, 18944, 1, 16, False), (6000, 18944, 1, 16, True), (200, 6144, 2, 16, False)])
-def test_one_token_with_column_orders_on_both_sides_of_the_dispatch(R, C, books, M, tables):
+@pytest.mark.parametrize("R,C,books,M,tables", [(64, 1024, 2, 4, False), (64, 18944, 1, 16, False), (6144, 18944, 1, 4, True), (6143, 1024, 1, 4, False),
+                                                (200, 6144, 2, 16, False), (2048, 3584, 1, 1, True), (2047, 3584, 1, 1, False)])
+def test_one_token_on_both_sides_of_the_dispatch(R, C, books, M, tables):
     from quantexperiments_b200.linear import PackedLinear
     m = orc.synth_matrix(R, C, seed=R + C + M, books=books, M=M)
-    t = lambda a: torch.as_tensor(a).cuda()
-    more = dict(words2=t(m["words"][1]), table2=t(m["table"][1])) if books == 2 else {}
-    lin = PackedLinear(t(m["words"][0]), t(m["table"][0]), t(m["row_scale"]), None, t(m["row_mask"]), t(m["perms"]), 4096, 8, **more)
+    lin = _linear(m)
     assert lin.use_l8() == tables
     x = torch.randn(1, C, generator=torch.Generator().manual_seed(R)).bfloat16()
     yref = orc.linear_ref(x.float().numpy(), orc.synth_decode(m))
     for _ in range(2):                                       # the second call takes the native path
         assert orc.max_rel_err(lin(x.cuda()).float().cpu().numpy(), yref) < _out_tol(torch.bfloat16)
+
+
+@pytest.mark.parametrize("R,C,books,M", [(512, 3584, 1, 1), (64, 1024, 2, 1), (260, 1032, 1, 4), (3584, 3584, 1, 16)])
+def test_one_token_of_few_rows_is_summed_in_fp32(R, C, books, M):
+    """Matrices whose rows do not fill tables of 16-bit entries multiply one token with products and sums of at least 32 bits: bf16
+    activations and fp16 codewords multiply exactly, C / 16 sums of 16 products are rounded (or truncated) at 2^-23 of the running sum.  (Tables
+    are off by some 1e-4.)"""
+    from quantexperiments_b200.linear import RunsLin
+    m = orc.synth_matrix(R, C, seed=R + C + M, books=books, M=M)
+    lin = _linear(m)
+    x = torch.randn(1, C, generator=torch.Generator().manual_seed(R)).bfloat16().float().cuda()
+    ref = x.double() @ torch.from_numpy(orc.synth_decode(m)).double().cuda().T
+    y = torch.empty(R, device="cuda")
+    RunsLin(lin).run(x[0], y)
+    for got in (lin(x), lin(x), lin.gemv(x[0]), y):          # Python path, native path, the engine's surfaces
+        assert (got.double() - ref).norm() <= books * (C / 16) * 2.0 ** -23 * ref.norm()
 
 
 def test_runs_lin_of_several_column_orders_is_ready_for_capture():
