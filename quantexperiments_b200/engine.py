@@ -367,11 +367,20 @@ class DecodeEngine:
                     self._side = torch.cuda.Stream(device=self.dev)
                 names = ("qkv", "o", "gu", "down")
                 ahead = _Ahead([S[k].dense for S in self.stacks for k in names][:4 * last + 1], self._side, self._scratch)
-            for li, L in enumerate(self.layers):
+
+            def product(stack, x, y, staged=None):
+                """Rows of a prompt are summed in fp32 like each other: no tables of 16-bit entries for the last one (a prompt of one
+                token runs as that token does by itself)."""
+                if ahead is not None:
+                    ahead.run(x, y, staged)
+                else:
+                    stack.run(x, y, staged, tables=T == 1 and stack.tables and all(l.use_l8() for l in stack.lins))
+
+            for li, (L, S) in enumerate(zip(self.layers, self.stacks)):
                 # behind the last layer's attention only the last position is asked for: everything that follows runs on one row
                 n = 1 if li == last else T
                 self._addnorm(h, add, L["ln1"], x, T, sh)
-                (ahead or self.stacks[li]["qkv"]).run(None if st else x, yqkv, sh)
+                product(S["qkv"], None if st else x, yqkv, sh)
                 if li == last:
                     ahead = None
                 kc, vc = self.kc[li], self.vc[li]
@@ -385,11 +394,11 @@ class DecodeEngine:
                 if n < T:
                     h, x, yo, ygu, act, yd = h[T - 1:].clone(), x[:1], yo[:1], ygu[:1], act[:1], yd[:1]
                     st, sh, si = False, None, None
-                (ahead or self.stacks[li]["o"]).run(ao, yo)
+                product(S["o"], ao, yo)
                 self._addnorm(h, yo, L["ln2"], x, n, sh)
-                (ahead or self.stacks[li]["gu"]).run(None if st else x, ygu, sh)
+                product(S["gu"], None if st else x, ygu, sh)
                 self._silu(ygu, act, n, si)
-                (ahead or self.stacks[li]["down"]).run(None if st else act, yd, si)
+                product(S["down"], None if st else act, yd, si)
                 add = yd
             xl = x[:1]
             self._addnorm(h, yd, self.final_norm, xl, 1)

@@ -244,20 +244,24 @@ class Stack:
         """Whether run() accepts the n tokens' activations staged by the operator before (cbl_prep_x's layout)."""
         return self.shared and self.lins[0].dm.M == 1 and (n > 1 or not self.tables) and (n < DENSE_MIN_TOKENS or self.dense is not None)
 
-    def run(self, x: torch.Tensor | None, y: torch.Tensor, staged: torch.Tensor | None = None) -> torch.Tensor:
+    def run(self, x: torch.Tensor | None, y: torch.Tensor, staged: torch.Tensor | None = None, tables: bool | None = None) -> torch.Tensor:
+        """tables: whether one token may run on table lookups (None: where the stack's rule says so)."""
         n = y.shape[0]
         if n >= DENSE_MIN_TOKENS and self.dense is not None:
             return self.dense.gemm(x, y, staged)
         ys = list(y.split(self.Rs, 1))
         if x is None:
             self.b3(n).run(None, ys, staged)
-        elif n == 1 and self.tables:
+        elif n == 1 and (self.tables if tables is None else tables):
             self.l8.run(x[0], [t[0] for t in ys])
         elif self.shared and n < DENSE_MIN_TOKENS:
             self.b3(n).run(x, ys)
         else:
             for l, t in zip(self.lins, ys):
-                l.forward_into(x, t)
+                if n == 1 and tables is False and l.dm.fast:
+                    l.group(1).run(x, [t])
+                else:
+                    l.forward_into(x, t)
         return y
 
     def bind(self):

@@ -548,6 +548,20 @@ def test_prompt_with_weights_decoded_ahead_matches_the_steps(n, M):
     eng.check()
 
 
+@pytest.mark.parametrize("T,M", [(20, 1), (140, 1), (33, 4)])
+def test_prompts_multiply_without_tables_of_16_bit_entries(T, M, monkeypatch):
+    """What follows the last layer's attention runs on one row of the prompt, with products and sums in fp32 like the rows before it."""
+    from quantexperiments_b200 import kernels
+    from quantexperiments_b200.engine import random_engine
+    eng = random_engine(_small_cfg(max_len=160), seed=3, M=M)
+    def refuse(*_):
+        raise AssertionError("table lookups in a prompt")
+    monkeypatch.setattr(kernels.L8Group, "run", refuse)
+    monkeypatch.setattr(kernels.L8Matrix, "run", refuse)
+    assert torch.isfinite(eng.prefill(list(range(T)))).all()
+    eng.check()
+
+
 def test_steps_of_matrices_with_column_orders_use_no_tables():
     """Engines of such matrices gather codewords at one token: their orders share no tables of 16-bit entries."""
     from quantexperiments_b200.engine import random_engine
