@@ -91,7 +91,8 @@ int cbl_gemv_generic(const cbl_packed* m, const void* x, int xdtype, int32_t nto
 
 /* Encoder side ("snap"): index of the nearest codeword of every chunk and its squared error,
  *   idx[i] = argmin_k (|c_k|^2 - 2 x_i . c_k)   (first k on ties),   err[i] = max(min + |x_i|^2, 0),
- * all in fp32 (8 FMAs per codeword from |c_k|^2, no reduced-precision contraction).  wt (optional, same shape as x):
+ * all in fp32 (8 FMAs per codeword from |c_k|^2; where the tensor cores look for candidates - fp16 book of whole 256 words, no
+ * weights, 512 chunks and more - every word that they cannot tell from the nearest is evaluated so, and the answer is the same).  wt (optional, same shape as x):
  * per-element weights, argmin_k sum_j wt_j (x_j - c_kj)^2 and err = that minimum.
  * x, wt fp32 [n, d]; book f16 / bf16 / f32 [K, d]; d = 8, K <= cbl_assign_max_codewords().
  * replaces shapequant/codebook.py:40-71 (_assign_batch, assign). */

@@ -124,8 +124,8 @@ k_assign(const float* __restrict__ x, const float* __restrict__ wt, int64_t n, c
 // so A1 B + A2 B = f |c|^2 - 2 x.c in fp32 (f: a power of two per chunk that keeps large chunks inside fp16; 1 otherwise).
 // Book and chunks are scaled by one more power of two when the book's largest value is not within 2 .. 64.
 // Sixteen warps read the 128 x 256 results out of tensor memory and keep the two groups of 16 codewords with the smallest
-// values per chunk; those of the best group - and of the second where it is closer than the arithmetic above can tell -
-// are then evaluated in fp32 exactly as k_assign does, in index order.
+// values per chunk and warpgroup; those of the best group - and of every group that is closer than the arithmetic above can
+// tell - are then evaluated in fp32 exactly as k_assign does, so that index and error are k_assign's, bit for bit.
 //
 // 8.49 M chunks x 4096 words: 11.1 ms by k_assign (0.65 of the fp32 FMA rate), 3.6 ms here.  The epilogue bounds it: three-input
 // minima issue at half rate; with the comparison left out it takes 2.5 ms, with the products left out the same 3.6.
@@ -134,7 +134,7 @@ constexpr int AT_PROD_WARP = 16, AT_MMA_WARP = 18;
 constexpr int AT_A_BYTES = 4096;                 // 128 rows x 16 fp16
 constexpr int AT_BOOK = 131072;
 constexpr int AT_STAGE = 2 * AT_A_BYTES + AT_TILE * 36;         // A1 | A2 | the chunks in fp32 | the scales f
-constexpr int AT_SMEM = AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * 16 + 4 * AT_TILE * 8;
+constexpr int AT_SMEM = AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * 12 + 4 * AT_TILE * 8;
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
 
 __device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity) {
@@ -209,7 +209,44 @@ __device__ __forceinline__ void at_chunk(const AtSource& s, int64_t ci, float (&
     for (int i = 0; i < 8; i++) v[i] = __fdiv_rn(v[i], sc);
 }
 
-struct AtPart { float best; int bg; float second; int sg; };
+struct AtPart { float best; int bg; float second; };
+
+// |c_k|^2 - 2 x.c_k of word k, added up as k_assign does (a book that was scaled down may have lost bits in shared memory).
+__device__ __forceinline__ float at_dist(const unsigned char* words, const __half* __restrict__ book, int q2, float ibs, const float (&x)[8], int k) {
+    const uint4 cw = q2 >= 0 ? *(const uint4*)(words + at_row(k)) : __ldg((const uint4*)book + k);
+    const __half2* h = (const __half2*)&cw;
+    float c[8], d = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float2 p = __half22float2(h[i]);
+        c[2 * i] = q2 > 0 ? p.x * ibs : p.x;
+        c[2 * i + 1] = q2 > 0 ? p.y * ibs : p.y;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) d += c[i] * c[i];
+#pragma unroll
+    for (int i = 0; i < 8; i++) d = fmaf(-2.0f * x[i], c[i], d);
+    return d;
+}
+
+// The nearest of words k0 .. k1 - 1 to one chunk, for a warp: {distance, index}, the first index that reaches the minimum.
+__device__ __forceinline__ float2 at_nearest(const unsigned char* words, const __half* __restrict__ book, int q2, float ibs, float4 x0, float4 x1, int k0, int k1) {
+    const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    float d0 = INFINITY;
+    int i0 = 0;
+#pragma unroll 1
+    for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) {
+        const float d = at_dist(words, book, q2, ibs, xs, k);
+        if (d < d0 || (d == d0 && k < i0)) { d0 = d; i0 = k; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float d1 = __shfl_xor_sync(0xffffffffu, d0, o);
+        const int i1 = __shfl_xor_sync(0xffffffffu, i0, o);
+        if (d1 < d0 || (d1 == d0 && i1 < i0)) { d0 = d1; i0 = i1; }
+    }
+    return make_float2(d0, __int_as_float(i0));
+}
 
 __global__ void __launch_bounds__(AT_THREADS, 1)
 k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int64_t* __restrict__ idx, float* __restrict__ err,
@@ -226,7 +263,7 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
     auto acc_full = [&](int b) { return bar0 + 32u + 8u * b; };
     auto acc_empty = [&](int b) { return bar0 + 48u + 8u * b; };
     AtPart* s_part = (AtPart*)(at_smem + AT_BOOK + 2 * AT_STAGE);
-    float2* s_ex = (float2*)(at_smem + AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * 16);
+    float2* s_ex = (float2*)(at_smem + AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * (int)sizeof(AtPart));
     const int64_t ntile = (n + AT_TILE - 1) / AT_TILE;
     const int nstep = K / AT_N;
     if (tid == 0) {
@@ -374,7 +411,7 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
         uint32_t base = 0;
         for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++, base += nstep) {
             float best = INFINITY, second = INFINITY;
-            int bg = 0, sg = 0;
+            int bg = 0;
             for (; use < base + nstep; use += 2) {
                 const int j = (int)(use - base), g0 = j * 16 + (w & 1) * 8;
                 wait(acc_full(b), (use >> 1) & 1);
@@ -387,10 +424,9 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
 #pragma unroll
                         for (int q = 3; q < 15; q += 2) m = as_min3(m, __uint_as_float(v[16 * h + q]), __uint_as_float(v[16 * h + q + 1]));
                         m = fminf(m, __uint_as_float(v[16 * h + 15]));
-                        if (m < second) {
+                        if (__builtin_expect(m < second, 0)) {      // a branch, not selects for every group: 3.61 ms against 3.77
                             const bool top = m < best;
                             second = top ? best : m;
-                            sg = top ? bg : g + h;
                             best = top ? m : best;
                             bg = top ? g + h : bg;
                         }
@@ -412,20 +448,14 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
                 if (lane == 0) mbar_arrive(acc_empty(b));
                 look(vb, g0 + 6);
             }
-            AtPart mine = {best, bg, second, sg};
+            AtPart mine = {best, bg, second};
             s_part[w * AT_TILE + row] = mine;
             asm volatile("bar.sync 1, %0;" ::"n"(AT_EPI) : "memory");
-            // all four warpgroups know the two best groups of their chunk; each evaluates a quarter of a group's words
+            // All four warpgroups know the two best groups that each of them has seen; each evaluates a quarter of a group's words.
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const AtPart p = s_part[q * AT_TILE + row];
-                if (q == 0) { best = p.best; bg = p.bg; second = p.second; sg = p.sg; continue; }
-                auto add = [&](float v, int g) {
-                    if (v < best || (v == best && g < bg)) { second = best; sg = bg; best = v; bg = g; }
-                    else if (v < second || (v == second && g < sg)) { second = v; sg = g; }
-                };
-                add(p.best, p.bg);
-                add(p.second, p.sg);
+                if (q == 0 || p.best < best) { best = p.best; bg = p.bg; }
             }
             const unsigned char* st = at_smem + AT_BOOK + (it & 1) * AT_STAGE;
             const float4 x0 = ((const float4*)(st + 2 * AT_A_BYTES))[row], x1 = ((const float4*)(st + 2 * AT_A_BYTES))[AT_TILE + row];
@@ -437,30 +467,41 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
             float bd = INFINITY;
             int bi = 0;
             const float ibs = ldexpf(1.f, -q2);
-            auto exact = [&](int g) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int k = g * 16 + w * 4 + q;
-                    // (a book that was scaled down may have lost bits in shared memory)
-                    const uint4 cw = q2 >= 0 ? *(const uint4*)(at_smem + at_row(k)) : __ldg((const uint4*)book + k);
-                    const __half2* h = (const __half2*)&cw;
-                    float c[8], d = 0.f;
+            for (int q = 0; q < 4; q++) {
+                const int k = bg * 16 + w * 4 + q;
+                const float d = at_dist(at_smem, book, q2, ibs, xv, k);
+                if (d < bd || (d == bd && k < bi)) { bd = d; bi = k; }
+            }
+            // What two groups' values can be off by against each other.  Relative to the largest term or sum, 2^-24 for each of the 17
+            // addends of an MMA, two MMAs, and 2^-23 of the products for the split; of two groups near the minimum d that is at
+            // most 2e-5 of |d| + |x|^2.  And the last place of the parts in fp16, 2^-25, times the sizes of a word's eight values.
+            // Every group that is no further from the best is evaluated; a warpgroup knows two, so where its second is among them
+            // (or the values are not finite) all words are.  A chunk at a time: of N(0, 1) chunks and words one in 1700 comes here.
+            const float margin = 2e-5f * (fabsf(best) + f * (bs * bs) * xx) + 0x1p-23f * (4.f * top * bs + 1.f);
+            bool close = false;
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const float2 p = __half22float2(h[i]);
-                        c[2 * i] = q2 > 0 ? p.x * ibs : p.x;
-                        c[2 * i + 1] = q2 > 0 ? p.y * ibs : p.y;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 8; i++) d += c[i] * c[i];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) d = fmaf(-2.0f * xv[i], c[i], d);
-                    if (d < bd || (d == bd && k < bi)) { bd = d; bi = k; }
+            for (int q = 0; q < 4; q++) {
+                const AtPart p = s_part[q * AT_TILE + row];
+                close |= !((p.bg == bg ? p.second : p.best) - best > margin);
+            }
+            for (uint32_t todo = __ballot_sync(0xffffffffu, close); todo; todo &= todo - 1) {
+                const int who = __ffs(todo) - 1, rw = (warp & 3) * 32 + who;
+                const float bw = __shfl_sync(0xffffffffu, best, who), mw = __shfl_sync(0xffffffffu, margin, who);
+                const float4* xw = (const float4*)(st + 2 * AT_A_BYTES) + rw;
+                bool all = false;
+#pragma unroll 1
+                for (int q = 0; q < 4; q++) all |= !(s_part[q * AT_TILE + rw].second - bw > mw);
+#pragma unroll 1
+                for (int q = 0; q < (all ? 1 : 4); q++) {
+                    const AtPart p = s_part[q * AT_TILE + rw];
+                    if (!all && !(p.best - bw <= mw)) continue;
+                    const int k0 = all ? w * (K / 4) : p.bg * 16 + w * 4;
+                    const float2 r = at_nearest(at_smem, book, q2, ibs, xw[0], xw[AT_TILE], k0, k0 + (all ? K / 4 : 4));
+                    const int i = __float_as_int(r.y);
+                    if (lane == who && (r.x < bd || (r.x == bd && i < bi))) { bd = r.x; bi = i; }
                 }
-            };
-            exact(bg);
-            // what the split operands and the accumulation can be off by, several times over
-            if ((second - best) <= 1e-5f * f * (bs * bs) * (fabsf(bd) + xx)) exact(sg);
+            }
             s_ex[w * AT_TILE + row] = make_float2(bd, __int_as_float(bi));
             asm volatile("bar.sync 1, %0;" ::"n"(AT_EPI) : "memory");
             if (w == 0) {

@@ -198,3 +198,28 @@ def test_snap_of_strided_rows(weighted):
         cw = torch.rand(w.shape[1], device="cuda", generator=g) + 0.5 if weighted else None
         got, want = cb.snap(w, book, col_weight=cw), cb.snap(w.clone(memory_format=torch.contiguous_format), book, col_weight=cw)
         assert torch.equal(got["idx"], want["idx"]) and torch.equal(got["row_scale"], want["row_scale"]) and torch.equal(got.err, want.err)
+
+
+def test_tensor_core_assign_equals_the_scalar_kernel_where_many_words_all_but_tie():
+    """Words that differ in the last bits of one fp16 value: many groups of 16 lie closer together than the tensor cores can tell. Also
+    chunks and words that are tiny beside the book's largest value, and chunks that are not finite.  Fewer than 512 chunks run on the scalar kernel."""
+    from quantexperiments_b200 import codebook as cb
+    g = torch.Generator().manual_seed(11)
+    centre = torch.randn(16, 8, generator=g)
+    near = centre[torch.randint(0, 16, (4096,), generator=g)].half()
+    near[torch.arange(4096), torch.randint(0, 8, (4096,), generator=g)] *= 1 + 2.0 ** -10
+    tiny = torch.randn(4096, 8, generator=g)
+    tiny[8:] *= 2.0 ** -10
+    for book, size in ((near, 1.0), (tiny.half(), 2.0 ** -10)):
+        x = (centre[torch.randint(0, 16, (6000,), generator=g)] if size == 1.0 else torch.randn(6000, 8, generator=g)) * size
+        x += 0.02 * size * torch.randn(6000, 8, generator=g)
+        x[3, 2], x[700, 0], x[1500] = float("inf"), float("-inf"), float("nan")
+        idx, err = cb.assign(x.cuda(), book.cuda())
+        few = [cb.assign(c.cuda(), book.cuda()) for c in x.split(500)]
+        want, werr = torch.cat([i for i, _ in few]), torch.cat([e for _, e in few])
+        fin = x.isfinite().all(1).cuda()
+        dist = lambda i: ((x.cuda().double() - book.cuda().double()[i]) ** 2).sum(1)
+        # the two kernels add |c|^2 in the same order; a word that both evaluate has the same distance bit for bit
+        assert torch.equal(idx, want), int((idx != want).sum())
+        assert torch.equal(err[fin], werr[fin])
+        assert ((dist(idx) - dist(want)).abs()[fin] == 0).all()
