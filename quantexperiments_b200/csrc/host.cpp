@@ -144,6 +144,14 @@ bool layout_for(const Plan& p, int64_t tokens) {
     return p.has_dense && tokens >= p.dense_from;
 }
 
+// Whether the plan's bias can be added by the kernel to products of x: one value per row, x's type and device, nobody's gradient.  Others
+// broadcast, convert or are recorded by the addition in Python.
+bool adds_in_kernel(const Plan& p, const at::Tensor& x) {
+    const at::Tensor& b = p.bias;
+    return b.dim() == 1 && b.size(0) == p.R && b.scalar_type() == x.scalar_type() && b.is_contiguous() && b.is_cuda() && b.get_device() == p.device &&
+           !b.requires_grad();
+}
+
 // forward(plan or tuple of plans, x): x [..., in] -> y [..., sum of R] in x's dtype (+ bias), or None.  Several plans write
 // column slices of one output (pieces of a stacked layer with column orders of their own).
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -168,7 +176,7 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     int64_t R = 0;
     for (int i = 0; i < np; i++) {
         const Plan& q = *plans[i];
-        if (!layout_for(q, tokens) || (q.bias.defined() && (q.bias.scalar_type() != x.scalar_type() || !q.bias.is_contiguous()))) Py_RETURN_NONE;
+        if (!layout_for(q, tokens) || (q.bias.defined() && !adds_in_kernel(q, x))) Py_RETURN_NONE;
         R += q.R;
     }
     try {

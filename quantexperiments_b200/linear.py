@@ -109,12 +109,12 @@ class PackedLinear(torch.nn.Module):
 
     def _bind(self) -> None:
         """(Re)makes the native call plan from the layouts that exist."""
-        dm = self.dm
-        if not dm.fast or (self.bias is not None and self.bias.requires_grad):
+        dm, b = self.dm, self.bias
+        if not dm.fast or (b is not None and (b.requires_grad or b.shape != (self.R,))):
             return
-        self._host_bias = self.bias
+        self._host_bias = b
         self._host = _cblhost.plan(dm.device.index, self.in_features, self.C, dm.M, [self.R], 0 if dm.perms is None else dm.perms.data_ptr(),
-                                   DENSE_MIN_TOKENS, self.bias)
+                                   DENSE_MIN_TOKENS, b)
         if self._l8 is not None and self.use_l8():
             _cblhost.set(self._host, "l8", bytes(self._l8.struct()))
         for g in self._b3.values():

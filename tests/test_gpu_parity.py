@@ -292,6 +292,28 @@ def test_one_token_of_few_rows_is_summed_in_fp32(R, C, books, M):
         assert (got.double() - ref).norm() <= books * (C / 16) * 2.0 ** -23 * ref.norm()
 
 
+@pytest.mark.parametrize("tokens", [1, 5, 200])
+def test_bias_of_another_shape_or_type_is_added_as_torch_would(tokens):
+    """The native call path adds a bias of one value per row and x's type; every other form gives what `y + bias` gives, on every call."""
+    m = orc.synth_matrix(2100, 256, seed=8)
+    plain = _linear(m)
+    x = torch.randn(tokens, 256, generator=torch.Generator().manual_seed(2)).bfloat16().cuda()
+    y = plain(x)
+    g = torch.Generator().manual_seed(3)
+    for bias in (torch.randn(1, generator=g).bfloat16(), torch.randn((), generator=g).bfloat16(), torch.randn(1, 2100, generator=g).bfloat16(),
+                 torch.randn(2100, generator=g), torch.randn(2100, 2, generator=g).bfloat16()[:, 0], torch.randn(2100, generator=g).bfloat16()):
+        lin = _linear(m, bias=bias.cuda())
+        for _ in range(3):
+            got = lin(x)
+            assert got.dtype == (y + lin.bias).dtype and torch.equal(got, y + lin.bias)
+    lin.bias.requires_grad_()
+    assert lin(x).requires_grad
+    lin(x).float().sum().backward()
+    assert torch.equal(lin.bias.grad, torch.full_like(lin.bias, tokens))
+    lin.bias = torch.nn.Parameter(lin.bias.detach()[:1])
+    assert torch.equal(lin(x), y + lin.bias)
+
+
 def test_runs_lin_of_several_column_orders_is_ready_for_capture():
     """RunsLin builds the layout that its one-token run reads in its constructor, not inside a captured region."""
     from quantexperiments_b200.linear import RunsLin
