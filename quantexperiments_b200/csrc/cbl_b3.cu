@@ -127,7 +127,7 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     __shared__ __align__(8) unsigned long long s_bar[B3_MAX_ST + 2 * B3_MAX_RX + 4];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_nfin;
-    __shared__ int s_parts[B3_MAX_PIECES][2];                 // for each of its books: first and last block, its number among the first block's pieces (8, 8, 8 bits)
+    __shared__ int s_parts[B3_MAX_PIECES][2];                 // for each of its books: first and last block, the first block's slot (8, 8, 8 bits)
     __shared__ int s_fin[B3_MAX_PIECES];                       // tiles (as gi of their first book) that this block has to finish
     const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     const int cta = (int)blockIdx.x;
@@ -150,7 +150,9 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     const uint32_t xbytes = (uint32_t)P.xrows * 128u, xstage = xbytes * (uint32_t)XU, a_col0 = 2u * (uint32_t)P.npad;
     auto seg_of = [&](int gi) { int s = 0; while (s + 1 < P.nseg && gi >= P.seg[s].gi1) s++; return s; };
     auto wait = [&](uint32_t bar, uint32_t parity) { return b3_wait(bar, parity, &s_abort); };
-    auto slot_of = [&](int c, int gi) { return P.partial + (size_t)(c * P.PP + gi - start(c) / nkb) * (size_t)(P.npad * B3_ROWS); };
+    // slot of a block for its piece of tile gi (with one book all but a block's first and last piece are whole tiles: two slots)
+    auto slot_no = [&](int c, int gi) { return min(gi - start(c) / nkb, P.PP - 1); };
+    auto slot_of = [&](int c, int gi) { return P.partial + (size_t)(c * P.PP + slot_no(c, gi)) * (size_t)(P.npad * B3_ROWS); };
 
     if (tid == 0) {
         s_abort = s_nfin = 0;
@@ -414,7 +416,7 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                     const int g = m.gi0 + k * m.ntile + tile, c0 = owner(g * nkb), ce = owner(g * nkb + nkb - 1);
                     np += ce - c0 + 1;
                     // a tile is the last piece of its first block and the first piece of the others
-                    if (warp == B3_EPI_WARP && lane == 0) s_parts[s_nfin][k] = c0 | ce << 8 | (g - start(c0) / nkb) << 16;
+                    if (warp == B3_EPI_WARP && lane == 0) s_parts[s_nfin][k] = c0 | ce << 8 | slot_no(c0, g) << 16;
                 }
             unsigned int* const ctr = P.counters + m.ctr0 + tile;
             T* const yr = (T*)m.y + max(r, 0);
@@ -653,13 +655,22 @@ __global__ void __launch_bounds__(256) k_repack_b3(cbl_packed m, const int32_t* 
 
 struct B3Plan { int T, U, G, PP, ks, npad, rows, NST, RX, XU; };
 
-int b3_plan(const cbl_b3* mats, int n, int ntok, B3Plan& pl) {
-    pl.T = 0;
-    int tiles = 0;
-    for (int i = 0; i < n; i++) { pl.T += mats[i].ntile * mats[i].books; tiles += mats[i].ntile; }
+// Tiles t0 .. t0 + nt - 1 of a matrix, and where its outputs go.
+struct B3Part { const cbl_b3* m; int t0, nt; void* y; const void* bias; };
+
+int b3_plan(const B3Part* parts, int n, int ntok, B3Plan& pl) {
+    const cbl_b3* mats = parts[0].m;
+    int64_t tiles = 0, all = 0;
+    bool two = false;
+    for (int i = 0; i < n; i++) {
+        all += (int64_t)parts[i].nt * parts[i].m->books;
+        tiles += parts[i].nt;
+        two |= parts[i].m->books == 2;
+    }
     if (tiles > B3_MAX_TILES) return CBL_EUNSUPPORTED;
     const int nkb = cbl_ceil_div(mats[0].C, B3_KB), S = cbl_sm_count();
-    if ((int64_t)pl.T * nkb > (1 << 30)) return CBL_EUNSUPPORTED;
+    if (all * nkb > (1 << 30)) return CBL_EUNSUPPORTED;
+    pl.T = (int)all;
     pl.U = pl.T * nkb;
     pl.npad = (ntok + 15) / 16 * 16;
     pl.NST = (512 - 2 * pl.npad) / 128;                        // stages of four decoded k-blocks in tensor memory, beside two accumulators
@@ -676,7 +687,8 @@ int b3_plan(const cbl_b3* mats, int n, int ntok, B3Plan& pl) {
     // SMs the cut follows them, so that a block has one piece; otherwise ranges run across tile borders.
     int G = S;
     pl.ks = 0;
-    if (pl.T < S) {
+    if (pl.T == 0) G = 1;                                      // no rows
+    else if (pl.T < S) {
         int ks = S / pl.T;
         const int least = 6 + ntok / 8, most = nkb / least > 1 ? nkb / least : 1;
         if (ks > most) ks = most;
@@ -685,11 +697,40 @@ int b3_plan(const cbl_b3* mats, int n, int ntok, B3Plan& pl) {
         const int waves = cbl_ceil_div(pl.T, S), g = cbl_ceil_div(pl.T, waves);
         if (pl.T % g == 0 && g * 100 >= 85 * S) G = g;
     }
-    if (G > pl.U) { G = pl.U; pl.ks = 0; }
+    if (pl.U > 0 && G > pl.U) { G = pl.U; pl.ks = 0; }
     pl.G = G;
     pl.PP = pl.U == 0 ? 1 : cbl_ceil_div(cbl_ceil_div(pl.U, G), nkb) + 1;
+    if (!two && pl.PP > 2) pl.PP = 2;
     return pl.PP > B3_MAX_PIECES ? CBL_EUNSUPPORTED : CBL_OK;
 }
+
+// Calls f(parts, n, plan) for the launches of a group: one, or, of matrices beyond a launch's limits (2 M rows), one per range of tiles.
+template <typename F>
+int b3_launches(const cbl_b3* mats, int n, void* const* ys, int esz, int ntok, F&& f) {
+    B3Part parts[B3_MAX_MATS];
+    B3Plan pl;
+    for (int i = 0; i < n; i++) parts[i] = {mats + i, 0, mats[i].ntile, ys ? ys[i] : nullptr, mats[i].bias};
+    if (b3_plan(parts, n, ntok, pl) == CBL_OK) return f(parts, n, pl);
+    const int64_t nkb = cbl_ceil_div(mats[0].C, B3_KB);
+    for (int i = 0; i < n; i++) {
+        // about 64 tiles of each book per block
+        int64_t most = (1 << 30) / (nkb * mats[i].books);
+        const int64_t per = 64 * cbl_sm_count() / mats[i].books;
+        most = most < per ? most : per;
+        if (most > B3_MAX_TILES) most = B3_MAX_TILES;
+        if (most < 1) return CBL_EUNSUPPORTED;
+        for (int64_t t0 = 0; t0 < mats[i].ntile; t0 += most) {
+            const int nt = (int)(mats[i].ntile - t0 < most ? mats[i].ntile - t0 : most);
+            const int64_t at = mats[i].tile_rows ? 0 : t0 * B3_ROWS * esz;          // bytes: rows in order start at the part's first
+            const B3Part part = {mats + i, (int)t0, nt, ys ? (char*)ys[i] + at : nullptr, mats[i].bias ? (const char*)mats[i].bias + at : nullptr};
+            int rc = b3_plan(&part, 1, ntok, pl);
+            if (!rc) rc = f(&part, 1, pl);
+            if (rc) return rc;
+        }
+    }
+    return CBL_OK;
+}
+
 
 int b3_check(const cbl_b3* m, const cbl_b3* first) {
     if (!m->words || !m->table || !m->row_scale) return CBL_EINVAL;
@@ -729,10 +770,16 @@ extern "C" int cbl_repack_b3(const cbl_packed* m, const int32_t* tile_rows, int3
 
 extern "C" size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int32_t ntok) {
     if (!mats || n < 1 || n > B3_MAX_MATS || ntok < 1 || ntok > cbl_gemm_b3_max_tokens(mats[0].copies) || mats[0].C <= 0) return 0;
-    B3Plan pl;
-    if (b3_plan(mats, n, ntok, pl)) return 0;
-    return (size_t)B3_CTL_WORDS * 4 + (size_t)pl.G * pl.PP * pl.npad * B3_ROWS * 4;
+    size_t most = 0;
+    const int rc = b3_launches(mats, n, nullptr, 0, ntok, [&](const B3Part*, int, const B3Plan& pl) {
+        const size_t bytes = (size_t)B3_CTL_WORDS * 4 + (size_t)pl.G * pl.PP * pl.npad * B3_ROWS * 4;
+        if (bytes > most) most = bytes;
+        return CBL_OK;
+    });
+    return rc ? 0 : most;
 }
+
+static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, int ntok, int64_t ldy, void* stage, void* workspace, cbl_stream s);
 
 extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
                            int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
@@ -746,16 +793,22 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
         if (rc) return rc;
         if (!ys[i] || (ntok > 1 && ldy < mats[i].R)) return CBL_EINVAL;
     }
-    const int C = mats[0].C, M = mats[0].M;
-    if (M > 1 && !perms) return CBL_EINVAL;
-    B3Plan pl;
-    int rc = b3_plan(mats, n, ntok, pl);
-    if (rc) return rc;
-    if (pl.U == 0) return CBL_OK;
-    if (x) {                                                   // x == NULL: the caller has staged the activations
-        rc = cbl_prep_x(x, xdtype, ntok, C, ldx, perms, M, stage, s);
-        if (rc) return rc;
-    }
+    if (mats[0].M > 1 && !perms) return CBL_EINVAL;
+    bool any = false, staged = x == nullptr;                   // x == NULL: the caller has staged the activations
+    for (int i = 0; i < n; i++) any |= mats[i].ntile > 0;
+    if (!any) return CBL_OK;
+    return b3_launches(mats, n, ys, ydtype == CBL_F32 ? 4 : 2, ntok, [&](const B3Part* parts, int k, const B3Plan& pl) {
+        if (!staged) {
+            const int rc = cbl_prep_x(x, xdtype, ntok, mats[0].C, ldx, perms, mats[0].M, stage, s);
+            if (rc) return rc;
+            staged = true;
+        }
+        return b3_launch(parts, k, pl, ydtype, ntok, ldy, stage, workspace, s);
+    });
+}
+
+static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, int ntok, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
+    const int C = parts[0].m->C, M = parts[0].m->M, copies = parts[0].m->copies;
     const int Bpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
     B3Launch P;
     P.nkb = cbl_ceil_div(C, B3_KB);
@@ -768,17 +821,19 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
     P.nseg = 0;
     int gi = 0, ctr = 0;
     for (int i = 0; i < n; i++) {
-        const cbl_b3& m = mats[i];
+        const cbl_b3& m = *parts[i].m;
+        const int t0 = parts[i].t0, nt = parts[i].nt, r0 = m.tile_rows ? 0 : t0 * B3_ROWS;
         B3Mat& o = P.mat[i];
-        o.row_scale = (const __half*)m.row_scale; o.tile_rows = m.tile_rows; o.tile_order = M > 1 ? m.tile_order : nullptr;
-        o.bias = m.bias; o.y = ys[i]; o.R = m.R; o.ntile = m.ntile; o.gi0 = gi; o.books = m.books; o.ctr0 = ctr;
-        ctr += m.ntile;
-        for (int k = 0; k < m.books && m.ntile > 0; k++) {
+        o.row_scale = (const __half*)m.row_scale + r0; o.tile_rows = m.tile_rows ? m.tile_rows + (size_t)t0 * B3_ROWS : nullptr;
+        o.tile_order = M > 1 ? m.tile_order + t0 : nullptr;
+        o.bias = parts[i].bias; o.y = parts[i].y; o.R = m.R - r0; o.ntile = nt; o.gi0 = gi; o.books = m.books; o.ctr0 = ctr;
+        ctr += nt;
+        for (int k = 0; k < m.books && nt > 0; k++) {
             B3Seg& sg = P.seg[P.nseg++];
-            sg.words = (const uint4*)m.words + (size_t)k * m.ntile * P.nkb * B3_ROWS;
+            sg.words = (const uint4*)m.words + ((size_t)k * m.ntile + t0) * P.nkb * B3_ROWS;
             sg.table = (const uint4*)(k ? m.table2 : m.table);
-            sg.gi0 = gi; sg.gi1 = gi + m.ntile; sg.mi = i;
-            gi += m.ntile;
+            sg.gi0 = gi; sg.gi1 = gi + nt; sg.mi = i;
+            gi += nt;
         }
     }
     if (pl.G > B3_MAX_BLOCKS) return CBL_EUNSUPPORTED;
@@ -833,7 +888,7 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
     cfg.gridDim = dim3(pl.G);
     cfg.blockDim = dim3(B3_THREADS);
     cfg.dynamicSmemBytes = B3_SMEM;
-    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[(mats[0].copies - 2) * 3 + ydtype], xmap, xmap1, P));
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[(copies - 2) * 3 + ydtype], xmap, xmap1, P));
     return cbl_check_launch();
 }
 

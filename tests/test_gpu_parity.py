@@ -952,3 +952,29 @@ def test_copy_layout_is_the_matrix_and_spreads_the_banks(copies, limit):
     banks = (slots & 7).reshape(b.ntile, -1, 16, 8, 8)                                         # groups of eight rows
     fullest = np.max([(banks == k).sum(3) for k in range(8)], axis=0)
     assert fullest[:4].mean() < limit
+
+
+@pytest.mark.parametrize("R,C,books,M", [(2_100_000, 64, 1, 1), (2_100_000, 72, 2, 3), (1_300_000, 8, 2, 1)])
+def test_gather_product_of_more_rows_than_a_launch_takes(R, C, books, M):
+    """Very tall matrices run as several launches over ranges of row tiles: outputs, biases, row scales and column orders keep their rows."""
+    from quantexperiments_b200.kernels import B3Group, B3Matrix, DeviceMatrix
+    g = torch.Generator(device="cuda").manual_seed(R + C)
+    W = (C // 8 * 12 + 31) // 32
+    words = [torch.randint(-2**31, 2**31 - 1, (R, W), dtype=torch.int32, device="cuda", generator=g) for _ in range(books)]
+    table = [torch.randn(4096, 8, device="cuda", generator=g).half() for _ in range(books)]
+    rs = (torch.rand(R, device="cuda", generator=g) + 0.5).half()
+    more = dict(tags2=words[1], table2=table[1]) if books == 2 else {}
+    mask = torch.randint(0, M, (R,), device="cuda", generator=g).to(torch.uint8) if M > 1 else None
+    perms = torch.from_numpy(orc.seeded_perms(C, M, 5)) if M > 1 else None
+    dm = DeviceMatrix(words[0], table[0], rs, None, mask, perms, K=4096, d=8, C=C, **more)
+    w = dm.dequant()
+    bias = torch.randn(R, device="cuda", generator=g)
+    for B, copies in ((1, 3), (20, 2)):
+        X = torch.randn(B, C, device="cuda", generator=g).half().float()
+        for b in (None, bias):
+            grp = B3Group([B3Matrix(dm, copies)], [b])
+            got = grp.run(X, [torch.full((B, R), float("nan"), device="cuda")])[0]
+            want = X @ w.T if b is None else X @ w.T + b
+            assert (got - want).abs().max() <= 1e-5 * C ** 0.5 * want.abs().max()
+            del got, want
+        grp.status()

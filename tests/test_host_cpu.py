@@ -173,3 +173,19 @@ def test_engine_sampling_helper_and_config_defaults():
     a = [_sample(logits, 1.0, 0.9, 0, torch.Generator().manual_seed(5)) for _ in range(3)]
     b = [_sample(logits, 1.0, 0.9, 0, torch.Generator().manual_seed(5)) for _ in range(3)]
     assert a == b                                                   # seeded draws repeat
+
+
+def test_gather_product_work_space_holds_what_is_written():
+    """cbl_gemm_b3: a block writes pieces of at most its first and last tile where a matrix has one book; any number of rows has a plan."""
+    lib = _lib.lib
+    def ws(R, C, books, ntok, copies=2, n=1):
+        mats = (_lib.B3 * n)(*[_lib.B3(R, C, books, 1, -(-R // 128), copies) for _ in range(n)])
+        return lib.cbl_gemm_b3_workspace_bytes(mats, n, ntok)
+    slot = 128 * 128 * 4                                       # a tile's rows x 128 tokens, fp32
+    for R, C in ((152064, 3584), (18944, 3584), (3584, 18944), (128, 64), (1, 8)):
+        assert 0 < ws(R, C, 1, 128) <= 65536 + 2 * 160 * slot
+    assert ws(152064, 3584, 2, 128) >= 65536 + 148 * 2 * slot
+    for R, C, books in ((4_000_000, 64, 1), (2_200_000, 8, 2), (2_080_000, 64, 2), (1 << 30, 64, 1)):
+        assert ws(R, C, books, 16, 3) > 65536, (R, C, books)
+    assert ws(1_200_000, 64, 1, 16, 3, n=4) > 65536
+    assert ws(0, 64, 1, 16) > 0
