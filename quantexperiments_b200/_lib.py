@@ -154,12 +154,16 @@ SIGNATURES = {
 }
 
 
-def _load() -> ctypes.CDLL:
+def _load() -> ctypes.PyDLL:
     if not LIB_PATH.exists():
         raise ImportError(f"{LIB_PATH} is missing: run `python -m quantexperiments_b200.build` "
                           "(there is no CPU or PyTorch fallback for these kernels)")
-    lib = ctypes.CDLL(str(LIB_PATH))
+    # A call that launches keeps the interpreter lock, so that the launches of one call (the activations' staging, then the product that
+    # reads it) are not interleaved with those of another thread that uses the stream's scratch.  Calls that wait for the GPU let go of it.
+    lib, waits = ctypes.PyDLL(str(LIB_PATH)), ctypes.CDLL(str(LIB_PATH))
     for name, (res, args) in SIGNATURES.items():
+        if name.endswith("_status") or name == "cbl_book_norm_exp":
+            setattr(lib, name, getattr(waits, name))
         fn = getattr(lib, name)          # AttributeError if the library lacks a declared symbol
         fn.restype, fn.argtypes = res, args
     return lib

@@ -6,12 +6,16 @@
 // does the work and fills the plan.  Per call the Python path spends 20 (one token) to 45 us (many tokens) on the host, which is more
 // than most products of a decode step run on the GPU; this one spends 4 to 8.
 //
-// Scratch buffers (staged activations, partial sums, decoded weights) belong to a (device, stream) pair, grow on demand and
-// live as long as the process; an outgrown one stays alive because a captured graph may still point at it.
+// Scratch buffers (staged activations, partial sums, decoded weights) belong to a (device, stream) pair and grow on demand; the
+// Python call paths take theirs from here as well (scratch()).  Calls on one stream share them in the order of the stream; graphs
+// captured on one stream share them too and are replayed one after another.  A buffer that a captured graph has been given lives as
+// long as the process (the graph holds its address); others go back to torch's allocator, in stream order, when they are outgrown,
+// when the last plan of their device is gone, or by release().
 #include <Python.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
+#include <ATen/ops/from_blob.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -48,27 +52,75 @@ struct Plan {
     int dense_from = 0;                                   // tokens from which the two-phase product runs
 };
 
+struct Buffer {
+    at::Tensor t;
+    bool in_graph = false;
+};
+enum Kind { L8, STAGE, PARTIAL, WEIGHTS, DENSE_STAGE, KINDS };
 struct Scratch {
-    at::Tensor l8, stage, partial, weights[2], dense_stage;
+    Buffer b[KINDS], second;                              // second: the other of the two alternating buffers of decoded weights
     int turn = 0;
 };
 
-std::mutex g_mu;
+std::mutex g_mu;                                          // (everything below also runs with the interpreter lock held)
 std::map<std::pair<int, void*>, Scratch> g_scratch;
-std::vector<at::Tensor> g_retired;
+std::vector<at::Tensor> g_kept;                           // outgrown buffers that a graph points at
+std::map<int, long> g_plans;                              // plans alive per device
 
-Scratch& scratch_of(int device, void* stream) {           // (call with g_mu held; the reference stays valid)
-    return g_scratch[{device, stream}];
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusActive;
 }
 
-void* need(at::Tensor& t, size_t bytes, size_t least, bool zero, int device) {
-    if (!t.defined() || (size_t)t.numel() < bytes) {
-        if (t.defined()) g_retired.push_back(t);
+// Memory for a captured region that first asks for it there: it must hold zeros now, not when the graph is replayed, and be no part
+// of the graph's own pool, whose blocks its earlier nodes may write.
+at::Tensor beside_graph(int64_t n, int device) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    TORCH_CHECK(cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess, "capture mode");
+    void* p = nullptr;
+    cudaStream_t own = nullptr;
+    cudaError_t e = cudaMalloc(&p, (size_t)n);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, (size_t)n, own);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+    if (own) cudaStreamDestroy(own);
+    if (e != cudaSuccess && p) cudaFree(p);
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    TORCH_CHECK(e == cudaSuccess, "scratch of ", n, " bytes for a captured region: ", cudaGetErrorString(e));
+    return at::from_blob(p, {n}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+}
+
+// The buffer of a kind on (device, current stream), at least `bytes` long; status words and arrival counters are zero when it is new.
+const at::Tensor& need(Kind kind, size_t bytes, int device, void* stream) {
+    static const size_t least[KINDS] = {16 << 20, 4 << 20, 16 << 20, 16, 16};
+    std::lock_guard<std::mutex> lock(g_mu);
+    Scratch& sc = g_scratch[{device, stream}];
+    if (kind == WEIGHTS) sc.turn ^= 1;                    // the decode of a product may run beside the GEMM of the one before
+    Buffer& b = kind == WEIGHTS && sc.turn ? sc.second : sc.b[kind];
+    const bool graph = capturing((cudaStream_t)stream);
+    if (!b.t.defined() || (size_t)b.t.numel() < bytes) {
+        if (b.in_graph) g_kept.push_back(b.t);
+        b = Buffer();
+        const int64_t n = (int64_t)std::max(bytes, least[kind]);
         const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device);
-        const int64_t n = (int64_t)std::max(bytes, least);
-        t = zero ? at::zeros({n}, opt) : at::empty({n}, opt);
+        b.t = graph ? beside_graph(n, device) : kind == STAGE || kind == WEIGHTS ? at::empty({n}, opt) : at::zeros({n}, opt);
     }
-    return t.data_ptr();
+    b.in_graph |= graph;
+    return b.t;
+}
+
+void drop(int device) {                                   // (with g_mu held)
+    for (auto& e : g_scratch) {
+        if (e.first.first != device) continue;
+        for (Buffer& b : e.second.b)
+            if (!b.in_graph) b = Buffer();
+        if (!e.second.second.in_graph) e.second.second = Buffer();
+    }
 }
 
 PyObject* fail(const char* fn, int rc) {
@@ -80,6 +132,28 @@ int dtype_of(at::ScalarType t) { return t == at::kBFloat16 ? CBL_BF16 : t == at:
 
 Plan* plan_of(PyObject* o) { return (Plan*)PyCapsule_GetPointer(o, PLAN); }
 
+// Matrices that read the same activations, decoded into the scratch and multiplied by the GEMM over the stacked rows.  `staged`: the
+// activations as cbl_prep_x lays them out (x NULL).  wide: C is the length of the activations that a column shard's orders name.
+int dense_product(const cbl_packed* m, int n, int32_t C, bool wide, const void* row_scale, const void* x, int xdt, int64_t tokens, int64_t ldx, void* staged,
+                  void* y, int ydt, int64_t ldy, const void* bias, int device, void* stream, const char** fn) {
+    const cbl_stream s = (cbl_stream)stream;
+    int64_t R = 0;
+    for (int i = 0; i < n; i++) R += m[i].R;
+    char* const w = (char*)need(WEIGHTS, cbl_dense_scratch_bytes((int32_t)R, C), device, stream).data_ptr();
+    const at::Tensor& st = need(DENSE_STAGE, cbl_gemm_stage_bytes(x ? (int32_t)tokens : 8, C) + 16, device, stream);
+    char* const stage = (char*)st.data_ptr();
+    const int64_t ld = ((int64_t)C + 7) / 8 * 8;
+    int64_t row = 0;
+    for (int i = 0; i < n; i++) {
+        *fn = wide ? "cbl_decode_raw_wide" : "cbl_decode_raw";
+        const int rc = wide ? cbl_decode_raw_wide(m + i, w + row * ld * 2, C, s) : cbl_decode_raw(m + i, w + row * ld * 2, s);
+        if (rc) return rc;
+        row += m[i].R;
+    }
+    *fn = "cbl_gemm_dense";
+    return cbl_gemm_dense_bias(w, (int32_t)R, C, row_scale, x, xdt, (int32_t)tokens, ldx, y, ydt, ldy, bias, x ? stage : staged, stage + st.numel() - 16, s);
+}
+
 // One product of `tokens` tokens into y [tokens, R] (row stride ldy); CBL_EUNSUPPORTED when the plan has no layout for them.
 int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* y, int ydt, int64_t ldy, const void* bias, void* stream, const char** fn) {
     const int esz = ydt == CBL_F32 ? 4 : 2;
@@ -87,11 +161,7 @@ int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* 
     for (int i = 0; i < p.n; i++) ys[i] = y + p.first[i] * esz;
     const cbl_stream s = (cbl_stream)stream;
     if (tokens == 1 && p.has_l8) {
-        void* ws;
-        {
-            std::lock_guard<std::mutex> lock(g_mu);
-            ws = need(scratch_of(p.device, stream).l8, p.l8_bytes, 16 << 20, true, p.device);
-        }
+        void* const ws = need(L8, p.l8_bytes, p.device, stream).data_ptr();
         const void* biases[MAX_PIECES] = {};
         if (bias) for (int i = 0; i < p.n; i++) biases[i] = (const char*)bias + p.first[i] * esz;
         *fn = "cbl_gemv_l8_bias";
@@ -102,13 +172,8 @@ int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* 
         if (!p.has_b3[k]) return CBL_EUNSUPPORTED;
         size_t& wb = p.ws_bytes[k][tokens];
         if (!wb) wb = cbl_gemm_b3_workspace_bytes(p.b3[k], p.n, (int32_t)tokens);
-        void *stage, *ws;
-        {
-            std::lock_guard<std::mutex> lock(g_mu);
-            Scratch& sc = scratch_of(p.device, stream);
-            stage = need(sc.stage, cbl_prep_x_bytes((int32_t)tokens, (int32_t)p.C, p.orders), 4 << 20, false, p.device);
-            ws = need(sc.partial, wb, 16 << 20, true, p.device);
-        }
+        void* const stage = need(STAGE, cbl_prep_x_bytes((int32_t)tokens, (int32_t)p.C, p.orders), p.device, stream).data_ptr();
+        void* const ws = need(PARTIAL, wb, p.device, stream).data_ptr();
         cbl_b3 mats[MAX_PIECES];
         for (int i = 0; i < p.n; i++) {
             mats[i] = p.b3[k][i];
@@ -118,24 +183,7 @@ int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* 
         return cbl_gemm_b3(mats, p.n, x, xdt, (int32_t)tokens, ldx, p.perms, ys, ydt, ldy, stage, ws, s);
     }
     if (!p.has_dense || tokens < p.dense_from) return CBL_EUNSUPPORTED;
-    char *w, *stage, *status;
-    {
-        // two scratch buffers alternate: the decode of this product may run beside the GEMM of the one before
-        std::lock_guard<std::mutex> lock(g_mu);
-        Scratch& sc = scratch_of(p.device, stream);
-        sc.turn ^= 1;
-        w = (char*)need(sc.weights[sc.turn], cbl_dense_scratch_bytes((int32_t)p.R, (int32_t)p.C), 0, false, p.device);
-        stage = (char*)need(sc.dense_stage, cbl_gemm_stage_bytes((int32_t)tokens, (int32_t)p.C) + 16, 0, true, p.device);
-        status = stage + sc.dense_stage.numel() - 16;
-    }
-    const int64_t ld = (p.C + 7) / 8 * 8;
-    for (int i = 0; i < p.n; i++) {
-        *fn = "cbl_decode_raw";
-        const int rc = cbl_decode_raw(&p.packed[i], w + p.first[i] * ld * 2, s);
-        if (rc) return rc;
-    }
-    *fn = "cbl_gemm_dense";
-    return cbl_gemm_dense_bias(w, (int32_t)p.R, (int32_t)p.C, p.row_scale, x, xdt, (int32_t)tokens, ldx, y, ydt, ldy, bias, stage, status, s);
+    return dense_product(p.packed, p.n, (int32_t)p.C, false, p.row_scale, x, xdt, tokens, ldx, nullptr, y, ydt, ldy, bias, p.device, stream, fn);
 }
 
 bool layout_for(const Plan& p, int64_t tokens) {
@@ -201,7 +249,15 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
 }
 
-void free_plan(PyObject* o) { delete plan_of(o); }
+void free_plan(PyObject* o) {
+    Plan* p = plan_of(o);
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        if (--g_plans[p->device] == 0) drop(p->device);
+    }
+    delete p;
+}
 
 // plan(device, in, C, orders, rows: list, perms pointer, dense_from, bias or None) -> capsule
 PyObject* py_plan(PyObject*, PyObject* args) {
@@ -221,6 +277,10 @@ PyObject* py_plan(PyObject*, PyObject* args) {
         p->l8_bytes += cbl_gemv_l8_workspace_bytes((int32_t)p->rows[i]);
     }
     if (bias != Py_None && THPVariable_Check(bias)) p->bias = THPVariable_Unpack(bias);
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        g_plans[device]++;
+    }
     return PyCapsule_New(p, PLAN, free_plan);
 }
 
@@ -268,13 +328,17 @@ PyObject* py_status(PyObject*, PyObject* args) {
         std::lock_guard<std::mutex> lock(g_mu);
         for (auto& e : g_scratch) {
             if (e.first.first != device) continue;
-            Scratch& s = e.second;
-            if (s.l8.defined() && cbl_gemv_l8_status(s.l8.data_ptr(), 0, nullptr)) bad |= 1;
-            if (s.partial.defined() && cbl_gemm_b3_status(s.partial.data_ptr(), nullptr)) bad |= 2;
-            if (s.dense_stage.defined()) {
+            const Buffer* const s = e.second.b;
+            if (s[L8].t.defined() && cbl_gemv_l8_status(s[L8].t.data_ptr(), 0, nullptr)) bad |= 1;
+            if (s[PARTIAL].t.defined() && cbl_gemm_b3_status(s[PARTIAL].t.data_ptr(), nullptr)) bad |= 2;
+            if (s[DENSE_STAGE].t.defined()) {
                 unsigned int v = 0;
-                cudaMemcpy(&v, (char*)s.dense_stage.data_ptr() + s.dense_stage.numel() - 16, 4, cudaMemcpyDeviceToHost);
-                if (v) bad |= 4;
+                char* const at = (char*)s[DENSE_STAGE].t.data_ptr() + s[DENSE_STAGE].t.numel() - 16;
+                cudaMemcpy(&v, at, 4, cudaMemcpyDeviceToHost);
+                if (v) {
+                    cudaMemset(at, 0, 4);
+                    bad |= 4;
+                }
             }
         }
     } catch (const std::exception& e) {
@@ -282,6 +346,57 @@ PyObject* py_status(PyObject*, PyObject* args) {
         return nullptr;
     }
     return PyLong_FromLong(bad);
+}
+
+// scratch(device, kind, bytes) -> the shared buffer of that kind on the device's current stream (uint8, at least that long)
+PyObject* py_scratch(PyObject*, PyObject* args) {
+    int device, kind;
+    unsigned long long bytes;
+    if (!PyArg_ParseTuple(args, "iiK", &device, &kind, &bytes)) return nullptr;
+    if (kind < 0 || kind >= KINDS) { PyErr_SetString(PyExc_ValueError, "unknown kind of scratch"); return nullptr; }
+    try {
+        const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+        return THPVariable_Wrap(need((Kind)kind, (size_t)bytes, device, (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream()));
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+// release(device): gives back every scratch buffer of the device that no captured graph points at
+PyObject* py_release(PyObject*, PyObject* args) {
+    int device;
+    if (!PyArg_ParseTuple(args, "i", &device)) return nullptr;
+    std::lock_guard<std::mutex> lock(g_mu);
+    drop(device);
+    Py_RETURN_NONE;
+}
+
+// dense(packed descriptors, device, C, wide, row scales, x, x type, tokens, row stride of x, staged, y, y type, row stride of y): decode and GEMM
+// in one call, addresses as integers
+PyObject* py_dense(PyObject*, PyObject* args) {
+    Py_buffer buf;
+    int device, C, wide, xdt, ydt;
+    unsigned long long row_scale, x, staged, y;
+    long long tokens, ldx, ldy;
+    if (!PyArg_ParseTuple(args, "y*iipKKiLLKKiL", &buf, &device, &C, &wide, &row_scale, &x, &xdt, &tokens, &ldx, &staged, &y, &ydt, &ldy)) return nullptr;
+    const size_t n = (size_t)buf.len / sizeof(cbl_packed);
+    std::vector<cbl_packed> m(n);
+    const bool ok = n >= 1 && n * sizeof(cbl_packed) == (size_t)buf.len && (x || staged);
+    if (ok) memcpy((void*)m.data(), buf.buf, buf.len);
+    PyBuffer_Release(&buf);
+    if (!ok) { PyErr_SetString(PyExc_ValueError, "wrong descriptor size, or no activations"); return nullptr; }
+    try {
+        const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+        const char* fn = "";
+        const int rc = dense_product(m.data(), (int)n, C, wide, (const void*)row_scale, (const void*)x, xdt, tokens, ldx, (void*)staged, (void*)y, ydt, ldy,
+                                     nullptr, device, (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(), &fn);
+        if (rc) return fail(fn, rc);
+        Py_RETURN_NONE;
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
 }
 
 // stream(): torch's current stream on the current device; device(): that device
@@ -383,6 +498,9 @@ PyMethodDef methods[] = {
     {"decode", py_decode, METH_VARARGS, "decode(packed, device, dtype, first row, end row) -> dense rows"},
     {"set_linear", py_set_linear, METH_O, "set_linear(fn): what shapequant::linear(x, handle) runs"},
     {"status", py_status, METH_VARARGS, "status(device) -> bits"},
+    {"scratch", py_scratch, METH_VARARGS, "scratch(device, kind, bytes) -> tensor"},
+    {"release", py_release, METH_VARARGS, "release(device): gives the scratch back"},
+    {"dense", py_dense, METH_VARARGS, "dense(packed, device, C, wide, row_scale, x, xdt, tokens, ldx, staged, y, ydt, ldy)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_cblhost", "native call path of the packed linears", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -145,14 +145,17 @@ class _Ahead:
     starts when product k - 1 has left the scratch buffer, and runs beside whatever stands between the two products."""
 
     def __init__(self, products: list, side: torch.cuda.Stream, scratch: list):
-        """`scratch`: two buffers (or None) of the caller's, taken in turn; grown here to what the products need."""
-        self.products, self.side, self.scratch, self.k, self.done = products, side, scratch, 0, None
+        """`scratch`: two (buffer, its stream) or None of the caller's, taken in turn; grown here to what the products need."""
+        self.products, self.side, self.k, self.done = products, side, 0, None
         dev = products[0].device
         self.main = torch.cuda.current_stream(dev)
         for i in range(2):
             need = max((p.scratch_bytes() for p in products[i::2]), default=0)
-            if need and (scratch[i] is None or scratch[i].numel() < need):
-                scratch[i] = torch.empty(need, dtype=torch.uint8, device=dev)
+            if need and (scratch[i] is None or scratch[i][0].numel() < need):
+                scratch[i] = (torch.empty(need, dtype=torch.uint8, device=dev), self.main)
+            elif need and scratch[i][1] != self.main:      # allocated by a prompt on another stream, which may free it
+                scratch[i][0].record_stream(self.main)
+        self.scratch = [s and s[0] for s in scratch]
         side.wait_stream(self.main)                  # the buffers' earlier users
         self.ready = self._decode(0)
 
@@ -318,7 +321,8 @@ class DecodeEngine:
         write, attention, o + add + norm, gate|up + silu * up, down + add + norm (of the next layer)."""
         from .kernels import l8_workspace
         c, dtc = self.cfg, _dt(self.dtype)
-        ws = l8_workspace(self.dev, 0, max(st.group.ws_bytes for S in self.stages for st in S.values())).data_ptr()
+        work = l8_workspace(self.dev, 0, max(st.group.ws_bytes for S in self.stages for st in S.values()))
+        ws = work.data_ptr()
         x, act, ao, h = self.x16.data_ptr(), self.act.data_ptr(), self.ao.data_ptr(), self.h.data_ptr()
         self._addnorm(self.h, None, self.layers[0]["ln1"], self.x16, 1)
         n = len(self.layers)

@@ -36,6 +36,22 @@ def _on(device: torch.device):
     return _HERE if _cblhost.device() == device.index else torch.cuda.device(device)
 
 
+# kinds of scratch (csrc/host.cpp)
+L8_WORK, STAGE, PARTIAL, DENSE_STAGE = 0, 1, 2, 4
+
+
+def scratch(device: torch.device, kind: int, nbytes: int) -> torch.Tensor:
+    """The buffer of a kind that the products on (device, current stream) share, at least `nbytes` long.  Hold the tensor until the
+    launches that use it are made; ask again for the next call (it may have been outgrown, or given back)."""
+    return _cblhost.scratch(torch.cuda.current_device() if device.index is None else device.index, kind, nbytes)
+
+
+def release_scratch(device="cuda") -> None:
+    """Gives back the scratch of the products on a device, but for what captured graphs point at."""
+    device = torch.device(device)
+    _cblhost.release(torch.cuda.current_device() if device.index is None else device.index)
+
+
 def _dt(t: torch.dtype) -> int:
     try:
         return _DT[t]
@@ -151,23 +167,9 @@ class DeviceMatrix:
             raise ValueError("Y must be [T, R] with unit column stride")
         if T == 0 or self.R == 0:
             return Y
-        key = (self.device.index, _stream())
-        need = lib.cbl_dense_scratch_bytes(self.R, Cx)
-        pair = DenseStack._scratch.setdefault(key, [None, None, 0])     # the two alternating scratches of the device and stream
-        pair[2] ^= 1
-        sc = pair[pair[2]]
-        if sc is None or sc.numel() < need:
-            sc = pair[pair[2]] = torch.empty(need, dtype=torch.uint8, device=self.device)
-        nst = lib.cbl_gemm_stage_bytes(T, Cx) + 16
-        st = DenseStack._stage.get(key)
-        if st is None or st.numel() < nst:
-            st = DenseStack._stage[key] = torch.zeros(nst, dtype=torch.uint8, device=self.device)
         with _on(self.device):
-            s = _stream()
-            _lib.check("cbl_decode_raw_wide", lib.cbl_decode_raw_wide(ctypes.byref(self.struct()), sc.data_ptr(), Cx, s))
-            _lib.check("cbl_gemm_dense", lib.cbl_gemm_dense(sc.data_ptr(), self.R, Cx, self.row_scale.data_ptr(), X.data_ptr(), _dt(X.dtype), T,
-                                                            X.stride(0), Y.data_ptr(), _dt(Y.dtype), Y.stride(0), st.data_ptr(),
-                                                            st.data_ptr() + st.numel() - 16, s))
+            _cblhost.dense(bytes(self.struct()), self.device.index, Cx, True, self.row_scale.data_ptr(), X.data_ptr(), _dt(X.dtype), T, X.stride(0), 0,
+                           Y.data_ptr(), _dt(Y.dtype), Y.stride(0))
         return Y
 
     @property
@@ -421,8 +423,6 @@ class B3Group:
     launch: run(X [B, >= C], ys) writes ys[i] [B, R_i]; the outputs share one row stride."""
 
     MAX = 4
-    _scratch: dict = {}
-    _retired: list = []                     # outgrown buffers stay alive: a captured graph may still point at them
 
     def __init__(self, mats: list[B3Matrix], biases: list | None = None):
         if not 1 <= len(mats) <= self.MAX:
@@ -434,7 +434,6 @@ class B3Group:
         self.biases = biases if biases is not None else [None] * len(mats)
         self._built = None
         self._ws_bytes: dict = {}
-        self._ys = (ctypes.c_void_p * len(mats))()
 
     @property
     def _structs(self):
@@ -446,19 +445,6 @@ class B3Group:
     @property
     def perms(self) -> torch.Tensor | None:
         return self.mats[0].dm.perms
-
-    @classmethod
-    def buffers(cls, device: torch.device, stage_bytes: int, ws_bytes: int) -> tuple[torch.Tensor, torch.Tensor]:
-        """Staging buffer and work space of the products on (device, current stream)."""
-        key = (device.index, _stream())
-        st, ws = cls._scratch.get(key, (None, None))
-        if st is None or st.numel() < stage_bytes or ws.numel() < ws_bytes:
-            if st is not None:
-                cls._retired.append((st, ws))
-            st = torch.empty(max(stage_bytes, 4 << 20), dtype=torch.uint8, device=device)
-            ws = torch.zeros(max(ws_bytes, 16 << 20), dtype=torch.uint8, device=device)
-            cls._scratch[key] = (st, ws)
-        return st, ws
 
     def run(self, X: torch.Tensor | None, ys: list[torch.Tensor], staged: torch.Tensor | None = None) -> list[torch.Tensor]:
         """`staged` (X None, one column order): the activations as cbl_prep_x lays them out, written by the operator before."""
@@ -473,27 +459,27 @@ class B3Group:
         if len(ys) != len(self.mats) or len({y.dtype for y in ys}) != 1:
             raise ValueError("one output per matrix, one dtype")
         ldy = ys[0].stride(0) if B > 1 else max(m.R for m in self.mats)
-        for i, (y, m) in enumerate(zip(ys, self.mats)):
+        for y, m in zip(ys, self.mats):
             if y.shape != (B, m.R) or y.stride(1) != 1 or (B > 1 and y.stride(0) != ldy):
                 raise ValueError("outputs must be [B, R_i] with unit column stride and a common row stride")
-            self._ys[i] = y.data_ptr()
+        out = (ctypes.c_void_p * len(ys))(*[y.data_ptr() for y in ys])
         st = self._structs
         need = self._ws_bytes.get(B)
         if need is None:
             need = self._ws_bytes[B] = (lib.cbl_prep_x_bytes(B, self.C, self.M), lib.cbl_gemm_b3_workspace_bytes(st, len(self.mats), B))
-        stage, ws = self.buffers(self.device, *need)
+        ws = scratch(self.device, PARTIAL, need[1])
         if X is None:
             stage, x = staged, (None, 0, B, 0)
         else:
-            x = (X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1])
+            stage, x = scratch(self.device, STAGE, need[0]), (X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1])
         with _on(self.device):
-            _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), *x, _ptr(self.perms), self._ys, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
+            _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), *x, _ptr(self.perms), out, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
         return ys
 
     def status(self) -> None:
         """Synchronises and raises CblError if a bounded device-side wait of an earlier run() expired."""
-        _, ws = self._scratch.get((self.device.index, _stream()), (None, None))
-        if ws is not None:
+        ws = scratch(self.device, PARTIAL, 0)
+        with _on(self.device):
             _lib.check("cbl_gemm_b3_status", lib.cbl_gemm_b3_status(ws.data_ptr(), _stream()))
 
 
@@ -502,9 +488,6 @@ class DenseStack:
     for matrices with several column orders: every matrix is decoded ONCE into a 16-bit scratch shared by
     all stacks of the device and stream (rows stacked in order), then one TMA-fed tensor-core GEMM writes
     Y [T, sum R]. d = 8, 12-bit tags, G = 1; one or two books; any number of column orders."""
-
-    _scratch: dict = {}
-    _stage: dict = {}
 
     def __init__(self, dms: list):
         for dm in dms:
@@ -540,59 +523,31 @@ class DenseStack:
             raise ValueError("Y must be [T, sum R] with unit column stride")
         if T == 0 or self.R == 0:
             return Y
-        key = (self.device.index, _stream())
-        sc = decoded
-        if sc is None:
-            need = self.scratch_bytes()
-            # two scratch buffers alternate: the decode of this stack may run beside the GEMM of the previous one
-            pair = DenseStack._scratch.setdefault(key, [None, None, 0])
-            pair[2] ^= 1
-            sc = pair[pair[2]]
-            if sc is None or sc.numel() < need:
-                sc = pair[pair[2]] = torch.empty(need, dtype=torch.uint8, device=self.device)
-            self.decode(sc)
-        need = lib.cbl_gemm_stage_bytes(T if X is not None else 8, self.C) + 16
-        st = DenseStack._stage.get(key)
-        if st is None or st.numel() < need:
-            st = DenseStack._stage[key] = torch.zeros(need, dtype=torch.uint8, device=self.device)
-        x = (None, 0, T, 0, staged.data_ptr()) if X is None else (X.data_ptr(), _dt(X.dtype), T, X.stride(0), st.data_ptr())
+        x = (0, 0, T, 0, staged.data_ptr()) if X is None else (X.data_ptr(), _dt(X.dtype), T, X.stride(0), 0)
         with _on(self.device):
-            _lib.check("cbl_gemm_dense_bias", lib.cbl_gemm_dense_bias(sc.data_ptr(), self.R, self.C, self.row_scale.data_ptr(), *x[:4], Y.data_ptr(),
-                                                                      _dt(Y.dtype), Y.stride(0), None, x[4], st.data_ptr() + st.numel() - 16, _stream()))
+            if decoded is None:
+                _cblhost.dense(b"".join(bytes(dm.struct()) for dm in self.dms), self.device.index, self.C, False, self.row_scale.data_ptr(), *x, Y.data_ptr(),
+                               _dt(Y.dtype), Y.stride(0))
+            else:
+                st = scratch(self.device, DENSE_STAGE, lib.cbl_gemm_stage_bytes(T if X is not None else 8, self.C) + 16)
+                _lib.check("cbl_gemm_dense_bias", lib.cbl_gemm_dense_bias(decoded.data_ptr(), self.R, self.C, self.row_scale.data_ptr(), x[0] or None, *x[1:4],
+                                                                          Y.data_ptr(), _dt(Y.dtype), Y.stride(0), None, x[4] or st.data_ptr(),
+                                                                          st.data_ptr() + st.numel() - 16, _stream()))
         return Y
 
     @classmethod
     def status(cls, device) -> None:
-        """Synchronises and raises CblError if a bounded device-side wait of an earlier gemm() expired."""
+        """Synchronises and raises CblError if a bounded device-side wait of an earlier product expired."""
         device = torch.device(device)
-        key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
-        st = cls._stage.get(key)
-        from . import _cblhost
-        if _cblhost.status(key[0]):
-            raise _lib.CblError("forward", _lib.ETIMEOUT, "a bounded device-side wait expired")
-        if st is not None:
-            torch.cuda.synchronize(device)
-            if int(st[-16:].view(torch.int32)[0]) != 0:
-                raise _lib.CblError("cbl_gemm_dense", _lib.ETIMEOUT, "a bounded device-side wait expired")
-
-
-_WORKSPACES: dict[tuple, torch.Tensor] = {}
-_RETIRED: list[torch.Tensor] = []       # outgrown work spaces stay alive: a captured graph may still point at them
+        if _cblhost.status(device.index if device.index is not None else torch.cuda.current_device()):
+            raise _lib.CblError("cbl_gemm_dense", _lib.ETIMEOUT, "a bounded device-side wait expired")
 
 
 def l8_workspace(device: torch.device, R: int, nbytes: int = 0) -> torch.Tensor:
-    """Zero-initialised work space shared by every L8 product on (device, current stream): the kernels
-    leave it zero. Products that may overlap on the device (different streams) get distinct buffers.
-    16 MB to begin with (a launch needs 5.3 MB of partial-sum slots plus 4 bytes per output row); a larger request
-    gets a new buffer and the old one is kept, so pointers handed out earlier (CUDA graphs) stay valid."""
-    key = (device.index, _stream())
-    need = max(lib.cbl_gemv_l8_workspace_bytes(R), nbytes)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < need:
-        if ws is not None:
-            _RETIRED.append(ws)
-        ws = _WORKSPACES[key] = torch.zeros(max(need, 16 << 20), dtype=torch.uint8, device=device)
-    return ws
+    """Work space shared by every L8 product on (device, current stream), zero when it is new: the kernels leave it zero.  Products
+    that may overlap on the device (different streams) get distinct buffers.  16 MB to begin with (a launch needs 5.3 MB of
+    partial-sum slots plus 4 bytes per output row)."""
+    return scratch(device, L8_WORK, max(lib.cbl_gemv_l8_workspace_bytes(R), nbytes))
 
 
 class L8Matrix:
@@ -763,10 +718,10 @@ class L8Group:
         self.Rs = [m.R for m in mats]
         self._built = None
         self._built_c = None                    # column-ordered variants, built on first use (gemm_rows)
-        self._ys = (ctypes.c_void_p * len(mats))()
         self.ws_bytes = sum(lib.cbl_gemv_l8_workspace_bytes(m.R) for m in mats)
         self.rows_ws_bytes = lib.cbl_gemm_rows_workspace_bytes(sum((m.R + 3) // 4 * 4 for m in mats))
         self._rows_stage: dict = {}
+        self._rows_ws: dict = {}
 
     @property
     def _structs(self):
@@ -798,19 +753,21 @@ class L8Group:
         if len(ys) != len(self.mats) or len({y.dtype for y in ys}) != 1:
             raise ValueError("one output per matrix, one dtype")
         ldy = ys[0].stride(0) if B > 1 else max(m.R for m in self.mats)
-        for i, (y, R) in enumerate(zip(ys, self.Rs)):
+        for y, R in zip(ys, self.Rs):
             if y.shape != (B, R) or y.stride(1) != 1 or (B > 1 and y.stride(0) != ldy):
                 raise ValueError("outputs must be [B, R_i] with unit column stride and a common row stride")
-            self._ys[i] = y.data_ptr()
+        out = (ctypes.c_void_p * len(ys))(*[y.data_ptr() for y in ys])
         key = _stream()
         st = self._rows_stage.get(key)
         if st is None:
             st = self._rows_stage[key] = torch.empty(lib.cbl_gemm_stage_bytes(lib.cbl_gemm_rows_max_tokens(), self.C), dtype=torch.uint8,
                                                      device=self.device)
-        ws = l8_workspace(self.device, 0, self.rows_ws_bytes)
+        ws = self._rows_ws.get(key)             # accumulators that are left zero: a buffer of the group's own
+        if ws is None:
+            ws = self._rows_ws[key] = torch.zeros(self.rows_ws_bytes, dtype=torch.uint8, device=self.device)
         with _on(self.device):
             _lib.check("cbl_gemm_rows_multi", lib.cbl_gemm_rows_multi(self._structs_c, len(self.mats), X.data_ptr(), _dt(X.dtype), B, X.stride(0),
-                                                                      self._ys, _dt(ys[0].dtype), ldy, st.data_ptr(), ws.data_ptr(), _stream()))
+                                                                      out, _dt(ys[0].dtype), ldy, st.data_ptr(), ws.data_ptr(), _stream()))
         return ys
 
     def run(self, x: torch.Tensor, ys: list[torch.Tensor]) -> list[torch.Tensor]:
@@ -820,12 +777,12 @@ class L8Group:
         if len(ys) != len(self.mats):
             raise ValueError("one output vector per matrix")
         dt = ys[0].dtype
-        for i, (y, R) in enumerate(zip(ys, self.Rs)):
+        for y, R in zip(ys, self.Rs):
             if y.numel() != R or not y.is_contiguous() or y.dtype != dt:
                 raise ValueError("outputs must be contiguous [R_i] vectors of one dtype")
-            self._ys[i] = y.data_ptr()
+        out = (ctypes.c_void_p * len(ys))(*[y.data_ptr() for y in ys])
         ws = l8_workspace(self.device, 0, self.ws_bytes)
         with _on(self.device):
-            _lib.check("cbl_gemv_l8_multi", lib.cbl_gemv_l8_multi(self._structs, len(self.mats), x.data_ptr(), _dt(x.dtype), self._ys,
+            _lib.check("cbl_gemv_l8_multi", lib.cbl_gemv_l8_multi(self._structs, len(self.mats), x.data_ptr(), _dt(x.dtype), out,
                                                                   _dt(dt), ws.data_ptr(), _stream()))
         return ys

@@ -978,3 +978,93 @@ def test_gather_product_of_more_rows_than_a_launch_takes(R, C, books, M):
             assert (got - want).abs().max() <= 1e-5 * C ** 0.5 * want.abs().max()
             del got, want
         grp.status()
+
+
+def test_scratch_first_asked_for_in_a_captured_region_is_zero_at_once():
+    """The products' work spaces hold zeros when they are new, also where the first request is part of a capture: before any replay, and
+    not in memory that earlier nodes of the graph write."""
+    from quantexperiments_b200 import kernels
+    s = torch.cuda.Stream()
+    pool = torch.cuda.graph_pool_handle()
+    dirty = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(dirty, pool=pool, stream=s):
+        t = torch.full((64 << 20,), 255, dtype=torch.uint8, device="cuda")
+        del t
+    dirty.replay()
+    torch.cuda.synchronize()
+    lin = _linear(orc.synth_matrix(2304, 512, seed=3))
+    x1, x5 = torch.randn(1, 512, device="cuda").bfloat16(), torch.randn(5, 512, device="cuda").bfloat16()
+    want1, want5 = lin(x1).clone(), lin(x5).clone()          # the layouts exist; another stream's scratch does not
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, pool=pool, stream=s):
+        t = torch.full((32 << 20,), 255, dtype=torch.uint8, device="cuda")
+        del t
+        y1, y5 = lin(x1), lin(x5)
+    with torch.cuda.stream(s):
+        work, partial = kernels.l8_workspace(lin.dm.device, 2304), kernels.scratch(lin.dm.device, kernels.PARTIAL, 0)
+        s.synchronize()
+        assert not work.any() and not partial[:65536].any()
+        assert torch.equal(lin(x1), want1) and torch.equal(lin(x5), want5)          # eager calls on that stream before the first replay
+        for _ in range(2):
+            g.replay()
+            assert torch.equal(y1, want1) and torch.equal(y5, want5)
+            assert torch.equal(lin(x1), want1) and torch.equal(lin(x5), want5)
+        s.synchronize()
+        assert not kernels.l8_workspace(lin.dm.device, 2304).any()
+
+
+def test_scratch_is_not_kept_twice_and_goes_back():
+    """Growing prompts do not leave their outgrown buffers behind, the first call of a layer shares its buffers with the later ones, and
+    release_scratch returns them."""
+    import gc
+    from quantexperiments_b200 import kernels
+    gc.collect()
+    kernels.release_scratch()
+    torch.cuda.synchronize()
+    m = orc.synth_matrix(512, 2048, seed=4)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        base = torch.cuda.memory_allocated()
+        lin = _linear(m)
+        weights = torch.cuda.memory_allocated() - base
+        for T in range(200, 2200, 100):
+            lin(torch.zeros(T, 2048, device="cuda", dtype=torch.bfloat16))
+        held = torch.cuda.memory_allocated() - base - weights
+        # two buffers of decoded weights and the staged activations of the longest prompt
+        assert held <= 2 * 512 * 2048 * 2 + 2112 * 2048 * 2 + (1 << 20), held
+        lin.gemv(torch.zeros(2048, device="cuda"))
+        kernels.release_scratch()
+        assert torch.cuda.memory_allocated() - base - weights <= sum(g.mats[0].nbytes() for g in lin._b3.values()) + (1 << 20)
+        lin(torch.zeros(300, 2048, device="cuda", dtype=torch.bfloat16))
+        s.synchronize()
+        del lin
+        gc.collect()
+        kernels.release_scratch()                            # (layers of other tests are alive; the last one to go gives it back by itself)
+        assert torch.cuda.memory_allocated() - base <= 1 << 20
+
+
+def test_threads_share_a_stream_without_mixing_their_activations():
+    """Two threads on one stream, each with calls of both Python and native paths: staging and product of a call stay together."""
+    import threading
+    from quantexperiments_b200.kernels import B3Group, B3Matrix, DenseStack
+    ms = [orc.synth_matrix(300, 1024, seed=40 + i) for i in range(2)]
+    lins = [_linear(m) for m in ms]
+    xs = [torch.randn(7, 1024, device="cuda").bfloat16() for _ in ms]
+    xl = [torch.randn(150, 1024, device="cuda").bfloat16() for _ in ms]
+    groups, stacks = [B3Group([B3Matrix(l.dm, 3)]) for l in lins], [DenseStack([l.dm]) for l in lins]
+    want = [(l(x).clone(), l(y).clone()) for l, x, y in zip(lins, xs, xl)]
+    bad, stream = [], torch.cuda.current_stream()
+    def work(i):
+        with torch.cuda.stream(stream):
+            out = torch.empty(7, 300, device="cuda", dtype=torch.bfloat16)
+            for _ in range(300):
+                groups[i].run(xs[i], [out])
+                a, b = stacks[i].gemm(xl[i]), lins[i](xs[i])
+                if not (torch.equal(out, want[i][0]) and torch.equal(a, want[i][1]) and torch.equal(b, want[i][0])):
+                    bad.append(i)
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
