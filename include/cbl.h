@@ -371,6 +371,11 @@ int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_
                 int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s);
 int cbl_gemm_b3_status(void* workspace, cbl_stream s);
 
+/* Orders a stream for kernels that start early (programmatic dependent launch): the products read tags, books and layouts, and
+ * cbl_decode_raw writes its output, while the kernel before them still runs.  Call it between the work that produced a matrix's
+ * tensors, or that last used the memory of a decode's output, and the first product (the re-layouts above end with it). */
+int cbl_order(cbl_stream s);
+
 /* Two-phase prefill for many tokens and for matrices with several column orders: decode the matrix ONCE
  * into a 16-bit scratch, then multiply with a TMA-fed tcgen05 GEMM (both operands by TMA, accumulators in
  * tensor memory).
@@ -379,7 +384,8 @@ int cbl_gemm_b3_status(void* workspace, cbl_stream s);
  * previous GEMM), and cbl_gemm_dense lets the next kernel start early.  `out` must therefore not be read or
  * written by any earlier work of the stream that may still be in flight: a caller that decodes matrix after
  * matrix keeps TWO scratch buffers and alternates them (decode A, gemm A, decode B, gemm B, decode A, ...), as
- * DenseStack does; with a single scratch put an event or another kernel between a GEMM and the next decode.
+ * DenseStack does; with a single scratch, or a new one in memory that other tensors have just left, put cbl_order
+ * before the decode.
  *   cbl_decode_raw: out fp16 [R, ld], ld = C rounded up to 8, = cbl_dense_scratch_bytes(R, C) bytes:
  *                   out[r, col] = fp16(A[tag]) or fp16(fp32(A[tag]) + fp32(B[tag2])), col the ORIGINAL column
  *                   (column orders undone), without the row scale.  d = 8, 12-bit tags, G = 1.
@@ -392,8 +398,7 @@ int cbl_decode_raw(const cbl_packed* m, void* out, cbl_stream s);
 /* The same for a column shard (tensor parallelism) of a matrix with several column orders: the shard's orders name
  * positions of the FULL activation vector, so a row of `out` is C_out >= m->C wide (ld = C_out rounded up to 8,
  * cbl_dense_scratch_bytes(R, C_out) bytes) and the shard's weights land at out[r, perms[row_mask[r]][c]]; every other
- * element must be ZERO on entry (the call writes only the shard's positions; every index in perms must be below
- * C_out).  The product is then cbl_gemm_dense over C_out columns against the full activations.
+ * element is set to zero (every index in perms must be below C_out).  The product is then cbl_gemm_dense over C_out columns against the full activations.
  * no counterpart in the reference (which refuses tensor parallelism, shapequant/vllm_ext/plugin.py:198-199). */
 int cbl_decode_raw_wide(const cbl_packed* m, void* out, int32_t C_out, cbl_stream s);
 int cbl_gemm_dense(const void* w16, int32_t R, int32_t C, const void* row_scale, const void* x, int xdtype, int32_t ntok, int64_t ldx,

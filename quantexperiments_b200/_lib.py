@@ -119,6 +119,7 @@ SIGNATURES = {
     "cbl_gemm_rows_workspace_bytes": (c_size_t, [c_int32]),
     "cbl_gemm_rows_multi": (c_int, [POINTER(L8), c_int32, c_void_p, c_int, c_int32, c_int64, POINTER(c_void_p), c_int, c_int64, c_void_p,
                                     c_void_p, c_void_p]),
+    "cbl_order": (c_int, [c_void_p]),
     "cbl_dense_scratch_bytes": (c_size_t, [c_int32, c_int32]),
     "cbl_decode_raw": (c_int, [POINTER(Packed), c_void_p, c_void_p]),
     "cbl_decode_raw_wide": (c_int, [POINTER(Packed), c_void_p, c_int32, c_void_p]),

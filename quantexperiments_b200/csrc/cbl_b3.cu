@@ -765,7 +765,7 @@ extern "C" int cbl_repack_b3(const cbl_packed* m, const int32_t* tile_rows, int3
     const int64_t n = (int64_t)m->books * ntile * 16 * nkb * 4;
     if (n == 0) return CBL_OK;
     k_repack_b3<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)s>>>(*m, tile_rows, ntile, nkb, copies, (uint32_t*)out, n);
-    return cbl_check_launch();
+    return cbl_order(s);                                       // the product reads the layout before it waits for its predecessor
 }
 
 extern "C" size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int32_t ntok) {

@@ -31,6 +31,13 @@ int cbl_sm_count() {
     return cached[dev];
 }
 
+// A kernel launched without early start waits for everything before it, and an early one after it reaches back no further than to it.
+__global__ void k_order() {}
+extern "C" int cbl_order(cbl_stream s) {
+    k_order<<<1, 32, 0, (cudaStream_t)s>>>();
+    return cbl_check_launch();
+}
+
 static int check_packed(const cbl_packed* m) {
     if (!m || !m->tags || !m->table || !m->row_scale) return CBL_EINVAL;
     if (m->R < 0 || m->C <= 0 || m->d < 1 || m->d > 16 || m->bits < 1 || m->bits > 16) return CBL_EINVAL;

@@ -109,6 +109,8 @@ const at::Tensor& need(Kind kind, size_t bytes, int device, void* stream) {
         const int64_t n = (int64_t)std::max(bytes, least[kind]);
         const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device);
         b.t = graph ? beside_graph(n, device) : kind == STAGE || kind == WEIGHTS ? at::empty({n}, opt) : at::zeros({n}, opt);
+        // a decode writes before it waits, and the memory may have been the output of a product that is still running
+        if (kind == WEIGHTS && !graph) cbl_order((cbl_stream)stream);
     }
     b.in_graph |= graph;
     return b.t;

@@ -103,6 +103,8 @@ class DeviceMatrix:
         self._packed = None                     # (addresses, descriptor)
         if self.x_cols is not None and (self.M == 1 or self.x_cols < self.C):
             raise ValueError("x_cols (wider activations than columns) needs several column orders and x_cols >= C")
+        with _on(self.device):                  # the products read these tensors before they wait for the work that has just written them
+            _lib.check("cbl_order", lib.cbl_order(_stream()))
 
     @classmethod
     def tags_only(cls, words: torch.Tensor, bits: int, n: int) -> "DeviceMatrix":

@@ -1068,3 +1068,18 @@ def test_threads_share_a_stream_without_mixing_their_activations():
     for t in ts:
         t.join()
     assert not bad
+
+
+def test_decode_into_memory_that_an_output_has_just_left():
+    """A product whose scratch is new takes memory that the output of the product before it, dropped at once, may have had; the decode
+    starts early and must not write there while that product still runs."""
+    from quantexperiments_b200 import kernels
+    lins = [_linear(orc.synth_matrix(R, 2048, seed=R)) for R in (1024, 4096)]
+    X = torch.randn(1500, 2048, device="cuda").bfloat16()
+    want = [lin(X).clone() for lin in lins]
+    for _ in range(20):
+        kernels.release_scratch()
+        for lin, w in zip(lins, want):
+            lin(X)
+            kernels.release_scratch()
+            assert torch.equal(lin(X), w)
