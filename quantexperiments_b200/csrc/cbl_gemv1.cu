@@ -136,8 +136,9 @@ __device__ __forceinline__ void l8_bar_arrive(int id) { asm volatile("bar.arrive
 __device__ __forceinline__ void l8_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(L8_THREADS) : "memory"); }
 __device__ __forceinline__ void l8_sync_block() { asm volatile("bar.sync 1, %0;" ::"n"(L8_NT) : "memory"); }
 
-__global__ void __launch_bounds__(L8_THREADS, 1) k_gemv_l8(const __grid_constant__ L8Launch P, const __grid_constant__ L8Plan plan,
-                                                           const void* __restrict__ x, int xdtype) {
+// (the launch's registers are stated, not left to the compiler: the roles share them out by setmaxnreg)
+__global__ void __maxnreg__(L8_REGS_LAUNCH) k_gemv_l8(const __grid_constant__ L8Launch P, const __grid_constant__ L8Plan plan,
+                                                      const void* __restrict__ x, int xdtype) {
     extern __shared__ __align__(128) unsigned char l8_smem[];              // two 64 KB tables | scaled activations of the builders' next tiles
     __shared__ float s_inv[L8_XSLOTS];                                      // factor that undoes a tile's scale
     __shared__ float s_tinv[2];                                             // the same, of the tile in a table
@@ -730,10 +731,11 @@ static int launch_l8(L8Launch& P, const void* x, int xdtype, cudaStream_t st, in
         std::lock_guard<std::mutex> lock(mu);
         if (!attr_set[dev]) {
             CBL_CUDA(cudaFuncSetAttribute(k_gemv_l8, cudaFuncAttributeMaxDynamicSharedMemorySize, L8_DYN_SMEM));
-            // the roles' registers come out of what the block is launched with: a build with fewer would wait for ever
+            // the roles' registers come out of what the block is launched with (in eights): a build with fewer would wait for ever.
+            // build.py refuses such a build; this looks at the one that is loaded
             cudaFuncAttributes fa;
             CBL_CUDA(cudaFuncGetAttributes(&fa, k_gemv_l8));
-            if (fa.numRegs != L8_REGS_LAUNCH) return CBL_EUNSUPPORTED;
+            if ((fa.numRegs + 7) / 8 * 8 != L8_REGS_LAUNCH) return CBL_EUNSUPPORTED;
             attr_set[dev] = true;
         }
         auto it = cache.find(key);

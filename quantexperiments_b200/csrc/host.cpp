@@ -512,4 +512,14 @@ TORCH_LIBRARY_FRAGMENT(shapequant, m) { m.def("linear(Tensor x, int handle) -> T
 TORCH_LIBRARY_IMPL(shapequant, CompositeExplicitAutograd, m) { m.impl("linear", linear_op); }
 TORCH_LIBRARY_IMPL(shapequant, Autograd, m) { m.impl("linear", linear_autograd); }
 
-PyMODINIT_FUNC PyInit__cblhost(void) { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__cblhost(void) {
+    // built against one torch, unusable with another
+    PyObject* torch = PyImport_ImportModule("torch");
+    PyObject* version = torch ? PyObject_GetAttrString(torch, "__version__") : nullptr;
+    const char* v = version ? PyUnicode_AsUTF8(version) : nullptr;
+    const bool same = v && std::string(v) == CBL_TORCH;
+    if (v && !same) PyErr_Format(PyExc_ImportError, "_cblhost.so was built for torch " CBL_TORCH ", this is %s: run `python -m quantexperiments_b200.build`", v);
+    Py_XDECREF(version);
+    Py_XDECREF(torch);
+    return same ? PyModule_Create(&module_def) : nullptr;
+}

@@ -189,3 +189,25 @@ def test_gather_product_work_space_holds_what_is_written():
         assert ws(R, C, books, 16, 3) > 65536, (R, C, books)
     assert ws(1_200_000, 64, 1, 16, 3, n=4) > 65536
     assert ws(0, 64, 1, 16) > 0
+
+
+def test_builds_that_could_not_run_are_refused(monkeypatch, tmp_path):
+    """The register count of the one-token kernel, read from the compiler's log; the torch that the host extension was built against."""
+    import torch
+    from quantexperiments_b200 import build
+    line = "ptxas info    : Compiling entry function '_Z9k_gemv_l88L8Launch' for 'sm_100a'\nptxas info    : Used {} registers, used 16 barriers\n"
+    build.check_registers(line.format(80))
+    build.check_registers(line.format(77))
+    for log in (line.format(72), line.format(88), line.replace("k_gemv_l8", "k_other").format(80)):
+        with pytest.raises(RuntimeError):
+            build.check_registers(log)
+    assert build.STAMP.read_text() == torch.__version__
+    ran = []
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **_: ran.append(cmd) or build.subprocess.CompletedProcess(cmd, 0, "", ""))
+    monkeypatch.setattr(build, "STAMP", tmp_path / "stamp")
+    build.STAMP.write_text(torch.__version__)
+    build.build_host()
+    assert not ran
+    build.STAMP.write_text("0.0")
+    build.build_host()
+    assert len(ran) == 1 and build.STAMP.read_text() == torch.__version__
