@@ -9,8 +9,8 @@
 // Scratch buffers (staged activations, partial sums, decoded weights) belong to a (device, stream) pair and grow on demand; the
 // Python call paths take theirs from here as well (scratch()).  Calls on one stream share them in the order of the stream; graphs
 // captured on one stream share them too and are replayed one after another.  A buffer that a captured graph has been given lives as
-// long as the process (the graph holds its address); others go back to torch's allocator, in stream order, when they are outgrown,
-// when the last plan of their device is gone, or by release().
+// long as the process (the graph holds its address); others go back to torch's allocator, in stream order, when they are outgrown, by
+// release() and, but for 36 MB per stream, when the last plan of their device is gone.
 #include <Python.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -57,6 +57,7 @@ struct Buffer {
     bool in_graph = false;
 };
 enum Kind { L8, STAGE, PARTIAL, WEIGHTS, DENSE_STAGE, KINDS };
+constexpr size_t LEAST[KINDS] = {16 << 20, 4 << 20, 16 << 20, 16, 16};
 struct Scratch {
     Buffer b[KINDS], second;                              // second: the other of the two alternating buffers of decoded weights
     int turn = 0;
@@ -97,7 +98,6 @@ at::Tensor beside_graph(int64_t n, int device) {
 
 // The buffer of a kind on (device, current stream), at least `bytes` long; status words and arrival counters are zero when it is new.
 const at::Tensor& need(Kind kind, size_t bytes, int device, void* stream) {
-    static const size_t least[KINDS] = {16 << 20, 4 << 20, 16 << 20, 16, 16};
     std::lock_guard<std::mutex> lock(g_mu);
     Scratch& sc = g_scratch[{device, stream}];
     if (kind == WEIGHTS) sc.turn ^= 1;                    // the decode of a product may run beside the GEMM of the one before
@@ -106,7 +106,7 @@ const at::Tensor& need(Kind kind, size_t bytes, int device, void* stream) {
     if (!b.t.defined() || (size_t)b.t.numel() < bytes) {
         if (b.in_graph) g_kept.push_back(b.t);
         b = Buffer();
-        const int64_t n = (int64_t)std::max(bytes, least[kind]);
+        const int64_t n = (int64_t)std::max(bytes, LEAST[kind]);
         const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device);
         b.t = graph ? beside_graph(n, device) : kind == STAGE || kind == WEIGHTS ? at::empty({n}, opt) : at::zeros({n}, opt);
         // a decode writes before it waits, and the memory may have been the output of a product that is still running
@@ -116,11 +116,14 @@ const at::Tensor& need(Kind kind, size_t bytes, int device, void* stream) {
     return b.t;
 }
 
-void drop(int device) {                                   // (with g_mu held)
+// Gives a device's buffers back; all: also those of the least size.  (with g_mu held)
+void drop(int device, bool all) {
     for (auto& e : g_scratch) {
         if (e.first.first != device) continue;
-        for (Buffer& b : e.second.b)
-            if (!b.in_graph) b = Buffer();
+        for (int k = 0; k < KINDS; k++) {
+            Buffer& b = e.second.b[k];
+            if (b.t.defined() && !b.in_graph && (all || (size_t)b.t.numel() > LEAST[k])) b = Buffer();
+        }
         if (!e.second.second.in_graph) e.second.second = Buffer();
     }
 }
@@ -256,7 +259,7 @@ void free_plan(PyObject* o) {
     if (!p) return;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (--g_plans[p->device] == 0) drop(p->device);
+        if (--g_plans[p->device] == 0) drop(p->device, false);
     }
     delete p;
 }
@@ -370,7 +373,7 @@ PyObject* py_release(PyObject*, PyObject* args) {
     int device;
     if (!PyArg_ParseTuple(args, "i", &device)) return nullptr;
     std::lock_guard<std::mutex> lock(g_mu);
-    drop(device);
+    drop(device, true);
     Py_RETURN_NONE;
 }
 
