@@ -4,6 +4,9 @@ staging buffers into ONE exact-size arena per device and re-laid out for the ker
     plan  = plan_arena(pf, names, layouts, rank, world, kinds)      # bytes per matrix, from the metadata alone
     lins  = load_linears(path, device="cuda", layouts=("l8",))       # {name: PackedLinear}, arena in lins.arena
 
+Layouts: "l8" (one token by table lookups), "b3" (codeword gathers of 1..16 tokens), "b3x2" (of 17..128); "t16" and "x16" serve
+callers that stage activations themselves.  More tokens read the file-order tags.
+
 While the copy engine moves matrix i to the device and the repack kernels of matrix i - 1 run, the host reads
 matrix i + 1 from the file into the other staging buffer. Column orders are regenerated from the stored seed and
 checked against the stored CRC (`PackedFile.perms`). With world > 1 each rank keeps its row range ("col" kind,
@@ -28,11 +31,12 @@ import torch
 from . import packed as pk
 from . import tp
 from ._lib import lib
-from .kernels import L8Matrix, T16Matrix, X16Matrix
+from .kernels import B3Group, B3Matrix, L8Matrix, T16Matrix, X16Matrix
 from .linear import PackedLinear
 
 ALIGN = 256
-LAYOUTS = ("l8", "t16", "x16")
+LAYOUTS = ("l8", "b3", "b3x2", "t16", "x16")
+B3_COPIES = {"b3": 3, "b3x2": 2}            # copies of the book that a layout's slots name
 
 
 def _al(n: int) -> int:
@@ -66,11 +70,12 @@ def _shard_meta(m: dict, kind: str | None, rank: int, world: int) -> tuple[int, 
     return R, C
 
 
-def _t16_tiles(R: int, M: int, row_mask: torch.Tensor | None) -> int:
+def _row_tiles(R: int, M: int, row_mask: torch.Tensor | None, rows: int) -> int:
+    """Tiles of `rows` rows of one column order each."""
     if M == 1 or row_mask is None:
-        return -(-R // 16)
+        return -(-R // rows)
     counts = torch.bincount(row_mask.to(torch.int64).flatten(), minlength=M)
-    return int(sum(-(-int(c) // 16) for c in counts if int(c) > 0))
+    return int(sum(-(-int(c) // rows) for c in counts if int(c) > 0))
 
 
 def _l8_positions(R: int, M: int, row_mask: torch.Tensor | None) -> int:
@@ -81,7 +86,7 @@ def _l8_positions(R: int, M: int, row_mask: torch.Tensor | None) -> int:
     return int(sum((int(c) + 31) // 32 * 32 for c in counts))
 
 
-def matrix_bytes(m: dict, R: int, C: int, layouts, ntile16: int, rpad8: int | None = None) -> dict:
+def matrix_bytes(m: dict, R: int, C: int, layouts, ntile16: int, rpad8: int | None = None, ntile128: int | None = None) -> dict:
     """Aligned device bytes of one matrix piece: file-order tensors and each requested layout."""
     bits = int(math.log2(m["K"]))
     W = pk.words_per_row(C // m["d"], bits)
@@ -100,6 +105,8 @@ def matrix_bytes(m: dict, R: int, C: int, layouts, ntile16: int, rpad8: int | No
         if lay == "l8":
             rp = rpad8 if rpad8 is not None else (R + 31) // 32 * 32
             out["l8"] = _al(max(lib.cbl_l8r_bytes(rp, C, 1), 16)) + _al(lib.cbl_book_frag_bytes())
+        elif lay in B3_COPIES:
+            out[lay] = _al(max(lib.cbl_b3_bytes(ntile128 if ntile128 is not None else -(-R // 128), C, 1), 16))
         elif lay == "x16":
             out["x16"] = _al(max(lib.cbl_x16_bytes(R, C, 1), 16))
         else:
@@ -117,12 +124,12 @@ def plan_arena(pf: pk.PackedFile, names=None, layouts=("l8",), rank: int = 0, wo
         kind = (kinds or {}).get(name)
         R, C = _shard_meta(m, kind, rank, world)
         mask = None
-        if m["M"] > 1 and ("t16" in layouts or "l8" in layouts):
+        if m["M"] > 1 and set(layouts) - {"x16"}:
             mask = pf.f.get_tensor(f"{name}.row_mask")
             if world > 1 and kind == "col":
                 r0, r1 = tp.row_range(m["R"], rank, world)
                 mask = mask[r0:r1]
-        plan[name] = matrix_bytes(m, R, C, layouts, _t16_tiles(R, m["M"], mask), _l8_positions(R, m["M"], mask))
+        plan[name] = matrix_bytes(m, R, C, layouts, _row_tiles(R, m["M"], mask, 16), _l8_positions(R, m["M"], mask), _row_tiles(R, m["M"], mask, 128))
     return plan
 
 
@@ -204,6 +211,8 @@ def load_linears(path_or_file, names=None, device="cuda", layouts=("l8",), rank:
                     continue
                 if lay == "l8":
                     lin._l8 = L8Matrix(lin.dm, alloc=arena.take)
+                elif lay in B3_COPIES:
+                    lin._b3[B3_COPIES[lay]] = B3Group([B3Matrix(lin.dm, B3_COPIES[lay], alloc=arena.take)])
                 elif lay == "x16":
                     lin._x16 = X16Matrix(lin.dm, alloc=arena.take)
                 else:

@@ -124,3 +124,29 @@ def test_rank_shards_and_pooling(tmp_path):
     assert torch.equal(built[0](x), before) or (built[0](x).float() - before.float()).abs().max() <= 1e-2 * before.float().abs().max()
     assert torch.equal(built[2].dense(), PackedLinear.from_packed(pf, "b.masks").dense())
     assert loader.pool_layouts(built) == 0
+
+
+@pytest.mark.gpu
+def test_layouts_of_the_gather_product_lie_in_the_arena(tmp_path):
+    """"b3" and "b3x2": every token count up to 128 runs on what the load has placed, and builds nothing more."""
+    from quantexperiments_b200 import loader, packed
+    path, raw = _file(tmp_path, SPECS)
+    lays = ("l8", "b3", "b3x2")
+    lins = loader.load_linears(path, layouts=lays)
+    plan = loader.plan_arena(packed.PackedFile(path), layouts=lays)
+    assert lins.stats["arena_bytes"] == sum(sum(p.values()) for p in plan.values()) == lins.arena.off
+    lo, hi = lins.arena.buf.data_ptr(), lins.arena.buf.data_ptr() + lins.arena.buf.numel()
+    for name, (R, C, K, d, G, M) in SPECS.items():
+        lin, tags = lins[name], raw[name][0]
+        if d != 8 or G != 1 or K != 4096:
+            assert not lin._b3
+            continue
+        placed = {c: g.mats[0].words.data_ptr() for c, g in lin._b3.items()}
+        assert set(placed) == {2, 3} and all(lo <= p < hi and p % loader.ALIGN == 0 for p in placed.values())
+        w = lin.dense()
+        for n in (1, 7, 16, 17, 128):
+            x = torch.randn(n, C, device="cuda").bfloat16()
+            ref = x.float() @ w.T
+            for _ in range(2):
+                assert (lin(x).float() - ref).abs().max() <= 1e-2 * ref.abs().max()
+        assert {c: g.mats[0].words.data_ptr() for c, g in lin._b3.items()} == placed
