@@ -5,8 +5,8 @@ Mirrors shapequant/vllm_ext/core.py of the reference: PackedShards (:212-486: fr
 dense, nbytes, R, C), register (:622-624) and linear_op with its fake implementation (:693-702), so
 that vLLM's LinearMethod.apply can stay `torch.ops.shapequant.linear(x, handle)`.
 
-Dispatch on the number of tokens: see linear.Stack (one token: table lookups; up to 128: codeword gathers on the tensor
-cores; more: decode once + GEMM over the stacked rows)."""
+Dispatch on the number of tokens: see linear.Stack (one token: table lookups where the rows fill tables; up to 128: codeword
+gathers on the tensor cores; more: decode once + GEMM over the stacked rows)."""
 
 from __future__ import annotations
 
@@ -56,6 +56,7 @@ class PackedShards:
         self.Rs = [lin.R for lin in lins]
         self.R = sum(self.Rs)
         self.offs = [sum(self.Rs[:i]) for i in range(len(lins))]
+        # bmax is accepted and kept for callers of the reference's class; which kernel multiplies how many tokens is Stack's rule
         self.bmax = self.cross = bmax
         self.device = lins[0].dm.device
         self.sq_name = ""

@@ -61,7 +61,7 @@ class ShapeQuantConfig(QuantizationConfig):
         if embed_head != "bf16":
             raise ValueError(f"embed_head {embed_head!r}: only 'bf16' (stock vLLM embedding and head) is supported")
         self.packed_file = packed_file
-        self.bmax = min(int(os.environ.get("SHAPEQUANT_BMAX", bmax)), core.BMAX)
+        self.bmax = min(int(os.environ.get("SHAPEQUANT_BMAX", bmax)), core.BMAX)      # accepted; the dispatch goes by token counts of its own
         self.embed_head = embed_head
         self.ignored = dict(ignored)
         self._pf = None
