@@ -304,9 +304,7 @@ def build_set(dev, rank: int, world: int, batch: int, model: str = "7b", layers:
                                words2=t.get("tags2"), table2=t.get("table2"), x_cols=C if wide else None)
             lin.kind = kind
             if batch == 1 and (lin.dm.M == 1 or lin.use_l8()):
-                lin.l8
-            else:
-                lin.small_batch(batch).xp_buffer(batch)
+                lin.l8                                   # (other layouts are built on first use of their token counts)
             lins.append(lin)
             kinds.append(kind)
             if keep_file_layout:
@@ -318,6 +316,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     import torch.distributed as dist
     from quantexperiments_b200 import kernels  # noqa: F401  (fails loudly if libcbl.so is missing)
     from quantexperiments_b200.kernels import L8Group
+    from quantexperiments_b200.linear import DENSE_MIN_TOKENS, Stack
     dev = torch.device("cuda", local_rank)
     torch.cuda.set_device(dev)
     B, model = args.batch, args.model
@@ -343,52 +342,55 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     xarena = torch.randn(n_in, device=dev, generator=g).bfloat16()
     yarena = torch.empty(sum(B * l.R for l in lins), device=dev, dtype=torch.bfloat16)
     xoff = yoff = 0
-    items = []                     # batch > 1: (lin, x [B, C], y [B, R], kind)
+    stacks = []                    # batch > 1: (Stack, x [B, C], y [B, sum R], kind)
     for l0 in range(0, len(lins), per_layer):
         q, k, v, o, gate, up, down = lins[l0:l0 + per_layer]
         for members, kind, nm in (((q, k, v), "col", "q"), ((o,), "row", "o"), ((gate, up), "col", "gate"), ((down,), "row", "down")):
             C = in_cols(members[0], nm)
             x = xarena[xoff:xoff + B * C].view(B, C)
             xoff += B * C
-            outs = []
-            for mm in members:
-                outs.append(yarena[yoff:yoff + B * mm.R].view(B, mm.R))
-                yoff += B * mm.R
-                items.append((mm, x, outs[-1], kind))
-            if B == 1:
-                # one token: the table-lookup kernel, unless the matrices have so many column orders for their rows that
-                # per-order tables do not pay (PackedLinear.use_l8); those run on the row-tile kernel
-                tables = all(mm.dm.M == 1 or mm.use_l8() for mm in members)
-                if arena is not None and kind == "row" and tables:
-                    groups.append((PeerReduceGemv(members[0].l8, arena), x[0], [outs[0][0]], "fused", members))
-                elif tables:
-                    groups.append((L8Group([mm.l8 for mm in members]), x[0], [o_[0] for o_ in outs], kind, members))
-                else:
-                    groups.append((None, x, outs, "t16", members))
+            n_out = B * sum(mm.R for mm in members)
+            y = yarena[yoff:yoff + n_out].view(B, -1)
+            yoff += n_out
+            outs = list(y.split([mm.R for mm in members], 1))
+            if B > 1:
+                stacks.append((Stack(members), x, y, kind))
+                stacks[-1][0].prepare(B)
+                continue
+            # one token: the grouped table-lookup launch, unless the matrices have so many column orders for their rows that
+            # they gather codewords (PackedLinear.use_l8)
+            tables = all(mm.dm.M == 1 or mm.use_l8() for mm in members)
+            if arena is not None and kind == "row" and tables:
+                groups.append((PeerReduceGemv(members[0].l8, arena), x[0], [outs[0][0]], "fused", members))
+            elif tables:
+                groups.append((L8Group([mm.l8 for mm in members]), x[0], [o_[0] for o_ in outs], kind, members))
+            else:
+                groups.append((None, x, outs, "single", members))
 
     def step_kernels():
         if B == 1:
             for grp, x, outs, kind, members in groups:
                 if kind == "fused":
                     grp.run(x, outs[0])
-                elif kind == "t16":
+                elif kind == "single":
                     for mm, y in zip(members, outs):
-                        mm.t16.run(x, y, 1, wide=mm.wide)
+                        mm.forward_into(x, y)
                         if world > 1 and mm.kind == "row":
                             dist.all_reduce(y)
                 else:
                     grp.run(x, outs)
             return
-        staged = (None, None)             # matrices that share their input share one staging pass of it
-        for lin, x, y, kind in items:
-            if staged[0] is not x:
-                staged = (x, lin.small_batch(B).prep(x, B))
-            lin.small_batch(B).run_prepped(staged[1], y, B)
+        for stack, x, y, kind in stacks:
+            stack.run(x, y)
             if world > 1 and kind == "row":
                 dist.all_reduce(y)
 
-    launches_per_step = (sum(2 * len(grp[4]) if grp[3] == "t16" else (2 if grp[3] == "fused" else 1) for grp in groups) if B == 1
-                         else len(lins) + 4 * (len(lins) // per_layer))
+    # a product that gathers codewords is two launches, the activations' staging and itself
+    if B == 1:
+        launches_per_step = sum({"single": sum(1 if mm.use_l8() else 2 for mm in grp[4]), "fused": 2}.get(grp[3], 1) for grp in groups)
+    else:
+        launches_per_step = sum(2 if st.shared and B < DENSE_MIN_TOKENS else len(st.lins) + 2 if st.dense is not None and B >= DENSE_MIN_TOKENS else 2 * len(st.lins)
+                                for st, *_ in stacks)
     stream = torch.cuda.Stream(device=dev)
 
     def barrier():
@@ -466,7 +468,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
             alg = set_bytes(model) / len(groups)
             peak, src = measured_peak()
             achieved = alg / per_launch_s / 1e9
-            roof = {"bound": "hbm", "kernel": "k_gemv_l8" if all(grp[3] != "t16" for grp in groups) else "k_gemv_l8 / k_gemv_t16 (per shape)", "achieved": achieved, "peak": peak, "peak_source": src, "unit": "GB/s",
+            roof = {"bound": "hbm", "kernel": "k_gemv_l8" if all(grp[3] != "single" for grp in groups) else "k_gemv_l8 / k_gemm_b3 (per shape)", "achieved": achieved, "peak": peak, "peak_source": src, "unit": "GB/s",
                     "frac": achieved / peak, "frac_of_nominal_8000": achieved / 8000.0,
                     "traffic": alg * NCU_TRAFFIC_GATEUP[0] / NCU_TRAFFIC_GATEUP[1], "algorithmic_bytes_per_launch": alg,
                     "us_per_launch": per_launch_s * 1e6, "launches_timed": args.steps * len(groups),
@@ -565,7 +567,7 @@ def run_prefill(args, rank: int, world: int, local_rank: int, emit: bool = True)
     torch.cuda.set_device(dev)
     T = args.tokens
     from quantexperiments_b200.kernels import DenseStack
-    from quantexperiments_b200.linear import DENSE_MIN_TOKENS
+    from quantexperiments_b200.linear import DENSE_MIN_TOKENS, Stack
     SHAPES = MODELS[args.model]["shapes"]
     lins, kinds, _ = build_set(dev, rank, world, 64, args.model)
     g = torch.Generator(device=dev).manual_seed(7)
@@ -574,26 +576,24 @@ def run_prefill(args, rank: int, world: int, local_rank: int, emit: bool = True)
     flops = sum(2.0 * T * l.R * l.C for l in lins)
     # q|k|v and gate|up share their activations: one stacked product each, as the reference's gemm(x, [pieces]) does.
     # From DENSE_MIN_TOKENS tokens on the stack is decoded once into a 16-bit scratch and multiplied by the TMA-fed
-    # tcgen05 GEMM; below, every piece runs the kernel that decodes weight tiles on the fly.
+    # tcgen05 GEMM; below, the pieces gather codewords (Stack.run).
     dense = T >= (args.dense_min if args.dense_min is not None else DENSE_MIN_TOKENS)
     groups, launches = [], 0
     for l0 in range(0, len(lins), len(SHAPES)):
         q, k, v, o, gate, up, down = lins[l0:l0 + len(SHAPES)]
         for members, kind in (((q, k, v), "col"), ((o,), "row"), ((gate, up), "col"), ((down,), "row")):
             y = torch.empty(T, sum(m.R for m in members), device=dev, dtype=torch.bfloat16)
-            groups.append((DenseStack([m.dm for m in members]) if dense and not members[0].wide else None, members, xs[members[0].in_features], y, kind))
-            launches += (len(members) + 2) if dense else 2 * len(members)
+            stack = Stack(members) if not dense else DenseStack([m.dm for m in members]) if not members[0].wide else None
+            groups.append((stack, members, xs[members[0].in_features], y, kind))
+            launches += (len(members) + 2) if dense else 2 if stack.shared else 2 * len(members)
 
     def run_group(stack, members, x, y, kind):
-        if stack is not None:
-            stack.gemm(x, y)
-        elif members[0].wide:
+        if stack is None:
             members[0].forward_into(x, y)              # wide decode into a zeroed scratch + the same GEMM over all columns
+        elif dense:
+            stack.gemm(x, y)
         else:
-            off = 0
-            for m in members:
-                m.l8.gemm(x, y[:, off:off + m.R])
-                off += m.R
+            stack.run(x, y)
         if world > 1 and kind == "row":
             dist.all_reduce(y)
 
@@ -865,7 +865,7 @@ def run_load(args, rank: int, world: int, local_rank: int) -> None:
         nbytes = os.path.getsize(path)
 
         def step():
-            lins = loader.load_linears(path, device=dev, layouts=("l8", "x16"), rank=rank, world=world, kinds=kinds)
+            lins = loader.load_linears(path, device=dev, layouts=("l8", "b3"), rank=rank, world=world, kinds=kinds)
             return lins.stats
 
         for _ in range(2):
@@ -927,6 +927,18 @@ def _case_gemv_l8(shapes):
     for rep in range(2):
         for grp in grps:
             grp.run(x, ys)
+
+
+def _case_gemm_b3(tokens: int, copies: int):
+    """gate|up of a few tokens by codeword gathers, distinct matrices (203 MB of layout) a few times."""
+    from quantexperiments_b200.kernels import B3Group, B3Matrix
+    grps = [B3Group([B3Matrix(_case_matrix(18944, 3584, seed=7 * i + j), copies) for j in range(2)]) for i in range(3)]
+    X = torch.randn(tokens, 3584, device="cuda").bfloat16()
+    Y = torch.empty(tokens, 2 * 18944, device="cuda", dtype=torch.bfloat16)
+    for rep in range(2):
+        for grp in grps:
+            grp.run(X, list(Y.split(18944, 1)))
+    grps[0].status()
 
 
 def _case_gemv_t16():
@@ -993,6 +1005,8 @@ PROFILE_CASES = {
     "gemv_l8_gateup": lambda: _case_gemv_l8([(18944, 3584), (18944, 3584)]),    # the largest batch-1 launch of the 7B set
     "gemv_l8_down": lambda: _case_gemv_l8([(3584, 18944)]),
     "gemv_l8_qkv": lambda: _case_gemv_l8([(3584, 3584), (512, 3584), (512, 3584)]),
+    "gemm_b3_gateup_12": lambda: _case_gemm_b3(12, 3),                          # three copies of the book
+    "gemm_b3_gateup_32": lambda: _case_gemm_b3(32, 2),                          # two
     "gemv_t16_gate": _case_gemv_t16,
     "gemv_x16_gateup": _case_gemv_x16,
     "gemm_dense_gate": lambda: _case_gemm(True),
