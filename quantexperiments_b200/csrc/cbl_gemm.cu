@@ -469,21 +469,18 @@ k_gemm_l8_2sm(const __grid_constant__ CUtensorMap xmap, cbl_l8 m, const float* _
 // ------------------------------------------------------------------------------------ up to 32 tokens: weight rows as M
 //
 // For a handful of tokens the product is bound by decoding alone, so the tile is turned around: 128 weight rows
-// are the M side of tcgen05.mma (decoded into the K-major swizzled A tile), the tokens the N side (16 or 32,
+// are the M side of tcgen05.mma, the tokens the N side (16 or 32,
 // brought in by TMA).  Every weight is decoded exactly once whatever the token count, the MMAs are negligible,
 // and there are no per-step activation fragments to fetch as in the mma.sync kernel.  512 decode threads = 128
-// rows x 4 k-blocks per hand-off (64 KB of A per stage, two stages).  Blocks = (row tile, k part): products with
+// rows x 4 k-blocks per hand-off.  Blocks = (row tile, k part): products with
 // few row tiles are split along k and summed with fp32 reductions into a work space, finished by a second
 // kernel.  Up to four matrices that share the activations run as one launch (each block stages its own
 // matrix's book).
 constexpr int GR_ROWS = 128;
 constexpr int GR_KBS = 4;                                  // k-blocks per stage
-constexpr int GR_STAGES = 2;
 constexpr int GR_NMAX = 32;                                // tokens per launch
-constexpr int GR_A_KB = GR_ROWS * 128;                     // one k-block of A: 16 KB
 constexpr int GR_X_KB = GR_NMAX * 128;                     // one k-block of the activations: 4 KB
-constexpr int GR_A_STAGE = GR_KBS * GR_A_KB, GR_X_STAGE = GR_KBS * GR_X_KB;
-constexpr int GR_SMEM = 65536 + GR_STAGES * (GR_A_STAGE + GR_X_STAGE);   // 224 KB
+constexpr int GR_X_STAGE = GR_KBS * GR_X_KB;
 constexpr int GR_DECODE_WARPS = 16, GR_THREADS = (GR_DECODE_WARPS + 2) * 32;
 constexpr int GR_MAX_GROUP = 4;
 
@@ -496,192 +493,7 @@ struct GRLaunch {
     int ksplit, npad;
 };
 
-__global__ void __launch_bounds__(GR_THREADS, 1)
-k_gemm_rows(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ GRLaunch P, const float* __restrict__ xinv, int ntok, int ydtype,
-            int64_t ldy, unsigned int* __restrict__ status) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) unsigned long long s_bar[3 * GR_STAGES + 1];    // full_a, full_x, empty per stage; tmem_full
-    __shared__ uint32_t s_tmem;
-    __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    int mi = 0;
-    while (mi + 1 < P.n && (int)blockIdx.x >= P.tile0[mi + 1]) mi++;
-    const cbl_l8& m = P.m[mi];
-    const int r0 = ((int)blockIdx.x - P.tile0[mi]) * GR_ROWS;
-    const int nkb = m.ntile, nkb1 = m.ntile / m.books;
-    // this block's k-blocks: part blockIdx.y of ksplit equal parts
-    const int kb_lo = (int)(((int64_t)nkb * blockIdx.y) / P.ksplit), kb_hi = (int)(((int64_t)nkb * (blockIdx.y + 1)) / P.ksplit);
-    const uint32_t sbase = cbl_smem_u32(smem), bar0 = cbl_smem_u32(s_bar);
-    auto full_a = [&](int s) { return bar0 + 8u * s; };
-    auto full_x = [&](int s) { return bar0 + 8u * (GR_STAGES + s); };
-    auto empty = [&](int s) { return bar0 + 8u * (2 * GR_STAGES + s); };
-    const uint32_t tmem_full = bar0 + 8u * (3 * GR_STAGES);
-    const uint32_t a_base = sbase + 65536, x_base = a_base + GR_STAGES * GR_A_STAGE;
-    // stages never straddle the two books: segment 0 = this part's k-blocks of the first book, segment 1 = of the second
-    const int seg_lo[2] = {kb_lo < nkb1 ? kb_lo : nkb1, kb_lo > nkb1 ? kb_lo : nkb1};
-    const int seg_hi[2] = {kb_hi < nkb1 ? kb_hi : nkb1, kb_hi > nkb1 ? kb_hi : nkb1};
-
-    if (tid == 0) {
-        s_abort = 0;
-        for (int s = 0; s < GR_STAGES; s++) { mbar_init(full_a(s), GR_DECODE_WARPS); mbar_init(full_x(s), 1); mbar_init(empty(s), 1); }
-        mbar_init(tmem_full, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == GR_DECODE_WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cbl_smem_u32(&s_tmem)), "r"(32u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (warp < GR_DECODE_WARPS) {                              // the book of the first segment that has work
-        const uint4* t0 = (const uint4*)((seg_lo[0] < seg_hi[0]) ? m.table : m.table2);
-        uint4* dst = (uint4*)smem;
-        for (int i = tid; i < 4096; i += GR_DECODE_WARPS * 32) dst[i] = __ldg(t0 + i);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem;
-    asm volatile("griddepcontrol.wait;" ::: "memory");          // the staged activations (and zeroed sums) come from earlier kernels
-    // A wait that expires marks the block aborted; every thread then keeps the shape of its loops (the decode
-    // warps meet at a named barrier when the book changes) but waits for nothing more.
-    auto wait = [&](uint32_t bar, uint32_t parity) {
-        if (*(volatile int*)&s_abort) return;
-        if (!mbar_wait(bar, parity)) s_abort = 1;
-    };
-
-    if (warp == GR_DECODE_WARPS) {
-        if (elect_one()) {                                      // TMA producer of the activations
-            int it = 0;
-            for (int sg = 0; sg < 2; sg++) {
-                for (int kb = seg_lo[sg]; kb < seg_hi[sg]; kb += GR_KBS, it++) {
-                    const int s = it % GR_STAGES, nv = min(GR_KBS, seg_hi[sg] - kb);
-                    wait(empty(s), ((it / GR_STAGES) & 1) ^ 1);
-                    if (*(volatile int*)&s_abort) break;              // no copies after an abort: nothing would wait for them
-                    mbar_expect_tx(full_x(s), (uint32_t)nv * (uint32_t)P.npad * 128u);
-                    for (int j = 0; j < nv; j++)
-                        tma_load_2d(x_base + s * GR_X_STAGE + j * GR_X_KB, &xmap, (kb + j - sg * nkb1) * GM_BK, 0, full_x(s));
-                }
-            }
-        }
-    } else if (warp == GR_DECODE_WARPS + 1) {
-        if (elect_one()) {                                      // MMA issuer
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(P.npad >> 3) << 17) | ((uint32_t)(GR_ROWS >> 4) << 24);
-            int it = 0;
-            uint32_t accumulate = 0;
-            for (int sg = 0; sg < 2; sg++) {
-                for (int kb = seg_lo[sg]; kb < seg_hi[sg]; kb += GR_KBS, it++) {
-                    const int s = it % GR_STAGES, nv = min(GR_KBS, seg_hi[sg] - kb);
-                    const uint32_t par = (it / GR_STAGES) & 1;
-                    wait(full_x(s), par);
-                    wait(full_a(s), par);
-                    if (*(volatile int*)&s_abort) break;              // no MMAs on tiles that never arrived
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int j = 0; j < nv; j++) {
-#pragma unroll
-                        for (int kk = 0; kk < GM_BK / 16; kk++) {
-                            umma_f16(tmem, umma_desc_sw128(a_base + s * GR_A_STAGE + j * GR_A_KB + kk * 32),
-                                     umma_desc_sw128(x_base + s * GR_X_STAGE + j * GR_X_KB + kk * 32), idesc, accumulate);
-                            accumulate = 1;
-                        }
-                    }
-                    umma_commit(empty(s));
-                }
-            }
-            umma_commit(tmem_full);
-        }
-    } else {
-        // ---------------- decode: thread = (W row r0 + (tid & 127), k-block tid >> 7 of the stage)
-        const int rl = tid & 127, kbs = tid >> 7, row = r0 + rl;
-        const bool live = row < m.Rpad;
-        const uint32_t* wp = (const uint32_t*)m.words + row;
-        const uint32_t sw = (uint32_t)(rl & 7);
-        const uint32_t rowoff = (uint32_t)kbs * GR_A_KB + (uint32_t)(rl >> 3) * 1024u + sw * 128u;
-        int it = 0;
-        for (int sg = 0; sg < 2; sg++) {
-            if (seg_lo[sg] >= seg_hi[sg]) continue;
-            if (sg == 1 && seg_lo[0] < seg_hi[0]) {
-                // switch books: every decode thread is done with the first one (barrier among the decode warps only)
-                asm volatile("bar.sync 1, %0;" ::"n"(GR_DECODE_WARPS * 32) : "memory");
-                const uint4* t1 = (const uint4*)m.table2;
-                uint4* dst = (uint4*)smem;
-                for (int i = tid; i < 4096; i += GR_DECODE_WARPS * 32) dst[i] = __ldg(t1 + i);
-                asm volatile("bar.sync 1, %0;" ::"n"(GR_DECODE_WARPS * 32) : "memory");
-            }
-            uint32_t wa = 0, wb = 0, wc = 0, na = 0, nb = 0, nc = 0;
-            auto load_tags = [&](int kb, uint32_t& a, uint32_t& b, uint32_t& c) {
-                a = b = c = 0;
-                if (live && kb < seg_hi[sg]) {
-                    const uint32_t* p = wp + (int64_t)kb * 3 * m.Rpad;
-                    a = __ldg(p); b = __ldg(p + m.Rpad); c = __ldg(p + 2 * (int64_t)m.Rpad);
-                }
-            };
-            load_tags(seg_lo[sg] + kbs, wa, wb, wc);
-            for (int kb = seg_lo[sg]; kb < seg_hi[sg]; kb += GR_KBS, it++) {
-                const int s = it % GR_STAGES;
-                load_tags(kb + GR_KBS + kbs, na, nb, nc);
-                wait(empty(s), ((it / GR_STAGES) & 1) ^ 1);
-                if (kb + kbs < seg_hi[sg]) {
-                    const uint32_t dst = a_base + s * GR_A_STAGE + rowoff;
-                    uint32_t off[8];
-                    off[0] = (wa << 4) & 0xFFF0u;
-                    off[1] = (wa >> 8) & 0xFFF0u;
-                    off[2] = __funnelshift_r(wa, wb, 20) & 0xFFF0u;
-                    off[3] = wb & 0xFFF0u;
-                    off[4] = (wb >> 12) & 0xFFF0u;
-                    off[5] = __funnelshift_r(wb, wc, 24) & 0xFFF0u;
-                    off[6] = (wc >> 4) & 0xFFF0u;
-                    off[7] = (wc >> 16) & 0xFFF0u;
-                    uint4 cw[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) cw[c] = cbl_lds128(sbase + off[c]);
-#pragma unroll
-                    for (int c = 0; c < 8; c++)
-                        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + (((uint32_t)c ^ sw) << 4)), "r"(cw[c].x), "r"(cw[c].y),
-                                     "r"(cw[c].z), "r"(cw[c].w)
-                                     : "memory");
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_a(s));
-                wa = na; wb = nb; wc = nc;
-            }
-        }
-        // ---------------- epilogue: decode warps 0..3 read TMEM lanes (= W rows) 32 w ..; columns = tokens
-        if (warp < 4) {
-            wait(tmem_full, 0);
-            const bool ok = *(volatile int*)&s_abort == 0;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int r = r0 + warp * 32 + lane;
-            if (ok) {
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (r < m.R) {
-                    if (P.ksplit == 1) {
-                        const float rs = __half2float(__ldg((const __half*)m.row_scale + r));
-#pragma unroll 4
-                        for (int n = 0; n < GR_NMAX; n++)
-                            if (n < ntok) cbl_store_out(P.y[mi], ydtype, (int64_t)n * ldy + r, __uint_as_float(v[n]) * xinv[n] * rs);
-                    } else {
-                        float* acc = P.acc[mi] + r;
-#pragma unroll 4
-                        for (int n = 0; n < GR_NMAX; n++)
-                            if (n < ntok) atomicAdd(acc + (int64_t)n * m.Rpad, __uint_as_float(v[n]));
-                    }
-                }
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (s_abort && tid == 0) atomicExch(status, 1u);
-    if (warp == GR_DECODE_WARPS) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32u) : "memory");
-    }
-}
-
-// Variant with the decoded A tile in TENSOR memory: a decode thread writes its row's codewords straight from
+// The decoded A tile lies in TENSOR memory: a decode thread writes its row's codewords straight from
 // registers into its TMEM lane (tcgen05.st) and the MMA takes A from TMEM, so neither the store of the A tile nor
 // the tensor cores' read of it touch shared memory - only the codeword gathers do.  TMEM columns: 0..31 the
 // accumulator, then GT_STAGES stages of 4 k-blocks x 32 columns (a k-block = 64 fp16 per row = 32 columns).
@@ -890,104 +702,11 @@ __global__ void __launch_bounds__(256) k_rows_finish(const __grid_constant__ GRL
 // carries the codeword gathers, the B-tile stores, the activation tiles and the tensor cores' operand
 // reads, and saturates before the tensor pipe does.  From about a thousand tokens on it is cheaper to
 // decode the matrix ONCE into a 16-bit scratch (cbl_decode_raw: raw codewords, or the sum of the two books'
-// codewords, column orders undone) and to run a plain TMA-fed tcgen05 GEMM over it (k_gemm_dense: both
+// codewords, column orders undone) and to run a plain TMA-fed tcgen05 GEMM over it (k_gemm_dense_2sm: both
 // operands arrive by TMA, nothing but the tensor cores reads shared memory).  Row scales and the tokens'
 // power-of-two scales are applied in the epilogue exactly as in the fused kernel.  The scratch also
 // serves matrices with several column orders, which the fused kernels do not execute.
-constexpr int GD_STAGES = 3;
-constexpr int GD_STAGE_BYTES = 2 * GM_A_BYTES + GM_B_BYTES;                 // 256 tokens + 256 rows of one k-block: 64 KB
-constexpr int GD_SMEM = GD_STAGES * GD_STAGE_BYTES + 1024;                  // + slack to align the ring to 1024 bytes
-constexpr int GD_EPI_WARPS = 8, GD_THREADS = (GD_EPI_WARPS + 2) * 32;
-
-__global__ void __launch_bounds__(GD_THREADS, 1)
-k_gemm_dense(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, cbl_l8 m, const float* __restrict__ xinv,
-             int ntok, void* __restrict__ y, int ydtype, int64_t ldy, int vec_ok, unsigned int* __restrict__ status) {
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long s_bar[2 * GD_STAGES + 1];
-    __shared__ uint32_t s_tmem;
-    __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
-    // token tiles vary fastest across the grid: blocks that run together share weight rows in L2
-    const int r0 = blockIdx.y * GM_BN, tok0 = blockIdx.x * GM_BM;
-    const int nkb = (m.C + GM_BK - 1) / GM_BK;
-    const uint32_t sbase = (cbl_smem_u32(smem_raw) + 1023u) & ~1023u, bar0 = cbl_smem_u32(s_bar);
-    auto full = [&](int s) { return bar0 + 8u * s; };
-    auto empty = [&](int s) { return bar0 + 8u * (GD_STAGES + s); };
-    const uint32_t tmem_full = bar0 + 8u * (2 * GD_STAGES);
-    if (tid == 0) {
-        s_abort = 0;
-        for (int s = 0; s < GD_STAGES; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        mbar_init(tmem_full, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == GD_EPI_WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cbl_smem_u32(&s_tmem)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem;
-
-    if (warp == GD_EPI_WARPS) {
-        if (elect_one()) {                                      // TMA producer: activations (2 x 128 tokens) and weights (256 rows)
-            for (int kb = 0; kb < nkb; kb++) {
-                const int s = kb % GD_STAGES;
-                if (!mbar_wait(empty(s), ((kb / GD_STAGES) & 1) ^ 1)) { s_abort = 1; break; }
-                mbar_expect_tx(full(s), GD_STAGE_BYTES);
-                const uint32_t dst = sbase + s * GD_STAGE_BYTES;
-                tma_load_2d(dst, &xmap, kb * GM_BK, tok0, full(s));
-                tma_load_2d(dst + GM_A_BYTES, &xmap, kb * GM_BK, tok0 + 128, full(s));
-                tma_load_2d(dst + 2 * GM_A_BYTES, &wmap, kb * GM_BK, r0, full(s));
-            }
-        }
-    } else if (warp == GD_EPI_WARPS + 1) {
-        if (elect_one()) {                                      // MMA issuer
-            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-            for (int kb = 0; kb < nkb; kb++) {
-                const int s = kb % GD_STAGES;
-                if (!mbar_wait(full(s), (kb / GD_STAGES) & 1)) { s_abort = 1; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = sbase + s * GD_STAGE_BYTES, b_addr = a_addr + 2 * GM_A_BYTES;
-#pragma unroll
-                for (int tb = 0; tb < 2; tb++) {
-#pragma unroll
-                    for (int kk = 0; kk < GM_BK / 16; kk++) {
-                        const uint64_t da = umma_desc_sw128(a_addr + tb * GM_A_BYTES + kk * 32);
-                        const uint64_t db = umma_desc_sw128(b_addr + kk * 32);
-                        umma_f16(tmem + tb * GM_BN, da, db, idesc, (kb | kk) ? 1u : 0u);
-                    }
-                }
-                umma_commit(empty(s));
-            }
-            umma_commit(tmem_full);
-        }
-    } else {
-        const bool ok = mbar_wait(tmem_full, 0);
-        if (!ok) s_abort = 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int q = warp & 3, tb = warp >> 2;
-        const int tok = tok0 + tb * 128 + q * 32 + lane;
-        const float tsc = (tok < ntok) ? xinv[tok] : 0.f;
-        if (ok) {
-            for (int c0 = 0; c0 < GM_BN; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(tb * GM_BN + c0), v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                gemm_store_row32(v, tok, ntok, r0 + c0, m, tsc, y, ydtype, ldy, vec_ok);
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (s_abort && tid == 0) atomicExch(status, 1u);
-    if (warp == GD_EPI_WARPS) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-    }
-}
-
-// The same GEMM on pairs of thread blocks, persistent, with the epilogue overlapped: a cluster of two blocks
+// It runs on pairs of thread blocks, persistent, with the epilogue overlapped: a cluster of two blocks
 // computes 256-token x 256-row tiles with tcgen05.mma.cta_group::2 (each block holds 128 tokens of the
 // activations and 128 rows of the weights per k-block, so the traffic from L2 per MMA cycle is the one of a
 // 256 x 256 tile although a block only accumulates 128 x 256).  A block's accumulator takes 256 of the 512
@@ -1229,20 +948,11 @@ extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const 
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
     }
-    {
-        // columns beyond C and rows beyond R are outside the map: TMA fills them with zeros
-        const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)R};
-        const cuuint64_t strides[1] = {(cuuint64_t)((C + 7) / 8 * 8) * 2};
-        const cuuint32_t box[2] = {GM_BK, GM_BN};
-        CUresult cr = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)w16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
-    }
     static bool attr_set[64] = {};
     int dev = 0;
     CBL_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        CBL_CUDA(cudaFuncSetAttribute(k_gemm_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM));
+        CBL_CUDA(cudaFuncSetAttribute(k_gemm_dense_2sm, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM));
         attr_set[dev] = true;
     }
     cbl_l8 m = {};
@@ -1252,56 +962,41 @@ extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const 
     const float* xinv = (const float*)((const __half*)stage + (int64_t)Mpad * Cpad);
     const int esz = ydtype == CBL_F32 ? 4 : 2;
     const int vec_ok = ((uintptr_t)y % 16 == 0) && ((ldy * esz) % 16 == 0) && ((uintptr_t)row_scale % 16 == 0);
-#ifdef CBL_DENSE_1SM
-    if (bias) return CBL_EUNSUPPORTED;
-    const int variant = 1;                                    // build option: the one-block kernel (for comparisons)
-#else
-    const int variant = 2;
-#endif
-    if (variant == 2) {
-        // Rows per tile: the fewest waves of SM pairs, each as long as its tile is wide (plus a tile's start and end, about
-        // 40 rows' worth).  700 tokens x 3584 rows: 69 tiles of 160 rows in one wave instead of 42 of 256.
-        const int ntt = cbl_ceil_div(ntok, 256), pairs = cbl_sm_count() / 2;
-        int bn = 256;
-        long best = -1;
-        for (int b = 256; b >= 64; b -= 32) {
-            const long cost = (long)cbl_ceil_div(ntt * cbl_ceil_div(R, b), pairs) * (b + 40);
-            if (best < 0 || cost < best) { best = cost; bn = b; }
-        }
-        // box of the pair kernel: 128 tokens / half of the tile's weight rows per block
-        {
-            const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)R};
-            const cuuint64_t strides[1] = {(cuuint64_t)((C + 7) / 8 * 8) * 2};
-            const cuuint32_t box[2] = {GM_BK, (cuuint32_t)(bn / 2)};
-            CUresult cr = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)w16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
-        }
-        static bool attr3_set[64] = {};
-        if (dev >= 0 && dev < 64 && !attr3_set[dev]) {
-            CBL_CUDA(cudaFuncSetAttribute(k_gemm_dense_2sm, cudaFuncAttributeMaxDynamicSharedMemorySize, G3_SMEM));
-            attr3_set[dev] = true;
-        }
-        const int ntiles = cbl_ceil_div(R, bn) * ntt;
-        int nclusters = pairs;
-        if (nclusters > ntiles) nclusters = ntiles;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * nclusters);
-        cfg.blockDim = dim3(G3_THREADS);
-        cfg.dynamicSmemBytes = G3_SMEM;
-        cfg.stream = st;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, bias, bn, (unsigned int*)workspace));
-        return cbl_check_launch();
+    // Rows per tile: the fewest waves of SM pairs, each as long as its tile is wide (plus a tile's start and end, about
+    // 40 rows' worth).  700 tokens x 3584 rows: 69 tiles of 160 rows in one wave instead of 42 of 256.
+    const int ntt = cbl_ceil_div(ntok, 256), pairs = cbl_sm_count() / 2;
+    int bn = 256;
+    long best = -1;
+    for (int b = 256; b >= 64; b -= 32) {
+        const long cost = (long)cbl_ceil_div(ntt * cbl_ceil_div(R, b), pairs) * (b + 40);
+        if (best < 0 || cost < best) { best = cost; bn = b; }
     }
-    dim3 grid(cbl_ceil_div(ntok, GM_BM), cbl_ceil_div(R, GM_BN));
-    k_gemm_dense<<<grid, GD_THREADS, GD_SMEM, st>>>(xmap, wmap, m, xinv, ntok, y, ydtype, ldy, vec_ok, (unsigned int*)workspace);
+    // box of the pair kernel: 128 tokens / half of the tile's weight rows per block; columns beyond C and rows beyond R are outside the
+    // map: TMA fills them with zeros
+    {
+        const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)R};
+        const cuuint64_t strides[1] = {(cuuint64_t)((C + 7) / 8 * 8) * 2};
+        const cuuint32_t box[2] = {GM_BK, (cuuint32_t)(bn / 2)};
+        CUresult cr = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)w16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
+    }
+    const int ntiles = cbl_ceil_div(R, bn) * ntt;
+    int nclusters = pairs;
+    if (nclusters > ntiles) nclusters = ntiles;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * nclusters);
+    cfg.blockDim = dim3(G3_THREADS);
+    cfg.dynamicSmemBytes = G3_SMEM;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, bias, bn, (unsigned int*)workspace));
     return cbl_check_launch();
 }
 
@@ -1371,15 +1066,9 @@ extern "C" int cbl_gemm_rows_multi(const cbl_l8* mats, int32_t n, const void* x,
     int dev = 0;
     CBL_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        CBL_CUDA(cudaFuncSetAttribute(k_gemm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
         CBL_CUDA(cudaFuncSetAttribute(k_gemm_rows_ta, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM));
         attr_set[dev] = true;
     }
-#ifdef CBL_ROWS_SMEM_A
-    const int ta = 0;                                          // build option: the A tile through shared memory (comparisons)
-#else
-    const int ta = 1;
-#endif
     const float* xinv = (const float*)((const __half*)stage + (int64_t)Mpad * Cpad);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1390,9 +1079,8 @@ extern "C" int cbl_gemm_rows_multi(const cbl_l8* mats, int32_t n, const void* x,
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(tiles, ksplit);
     cfg.blockDim = dim3(GR_THREADS);
-    cfg.dynamicSmemBytes = ta ? GT_SMEM : GR_SMEM;
-    if (ta) CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_rows_ta, xmap, P, xinv, (int)ntok, ydtype, ldy, status));
-    else CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_rows, xmap, P, xinv, (int)ntok, ydtype, ldy, status));
+    cfg.dynamicSmemBytes = GT_SMEM;
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_rows_ta, xmap, P, xinv, (int)ntok, ydtype, ldy, status));
     if (ksplit > 1) {
         int maxR = 0;
         for (int i = 0; i < P.n; i++) maxR = maxR > P.m[i].R ? maxR : P.m[i].R;
