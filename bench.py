@@ -896,7 +896,7 @@ def run_load(args, rank: int, world: int, local_rank: int) -> None:
     line = {"metric": "packed_load_gbs", "value": nbytes / s / 1e9, "unit": "GB/s", "n_gpus": world, "steps": args.steps, "warmup": 2,
             "ms_per_step": s * 1e3, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "u8", "data": "synthetic",
             "config": {"workload": f"load of a packed file with {layers} layers of Qwen2.5-7B shapes ({nbytes} bytes, page cache warm) into one arena "
-                                   f"with the l8 and x16 kernel layouts", "parallelism": f"tp{world}" if world > 1 else "single",
+                                   f"with the l8 and b3 kernel layouts", "parallelism": f"tp{world}" if world > 1 else "single",
                        "timing": "host wall clock around load_linears (the path is host-driven: file read, pinned copy, H2D, repack kernels)"},
             "gpu_launches": 3 * len(kinds) * args.steps, "arena_bytes": stats["arena_bytes"], "h2d_bytes_per_step": stats["h2d_bytes"],
             "tensor_by_tensor_ms": s_one * 1e3}
@@ -930,7 +930,7 @@ def _case_gemv_l8(shapes):
 
 
 def _case_gemm_b3(tokens: int, copies: int):
-    """gate|up of a few tokens by codeword gathers, distinct matrices (203 MB of layout) a few times."""
+    """gate|up of a few tokens by codeword gathers, three pairs (17 MB of layout per matrix) twice."""
     from quantexperiments_b200.kernels import B3Group, B3Matrix
     grps = [B3Group([B3Matrix(_case_matrix(18944, 3584, seed=7 * i + j), copies) for j in range(2)]) for i in range(3)]
     X = torch.randn(tokens, 3584, device="cuda").bfloat16()

@@ -37,7 +37,7 @@
 #include "cbl_common.cuh"
 
 
-constexpr int L8_NT = 512;                       // threads per block; a thread handles 4 consecutive rows per ring stage
+constexpr int L8_NT = 512;                       // threads that look up; each handles 4 consecutive rows per step
 constexpr int L8_NWARP = L8_NT / 32;
 constexpr int L8_BUILDERS = 8;                   // warps that build the tables after the first
 constexpr int L8_FRAGS = 128 / L8_BUILDERS;      // pairs of 16 codewords that one of them holds

@@ -1,9 +1,11 @@
 """Device-side matrices and kernel launchers over libcbl (thin, allocation-aware Python).
 
 DeviceMatrix  the file layout resident on the GPU: dense decode, tag unpacking
-T16Matrix     row-tile re-layout + tensor-core product for batches up to 64 (column orders and
-              two summed books supported)
-L8Matrix      column-tile re-layout + batch-1 product by activation-side tables
+L8Matrix      column-tile re-layout + one-token product by activation-side tables (L8Group: several matrices per launch)
+B3Matrix      slots of rotated book copies + product of 1..128 tokens by codeword gathers (B3Group)
+DenseStack    decode once + GEMM, for many tokens
+T16Matrix, X16Matrix, L8Group.gemm_rows, L8Matrix.gemm
+              earlier products of small and large batches: callers may use them, nothing in the package does
 
 All launches go to torch's current CUDA stream; outputs can be caller-provided so that steady-state
 calls allocate nothing (CUDA-graph capturable)."""

@@ -206,7 +206,7 @@ class RowParallelLinear:
         lead = x.shape[:-1]
         n = math.prod(lead)
         y = torch.empty(n, self.R, dtype=torch.float32, device=x.device)
-        self.lin.forward_into(x.reshape(n, self.lin.in_features), y)    # one token: table lookups; <= 64: row tiles; more: decode + GEMM
+        self.lin.forward_into(x.reshape(n, self.lin.in_features), y)    # up to 128 tokens: table lookups or codeword gathers; more: decode + GEMM
         return y.reshape(*lead, self.R)
 
     @property

@@ -443,7 +443,7 @@ def test_engine_steps_match_the_torch_restatement(dtype, books, M):
 def test_engine_graph_replay_prefill_and_batched_engine_agree():
     from quantexperiments_b200.engine import Qwen2BatchEngine, generate, random_engine
     eng = random_engine(_small_cfg(max_len=160), seed=9)
-    prompt = torch.randint(0, 1000, (70,), generator=torch.Generator().manual_seed(1)).tolist()      # > 64 tokens: the GEMM path
+    prompt = torch.randint(0, 1000, (70,), generator=torch.Generator().manual_seed(1)).tolist()      
     # eager token-by-token feed of the prompt, then greedy continuation
     eng.reset(prompt[0])
     for i, t in enumerate(prompt):

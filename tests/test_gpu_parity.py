@@ -466,11 +466,11 @@ def test_packed_linear_matches_reference_fixture_and_dispatches_by_token_count()
     assert lin.stored_bytes() == int(z["stored_bytes"][0])
     assert float(lin.dense().double().sum()) == float(z["dense_sum"][0])
     x = _t(z["x"]).cuda()
-    y = lin(x)                                    # 3 tokens -> small-batch kernel
+    y = lin(x)                                    # 3 tokens -> codeword gathers
     assert orc.max_rel_err(y.cpu().numpy(), z["y"]) < TOL
     y1 = lin(x[:1])                               # 1 token -> batch-1 path
     assert orc.max_rel_err(y1.cpu().numpy(), z["y"][:1]) < TOL
-    xb = torch.randn(2, 40, C, device="cuda", dtype=torch.bfloat16)      # 80 tokens, column orders -> decode + library GEMM
+    xb = torch.randn(2, 40, C, device="cuda", dtype=torch.bfloat16)      # 80 tokens
     yb = lin(xb)
     ref = xb.float().reshape(80, C) @ lin.dense().T
     assert yb.shape == (2, 40, R) and orc.max_rel_err(yb.float().reshape(80, R).cpu().numpy(), ref.cpu().numpy()) < 1e-2
@@ -675,7 +675,7 @@ def test_qwen32b_shaped_rows_with_two_books_and_sixteen_column_orders(C):
     Y = l8.gemm(x.cuda(), torch.empty(300, 2304, device="cuda"))
     l8.status()
     assert orc.max_rel_err(Y.cpu().numpy(), yref) < TOL
-    # the module dispatches 300 tokens of a 16-order matrix to decode + library GEMM
+    # the module dispatches 300 tokens of a 16-order matrix to decode + GEMM
     lin = PackedLinear(_t(m["words"][0]).cuda(), _t(m["table"][0]).cuda(), _t(m["row_scale"]).cuda(), None, _t(m["row_mask"]).cuda(),
                        _t(m["perms"]).cuda(), 4096, 8, words2=_t(m["words"][1]).cuda(), table2=_t(m["table"][1]).cuda())
     yl = lin(x.cuda())
@@ -889,7 +889,7 @@ def test_large_decode_with_the_book_in_shared_memory_equals_the_generic_decode(R
     assert torch.equal(big[:R, :C], dm.dequant(dtype=torch.bfloat16)) and torch.isnan(big[:R, C:]).all() and torch.isnan(big[R:]).all()
 
 
-# ------------------------------------------------------------------------------------------ 1..64 tokens, book in three copies
+# ------------------------------------------------------------------------------------------ 1..128 tokens, book in two or three copies
 @pytest.mark.parametrize("Rs,C,books,M", [((1,), 8, 1, 1), ((130,), 64, 1, 1), ((300,), 264, 2, 1), ((1000, 129, 40), 520, 1, 1), ((260, 130), 1032, 2, 4),
                                           ((2304,), 8200, 1, 16), ((3584, 512, 512), 3584, 1, 1), ((20000,), 456, 1, 1), ((9000, 9000), 904, 2, 1),
                                           ((19000,), 128, 2, 16), ((18950,), 2248, 1, 1)])

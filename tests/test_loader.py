@@ -99,7 +99,7 @@ def test_rank_shards_and_pooling(tmp_path):
         ref = full["a.gate"][:, rank * 512:(rank + 1) * 512] @ x.float()
         assert (y.float() - ref).abs().max() <= 1e-2 * ref.abs().max()
     # an input shard of a matrix with several column orders keeps orders that name positions of the full activation
-    # vector: the ranks' partial products (1, 5 and 100 tokens: table lookups, row tiles, wide decode + GEMM) add up
+    # vector: the ranks' partial products (1, 5 and 100 tokens) add up
     masks_full = PackedLinear.from_packed(pf, "b.masks")
     Cm = masks_full.C
     for T in (1, 5, 100):
