@@ -4,7 +4,7 @@
 // activations, picks the product for their token count, allocates the output and launches on torch's current stream.  It
 // returns None for whatever it does not handle (a layout that is not built yet, an unusual dtype): the Python path then
 // does the work and fills the plan.  Per call the Python path spends 20 (one token) to 45 us (many tokens) on the host, which is more
-// than most products of a decode step run on the GPU; this one spends 4 to 8.
+// than most products of a decode step run on the GPU; this one spends 6 (one launch) to 10.
 //
 // Scratch buffers (staged activations, partial sums, decoded weights) belong to a (device, stream) pair and grow on demand; the
 // Python call paths take theirs from here as well (scratch()).  Calls on one stream share them in the order of the stream; graphs
@@ -47,6 +47,7 @@ struct Plan {
     cbl_packed packed[MAX_PIECES];
     const void* row_scale = nullptr;                      // of the stacked rows
     at::Tensor bias;
+    PyObject* keep = nullptr;                             // the tensors whose addresses the descriptors hold
     size_t ws_bytes[2][129] = {};
     size_t l8_bytes = 0;
     int dense_from = 0;                                   // tokens from which the two-phase product runs
@@ -261,16 +262,17 @@ void free_plan(PyObject* o) {
         std::lock_guard<std::mutex> lock(g_mu);
         if (--g_plans[p->device] == 0) drop(p->device, false);
     }
+    Py_XDECREF(p->keep);
     delete p;
 }
 
-// plan(device, in, C, orders, rows: list, perms pointer, dense_from, bias or None) -> capsule
+// plan(device, in, C, orders, rows: list, perms pointer, dense_from, bias or None, tensors to keep alive) -> capsule
 PyObject* py_plan(PyObject*, PyObject* args) {
     int device, orders, dense_from;
     long long in, C;
     unsigned long long perms;
-    PyObject *rows, *bias;
-    if (!PyArg_ParseTuple(args, "iLLiOKiO", &device, &in, &C, &orders, &rows, &perms, &dense_from, &bias)) return nullptr;
+    PyObject *rows, *bias, *keep;
+    if (!PyArg_ParseTuple(args, "iLLiOKiOO", &device, &in, &C, &orders, &rows, &perms, &dense_from, &bias, &keep)) return nullptr;
     const Py_ssize_t n = PyList_Size(rows);
     if (n < 1 || n > MAX_PIECES) { PyErr_SetString(PyExc_ValueError, "a plan holds 1..4 matrices"); return nullptr; }
     Plan* p = new Plan;
@@ -282,6 +284,8 @@ PyObject* py_plan(PyObject*, PyObject* args) {
         p->l8_bytes += cbl_gemv_l8_workspace_bytes((int32_t)p->rows[i]);
     }
     if (bias != Py_None && THPVariable_Check(bias)) p->bias = THPVariable_Unpack(bias);
+    Py_INCREF(keep);
+    p->keep = keep;
     {
         std::lock_guard<std::mutex> lock(g_mu);
         g_plans[device]++;
@@ -496,7 +500,7 @@ PyObject* py_set_linear(PyObject*, PyObject* fn) {
 
 PyMethodDef methods[] = {
     {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "forward(plan, x) -> y or None"},
-    {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias)"},
+    {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias, keep)"},
     {"set", py_set, METH_VARARGS, "set(plan, kind, descriptors, row_scale=0)"},
     {"stream", py_stream, METH_NOARGS, "stream(): torch's current stream of the current device"},
     {"device", py_device, METH_NOARGS, "device(): the current device"},

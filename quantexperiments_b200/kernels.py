@@ -61,10 +61,36 @@ def _dt(t: torch.dtype) -> int:
         raise ValueError(f"dtype {t} is not supported (float32, float16, bfloat16)") from None
 
 
-class DeviceMatrix:
+def _where(*ts: torch.Tensor | None) -> tuple:
+    """Addresses, for telling whether a cached descriptor still describes these tensors."""
+    return tuple(0 if t is None else t.data_ptr() for t in ts)
+
+
+class _Uncopied:
+    """Copies and pickles without the named attributes (cached descriptors, which hold addresses): None in their place."""
+
+    _uncopied: tuple = ()
+
+    def __getstate__(self):
+        return {k: None if k in self._uncopied else v for k, v in self.__dict__.items()}
+
+
+# counts tensors that have been put in the place of others (DeviceMatrix attributes, loader.pool_layouts()): native call plans made
+# before hold old addresses and are made again
+epoch = [0]
+
+
+class DeviceMatrix(_Uncopied):
     """One packed matrix in the file layout on a CUDA device (tags int32 [R, W], table fp16
     [G*K, d], row_scale fp16 [R], optional row_book / row_mask uint8 [R], perms int32 [M, C];
     optional second tag plane + table for two summed books)."""
+
+    _uncopied = ("_packed",)
+
+    def __setattr__(self, name, value):
+        if isinstance(value, torch.Tensor) and name in self.__dict__:
+            epoch[0] += 1
+        object.__setattr__(self, name, value)
 
     def __init__(self, tags, table, row_scale, row_book=None, row_mask=None, perms=None, *, K: int, d: int,
                  C: int | None = None, device="cuda", tags2=None, table2=None, x_cols: int | None = None):
@@ -116,7 +142,7 @@ class DeviceMatrix:
                    torch.ones(words.shape[0], dtype=torch.float16, device=dev), K=1 << bits, d=1, C=n, device=dev)
 
     def struct(self) -> _lib.Packed:
-        key = (self.tags.data_ptr(), self.table.data_ptr(), self.row_scale.data_ptr())
+        key = _where(self.tags, self.tags2, self.table, self.table2, self.row_scale, self.row_book, self.row_mask, self.perms)
         if self._packed is None or self._packed[0] != key:
             self._packed = (key, self._make_struct())
         return self._packed[1]
@@ -422,11 +448,12 @@ class B3Matrix:
         return self.words.numel() * 4 + (0 if self.tile_rows is None else (self.tile_rows.numel() + self.tile_order.numel()) * 4)
 
 
-class B3Group:
+class B3Group(_Uncopied):
     """Up to four matrices that read the same activations through the same column orders (q|k|v, gate|up), run as one
     launch: run(X [B, >= C], ys) writes ys[i] [B, R_i]; the outputs share one row stride."""
 
     MAX = 4
+    _uncopied = ("_built",)
 
     def __init__(self, mats: list[B3Matrix], biases: list | None = None):
         if not 1 <= len(mats) <= self.MAX:
@@ -441,7 +468,7 @@ class B3Group:
 
     @property
     def _structs(self):
-        key = tuple(m.words.data_ptr() for m in self.mats)
+        key = tuple(_where(m.words, m.tile_rows, m.tile_order, m.dm.table, m.dm.table2, m.dm.row_scale) for m in self.mats)
         if self._built is None or self._built[0] != key:
             self._built = (key, (_lib.B3 * len(self.mats))(*[m.struct(b) for m, b in zip(self.mats, self.biases)]))
         return self._built[1]
@@ -487,11 +514,13 @@ class B3Group:
             _lib.check("cbl_gemm_b3_status", lib.cbl_gemm_b3_status(ws.data_ptr(), _stream()))
 
 
-class DenseStack:
+class DenseStack(_Uncopied):
     """Matrices that multiply the same activations (q|k|v, gate|up, or a single matrix), for many tokens or
     for matrices with several column orders: every matrix is decoded ONCE into a 16-bit scratch shared by
     all stacks of the device and stream (rows stacked in order), then one TMA-fed tensor-core GEMM writes
     Y [T, sum R]. d = 8, 12-bit tags, G = 1; one or two books; any number of column orders."""
+
+    _uncopied = ("_scales",)
 
     def __init__(self, dms: list):
         for dm in dms:
@@ -500,8 +529,16 @@ class DenseStack:
             raise ValueError("stacked matrices share the input size and the device")
         self.dms, self.C, self.device = dms, dms[0].C, dms[0].device
         self.R = sum(dm.R for dm in dms)
-        self.row_scale = dms[0].row_scale if len(dms) == 1 else torch.cat([dm.row_scale for dm in dms])
         self.ld = (self.C + 7) // 8 * 8
+        self._scales = None                     # (addresses, the stacked rows' scales)
+        self.row_scale
+
+    @property
+    def row_scale(self) -> torch.Tensor:
+        key = _where(*[dm.row_scale for dm in self.dms])
+        if self._scales is None or self._scales[0] != key:
+            self._scales = (key, self.dms[0].row_scale if len(self.dms) == 1 else torch.cat([dm.row_scale for dm in self.dms]))
+        return self._scales[1]
 
     def scratch_bytes(self) -> int:
         return lib.cbl_dense_scratch_bytes(self.R, self.C)
@@ -707,11 +744,12 @@ class L8Matrix:
         return y
 
 
-class L8Group:
+class L8Group(_Uncopied):
     """Up to four column-tile matrices that read the same activation vector (q|k|v, gate|up), run as
     one launch: run(x, ys) writes each matrix's output into its own contiguous vector."""
 
     MAX = 4
+    _uncopied = ("_built", "_built_c")
 
     def __init__(self, mats: list[L8Matrix]):
         if not 1 <= len(mats) <= self.MAX:
@@ -730,7 +768,7 @@ class L8Group:
     @property
     def _structs(self):
         """The matrices' batch-1 descriptors; rebuilt when a matrix's buffers have moved (loader.pool_layouts)."""
-        key = tuple(m.words.data_ptr() for m in self.mats)
+        key = tuple(_where(m.words, m.frag, m.frag2, m.row_index, m.dm.table, m.dm.table2, m.dm.row_scale, m.dm.perms) for m in self.mats)
         if self._built is None or self._built[0] != key:
             self._built = (key, (_lib.L8 * len(self.mats))(*[m.struct() for m in self.mats]))
         return self._built[1]

@@ -20,7 +20,7 @@ import math
 import torch
 
 from . import _cblhost, _lib
-from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix
+from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix, _Uncopied, epoch
 
 # Rows from which one token runs on activation-side tables (L8Matrix) instead of codeword gathers (B3Matrix); of a matrix with
 # several column orders, rows per order: every order needs tables of its own, and a build costs as much as the lookups of some
@@ -34,14 +34,19 @@ L8_MIN_ROWS_PER_ORDER = 1536
 B3_MAX_3COPIES = 16
 # Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM.
 DENSE_MIN_TOKENS = 129
-# counts loader.pool_layouts() calls: native plans made before one hold old addresses
-pool_epoch = 0
 
 
-class PackedLinear(torch.nn.Module):
+def _tensors(objs) -> tuple:
+    """Every tensor of some objects: what a native plan keeps alive, since it holds their addresses."""
+    return tuple(v for o in objs for v in vars(o).values() if isinstance(v, torch.Tensor))
+
+
+class PackedLinear(_Uncopied, torch.nn.Module):
     """A block linear run from packed tensors: one token -> batch-1 kernel, up to 128 tokens -> the
     codeword-gather tensor-core kernel, more -> decode once + tcgen05 GEMM. Constructor arguments follow the
     reference (words, table, row_scale, row_book, row_mask, perms, K, d, bias)."""
+
+    _uncopied = ("_host", "_host_bias")
 
     def __init__(self, words, table, row_scale, row_book, row_mask, perms, K: int, d: int, bias=None,
                  words2=None, table2=None, x_cols: int | None = None):
@@ -112,9 +117,9 @@ class PackedLinear(torch.nn.Module):
         dm, b = self.dm, self.bias
         if not dm.fast or (b is not None and (b.requires_grad or b.shape != (self.R,))):
             return
-        self._host_bias = b
+        self._host_bias, self._host_epoch = b, epoch[0]
         self._host = _cblhost.plan(dm.device.index, self.in_features, self.C, dm.M, [self.R], 0 if dm.perms is None else dm.perms.data_ptr(),
-                                   DENSE_MIN_TOKENS, b)
+                                   DENSE_MIN_TOKENS, b, _tensors([dm, *([] if self._l8 is None else [self._l8]), *(g.mats[0] for g in self._b3.values())]))
         if self._l8 is not None and self.use_l8():
             _cblhost.set(self._host, "l8", bytes(self._l8.struct()))
         for g in self._b3.values():
@@ -164,7 +169,7 @@ class PackedLinear(torch.nn.Module):
         return y
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if self._host is not None and self._host_bias is self.bias:
+        if self._host is not None and self._host_bias is self.bias and self._host_epoch == epoch[0]:
             y = _cblhost.forward(self._host, x)
             if y is not None:
                 return y
@@ -269,7 +274,9 @@ class Stack:
         if not self.fast or len(self.lins) > B3Group.MAX:
             return None, None
         dm = self.lins[0].dm
-        h = _cblhost.plan(dm.device.index, self.C, self.C, dm.M, self.Rs, 0 if dm.perms is None else dm.perms.data_ptr(), DENSE_MIN_TOKENS, None)
+        held = [l.dm for l in self.lins] + ([] if self._l8 is None else self._l8.mats)
+        keep = _tensors(held + [m for g in self._b3.values() for m in g.mats]) + (() if self.dense is None else (self.dense.row_scale,))
+        h = _cblhost.plan(dm.device.index, self.C, self.C, dm.M, self.Rs, 0 if dm.perms is None else dm.perms.data_ptr(), DENSE_MIN_TOKENS, None, keep)
         if self._l8 is not None:
             _cblhost.set(h, "l8", bytes(self._l8._structs))
         for g in self._b3.values():

@@ -233,8 +233,8 @@ def pool_layouts(linears) -> int:
     that use these matrices: single-matrix launchers and L8Group read the pointers at every call, but a captured
     graph, a PeerReduceGemv or a decode engine built earlier keeps the old addresses (build those afterwards).
     Returns the bytes now pooled."""
-    from . import linear
-    linear.pool_epoch += 1
+    from .kernels import epoch
+    epoch[0] += 1
     lins = [l for l in linears if not getattr(l, "_pooled", False)]
     pooled = 0
     for dev in {l.dm.device for l in lins}:

@@ -13,8 +13,8 @@ from __future__ import annotations
 
 import torch
 
-from .. import _cblhost, linear
-from ..kernels import T16Matrix
+from .. import _cblhost
+from ..kernels import T16Matrix, _Uncopied, epoch
 from ..linear import DENSE_MIN_TOKENS, PackedLinear, Stack
 
 BMAX = T16Matrix.BMAX
@@ -42,7 +42,9 @@ def packed_pieces(prefix: str, names) -> list[str] | None:
     return None
 
 
-class PackedShards:
+class PackedShards(_Uncopied):
+    _uncopied = ("_host",)
+
     def __init__(self, lins: list[PackedLinear], *, bmax: int = BMAX, **_ignored):
         if not lins:
             raise ValueError("no pieces")
@@ -63,7 +65,7 @@ class PackedShards:
         # Kernel layouts are second copies of the tags in a kernel's order: each is built when its token-count class
         # is first used (or by prepare()), so a layer that only ever decodes keeps one extra copy, not three.
         self.stack = Stack(lins)
-        self._host = (None, None)               # native call plans: up to 128 tokens, more
+        self._host = None                       # native call plans: up to 128 tokens, more
         self.prepare(1)
 
     def prepare(self, M: int) -> None:
@@ -73,9 +75,9 @@ class PackedShards:
             if torch.cuda.is_current_stream_capturing():
                 raise RuntimeError(f"PackedShards.prepare({M}) must run before the stream is captured (layouts are allocated on first use)")
             self.stack.prepare(M)
-            self._host = (None, None)
-        if self._host[1] is None or self._epoch != linear.pool_epoch:
-            self._host, self._epoch = self.stack.bind(), linear.pool_epoch
+            self._host = None
+        if self._host is None or self._host[1] is None or self._epoch != epoch[0]:
+            self._host, self._epoch = self.stack.bind(), epoch[0]
 
     @classmethod
     def from_packed(cls, pf, names: list[str], dev="cuda", **kw) -> "PackedShards":
@@ -99,8 +101,8 @@ class PackedShards:
         """x [..., C] -> [..., R] in x's dtype."""
         shp = x.shape
         M = x.numel() // self.C
-        host = self._host[M >= DENSE_MIN_TOKENS]
-        if host is not None and self._epoch == linear.pool_epoch and x.dtype in (torch.float16, torch.bfloat16):
+        host = self._host and self._host[M >= DENSE_MIN_TOKENS]
+        if host is not None and self._epoch == epoch[0] and x.dtype in (torch.float16, torch.bfloat16):
             y = _cblhost.forward(host, x)
             if y is not None:
                 return y

@@ -1083,3 +1083,41 @@ def test_decode_into_memory_that_an_output_has_just_left():
             lin(X)
             kernels.release_scratch()
             assert torch.equal(lin(X), w)
+
+
+@pytest.mark.parametrize("M", [1, 3])
+def test_layers_copy_and_pickle_after_use(M):
+    """A layer that has run (layouts, native plan, cached descriptors) still copies and pickles; the copy owns its tensors."""
+    import copy
+    import gc
+    import pickle
+    m = orc.synth_matrix(2100, 512, seed=60 + M, M=M)
+    lin = _linear(m, bias=torch.randn(2100, device="cuda").bfloat16())
+    xs = [torch.randn(n, 512, device="cuda").bfloat16() for n in (1, 5, 40, 200)]
+    want = [lin(x) for x in xs]
+    lin.dense(), lin.gemv(xs[0][0])
+    twins = [copy.deepcopy(lin), pickle.loads(pickle.dumps(lin))]
+    del lin
+    gc.collect()
+    for twin in twins:
+        for _ in range(2):
+            assert all(torch.equal(twin(x), w) for x, w in zip(xs, want))
+
+
+@pytest.mark.parametrize("M", [1, 2])
+def test_tensors_given_to_a_matrix_later_are_used(M):
+    """Row scales put in the place of a matrix's are honoured by the next call on every path, and the old ones are not read again."""
+    from quantexperiments_b200.vllm_ext import core
+    ms = [orc.synth_matrix(4200, 256, seed=70 + i, M=M) for i in range(2)]
+    lins = [_linear(m) for m in ms]
+    ps = core.PackedShards(lins)
+    xs = [torch.randn(n, 256, device="cuda").bfloat16() for n in (1, 5, 40, 200)]
+    for _ in range(2):
+        before = [(lins[0](x), ps.forward(x)) for x in xs]
+    for lin in lins:
+        lin.dm.row_scale = lin.dm.row_scale * 2
+    junk = [torch.full_like(lins[0].dm.row_scale, float("nan")) for _ in range(8)]          # takes the freed memory
+    for _ in range(2):
+        for x, (a, b) in zip(xs, before):
+            assert torch.equal(lins[0](x), 2 * a) and torch.equal(ps.forward(x), 2 * b)
+    assert all(t.isnan().all() for t in junk) and torch.equal(lins[0].dense(), torch.from_numpy(orc.synth_decode(ms[0])).cuda() * 2)
