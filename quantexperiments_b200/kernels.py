@@ -432,6 +432,9 @@ class B3Matrix:
         _need_fast(dm)
         self.dm, self.R, self.C, self.M, self.books, self.device = dm, dm.R, dm.C, dm.M, dm.books, dm.device
         self.copies, self.bmax = copies, lib.cbl_gemm_b3_max_tokens(copies)
+        if torch.cuda.is_current_stream_capturing():
+            # it would be written by a node of the graph: garbage to every other caller until the first replay
+            raise RuntimeError("the layout of a token count is built by its first call (or prepare()): make that before the stream is captured")
         self.tile_rows, self.tile_order, self.ntile = order_tiles(dm, 128)
         nbytes = lib.cbl_b3_bytes(self.ntile, dm.C, dm.books)
         self.words = _alloc_i32(max(nbytes, 16) // 4, dm.device, alloc)

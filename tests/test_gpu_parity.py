@@ -1121,3 +1121,22 @@ def test_tensors_given_to_a_matrix_later_are_used(M):
         for x, (a, b) in zip(xs, before):
             assert torch.equal(lins[0](x), 2 * a) and torch.equal(ps.forward(x), 2 * b)
     assert all(t.isnan().all() for t in junk) and torch.equal(lins[0].dense(), torch.from_numpy(orc.synth_decode(ms[0])).cuda() * 2)
+
+
+def test_layouts_are_not_built_inside_a_captured_region():
+    """A first call inside a capture is refused (the layout would hold garbage until the first replay); after a first call it captures."""
+    lin = _linear(orc.synth_matrix(300, 512, seed=90))
+    x = torch.randn(12, 512, device="cuda").bfloat16()
+    s = torch.cuda.Stream()
+    with pytest.raises(RuntimeError, match="before the stream is captured"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=s):
+            lin(x)
+    torch.cuda.synchronize()
+    assert not lin._b3
+    want = lin(x).clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        y = lin(x)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
