@@ -64,7 +64,7 @@ struct Scratch {
     int turn = 0;
 };
 
-std::mutex g_mu;                                          // (everything below also runs with the interpreter lock held)
+std::recursive_mutex g_mu;                                          // (everything below also runs with the interpreter lock held)
 std::map<std::pair<int, void*>, Scratch> g_scratch;
 std::vector<at::Tensor> g_kept;                           // outgrown buffers that a graph points at
 std::map<int, long> g_plans;                              // plans alive per device
@@ -99,7 +99,7 @@ at::Tensor beside_graph(int64_t n, int device) {
 
 // The buffer of a kind on (device, current stream), at least `bytes` long; status words and arrival counters are zero when it is new.
 const at::Tensor& need(Kind kind, size_t bytes, int device, void* stream) {
-    std::lock_guard<std::mutex> lock(g_mu);
+    std::lock_guard<std::recursive_mutex> lock(g_mu);
     Scratch& sc = g_scratch[{device, stream}];
     if (kind == WEIGHTS) sc.turn ^= 1;                    // the decode of a product may run beside the GEMM of the one before
     Buffer& b = kind == WEIGHTS && sc.turn ? sc.second : sc.b[kind];
@@ -259,7 +259,7 @@ void free_plan(PyObject* o) {
     Plan* p = plan_of(o);
     if (!p) return;
     {
-        std::lock_guard<std::mutex> lock(g_mu);
+        std::lock_guard<std::recursive_mutex> lock(g_mu);
         if (--g_plans[p->device] == 0) drop(p->device, false);
     }
     Py_XDECREF(p->keep);
@@ -287,7 +287,7 @@ PyObject* py_plan(PyObject*, PyObject* args) {
     Py_INCREF(keep);
     p->keep = keep;
     {
-        std::lock_guard<std::mutex> lock(g_mu);
+        std::lock_guard<std::recursive_mutex> lock(g_mu);
         g_plans[device]++;
     }
     return PyCapsule_New(p, PLAN, free_plan);
@@ -334,7 +334,7 @@ PyObject* py_status(PyObject*, PyObject* args) {
     try {
         const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
         cudaDeviceSynchronize();
-        std::lock_guard<std::mutex> lock(g_mu);
+        std::lock_guard<std::recursive_mutex> lock(g_mu);
         for (auto& e : g_scratch) {
             if (e.first.first != device) continue;
             const Buffer* const s = e.second.b;
@@ -376,7 +376,7 @@ PyObject* py_scratch(PyObject*, PyObject* args) {
 PyObject* py_release(PyObject*, PyObject* args) {
     int device;
     if (!PyArg_ParseTuple(args, "i", &device)) return nullptr;
-    std::lock_guard<std::mutex> lock(g_mu);
+    std::lock_guard<std::recursive_mutex> lock(g_mu);
     drop(device, true);
     Py_RETURN_NONE;
 }
