@@ -373,7 +373,8 @@ int cbl_gemm_b3_status(void* workspace, cbl_stream s);
 
 /* Orders a stream for kernels that start early (programmatic dependent launch): the products read tags, books and layouts, and
  * cbl_decode_raw writes its output, while the kernel before them still runs.  Call it between the work that produced a matrix's
- * tensors, or that last used the memory of a decode's output, and the first product (the re-layouts above end with it). */
+ * tensors, or that last used the memory of a decode's output, and the first product.  cbl_repack_b3 ends with it; after
+ * cbl_repack_l8r and cbl_repack_book the host waits in cbl_book_norm_exp, which does as well when it is called last. */
 int cbl_order(cbl_stream s);
 
 /* Two-phase prefill for many tokens and for matrices with several column orders: decode the matrix ONCE

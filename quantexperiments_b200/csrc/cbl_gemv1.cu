@@ -597,7 +597,7 @@ extern "C" int cbl_repack_book(const void* table, void* out, cbl_stream s) {
     if (!table || !out || ((uintptr_t)table % 4) || ((uintptr_t)out % 16)) return CBL_EINVAL;
     CBL_CUDA(cudaMemsetAsync((char*)out + 65536, 0, 16, (cudaStream_t)s));
     k_repack_book<<<16, 256, 0, (cudaStream_t)s>>>((const uint32_t*)table, (uint4*)out, (unsigned int*)((char*)out + 65536));
-    return cbl_order(s);                                // the product reads the layout before it waits for its predecessor
+    return cbl_check_launch();
 }
 
 // Rotated column-tile layout: uint32 [ntile][3][Rpad].  Position p of the row order holds source row row_index[p]
@@ -647,7 +647,7 @@ extern "C" int cbl_repack_l8r(const cbl_packed* m, const int32_t* row_index, int
     const int64_t n = (int64_t)m->books * ntile1 * Rpad;
     if (n == 0) return CBL_OK;
     k_repack_l8r<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)s>>>(*m, row_index, ntile1, Rpad, (uint32_t*)out, n);
-    return cbl_order(s);
+    return cbl_check_launch();
 }
 
 // ------------------------------------------------------------------------------------ launch

@@ -638,7 +638,8 @@ class L8Matrix:
             _lib.check("cbl_repack_book", lib.cbl_repack_book(dm.table.data_ptr(), self.frag.data_ptr(), _stream()))
             if dm.books == 2:
                 _lib.check("cbl_repack_book", lib.cbl_repack_book(dm.table2.data_ptr(), self.frag2.data_ptr(), _stream()))
-            # the exponent that scales the kernel's tables, read back once so that no launch has to fetch it
+            # the exponent that scales the kernel's tables, read back once so that no launch has to fetch it (the wait also puts the
+            # layouts behind it: the product reads them before it waits for its predecessor)
             e = ctypes.c_int32(0)
             _lib.check("cbl_book_norm_exp", lib.cbl_book_norm_exp(self.frag.data_ptr(), ctypes.byref(e), _stream()))
             self.book_exp, self.book_exp2 = e.value, 0
