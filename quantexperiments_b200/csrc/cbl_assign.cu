@@ -10,6 +10,7 @@
 // k_pack_tags  one thread per 32-bit word of the stream.
 #include "cbl_tc.cuh"
 #include <cmath>
+#include <type_traits>
 
 constexpr int AS_THREADS = 256, AS_GROUP = 8;
 
@@ -123,30 +124,37 @@ k_assign(const float* __restrict__ x, const float* __restrict__ wt, int64_t n, c
 //     A1 = [hi(-2 x) | f f f 0 0 0 0 0]   A2 = [lo(-2 x) | 0]   B = [c | hi, mid, lo of |c|^2 | 0]
 // so A1 B + A2 B = f |c|^2 - 2 x.c in fp32 (f: a power of two per chunk that keeps large chunks inside fp16; 1 otherwise).
 // Book and chunks are scaled by one more power of two when the book's largest value is not within 2 .. 64.
-// Sixteen warps read the 128 x 256 results out of tensor memory and keep the two groups of 16 codewords with the smallest
-// values per chunk and warpgroup; those of the best group - and of every group that is closer than the arithmetic above can
-// tell - are then evaluated in fp32 exactly as k_assign does, so that index and error are k_assign's, bit for bit.
+// Twelve warps read the distances out of tensor memory (four accumulators of 128 words, taken in turn by three warpgroups) and keep
+// the smallest values of the two best groups of 32 words per chunk and warpgroup, the group's number in the value's last six bits.
+// Four other warps evaluate the words of the best group - and of every group that is closer than the arithmetic above can tell -
+// in fp32 exactly as k_assign does, so that index and error are k_assign's, bit for bit, while the twelve read the next tile.
 //
-// 8.49 M chunks x 4096 words: 11.1 ms by k_assign (0.65 of the fp32 FMA rate), 3.6 ms here.  The epilogue bounds it: three-input
-// minima issue at half rate; with the comparison left out it takes 2.5 ms, with the products left out the same 3.6.
-constexpr int AT_TILE = 128, AT_N = 256, AT_EPI = 512, AT_THREADS = AT_EPI + 64 + 32;
-constexpr int AT_PROD_WARP = 16, AT_MMA_WARP = 18;
+// 8.49 M chunks x 4096 words: 11.1 ms by k_assign (0.65 of the fp32 FMA rate), 2.42 ms here.  The ALU pipe bounds it (77 % busy): a
+// three-input minimum takes it two clocks per two values, and the groups' numbers, the two smallest and the exact evaluation
+// make 0.9 instructions per value.  With 512 threads that met at a barrier after every tile, a branch per group of 16 and one
+// warp that issued all products it took 3.6 ms; four warpgroups of 64 values at a time take 2.5.
+constexpr int AT_TILE = 128, AT_N = 128, AT_GROUP = 32, AT_WG = 3, AT_EPI = AT_WG * 128, AT_THREADS = AT_EPI + 256;
+constexpr int AT_AUX_WARP = AT_EPI / 32, AT_MMA_WARP = AT_AUX_WARP + 4;
 constexpr int AT_A_BYTES = 4096;                 // 128 rows x 16 fp16
-constexpr int AT_BOOK = 131072;
+constexpr int AT_SQ = 131072;                    // behind the book in MMA order: |c|^2 of every word, as k_assign adds it up
+constexpr int AT_BOOK = AT_SQ + 16384;
 constexpr int AT_STAGE = 2 * AT_A_BYTES + AT_TILE * 36;         // A1 | A2 | the chunks in fp32 | the scales f
-constexpr int AT_SMEM = AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * 12 + 4 * AT_TILE * 8;
+constexpr int AT_SMEM = AT_BOOK + 2 * AT_STAGE + 2 * AT_WG * AT_TILE * 12;
+constexpr uint32_t AT_ID = 63;                   // a warpgroup sees a third of 4096 words: 44 groups
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
 
-__device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < AT_WAIT_LIMIT; i++) {
+// Bounded wait.  One that expires is remembered (the errors of the block become NaN) and ends the waits after it at once; the roles
+// keep their step.
+__device__ __forceinline__ void at_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+    for (uint32_t i = 1; i <= AT_WAIT_LIMIT; i++) {
         uint32_t ok;
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                      : "=r"(ok)
                      : "r"(bar), "r"(parity)
                      : "memory");
-        if (ok) return true;
+        if (ok || ((i & 255u) == 0 && *abort)) return;
     }
-    return false;
+    *abort = 1;
 }
 __device__ __forceinline__ void at_umma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -161,24 +169,23 @@ __device__ __forceinline__ uint64_t at_desc(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)(128 >> 4) << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46;
 }
 __device__ __forceinline__ uint32_t at_row(int r) { return (uint32_t)((r >> 3) * 256 + (r & 7) * 16); }      // first half; the second 128 bytes on
-__device__ __forceinline__ void at_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+// 64 columns, landed: load and wait are one statement, so that the values are not copied to be tied to the wait.
+__device__ __forceinline__ void at_ld64(uint32_t taddr, uint32_t (&v)[32], uint32_t (&u)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, "
+        "%52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
           "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-
-// Waits for the loads issued so far; the values cannot be used ahead of it.
-__device__ __forceinline__ void at_landed(uint32_t (&v)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), 
-                   "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
-                 :
-                 : "memory");
+          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]),
+          "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]),
+          "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]),
+          "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
+        : "r"(taddr), "r"(taddr + 32)
+        : "memory");
 }
 
 // Where the chunks come from: an array of them, or rows of a matrix divided by their fp16 scale (zero columns appended).
@@ -209,35 +216,47 @@ __device__ __forceinline__ void at_chunk(const AtSource& s, int64_t ci, float (&
     for (int i = 0; i < 8; i++) v[i] = __fdiv_rn(v[i], sc);
 }
 
-struct AtPart { float best; int bg; float second; };
+struct AtPart { float best; int bg; float second; };           // bg: the best value's group of 32 words
 
-// |c_k|^2 - 2 x.c_k of word k, added up as k_assign does (a book that was scaled down may have lost bits in shared memory).
-__device__ __forceinline__ float at_dist(const unsigned char* words, const __half* __restrict__ book, int q2, float ibs, const float (&x)[8], int k) {
-    const uint4 cw = q2 >= 0 ? *(const uint4*)(words + at_row(k)) : __ldg((const uint4*)book + k);
+// Word k in fp32.  HOW: 0 as it lies in shared memory, 1 there scaled up, 2 from the book itself (scaled down it may have lost bits).
+template <int HOW>
+__device__ __forceinline__ void at_word(const unsigned char* smem, const __half* __restrict__ book, float ibs, int k, float (&c)[8]) {
+    const uint4 cw = HOW < 2 ? *(const uint4*)(smem + at_row(k)) : __ldg((const uint4*)book + k);
     const __half2* h = (const __half2*)&cw;
-    float c[8], d = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const float2 p = __half22float2(h[i]);
-        c[2 * i] = q2 > 0 ? p.x * ibs : p.x;
-        c[2 * i + 1] = q2 > 0 ? p.y * ibs : p.y;
+        c[2 * i] = HOW == 1 ? p.x * ibs : p.x;
+        c[2 * i + 1] = HOW == 1 ? p.y * ibs : p.y;
     }
-#pragma unroll
-    for (int i = 0; i < 8; i++) d += c[i] * c[i];
+}
+__device__ __forceinline__ uint64_t at_pair(float lo, float hi) { return (uint64_t)__float_as_uint(hi) << 32 | __float_as_uint(lo); }
+
+// |c_k|^2 - 2 x.c_k of word k, added up as k_assign does.
+__device__ __forceinline__ float at_dist(const unsigned char* smem, const __half* __restrict__ book, int q2, float ibs, const float (&x)[8], int k) {
+    float c[8];
+    if (q2 >= 0) at_word<1>(smem, book, ibs, k, c);
+    else at_word<2>(smem, book, ibs, k, c);
+    float d = *(const float*)(smem + AT_SQ + 4 * k);
 #pragma unroll
     for (int i = 0; i < 8; i++) d = fmaf(-2.0f * x[i], c[i], d);
     return d;
 }
 
-// The nearest of words k0 .. k1 - 1 to one chunk, for a warp: {distance, index}, the first index that reaches the minimum.
-__device__ __forceinline__ float2 at_nearest(const unsigned char* words, const __half* __restrict__ book, int q2, float ibs, float4 x0, float4 x1, int k0, int k1) {
+// The nearest of words k0 .. k0 + 127, k0 + step .. k0 + step + 127 and so on below k1 to one chunk, for a warp: {distance, index}, the
+// first index that reaches the minimum.
+__device__ __forceinline__ float2 at_nearest(const unsigned char* words, const __half* __restrict__ book, int q2, float ibs, float4 x0, float4 x1, int k0, int k1, int step) {
     const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
     float d0 = INFINITY;
     int i0 = 0;
 #pragma unroll 1
-    for (int k = k0 + (threadIdx.x & 31); k < k1; k += 32) {
-        const float d = at_dist(words, book, q2, ibs, xs, k);
-        if (d < d0 || (d == d0 && k < i0)) { d0 = d; i0 = k; }
+    for (; k0 < k1; k0 += step) {
+#pragma unroll
+        for (int h = 0; h < AT_N; h += 32) {
+            const int k = k0 + h + (threadIdx.x & 31);
+            const float d = at_dist(words, book, q2, ibs, xs, k);
+            if (d < d0 || (d == d0 && k < i0)) { d0 = d; i0 = k; }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -252,29 +271,33 @@ __global__ void __launch_bounds__(AT_THREADS, 1)
 k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int64_t* __restrict__ idx, float* __restrict__ err,
             unsigned char* __restrict__ used) {
     extern __shared__ __align__(1024) unsigned char at_smem[];
-    __shared__ __align__(8) unsigned long long s_bar[8];
+    __shared__ __align__(8) unsigned long long s_bar[22];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     __shared__ unsigned int s_max;
     const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
     const uint32_t sb = cbl_smem_u32(at_smem), bar0 = cbl_smem_u32(s_bar);
     auto full_a = [&](int s) { return bar0 + 8u * s; };
-    auto empty_a = [&](int s) { return bar0 + 16u + 8u * s; };
-    auto acc_full = [&](int b) { return bar0 + 32u + 8u * b; };
-    auto acc_empty = [&](int b) { return bar0 + 48u + 8u * b; };
-    AtPart* s_part = (AtPart*)(at_smem + AT_BOOK + 2 * AT_STAGE);
-    float2* s_ex = (float2*)(at_smem + AT_BOOK + 2 * AT_STAGE + 4 * AT_TILE * (int)sizeof(AtPart));
+    auto acc_empty = [&](int b) { return bar0 + 16u + 8u * b; };
+    auto part_full = [&](int s) { return bar0 + 48u + 8u * s; };
+    auto part_empty = [&](int s) { return bar0 + 64u + 8u * s; };
+    // use u is announced at barrier u % 12: that one is waited for by one warpgroup only (the four accumulators' uses are finished in
+    // no certain order, so a barrier per accumulator could be two phases behind the one that looks at its parity)
+    auto use_full = [&](uint32_t i) { return bar0 + 80u + 8u * i; };
+    AtPart* s_part = (AtPart*)(at_smem + AT_BOOK + 2 * AT_STAGE);      // [2 tiles][3 warpgroups][128 chunks]
     const int64_t ntile = (n + AT_TILE - 1) / AT_TILE;
-    const int nstep = K / AT_N;
+    // A use of an accumulator: 128 words of a tile; uses are numbered over all of the block's tiles, use u is one of accumulator u & 3.
+    const uint32_t nuse = K / AT_N, uses = blockIdx.x < ntile ? (uint32_t)((ntile - blockIdx.x + gridDim.x - 1) / gridDim.x) * nuse : 0u;
     if (tid == 0) {
         s_abort = 0;
         s_max = 0u;
         for (int s = 0; s < 2; s++) {
-            mbar_init(full_a(s), 2);
-            mbar_init(empty_a(s), 1 + 4);                      // the MMAs, and the epilogue's last look at the fp32 chunks
-            mbar_init(acc_full(s), 1);
-            mbar_init(acc_empty(s), 8);
+            mbar_init(full_a(s), 4);
+            mbar_init(part_full(s), AT_EPI / 32);
+            mbar_init(part_empty(s), 4);
         }
+        for (int b = 0; b < 4; b++) mbar_init(acc_empty(b), 4);
+        for (int i = 0; i < 12; i++) mbar_init(use_full(i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == AT_MMA_WARP) {
@@ -310,6 +333,7 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
             sq += f.x * f.x;
             sq += f.y * f.y;
         }
+        ((float*)(at_smem + AT_SQ))[k] = sq;
         sq = sq * bs * bs;
         __align__(16) __half part[8];
 #pragma unroll
@@ -328,133 +352,85 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
-    // A wait that expires is remembered (the errors of the block become NaN); the roles keep their step (they meet at named barriers).
     auto wait = [&](uint32_t bar, uint32_t parity) {
-        if (!at_wait(bar, parity)) s_abort = 1;
+        at_wait(bar, parity, &s_abort);
         __syncwarp();
     };
 
-    if (warp == AT_MMA_WARP) {
+    if (warp >= AT_MMA_WARP) {
+        // ---------------- MMA issue: a warp per accumulator (one warp for all of them needs some 200 clocks per use, wait and commit
+        // included; the products take 128)
         const uint32_t idesc = (1u << 4) | ((uint32_t)(AT_N >> 3) << 17) | ((uint32_t)(AT_TILE >> 4) << 24);
-        int it = 0;
-        uint32_t use = 0;                                      // uses of the two accumulators so far
-        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++) {
-            const int ab = it & 1;
-            wait(full_a(ab), (it >> 1) & 1);
-            const uint64_t a1 = at_desc(sb + AT_BOOK + ab * AT_STAGE), a2 = at_desc(sb + AT_BOOK + ab * AT_STAGE + AT_A_BYTES);
-            for (int j = 0; j < nstep; j++, use++) {
-                const int b = use & 1;
-                wait(acc_empty(b), ((use >> 1) & 1) ^ 1);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t bd = at_desc(sb + (uint32_t)j * (AT_N * 32));
-                if (elect_one()) {
-                    at_umma(tmem + b * AT_N, a1, bd, idesc, 0u);
-                    at_umma(tmem + b * AT_N, a2, bd, idesc, 1u);
-                    umma_commit(acc_full(b));
-                    if (j == nstep - 1) umma_commit(empty_a(ab));
-                }
-                __syncwarp();
+        const int b = warp - AT_MMA_WARP;
+        // descriptors hold addresses / 16, in their lowest bits
+        const uint64_t stage0 = at_desc(sb + AT_BOOK), book0 = at_desc(sb);
+        uint32_t it = 0, j = b, i12 = b, par = 1;
+        for (uint32_t use = b; use < uses; use += 4, j += 4, par ^= 1u) {
+            for (; j >= nuse; j -= nuse) it++;
+            wait(full_a(it & 1), (it >> 1) & 1);
+            wait(acc_empty(b), par);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t a1 = stage0 + (it & 1) * (AT_STAGE / 16), bd = book0 + j * (AT_N * 32 / 16);
+            if (elect_one()) {
+                at_umma(tmem + b * AT_N, a1, bd, idesc, 0u);
+                at_umma(tmem + b * AT_N, a1 + AT_A_BYTES / 16, bd, idesc, 1u);
+                umma_commit(use_full(i12));
             }
+            __syncwarp();
+            i12 = i12 == b + 8u ? b : i12 + 4u;
         }
-    } else if (warp >= AT_PROD_WARP) {
-        // ---------------- producer: two chunks of the tile per thread
-        int it = 0;
-        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++) {
-            const int ab = it & 1;
-            float v[2][8];
+    } else if (warp >= AT_AUX_WARP) {
+        // ---------------- a thread a chunk of the tile: stages the next tile, then names the nearest words of this one.  A stage
+        // is free when its tile is finished (its products were complete before the epilogue's results were).
+        const int row = tid - AT_EPI;
+        const float ibs = ldexpf(1.f, -q2);
+        auto stage = [&](int64_t t, int ab) {
+            float v[8];
+            const int64_t ci = t * AT_TILE + row;
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const int64_t ci = t * AT_TILE + c * 64 + tid - AT_EPI;
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[c][i] = 0.f;
-                if (ci < n) at_chunk(src, ci, v[c]);
-            }
-            wait(empty_a(ab), ((it >> 1) & 1) ^ 1);
+            for (int i = 0; i < 8; i++) v[i] = 0.f;
+            if (ci < n) at_chunk(src, ci, v);
             unsigned char* st = at_smem + AT_BOOK + ab * AT_STAGE;
+            float mx = 0.f;
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const int r = c * 64 + tid - AT_EPI;
-                float mx = 0.f;
+            for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[i]));
+            mx *= bs;
+            const int e = mx > 8192.f && mx < 3.0e38f ? ilogbf(mx) - 12 : 0;      // |2 x| f < 2^14 (f only shrinks)
+            const float f = ldexpf(1.f, -e), fs = -2.0f * f * bs;
+            __align__(16) __half hi[8], lo[8], ff[8];
 #pragma unroll
-                for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[c][i]));
-                mx *= bs;
-                const int e = mx > 8192.f && mx < 3.0e38f ? ilogbf(mx) - 12 : 0;      // |2 x| f < 2^14 (f only shrinks)
-                const float f = ldexpf(1.f, -e), fs = -2.0f * f * bs;
-                __align__(16) __half hi[8], lo[8], ff[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float a = fs * v[c][i];
-                    hi[i] = __float2half_rn(a);
-                    lo[i] = __float2half_rn(a - __half2float(hi[i]));
-                    ff[i] = __float2half_rn(i < 3 ? f : 0.f);
-                }
-                const uint32_t o = at_row(r);
-                *(uint4*)(st + o) = *(const uint4*)hi;
-                *(uint4*)(st + o + 128) = *(const uint4*)ff;
-                *(uint4*)(st + AT_A_BYTES + o) = *(const uint4*)lo;
-                *(uint4*)(st + AT_A_BYTES + o + 128) = make_uint4(0, 0, 0, 0);
-                float4* xs = (float4*)(st + 2 * AT_A_BYTES) + r;       // [2][128]: the two halves of the chunks
-                xs[0] = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
-                xs[AT_TILE] = make_float4(v[c][4], v[c][5], v[c][6], v[c][7]);
-                ((float*)(st + 2 * AT_A_BYTES + AT_TILE * 32))[r] = f;
+            for (int i = 0; i < 8; i++) {
+                const float a = fs * v[i];
+                hi[i] = __float2half_rn(a);
+                lo[i] = __float2half_rn(a - __half2float(hi[i]));
+                ff[i] = __float2half_rn(i < 3 ? f : 0.f);
             }
+            const uint32_t o = at_row(row);
+            *(uint4*)(st + o) = *(const uint4*)hi;
+            *(uint4*)(st + o + 128) = *(const uint4*)ff;
+            *(uint4*)(st + AT_A_BYTES + o) = *(const uint4*)lo;
+            *(uint4*)(st + AT_A_BYTES + o + 128) = make_uint4(0, 0, 0, 0);
+            float4* xs = (float4*)(st + 2 * AT_A_BYTES) + row;         // [2][128]: the two halves of the chunks
+            xs[0] = make_float4(v[0], v[1], v[2], v[3]);
+            xs[AT_TILE] = make_float4(v[4], v[5], v[6], v[7]);
+            ((float*)(st + 2 * AT_A_BYTES + AT_TILE * 32))[row] = f;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(full_a(ab));
-        }
-    } else {
-        // ---------------- epilogue: warpgroup w reads half w & 1 of accumulator w >> 1; a thread's lane is a chunk of the tile
-        const int w = warp >> 2, row = (warp & 3) * 32 + lane, b = w >> 1;
-        const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(b * AT_N + (w & 1) * 128);
-        uint32_t use = b;                                      // accumulator uses are numbered over all tiles; this warpgroup takes every other
+        };
+        if (blockIdx.x < ntile) stage(blockIdx.x, 0);
         int it = 0;
-        uint32_t base = 0;
-        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++, base += nstep) {
-            float best = INFINITY, second = INFINITY;
+        uint32_t base = 0;                                     // number of the tile's first use
+        for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x, it++, base += nuse) {
+            if (t + gridDim.x < ntile) stage(t + gridDim.x, (it + 1) & 1);
+            wait(part_full(it & 1), (it >> 1) & 1);
+            const AtPart* const part = s_part + (it & 1) * AT_WG * AT_TILE;
+            // the two best groups that each warpgroup has seen
+            float best = INFINITY;
             int bg = 0;
-            for (; use < base + nstep; use += 2) {
-                const int j = (int)(use - base), g0 = j * 16 + (w & 1) * 8;
-                wait(acc_full(b), (use >> 1) & 1);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t va[32], vb[32];
-                auto look = [&](const uint32_t (&v)[32], int g) {
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        float m = as_min3(__uint_as_float(v[16 * h]), __uint_as_float(v[16 * h + 1]), __uint_as_float(v[16 * h + 2]));
-#pragma unroll
-                        for (int q = 3; q < 15; q += 2) m = as_min3(m, __uint_as_float(v[16 * h + q]), __uint_as_float(v[16 * h + q + 1]));
-                        m = fminf(m, __uint_as_float(v[16 * h + 15]));
-                        if (__builtin_expect(m < second, 0)) {      // a branch, not selects for every group: 3.61 ms against 3.77
-                            const bool top = m < best;
-                            second = top ? best : m;
-                            best = top ? m : best;
-                            bg = top ? g + h : bg;
-                        }
-                    }
-                };
-                at_ld32(ta, va);
-                at_landed(va);
-                at_ld32(ta + 32, vb);
-                look(va, g0);
-                at_landed(vb);
-                at_ld32(ta + 64, va);
-                look(vb, g0 + 2);
-                at_landed(va);
-                at_ld32(ta + 96, vb);
-                look(va, g0 + 4);
-                at_landed(vb);
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty(b));
-                look(vb, g0 + 6);
-            }
-            AtPart mine = {best, bg, second};
-            s_part[w * AT_TILE + row] = mine;
-            asm volatile("bar.sync 1, %0;" ::"n"(AT_EPI) : "memory");
-            // All four warpgroups know the two best groups that each of them has seen; each evaluates a quarter of a group's words.
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const AtPart p = s_part[q * AT_TILE + row];
+            for (int q = 0; q < AT_WG; q++) {
+                const AtPart p = part[q * AT_TILE + row];
                 if (q == 0 || p.best < best) { best = p.best; bg = p.bg; }
             }
             const unsigned char* st = at_smem + AT_BOOK + (it & 1) * AT_STAGE;
@@ -466,60 +442,116 @@ k_assign_tc(AtSource src, int64_t n, const __half* __restrict__ book, int K, int
             for (int i = 0; i < 8; i++) xx += xv[i] * xv[i];
             float bd = INFINITY;
             int bi = 0;
-            const float ibs = ldexpf(1.f, -q2);
+            // two words at a time, every lane at another place of its group (a group is 32 x 16 bytes: at the same place, all lanes
+            // would read the same four banks)
+            auto words = [&](auto how) {
+                uint64_t m2x[8];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int k = bg * 16 + w * 4 + q;
-                const float d = at_dist(at_smem, book, q2, ibs, xv, k);
-                if (d < bd || (d == bd && k < bi)) { bd = d; bi = k; }
-            }
+                for (int i = 0; i < 8; i++) m2x[i] = at_pair(-2.0f * xv[i], -2.0f * xv[i]);
+#pragma unroll 2
+                for (int q = 0; q < AT_GROUP / 2; q++) {
+                    const int k0 = bg * AT_GROUP + ((q + lane) & (AT_GROUP / 2 - 1)), k1 = k0 + AT_GROUP / 2;
+                    float c0[8], c1[8];
+                    at_word<decltype(how)::value>(at_smem, book, ibs, k0, c0);
+                    at_word<decltype(how)::value>(at_smem, book, ibs, k1, c1);
+                    uint64_t d = at_pair(*(const float*)(at_smem + AT_SQ + 4 * k0), *(const float*)(at_smem + AT_SQ + 4 * k1));
+#pragma unroll
+                    for (int i = 0; i < 8; i++) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(m2x[i]), "l"(at_pair(c0[i], c1[i])));
+                    const float d0 = __uint_as_float((uint32_t)d), d1 = __uint_as_float((uint32_t)(d >> 32));
+                    if (d0 < bd || (d0 == bd && k0 < bi)) { bd = d0; bi = k0; }
+                    if (d1 < bd || (d1 == bd && k1 < bi)) { bd = d1; bi = k1; }
+                }
+            };
+            if (q2 == 0) words(std::integral_constant<int, 0>());
+            else if (q2 > 0) words(std::integral_constant<int, 1>());
+            else words(std::integral_constant<int, 2>());
             // What two groups' values can be off by against each other.  Relative to the largest term or sum, 2^-24 for each of the 17
             // addends of an MMA, two MMAs, and 2^-23 of the products for the split; of two groups near the minimum d that is at
-            // most 2e-5 of |d| + |x|^2.  And the last place of the parts in fp16, 2^-25, times the sizes of a word's eight values.
+            // most 2e-5 of |d| + |x|^2.  The group's number in place of the last six bits: 2 x 63 x 2^-23 of |d|.  And the last
+            // place of the parts in fp16, 2^-25, times the sizes of a word's eight values.
             // Every group that is no further from the best is evaluated; a warpgroup knows two, so where its second is among them
-            // (or the values are not finite) all words are.  A chunk at a time: of N(0, 1) chunks and words one in 1700 comes here.
-            const float margin = 2e-5f * (fabsf(best) + f * (bs * bs) * xx) + 0x1p-23f * (4.f * top * bs + 1.f);
+            // (or the values are not finite) all words that it has seen are, a chunk at a time.
+            const float margin = 2e-5f * (fabsf(best) + f * (bs * bs) * xx) + 1.6e-5f * fabsf(best) + 0x1p-23f * (4.f * top * bs + 1.f);
             bool close = false;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const AtPart p = s_part[q * AT_TILE + row];
+            for (int q = 0; q < AT_WG; q++) {
+                const AtPart p = part[q * AT_TILE + row];
                 close |= !((p.bg == bg ? p.second : p.best) - best > margin);
             }
             for (uint32_t todo = __ballot_sync(0xffffffffu, close); todo; todo &= todo - 1) {
-                const int who = __ffs(todo) - 1, rw = (warp & 3) * 32 + who;
+                const int who = __ffs(todo) - 1, rw = (warp - AT_AUX_WARP) * 32 + who;
                 const float bw = __shfl_sync(0xffffffffu, best, who), mw = __shfl_sync(0xffffffffu, margin, who);
                 const float4* xw = (const float4*)(st + 2 * AT_A_BYTES) + rw;
-                bool all = false;
 #pragma unroll 1
-                for (int q = 0; q < 4; q++) all |= !(s_part[q * AT_TILE + rw].second - bw > mw);
-#pragma unroll 1
-                for (int q = 0; q < (all ? 1 : 4); q++) {
-                    const AtPart p = s_part[q * AT_TILE + rw];
+                for (int q = 0; q < AT_WG; q++) {
+                    const AtPart p = part[q * AT_TILE + rw];
+                    const bool all = !(p.second - bw > mw);
                     if (!all && !(p.best - bw <= mw)) continue;
-                    const int k0 = all ? w * (K / 4) : p.bg * 16 + w * 4;
-                    const float2 r = at_nearest(at_smem, book, q2, ibs, xw[0], xw[AT_TILE], k0, k0 + (all ? K / 4 : 4));
+                    // its steps of 128 words, or the one that its best group lies in
+                    const uint32_t mine = (uint32_t)(q + AT_WG - base % AT_WG) % AT_WG;
+                    const int k0 = all ? (int)mine * AT_N : p.bg * AT_GROUP / AT_N * AT_N;
+                    const float2 r = at_nearest(at_smem, book, q2, ibs, xw[0], xw[AT_TILE], k0, all ? K : k0 + 1, AT_WG * AT_N);
                     const int i = __float_as_int(r.y);
                     if (lane == who && (r.x < bd || (r.x == bd && i < bi))) { bd = r.x; bi = i; }
                 }
             }
-            s_ex[w * AT_TILE + row] = make_float2(bd, __int_as_float(bi));
-            asm volatile("bar.sync 1, %0;" ::"n"(AT_EPI) : "memory");
-            if (w == 0) {
-#pragma unroll
-                for (int q = 1; q < 4; q++) {
-                    const float2 p = s_ex[q * AT_TILE + row];
-                    const int k = __float_as_int(p.y);
-                    if (p.x < bd || (p.x == bd && k < bi)) { bd = p.x; bi = k; }
-                }
-                const int64_t ci = t * AT_TILE + row;
-                if (ci < n) {
-                    idx[ci] = bi;
-                    err[ci] = s_abort ? __int_as_float(0x7fc00000) : fmaxf(bd + xx, 0.f);      // an expired wait shows as NaN
-                    if (used) used[bi] = 1;
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(empty_a(it & 1));
+            const int64_t ci = t * AT_TILE + row;
+            if (ci < n) {
+                idx[ci] = bi;
+                err[ci] = s_abort ? __int_as_float(0x7fc00000) : fmaxf(bd + xx, 0.f);          // an expired wait shows as NaN
+                if (used) used[bi] = 1;
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(part_empty(it & 1));
+        }
+    } else {
+        // ---------------- epilogue: warpgroup w takes every third use; a thread's lane is a chunk of the tile
+        const int w = warp >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t t0 = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t zero = (uint32_t)K & 255u;              // orders a load behind the values before it: started early, it would take their registers
+        uint32_t use = w, base = 0, i12 = w, par = 0;
+        for (int it = 0; base < uses; it++, base += nuse) {
+            float best = INFINITY, second = INFINITY;
+            const uint32_t j0 = use - base;                    // this warpgroup's first step of the tile
+            for (uint32_t g0 = 0; use < base + nuse; use += AT_WG, g0 += 4) {
+                const uint32_t ta = t0 + (use & 3) * AT_N;
+                wait(use_full(i12), par);
+                if ((i12 += AT_WG) >= 12) { i12 -= 12; par ^= 1u; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t va[32], vb[32];
+                // minima of two groups with the groups' numbers in their last bits, and the two smallest of all so far: no branch (in some
+                // of a warp's lanes nearly every group is among the best two so far)
+                auto least = [&](const uint32_t (&v)[32], uint32_t g) {
+                    float m = as_min3(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2])),
+                          o = as_min3(__uint_as_float(v[16]), __uint_as_float(v[17]), __uint_as_float(v[18]));
+#pragma unroll
+                    for (int q = 3; q < 15; q += 2) {
+                        m = as_min3(m, __uint_as_float(v[q]), __uint_as_float(v[q + 1]));
+                        o = as_min3(o, __uint_as_float(v[16 + q]), __uint_as_float(v[17 + q]));
+                    }
+                    m = fminf(as_min3(m, __uint_as_float(v[15]), __uint_as_float(v[31])), o);
+                    return __uint_as_float((__float_as_uint(m) & ~AT_ID) | g);
+                };
+                auto look = [&](uint32_t g) {
+                    const float m0 = least(va, g), m1 = least(vb, g + 1), lo = fminf(m0, m1);
+                    second = as_min3(second, fmaxf(m0, m1), fmaxf(best, lo));
+                    best = fminf(best, lo);
+                };
+                at_ld64((__float_as_uint(best) & zero) | ta, va, vb);
+                look(g0);
+                at_ld64((__float_as_uint(best) & zero) | (ta + 64), va, vb);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(use & 3));
+                look(g0 + 2);
+            }
+            wait(part_empty(it & 1), ((it >> 1) & 1) ^ 1);
+            const uint32_t id = __float_as_uint(best) & AT_ID;
+            // the group's number among all words; 0 where no value was finite
+            const AtPart mine = {best, best < INFINITY ? (int)((j0 + AT_WG * (id >> 2)) * (AT_N / AT_GROUP) + (id & 3)) : 0, second};
+            s_part[((it & 1) * AT_WG + w) * AT_TILE + row] = mine;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(part_full(it & 1));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -554,7 +586,7 @@ extern "C" int cbl_assign(const float* x, const float* wt, int64_t n, int32_t d,
     if (((uintptr_t)x % 16) || (wt && ((uintptr_t)wt % 16))) return CBL_EINVAL;
     if (n == 0) return CBL_OK;
     // fp16 books of whole MMA tiles, unweighted, at least a few tiles of chunks: the tensor cores find the candidates
-    if (!wt && bdtype == CBL_F16 && K % AT_N == 0 && (uintptr_t)book % 16 == 0 && n >= 4 * AT_TILE)
+    if (!wt && bdtype == CBL_F16 && K % 256 == 0 && (uintptr_t)book % 16 == 0 && n >= 4 * AT_TILE)
         return launch_assign_tc(AtSource{x, nullptr, 0, 0, 0}, n, book, K, idx, err, nullptr, (cudaStream_t)s);
     const int Kpad = (K + AS_GROUP - 1) / AS_GROUP * AS_GROUP;
     const size_t smem = (size_t)Kpad * 36;
@@ -580,7 +612,7 @@ extern "C" int cbl_assign(const float* x, const float* wt, int64_t n, int32_t d,
 extern "C" int cbl_snap_rows(const float* w, int64_t R, int32_t C, int64_t ld, const void* scale, const void* book, int32_t K, int64_t* idx, float* err,
                              unsigned char* used, cbl_stream s) {
     if (!w || !scale || !book || !idx || !err || R < 0 || C < 1 || ld < C) return CBL_EINVAL;
-    if (K < AT_N || K > 4096 || K % AT_N || (uintptr_t)book % 16) return CBL_EUNSUPPORTED;
+    if (K < 256 || K > 4096 || K % 256 || (uintptr_t)book % 16) return CBL_EUNSUPPORTED;
     if (R == 0) return CBL_OK;
     const int nch = cbl_ceil_div(C, 8);
     return launch_assign_tc(AtSource{w, (const __half*)scale, C, nch, ld}, R * nch, book, K, idx, err, used, (cudaStream_t)s);

@@ -172,6 +172,19 @@ def test_tensor_core_assign_finds_the_exact_minimum(K, scale_x, scale_c):
         assert int(idx[6]) == K - 1 or torch.equal(book[int(idx[6])], book[K - 1])
 
 
+@pytest.mark.parametrize("K", [256, 512, 768, 1280, 3840])
+def test_tensor_core_assign_of_books_between_equals_the_scalar_kernel(K):
+    """Books whose uses of the accumulators fall unevenly to the three warpgroups and the four issuing warps; one tile and many per block."""
+    from quantexperiments_b200 import codebook as cb
+    g = torch.Generator().manual_seed(K)
+    book = torch.randn(K, 8, generator=g).half().cuda()
+    x = torch.randn(148 * 128 * 3 + 77, 8, generator=g).cuda()
+    for n in (512, x.shape[0]):
+        idx, err = cb.assign(x[:n], book)
+        few = [cb.assign(c.contiguous(), book) for c in x[:n].split(500)]          # fewer than 512 chunks: the scalar kernel
+        assert torch.equal(idx, torch.cat([i for i, _ in few])) and torch.equal(err, torch.cat([e for _, e in few]))
+
+
 def test_snap_rows_equals_snap_by_chunks():
     """snap() of a plain matrix (division and chunking inside the kernel, ragged columns) against assign() of the chunks."""
     from quantexperiments_b200 import codebook as cb
@@ -201,7 +214,7 @@ def test_snap_of_strided_rows(weighted):
 
 
 def test_tensor_core_assign_equals_the_scalar_kernel_where_many_words_all_but_tie():
-    """Words that differ in the last bits of one fp16 value: many groups of 16 lie closer together than the tensor cores can tell. Also
+    """Words that differ in the last bits of one fp16 value: many groups of 32 lie closer together than the tensor cores can tell. Also
     chunks and words that are tiny beside the book's largest value, and chunks that are not finite.  Fewer than 512 chunks run on the scalar kernel."""
     from quantexperiments_b200 import codebook as cb
     g = torch.Generator().manual_seed(11)
