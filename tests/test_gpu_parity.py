@@ -292,6 +292,26 @@ def test_one_token_of_few_rows_is_summed_in_fp32(R, C, books, M):
         assert (got.double() - ref).norm() <= books * (C / 16) * 2.0 ** -23 * ref.norm()
 
 
+@pytest.mark.parametrize("n,C,M", [(1, 8, 2), (1, 18944, 16), (3, 2056, 4), (9, 3584, 16), (128, 1032, 3)])
+def test_activations_staged_through_column_orders(n, C, M):
+    """Rows as long as the orders are picked from shared memory, rows further apart from memory: the same buffer, bit for bit."""
+    from quantexperiments_b200 import _lib
+    from quantexperiments_b200.packed import seeded_perms
+    perms = seeded_perms(C, M, torch.Generator().manual_seed(C)).to(torch.int32).cuda()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    for dt, code in ((torch.bfloat16, _lib.BF16), (torch.float16, _lib.F16), (torch.float32, _lib.F32)):
+        for at in (0, 1):                                    # on 16-byte boundaries and off them
+            buf = torch.randn(n * C + at, device="cuda", generator=g).mul_(300).to(dt)
+            x = buf[at:].view(n, C)
+            apart = torch.empty(n, C + 16, device="cuda", dtype=dt)
+            apart[:, :C] = x
+            out = [torch.full((_lib.lib.cbl_prep_x_bytes(n, C, M),), 255, dtype=torch.uint8, device="cuda") for _ in range(2)]
+            for t, o in zip((x, apart), out):
+                assert _lib.lib.cbl_prep_x(t.data_ptr(), code, n, C, t.stride(0) if n > 1 or t is apart else C, perms.data_ptr(), M, o.data_ptr(), 0) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(*out)
+
+
 @pytest.mark.parametrize("tokens", [1, 5, 200])
 def test_bias_of_another_shape_or_type_is_added_as_torch_would(tokens):
     """The native call path adds a bias of one value per row and x's type; every other form gives what `y + bias` gives, on every call."""
