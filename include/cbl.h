@@ -78,6 +78,18 @@ typedef struct cbl_packed {
  *          shapequant/kernels/batched_runs.py:935-961 (dequant_tile, fp16 / bf16 output). */
 int cbl_dequant(const cbl_packed* m, void* out, int dtype, int64_t ld, int32_t r0, int32_t r1, cbl_stream s);
 
+/* Products of 1..4 tokens of up to four small matrices (d = 8, 12-bit tags, G = 1; the same C, W and column orders) straight from the
+ * file layout, fp32 accumulate, one launch (two with several column orders, or where a row of x is not on a 16-byte boundary:
+ * `stage`, cbl_prep_x_bytes() long, is used then and may be NULL otherwise).
+ *   ys[i][t * ldy + r] = round(row_scale[r] * sum_c W_i[r, c] * x[t * ldx + c]); biases (NULL, or one pointer or NULL per matrix, in y's
+ * type) are added to the rounded product and the sum is rounded again.
+ * cbl_direct_serves: whether it is the faster product for these matrices and token count; `tables`: where table lookups (cbl_gemv_l8) would
+ * serve them otherwise, not codeword gathers (cbl_gemm_b3).
+ * replaces shapequant/kernels/gemv.py:28-64 (_gemv_kernel) for them. */
+int32_t cbl_direct_serves(const cbl_packed* mats, int32_t n, int32_t ntok, int32_t tables);
+int cbl_gemv_direct(const cbl_packed* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
+                    int ydtype, int64_t ldy, const void* const* biases, void* stage, cbl_stream s);
+
 /* Product for EVERY format the file layout can hold (any d <= 16, tags of up to 16 bits, several books per matrix
  * through row_book, one or two summed books, several column orders), the formats outside the benchmark's d = 8 /
  * 12-bit / one-book-per-matrix that the table-lookup and tensor-core kernels execute:

@@ -71,6 +71,9 @@ SIGNATURES = {
     "cbl_last_cuda_error": (c_int, []),
     "cbl_dequant": (c_int, [POINTER(Packed), c_void_p, c_int, c_int64, c_int32, c_int32, c_void_p]),
     "cbl_gemv_generic": (c_int, [POINTER(Packed), c_void_p, c_int, c_int32, c_int64, c_void_p, c_int, c_int64, c_void_p]),
+    "cbl_direct_serves": (c_int32, [POINTER(Packed), c_int32, c_int32, c_int32]),
+    "cbl_gemv_direct": (c_int, [POINTER(Packed), c_int32, c_void_p, c_int, c_int32, c_int64, c_void_p, POINTER(c_void_p), c_int, c_int64,
+                                POINTER(c_void_p), c_void_p, c_void_p]),
     "cbl_unpack_tags": (c_int, [POINTER(Packed), c_int, c_void_p, c_void_p]),
     "cbl_assign_max_codewords": (c_int, []),
     "cbl_assign": (c_int, [c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_int, c_int32, c_void_p, c_void_p, c_void_p]),

@@ -1,0 +1,285 @@
+// Products of 1..4 tokens of small matrices, straight from the file layout (d = 8, 12-bit tags, 4096-entry fp16 books, one or two
+// summed books, any number of column orders): no kernel layout, no book in shared memory, no pieces to add, one launch.
+//
+// A warp takes two rows (four for one token) and every nw-th group of 32 chunks of them, a lane a chunk: the tag, its 16-byte codeword by a
+// global load (the book is 64 KB and stays in L1), the chunk's activations as they come, fp32 FMAs.  The nw warps of a row set
+// add their sums in shared memory in a fixed order.  Tags and codewords are on their way before the kernel waits for its predecessor.
+//
+// What bounds it is latency while a warp has one or two groups - tag, codeword, sum, one after the other: 512 x 3584, one token, 2.3 us
+// where the product that loads the book into shared memory takes 7.9 (staging of x, 2.7 us of book, the pieces' addition) - and beyond that the L1's
+// rate of random 16-byte reads, about one per clock and SM (shared memory gives four to six).  64 registers, so that two blocks share an SM
+// (two tokens of 896 x 4864: 5.2 us, 6.8 with more registers and one block).  cbl_direct_serves() draws the line.
+#include "cbl_common.cuh"
+
+namespace {
+
+constexpr int DR_WARPS = 16, DR_MAX_MATS = 4, DR_MAX_TOKENS = 4;
+
+struct DrMat {
+    const uint32_t* tags;
+    const uint32_t* tags2;
+    const uint4* table;
+    const uint4* table2;
+    const __half* row_scale;
+    const uint8_t* row_mask;
+    const void* bias;
+    void* y;
+    int R, blk0;
+};
+struct DrLaunch {
+    DrMat m[DR_MAX_MATS];
+    int n, W, nch, nw, ntok, ydtype, bpad;
+    int64_t ldx, ldy;                            // in values; staged rows are ldx apart too
+    const void* x;
+    const float* xinv;                           // staged activations: the factors that undo the token scales
+};
+
+enum { DR_F32 = CBL_F32, DR_F16 = CBL_F16, DR_BF16 = CBL_BF16, DR_STAGED };
+
+// Eight values of an activation row at a 16-byte boundary: as they lie (past the L1: the kernel before may still have been writing
+// when this one's blocks arrived), and in fp32.
+template <int XT>
+struct DrX {
+    uint4 u[XT == DR_F32 ? 2 : 1];
+    __device__ __forceinline__ void load(const void* __restrict__ x, int64_t at) {
+        const uint4* p = (const uint4*)((const char*)x + at * (XT == DR_F32 ? 4 : 2));
+        u[0] = __ldcg(p);
+        if (XT == DR_F32) u[XT == DR_F32] = __ldcg(p + 1);
+    }
+    __device__ __forceinline__ void get(float (&v)[8]) const {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t w = k == 0 ? u[0].x : k == 1 ? u[0].y : k == 2 ? u[0].z : u[0].w;
+            if (XT == DR_F32) {
+                const uint4& h = u[XT == DR_F32];
+                v[k] = __uint_as_float(w);
+                v[4 + k] = __uint_as_float(k == 0 ? h.x : k == 1 ? h.y : k == 2 ? h.z : h.w);
+            } else {
+                const float2 f = XT == DR_BF16 ? __bfloat1622float2(*(const __nv_bfloat162*)&w) : __half22float2(*(const __half2*)&w);
+                v[2 * k] = f.x;
+                v[2 * k + 1] = f.y;
+            }
+        }
+    }
+};
+
+template <int XT, int NT>
+__global__ void __launch_bounds__(DR_WARPS * 32, 2)
+k_direct(const __grid_constant__ DrLaunch P) {
+    constexpr int RB = NT >= 2 || XT == DR_STAGED ? 2 : 4, NV = RB * NT;
+    __shared__ float s_sum[DR_WARPS][NV];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int mi = 0;
+    while (mi + 1 < P.n && (int)blockIdx.x >= P.m[mi + 1].blk0) mi++;
+    const DrMat& m = P.m[mi];
+    const int nw = P.nw, sets = DR_WARPS / nw, set = warp / nw, nch = P.nch, W = P.W;
+    const int r0 = (((int)blockIdx.x - m.blk0) * sets + set) * RB;
+    const bool two = m.tags2 != nullptr;
+    // tags (two words that may hold one) and codewords of this lane's chunk of group g
+    auto words = [&](const uint32_t* __restrict__ tags, int r, int c) {
+        const uint32_t* p = tags + (int64_t)r * W;
+        const int b = c * 12, w = b >> 5;
+        return __funnelshift_r(__ldg(p + w), __ldg(p + min(w + 1, W - 1)), b & 31) & 4095u;
+    };
+    uint32_t t1[RB], t2[RB];
+    auto fetch = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < RB; i++) {
+            const int r = min(r0 + i, m.R - 1);
+            t1[i] = words(m.tags, r, c);
+            if (two) t2[i] = words(m.tags2, r, c);
+        }
+    };
+    float acc[RB][NT];
+#pragma unroll
+    for (int i = 0; i < RB; i++)
+#pragma unroll
+        for (int t = 0; t < NT; t++) acc[i][t] = 0.f;
+    int xrow[RB];                                              // staged: the rows' column orders start here
+#pragma unroll
+    for (int i = 0; i < RB; i++) xrow[i] = XT == DR_STAGED && m.row_mask ? (int)__ldg(m.row_mask + min(r0 + i, m.R - 1)) * P.bpad : 0;
+    bool first = true;
+    int c = r0 < m.R ? (warp % nw) * 32 + lane : nch;
+    if (c < nch) fetch(c);
+    while (c < nch) {
+        const int at = c;
+        float w[RB][8];
+#pragma unroll
+        for (int i = 0; i < RB; i++) {
+            const uint4 u = __ldg(m.table + t1[i]);
+            const __half2* h = (const __half2*)&u;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float2 f = __half22float2(h[k]);
+                w[i][2 * k] = f.x;
+                w[i][2 * k + 1] = f.y;
+            }
+        }
+        if (two) {
+#pragma unroll
+            for (int i = 0; i < RB; i++) {
+                const uint4 u = __ldg(m.table2 + t2[i]);
+                const __half2* h = (const __half2*)&u;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const float2 f = __half22float2(h[k]);
+                    w[i][2 * k] += f.x;
+                    w[i][2 * k + 1] += f.y;
+                }
+            }
+        }
+        c += nw * 32;
+        if (c < nch) fetch(c);
+        if (first) {                                           // nothing above depends on the kernel before this one
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            first = false;
+        }
+        // the loads of several tokens before their sums, as many as the registers hold; tokens beyond ntok repeat the first
+        constexpr int TB = NT < 4 || XT == DR_F16 || XT == DR_BF16 ? NT : 2;
+#pragma unroll
+        for (int t0 = 0; t0 < NT; t0 += TB) {
+            DrX<XT> x[XT == DR_STAGED ? RB : 1][TB];
+#pragma unroll
+            for (int i = 0; i < (XT == DR_STAGED ? RB : 1); i++)
+#pragma unroll
+                for (int t = 0; t < TB; t++) x[i][t].load(P.x, (xrow[i] + (t0 + t < P.ntok ? t0 + t : 0)) * P.ldx + 8 * (int64_t)at);
+#pragma unroll
+            for (int t = 0; t < TB; t++) {
+                float xv[8];
+#pragma unroll
+                for (int i = 0; i < RB; i++) {
+                    if (i == 0 || XT == DR_STAGED) x[XT == DR_STAGED ? i : 0][t].get(xv);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) acc[i][t0 + t] = fmaf(w[i][k], xv[k], acc[i][t0 + t]);
+                }
+            }
+        }
+    }
+    if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the lanes' sums of NV values: halves are exchanged, so that a lane adds up one value in the end (NV + 1 shuffles or so, not 5 NV)
+    float v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) v[i] = acc[i / NT][i % NT];
+    int mine = 0, o = 16;
+#pragma unroll
+    for (int half = NV / 2; half > 0; half /= 2, o /= 2) {
+        const bool up = lane & o;
+        mine += up ? half : 0;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const float give = up ? v[i] : v[i + half];
+            v[i] = (up ? v[i + half] : v[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    const int same = 2 * o - 1;                                // lanes that hold the same value
+#pragma unroll
+    for (; o > 0; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    if ((lane & same) == 0) s_sum[warp][mine] = v[0];
+    __syncthreads();
+    if (tid < sets * NV) {
+        const int s = tid / NV, v = tid % NV, t = v % NT, r = (((int)blockIdx.x - m.blk0) * sets + s) * RB + v / NT;
+        if (r < m.R && t < P.ntok) {
+            float sum = 0.f;
+            for (int k = 0; k < nw; k++) sum += s_sum[s * nw + k][v];
+            if (XT == DR_STAGED) sum *= __ldcg(P.xinv + (m.row_mask ? (int)__ldg(m.row_mask + r) * P.bpad : 0) + t);
+            float o = sum * __half2float(__ldg(m.row_scale + r));
+            if (m.bias) {                                      // two roundings, as two operators would give
+                if (P.ydtype == CBL_BF16) o = __bfloat162float(__float2bfloat16_rn(o));
+                else if (P.ydtype == CBL_F16) o = __half2float(__float2half_rn(o));
+                o += cbl_load_in(m.bias, P.ydtype, r);
+            }
+            cbl_store_out(m.y, P.ydtype, t * P.ldy + r, o);
+        }
+    }
+}
+
+}  // namespace
+
+// Chunks of the matrices (of two books: a quarter more) up to which this product is the faster one.  Measured against the codeword gathers
+// with the book in shared memory, us, here / there (rows x columns, GPU time): one token, 1024 x 18944 9.7 / 11.8, 512 x 3584 2.3 / 7.9; two,
+// 1024 x 8192 7.6 / 9.4, 4096 x 4096 12.2 / 9.1; four, 1024 x 3584 5.8 / 8.3, 4864 x 896 7.6 / 7.5.  Against table lookups (one token, 2048 rows and more):
+// 3584 x 896 3.3 / 4.7, 4864 x 896 5.6 / 4.8.  With column orders, staging included: one token, 4 orders, 1024 x 3584 7.8 / 8.6, 4864 x 896
+// 8.1 / 7.6, 16 orders, 1024 x 8192 10.5 / 12.3, 4096 x 4096 14.0 / 13.2; four, 512 x 3584 5.2 / 8.3, 1024 x 3584 9.5 / 9.4.
+// (Eight tokens of the smallest matrices would gain as well, 512 x 3584 3.9 / 8.5: from five on the gathers keep them, whose sums callers compare.)
+extern "C" int32_t cbl_direct_serves(const cbl_packed* mats, int32_t n, int32_t ntok, int32_t tables) {
+    if (!mats || n < 1 || n > DR_MAX_MATS || ntok < 1 || ntok > DR_MAX_TOKENS) return 0;
+    int64_t chunks = 0;
+    for (int i = 0; i < n; i++) {
+        const cbl_packed& m = mats[i];
+        if (m.d != 8 || m.bits != 12 || m.G != 1) return 0;
+        const int64_t c = (int64_t)m.R * (m.C / 8);
+        chunks += m.books == 2 ? c + c / 4 : c;
+    }
+    const int M = mats[0].M;
+    if (M > 1) return !tables && chunks <= (ntok <= 2 ? 400000 + 30000 * (M < 16 ? M : 16) : 360000);
+    if (ntok == 1) return chunks <= (tables ? 450000 : 2500000);
+    return chunks <= (ntok == 2 ? 1200000 : 600000);
+}
+
+extern "C" int cbl_gemv_direct(const cbl_packed* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
+                               int ydtype, int64_t ldy, const void* const* biases, void* stage, cbl_stream s) {
+    if (!mats || !ys || !x || n < 1) return CBL_EINVAL;
+    if (n > DR_MAX_MATS || ntok > DR_MAX_TOKENS) return CBL_EUNSUPPORTED;
+    const int C = mats[0].C, M = mats[0].M;
+    if (ntok < 1 || ldx < C || (M > 1 && !perms)) return CBL_EINVAL;
+    if (xdtype != CBL_F32 && xdtype != CBL_F16 && xdtype != CBL_BF16) return CBL_EINVAL;
+    if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
+    // column orders, or rows that are not on 16-byte boundaries: staged
+    const int esz = xdtype == CBL_F32 ? 4 : 2;
+    const bool staged = M > 1 || (uintptr_t)x % 16 || (ntok > 1 && ldx * esz % 16);
+    if (staged && (!stage || (uintptr_t)stage % 16)) return CBL_EINVAL;
+    const int rb = ntok >= 2 || staged ? 2 : 4;
+    DrLaunch P;
+    P.n = 0;
+    int64_t sets = 0;
+    for (int i = 0; i < n; i++) {
+        const cbl_packed& m = mats[i];
+        if (m.d != 8 || m.bits != 12 || m.G != 1) return CBL_EUNSUPPORTED;
+        if (!m.tags || !m.table || !m.row_scale || !ys[i] || (m.books != 1 && m.books != 2) || (m.books == 2 && (!m.tags2 || !m.table2))) return CBL_EINVAL;
+        if (m.R < 0 || m.C <= 0 || m.C % 8 || (int64_t)m.W * 32 < (int64_t)(m.C / 8) * 12 || (ntok > 1 && ldy < m.R)) return CBL_EINVAL;
+        if (m.C != C || m.M != M || m.W != mats[0].W || (M > 1 && !m.row_mask)) return CBL_EINVAL;
+        if ((uintptr_t)m.table % 16 || (m.books == 2 && (uintptr_t)m.table2 % 16)) return CBL_EINVAL;
+        sets += cbl_ceil_div(m.R, rb);
+    }
+    if (sets == 0) return CBL_OK;
+    P.W = mats[0].W; P.nch = C / 8; P.ntok = ntok; P.ydtype = ydtype; P.ldx = ldx; P.ldy = ldy; P.x = x; P.xinv = nullptr; P.bpad = 0;
+    // warps of a row set: one per group of 32 chunks, fewer where that would be more than 64 warps per SM
+    P.nw = 1;
+    while (P.nw < DR_WARPS && P.nw * 32 < P.nch && sets * P.nw * 2 <= 64 * cbl_sm_count()) P.nw *= 2;
+    const int per = DR_WARPS / P.nw;
+    int64_t blocks = 0;
+    for (int i = 0; i < n; i++) {
+        const cbl_packed& m = mats[i];
+        if (m.R == 0) continue;
+        P.m[P.n++] = {(const uint32_t*)m.tags, m.books == 2 ? (const uint32_t*)m.tags2 : nullptr, (const uint4*)m.table, (const uint4*)m.table2,
+                      (const __half*)m.row_scale, M > 1 ? m.row_mask : nullptr, biases ? biases[i] : nullptr, ys[i], m.R, (int)blocks};
+        blocks += cbl_ceil_div(cbl_ceil_div(m.R, rb), per);
+    }
+    int kind = xdtype;
+    if (staged) {
+        const int rc = cbl_prep_x(x, xdtype, ntok, C, ldx, perms, M, stage, s);
+        if (rc) return rc;
+        kind = DR_STAGED;
+        P.bpad = (ntok + 7) / 8 * 8;
+        P.ldx = (C + 511) / 512 * 512;
+        P.x = stage;
+        P.xinv = (const float*)((const __half*)stage + (int64_t)M * P.bpad * P.ldx);
+    }
+    typedef void (*kernel_fn)(const DrLaunch);
+    static const kernel_fn fns[4][3] = {{k_direct<DR_F32, 1>, k_direct<DR_F32, 2>, k_direct<DR_F32, 4>},
+                                        {k_direct<DR_F16, 1>, k_direct<DR_F16, 2>, k_direct<DR_F16, 4>},
+                                        {k_direct<DR_BF16, 1>, k_direct<DR_BF16, 2>, k_direct<DR_BF16, 4>},
+                                        {k_direct<DR_STAGED, 1>, k_direct<DR_STAGED, 2>, k_direct<DR_STAGED, 4>}};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = (cudaStream_t)s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(DR_WARPS * 32);
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[kind][ntok == 1 ? 0 : ntok == 2 ? 1 : 2], P));
+    return cbl_check_launch();
+}

@@ -50,6 +50,8 @@ struct Plan {
     PyObject* keep = nullptr;                             // the tensors whose addresses the descriptors hold
     size_t ws_bytes[2][129] = {};
     size_t l8_bytes = 0;
+    bool tables = false;                                  // whether one token's product is one of table lookups
+    bool direct[5] = {};                                  // token counts of a single small matrix that run straight from the file layout
     int dense_from = 0;                                   // tokens from which the two-phase product runs
 };
 
@@ -166,12 +168,20 @@ int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* 
     void* ys[MAX_PIECES];
     for (int i = 0; i < p.n; i++) ys[i] = y + p.first[i] * esz;
     const cbl_stream s = (cbl_stream)stream;
-    if (tokens == 1 && p.has_l8) {
+    if (tokens == 1 && p.has_l8 && !p.direct[1]) {
         void* const ws = need(L8, p.l8_bytes, p.device, stream).data_ptr();
         const void* biases[MAX_PIECES] = {};
         if (bias) for (int i = 0; i < p.n; i++) biases[i] = (const char*)bias + p.first[i] * esz;
         *fn = "cbl_gemv_l8_bias";
         return cbl_gemv_l8_bias(p.l8, p.n, x, xdt, ys, ydt, bias ? biases : nullptr, ws, s);
+    }
+    if (tokens <= 4 && p.direct[tokens]) {
+        // staging of activations through several column orders, or from rows that are not on 16-byte boundaries
+        const bool staged = p.orders > 1 || (uintptr_t)x % 16 || (tokens > 1 && ldx * (xdt == CBL_F32 ? 4 : 2) % 16);
+        void* const stage = staged ? need(STAGE, cbl_prep_x_bytes((int32_t)tokens, (int32_t)p.C, p.orders), p.device, stream).data_ptr() : nullptr;
+        const void* biases[1] = {bias};
+        *fn = "cbl_gemv_direct";
+        return cbl_gemv_direct(p.packed, 1, x, xdt, (int32_t)tokens, ldx, p.perms, ys, ydt, ldy, biases, stage, s);
     }
     const int k = tokens <= cbl_gemm_b3_max_tokens(3) ? 1 : 0;
     if (tokens <= cbl_gemm_b3_max_tokens(2)) {
@@ -193,7 +203,7 @@ int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* 
 }
 
 bool layout_for(const Plan& p, int64_t tokens) {
-    if (tokens == 1 && p.has_l8) return true;
+    if ((tokens == 1 && p.has_l8) || (tokens <= 4 && p.direct[tokens])) return true;
     if (tokens <= cbl_gemm_b3_max_tokens(2)) return p.has_b3[tokens <= cbl_gemm_b3_max_tokens(3) ? 1 : 0];
     return p.has_dense && tokens >= p.dense_from;
 }
@@ -266,17 +276,17 @@ void free_plan(PyObject* o) {
     delete p;
 }
 
-// plan(device, in, C, orders, rows: list, perms pointer, dense_from, bias or None, tensors to keep alive) -> capsule
+// plan(device, in, C, orders, rows: list, perms pointer, dense_from, bias or None, tensors to keep alive, tables) -> capsule
 PyObject* py_plan(PyObject*, PyObject* args) {
-    int device, orders, dense_from;
+    int device, orders, dense_from, tables;
     long long in, C;
     unsigned long long perms;
     PyObject *rows, *bias, *keep;
-    if (!PyArg_ParseTuple(args, "iLLiOKiOO", &device, &in, &C, &orders, &rows, &perms, &dense_from, &bias, &keep)) return nullptr;
+    if (!PyArg_ParseTuple(args, "iLLiOKiOOp", &device, &in, &C, &orders, &rows, &perms, &dense_from, &bias, &keep, &tables)) return nullptr;
     const Py_ssize_t n = PyList_Size(rows);
     if (n < 1 || n > MAX_PIECES) { PyErr_SetString(PyExc_ValueError, "a plan holds 1..4 matrices"); return nullptr; }
     Plan* p = new Plan;
-    p->device = device; p->in = in; p->C = C; p->orders = orders; p->n = (int)n; p->perms = (const int32_t*)perms; p->dense_from = dense_from;
+    p->device = device; p->in = in; p->C = C; p->orders = orders; p->n = (int)n; p->perms = (const int32_t*)perms; p->dense_from = dense_from; p->tables = tables;
     for (Py_ssize_t i = 0; i < n; i++) {
         p->first[i] = p->R;
         p->rows[i] = PyLong_AsLongLong(PyList_GetItem(rows, i));
@@ -317,6 +327,7 @@ PyObject* py_set(PyObject*, PyObject* args) {
             if (ok) p->has_b3[copies - 2] = true;
         } else if (k == "dense") {
             ok = p->has_dense = take(p->packed);
+            for (int t = 1; t <= 4; t++) p->direct[t] = ok && p->n == 1 && cbl_direct_serves(p->packed, 1, t, p->tables);
             p->row_scale = (const void*)row_scale;
         } else ok = false;
         if (!ok) PyErr_SetString(PyExc_ValueError, "unknown layout or wrong descriptor size");
@@ -500,7 +511,7 @@ PyObject* py_set_linear(PyObject*, PyObject* fn) {
 
 PyMethodDef methods[] = {
     {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "forward(plan, x) -> y or None"},
-    {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias, keep)"},
+    {"plan", py_plan, METH_VARARGS, "plan(device, in, C, orders, rows, perms, dense_from, bias, keep, tables)"},
     {"set", py_set, METH_VARARGS, "set(plan, kind, descriptors, row_scale=0)"},
     {"stream", py_stream, METH_NOARGS, "stream(): torch's current stream of the current device"},
     {"device", py_device, METH_NOARGS, "device(): the current device"},

@@ -225,6 +225,23 @@ class DeviceMatrix(_Uncopied):
                                                                 Y.data_ptr(), _dt(Y.dtype), Y.stride(0) if T > 1 else self.R, _stream()))
         return Y
 
+    def gemv_direct(self, X: torch.Tensor, Y: torch.Tensor) -> torch.Tensor:
+        """Y [T, R] = X [T, C] . W^T of up to 4 tokens straight from the file layout (small matrices: see cbl_direct_serves)."""
+        T = X.shape[0]
+        if X.dim() != 2 or X.shape[1] != self.C or X.stride(1) != 1 or X.device != self.device:
+            raise ValueError("X must be [T, C] with unit column stride on the matrix's device")
+        if Y.shape != (T, self.R) or Y.stride(1) != 1:
+            raise ValueError("Y must be [T, R] with unit column stride")
+        ldx = X.stride(0) if T > 1 else self.C
+        stage = None
+        if self.M > 1 or X.data_ptr() % 16 or (T > 1 and ldx * X.element_size() % 16):
+            stage = scratch(self.device, STAGE, lib.cbl_prep_x_bytes(T, self.C, self.M))
+        with _on(self.device):
+            _lib.check("cbl_gemv_direct", lib.cbl_gemv_direct(ctypes.byref(self.struct()), 1, X.data_ptr(), _dt(X.dtype), T, ldx, _ptr(self.perms),
+                                                              (ctypes.c_void_p * 1)(Y.data_ptr()), _dt(Y.dtype), Y.stride(0) if T > 1 else self.R, None, _ptr(stage),
+                                                              _stream()))
+        return Y
+
     def unpack(self, plane: int = 0) -> torch.Tensor:
         out = torch.empty(self.R, self.nch, dtype=torch.int32, device=self.device)
         with _on(self.device):

@@ -15,19 +15,21 @@ pass the plain activation vector, not permuted copies.
 
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
 
 from . import _cblhost, _lib
+from ._lib import lib
 from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix, _Uncopied, epoch
 
 # Rows from which one token runs on activation-side tables (L8Matrix) instead of codeword gathers (B3Matrix); of a matrix with
 # several column orders, rows per order: every order needs tables of its own, and a build costs as much as the lookups of some
 # 1300 rows.  The tables hold 16-bit integers (results off by about 1e-4), the gathers sum fp16 products in fp32 (3e-7).  Above the
-# line the tables serve (2048 x 3584: 5.5 us against 9.0 by gathers; 27648 x 5120, two books, 16 orders: 34.1 against 50.8); below
-# it they would be faster as well (512 x 3584: 4.6 against 7.6; 3584 x 3584 in 16 orders: 10.2 against 13.6), but a small
-# matrix gains three to six microseconds at most and keeps its exact sums.
+# line the tables serve (2048 x 3584: 5.5 us against 8.8 by gathers; 27648 x 5120, two books, 16 orders: 34.1 against 50.8); below
+# it they would be faster than gathers as well, but a small matrix keeps its exact sums, and straight from the file layout
+# (PackedLinear.direct) it is about as fast (512 x 3584: 2.3 us, tables 4.7, gathers 7.9; 2047 x 3584: 6.4, 5.6, 8.5).
 L8_MIN_ROWS = 2048
 L8_MIN_ROWS_PER_ORDER = 1536
 # Tokens up to which the book lies three times in shared memory (the activations of more tokens need the room: two copies).
@@ -42,8 +44,8 @@ def _tensors(objs) -> tuple:
 
 
 class PackedLinear(_Uncopied, torch.nn.Module):
-    """A block linear run from packed tensors: one token -> batch-1 kernel, up to 128 tokens -> the
-    codeword-gather tensor-core kernel, more -> decode once + tcgen05 GEMM. Constructor arguments follow the
+    """A block linear run from packed tensors: up to 4 tokens of a small matrix -> straight from the file layout, one token ->
+    batch-1 kernel, up to 128 tokens -> the codeword-gather tensor-core kernel, more -> decode once + tcgen05 GEMM. Constructor arguments follow the
     reference (words, table, row_scale, row_book, row_mask, perms, K, d, bias)."""
 
     _uncopied = ("_host", "_host_bias")
@@ -119,7 +121,7 @@ class PackedLinear(_Uncopied, torch.nn.Module):
             return
         self._host_bias, self._host_epoch = b, epoch[0]
         self._host = _cblhost.plan(dm.device.index, self.in_features, self.C, dm.M, [self.R], 0 if dm.perms is None else dm.perms.data_ptr(),
-                                   DENSE_MIN_TOKENS, b, _tensors([dm, *([] if self._l8 is None else [self._l8]), *(g.mats[0] for g in self._b3.values())]))
+                                   DENSE_MIN_TOKENS, b, _tensors([dm, *([] if self._l8 is None else [self._l8]), *(g.mats[0] for g in self._b3.values())]), self.use_l8())
         if self._l8 is not None and self.use_l8():
             _cblhost.set(self._host, "l8", bytes(self._l8.struct()))
         for g in self._b3.values():
@@ -128,9 +130,13 @@ class PackedLinear(_Uncopied, torch.nn.Module):
             _cblhost.set(self._host, "dense", bytes(dm.struct()), dm.row_scale.data_ptr())
 
     def use_l8(self) -> bool:
-        """One token runs on the table-lookup kernel (any number of column orders up to its limit)."""
+        """One token runs on the table-lookup kernel (any number of column orders up to its limit), unless direct() says otherwise."""
         least = L8_MIN_ROWS if self.dm.M == 1 else L8_MIN_ROWS_PER_ORDER * self.dm.M
         return self.dm.fast and not self.wide and self.dm.M <= L8Matrix.MAX_ORDERS and self.R >= least
+
+    def direct(self, n: int) -> bool:
+        """n tokens run straight from the file layout, without a kernel layout: few tokens of a small matrix."""
+        return n <= 4 and self.dm.fast and not self.wide and bool(lib.cbl_direct_serves(ctypes.byref(self.dm.struct()), 1, n, self.use_l8()))
 
     def gemv(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x [C] (fp16 / bf16 / fp32, contiguous) -> y [R] in x's dtype (or `out`'s)."""
@@ -138,10 +144,13 @@ class PackedLinear(_Uncopied, torch.nn.Module):
             y = out if out is not None else torch.empty(self.R, dtype=x.dtype, device=x.device)
             self.dm.gemv_generic(x.reshape(1, -1), y.reshape(1, -1))
             return y
-        if self.use_l8():
+        if self.use_l8() and not self.direct(1):
             return self.l8.run(x, out)
         y = out if out is not None else torch.empty(self.R, dtype=x.dtype, device=x.device)
-        self.group(1).run(x.reshape(1, -1), [y.reshape(1, -1)])
+        if self.direct(1):
+            self.dm.gemv_direct(x.reshape(1, -1), y.reshape(1, -1))
+        else:
+            self.group(1).run(x.reshape(1, -1), [y.reshape(1, -1)])
         return y
 
     def dense(self) -> torch.Tensor:
@@ -159,7 +168,9 @@ class PackedLinear(_Uncopied, torch.nn.Module):
             self.dm.gemv_generic(x2 if x2.stride(1) == 1 else x2.contiguous(), y)
             return y
         x2 = x2 if x2.stride(1) == 1 else x2.contiguous()
-        if n == 1 and self.use_l8() and y.is_contiguous():
+        if self.direct(n):
+            self.dm.gemv_direct(x2, y)
+        elif n == 1 and self.use_l8() and y.is_contiguous():
             self.l8.run(x2[0], y[0])
         elif n < DENSE_MIN_TOKENS:
             self.group(n).run(x2, [y])
@@ -195,7 +206,7 @@ class Stack:
 
     def __init__(self, lins: list, step: bool = False):
         from .kernels import DenseStack, L8Group
-        self.lins, self.C, self.device = lins, lins[0].C, lins[0].dm.device
+        self.lins, self.C, self.device, self.step = lins, lins[0].C, lins[0].dm.device, step
         self.Rs = [l.R for l in lins]
         self.R = sum(self.Rs)
         p0 = lins[0].dm.perms
@@ -229,13 +240,15 @@ class Stack:
         """Whether run() on n tokens builds no layout."""
         if not self.fast or n >= DENSE_MIN_TOKENS:
             return True
+        if self._direct(n):
+            return True
         if n == 1 and self.tables:
             return self._l8 is not None
         copies = 3 if n <= B3_MAX_3COPIES else 2
         return copies in self._b3 if self.shared else all(copies in l._b3 for l in self.lins)
 
     def prepare(self, n: int) -> None:
-        if not self.fast or n >= DENSE_MIN_TOKENS:
+        if not self.fast or n >= DENSE_MIN_TOKENS or self._direct(n):
             return
         if n == 1 and self.tables:
             self.l8._structs
@@ -244,6 +257,9 @@ class Stack:
         else:
             for l in self.lins:
                 l.group(n)
+
+    def _direct(self, n: int) -> bool:
+        return not self.step and len(self.lins) == 1 and self.lins[0].direct(n)
 
     def takes_staged(self, n: int) -> bool:
         """Whether run() accepts the n tokens' activations staged by the operator before (cbl_prep_x's layout)."""
@@ -257,6 +273,8 @@ class Stack:
         ys = list(y.split(self.Rs, 1))
         if x is None:
             self.b3(n).run(None, ys, staged)
+        elif self._direct(n):
+            self.lins[0].forward_into(x, y)
         elif n == 1 and (self.tables if tables is None else tables):
             self.l8.run(x[0], [t[0] for t in ys])
         elif self.shared and n < DENSE_MIN_TOKENS:
@@ -276,7 +294,8 @@ class Stack:
         dm = self.lins[0].dm
         held = [l.dm for l in self.lins] + ([] if self._l8 is None else self._l8.mats)
         keep = _tensors(held + [m for g in self._b3.values() for m in g.mats]) + (() if self.dense is None else (self.dense.row_scale,))
-        h = _cblhost.plan(dm.device.index, self.C, self.C, dm.M, self.Rs, 0 if dm.perms is None else dm.perms.data_ptr(), DENSE_MIN_TOKENS, None, keep)
+        h = _cblhost.plan(dm.device.index, self.C, self.C, dm.M, self.Rs, 0 if dm.perms is None else dm.perms.data_ptr(), DENSE_MIN_TOKENS, None, keep,
+                         all(l.use_l8() for l in self.lins))
         if self._l8 is not None:
             _cblhost.set(h, "l8", bytes(self._l8._structs))
         for g in self._b3.values():
@@ -300,7 +319,7 @@ class RunsLin:
         # build the layouts now, not inside a captured region (fused epilogues take the tables whatever the rows)
         if lin.use_l8() or self._epilogues():
             lin.l8
-        if not lin.use_l8():
+        if not lin.use_l8() and not lin.direct(1):
             lin.group(1)
 
     def _epilogues(self) -> bool:
@@ -321,7 +340,6 @@ class RunsLin:
             else:
                 self.lin.forward_into(x, y)
             return y
-        import ctypes
         from .kernels import L8Group, _dt, _stream, l8_workspace
         if epi.get("perms") is not None:
             raise ValueError("epi['perms']: permuted copies of the output are not produced here (the next product applies its column orders itself)")

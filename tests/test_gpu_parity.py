@@ -292,6 +292,45 @@ def test_one_token_of_few_rows_is_summed_in_fp32(R, C, books, M):
         assert (got.double() - ref).norm() <= books * (C / 16) * 2.0 ** -23 * ref.norm()
 
 
+@pytest.mark.parametrize("R,C,books,M", [(1, 8, 1, 1), (63, 264, 1, 1), (64, 256, 2, 1), (515, 3592, 1, 1), (1000, 8184, 2, 1), (3584, 896, 1, 1), (66, 776, 1, 4),
+                                         (515, 2048, 2, 16), (5, 18944, 1, 3)])
+def test_small_products_straight_from_the_file_layout(R, C, books, M):
+    """1..4 tokens of small matrices: fp32 sums of exact products (a lane's C / 256 chunks, a tree over lanes and warps: less than C / 16 roundings at
+    2^-23 in a row), no further from float64 than the codeword gathers; every activation type, rows off the 16-byte boundaries (staged in fp16),
+    rows apart, outputs apart, a bias."""
+    m = orc.synth_matrix(R, C, seed=R + C + M, books=books, M=M)
+    lin = _linear(m)
+    W = torch.from_numpy(orc.synth_decode(m)).double().cuda()
+    g = torch.Generator().manual_seed(R + C)
+    for n in range(1, 5):
+        if not lin.direct(n):
+            assert n > 1 and R * C > 2800000
+            continue
+        for dt in (torch.bfloat16, torch.float16, torch.float32):
+            buf = torch.randn(n * C + 1, generator=g).to(dt).cuda()
+            for x in (buf[:n * C].view(n, C), buf[1:].view(n, C)):
+                ref = x.double() @ W.T
+                y = torch.full((n, R + 3), float("nan"), device="cuda")
+                lin.forward_into(x, y[:, :R])
+                exact = dt == torch.bfloat16 or dt == torch.float16 or (M == 1 and x.data_ptr() % 16 == 0 and C % 4 == 0)
+                # staged fp32: independent errors of at most 2^-11 of each value, so 2^-11 sqrt(sum w^2 x^2) at most in the root mean square of an
+                # output; twice that for the few outputs of a small case
+                bound = books * max(C / 16, 8) * 2.0 ** -23 * ref.norm() if exact else 2.0 ** -10 * (W.square() @ x.double().square().T).sum().sqrt()
+                off = (y[:, :R].double() - ref).norm()
+                assert off <= bound and y[:, R:].isnan().all()
+                z = torch.empty(n, R, device="cuda")
+                lin.group(n).run(x, [z])
+                assert off <= 1.1 * (z.double() - ref).norm() + 2.0 ** -22 * ref.norm()
+                for _ in range(2):                           # Python path, native path
+                    assert torch.equal(lin(x), y[:, :R].to(dt))
+        wide = torch.randn(n, C + 24, generator=g).bfloat16().cuda()
+        assert torch.equal(lin.forward_into(wide[:, 8:C + 8], torch.empty(n, R, device="cuda")), lin.forward_into(wide[:, 8:C + 8].contiguous(), torch.empty(n, R, device="cuda")))
+        biased = _linear(m, bias=torch.randn(R, generator=g).bfloat16().cuda())
+        xb = wide[:, :C].contiguous()
+        for _ in range(2):
+            assert torch.equal(biased(xb), lin(xb) + biased.bias)
+
+
 @pytest.mark.parametrize("n,C,M", [(1, 8, 2), (1, 18944, 16), (3, 2056, 4), (9, 3584, 16), (128, 1032, 3)])
 def test_activations_staged_through_column_orders(n, C, M):
     """Rows as long as the orders are picked from shared memory, rows further apart from memory: the same buffer, bit for bit."""
