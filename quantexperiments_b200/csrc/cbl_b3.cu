@@ -198,7 +198,7 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     // The stages of the ring that are free, seen from its next one on: every lane tests one barrier, how many in a row
     // have completed their phase (at least one, also when the wait has expired).  A test queues behind the gathers, some
     // hundred clocks, so it is made for all stages at once.
@@ -250,13 +250,15 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         int mine = 0;                                          // units this warpgroup has decoded
         for (int u = u0; u < u1;) {
             if (rj < rn) gather(q0.x, q0.y, ca);
-            for (int j = rj; j < rn; j += 16) {                // (beyond the run the tags are zero: slot 0)
-                uint4 c = q0;
-                q0 = tags(j + 16);
-                unit(c, q1);
-                if (j + 4 < rn) { c = q1; q1 = tags(j + 20); unit(c, q2); }
-                if (j + 8 < rn) { c = q2; q2 = tags(j + 24); unit(c, q3); }
-                if (j + 12 < rn) { c = q3; q3 = tags(j + 28); unit(c, q0); }
+            const uint4* tq = tp + (int64_t)(rj + 16) * B3_ROWS;
+#pragma unroll 1
+            for (int j = rj; j < rn; j += 4) {                 // (beyond the run the tags are zero: slot 0; one copy of the code, which stays in the
+                                                               // instruction cache: gate|up of 12 tokens 21.0 us unrolled by four, 20.3 so)
+                const uint4 c = q0;
+                q0 = q1; q1 = q2; q2 = q3;
+                q3 = j + 16 < rn ? cbl_ldg_stream(tq) : make_uint4(0, 0, 0, 0);
+                tq += 4 * B3_ROWS;
+                unit(c, q0);
             }
             if (rj < rn) mine += (rn - rj + 3) / 4;
             u += rn;
@@ -270,67 +272,79 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
         }
         if (mine < nq) { room(); done(); }                     // no unit of the last stage: arrive all the same
     } else if (warp == B3_MMA_WARP) {
-        // ---------------- MMA issue, four units at a time.  A stage is announced through a named barrier, which does not
-        // queue with the gathers; counters depend on nothing but the block's range, so that they stay in uniform registers.
+        // ---------------- MMA issue, a piece at a time, in stages of four units.  A stage is announced through a named barrier, which does not
+        // queue with the gathers.  This warp sets the pace: its instructions come from far away (the decode warps' fill the caches) and
+        // a stage's 16 MMAs take 280 of the clocks, so everything else is kept short; counters depend on nothing but the block's
+        // range, so that they stay in uniform registers.
         const uint32_t idesc = (1u << 4) | ((uint32_t)(P.npad >> 3) << 17) | ((uint32_t)(B3_ROWS >> 4) << 24);
-        int st = 0, xs = 0, xk = 0, pc = 0, kb = u0 % nkb;
-        for (int i = 0; i < nu; i += 4) {
-            asm volatile("bar.sync %0, %1;" ::"r"(B3_BAR_STAGE + st), "n"(B3_DEC + 64) : "memory");
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int n = min(4, nu - i);
-            for (int k = 0; k < n;) {                          // the units of one piece at a time
-                const int m = min(n - k, nkb - kb), b = pc & 1;
-                const bool first = kb == 0 || (i == 0 && k == 0), end = i + k + m == nu, last = kb + m == nkb || end;
-                if (first && pc > 1) {
-                    wait(acc_empty(b), ((pc >> 1) & 1) ^ 1);
-                    __syncwarp();
+        const uint64_t x_desc = umma_desc_sw128(x_base);       // a descriptor's low word holds the address / 16
+        const uint32_t xlo = (uint32_t)x_desc, xhi = (uint32_t)(x_desc >> 32), xw = xbytes >> 4, xst = xstage >> 4;
+        auto desc = [&](uint32_t lo) { return (uint64_t)xhi << 32 | lo; };
+        int st = 0, xs = 0, so = 0, pc = 0, kb = u0 % nkb;     // stage, place of its activations, units of it that are done
+        for (int i = 0; i < nu; pc++) {
+            int left = min(nkb - kb, nu - i);                  // units of the piece
+            kb = 0;
+            if (pc > 1) {
+                wait(acc_empty(pc & 1), ((pc >> 1) & 1) ^ 1);
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            const uint32_t d = tmem + (uint32_t)((pc & 1) * P.npad);
+            uint32_t acc = 0;
+            while (left > 0) {
+                if (so == 0) {
+                    asm volatile("bar.sync %0, %1;" ::"r"(B3_BAR_STAGE + st), "n"(B3_DEC + 64) : "memory");
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-                // nothing but straight code in here: with a wait inside, the compiler no longer sees a single thread and issues an
-                // MMA every 130 clocks (measured) instead of every 20
-                const uint32_t d = tmem + (uint32_t)(b * P.npad);
-                if (m == 4) {                                  // all of a stage: no loop either
-                    const int xs1 = XU == 4 ? xs : (xs + 1 == RX ? 0 : xs + 1);
-                    const uint64_t x0 = umma_desc_sw128(x_base + (uint32_t)xs * xstage), x1 = umma_desc_sw128(x_base + (uint32_t)xs1 * xstage + (XU == 4 ? 2 * xbytes : 0u));
-                    const uint32_t a = tmem + a_col0 + (uint32_t)(st * 128), xw = xbytes >> 4;
-                    const uint32_t acc0 = first ? 0u : 1u;
+                const int xs1 = XU == 4 ? xs : (xs + 1 == RX ? 0 : xs + 1);          // where units 2 and 3 are
+                const uint32_t a = tmem + a_col0 + (uint32_t)(st * 128), x0 = xlo + (uint32_t)xs * xst, x1 = XU == 4 ? x0 + 2 * xw : xlo + (uint32_t)xs1 * xst;
+                bool done = true;
+                // nothing but straight code behind the election: with a wait in there, the compiler no longer sees a single thread and
+                // issues an MMA every 130 clocks (measured) instead of every 17
+                if (so == 0 && left >= 4) {
                     if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + kk * 8, x0 + kk * 2, idesc, kk == 0 ? acc0 : 1u);
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + kk * 8, desc(x0 + kk * 2), idesc, kk == 0 ? acc : 1u);
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 32 + kk * 8, x0 + xw + kk * 2, idesc, 1u);
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 32 + kk * 8, desc(x0 + xw + kk * 2), idesc, 1u);
                         if (XU == 2) umma_commit(empty_x(xs));
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 64 + kk * 8, x1 + kk * 2, idesc, 1u);
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 64 + kk * 8, desc(x1 + kk * 2), idesc, 1u);
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 96 + kk * 8, x1 + xw + kk * 2, idesc, 1u);
+                        for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + 96 + kk * 8, desc(x1 + xw + kk * 2), idesc, 1u);
                         umma_commit(empty_x(xs1));
                         umma_commit(empty_a(st));
-                        if (last) umma_commit(acc_full(b));
                     }
-                } else if (elect_one()) {
-                    int x = xs, xi = xk;
-                    for (int t = 0; t < m; t++) {
-                        const uint64_t xd = umma_desc_sw128(x_base + (uint32_t)x * xstage + (uint32_t)xi * xbytes);
-                        const uint32_t a = tmem + a_col0 + (uint32_t)(st * 128 + (k + t) * 32);
+                    left -= 4;
+                    i += 4;
+                } else {
+                    const int m = min(4 - so, left), to = so + m;
+                    done = to == 4 || i + m == nu;
+                    if (elect_one()) {
+                        for (int t = so; t < to; t++) {
+                            const uint32_t x = t < 2 ? x0 + t * xw : x1 + (t - 2) * xw;
 #pragma unroll
-                        for (int kk = 0; kk < B3_KB / 16; kk++) umma_f16_ta(d, a + kk * 8, xd + kk * 2, idesc, (first && t == 0 && kk == 0) ? 0u : 1u);
-                        if (++xi == XU || (end && t == m - 1)) {
-                            umma_commit(empty_x(x));
-                            xi = 0;
-                            if (++x == RX) x = 0;
+                            for (int kk = 0; kk < 4; kk++) umma_f16_ta(d, a + t * 32 + kk * 8, desc(x + kk * 2), idesc, kk == 0 && t == so ? acc : 1u);
+                            if (XU == 2 && t == 1) umma_commit(empty_x(xs));
+                        }
+                        if (done) {
+                            if (XU == 4 || to != 2) umma_commit(empty_x(to > 2 ? xs1 : xs));
+                            umma_commit(empty_a(st));
                         }
                     }
-                    if (last) umma_commit(acc_full(b));
-                    if (k + m == n) umma_commit(empty_a(st));
+                    left -= m;
+                    i += m;
+                    so = done ? 0 : to;
                 }
                 __syncwarp();
-                kb += m;
-                if (last) { kb = 0; pc++; }
-                for (xk += m; xk >= XU; xk -= XU) xs = xs + 1 == RX ? 0 : xs + 1;
-                k += m;
+                acc = 1;
+                if (done) {
+                    if (++st == NST) st = 0;
+                    xs = xs1 + 1 == RX ? 0 : xs1 + 1;
+                }
             }
-            if (++st == NST) st = 0;
+            if (elect_one()) umma_commit(acc_full(pc & 1));
+            __syncwarp();
         }
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next kernel's blocks may take the SMs as they empty
     } else if (warp == B3_X_WARP) {
