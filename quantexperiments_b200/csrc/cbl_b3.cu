@@ -455,11 +455,20 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
 #pragma unroll
                     for (int j = 0; j < 16; j++)
                         if (j < nn) __stcg(o + j * B3_ROWS, __uint_as_float(v[j]));
-                } else if (put) {
+                } else {
+                    // all values, then all stores: a branch between two of them costs a hundred clocks a token
                     T* o = yr + n0 * ldy;
+                    T t[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) t[j] = cbl_cvt_out<T>(__uint_as_float(v[j]) * rs);
+                    if (bias) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) t[j] = cbl_cvt_out<T>((float)t[j] + brow);
+                    }
+                    const int left = put ? nn : 0;
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
-                        if (j < nn) *o = b3_round<T>(__uint_as_float(v[j]) * rs, bias, brow);
+                        if (j < left) *o = t[j];
                         o += ldy;
                     }
                 }
