@@ -381,6 +381,12 @@ int cbl_repack_b3(const cbl_packed* m, const int32_t* tile_rows, int32_t ntile, 
 size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int32_t ntok);
 int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
                 int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s);
+/* The same product for 129 tokens and more of matrices with one column order and two copies of the book (pairs of SMs, 256 tokens at a time):
+ * x NULL: `stage` holds the activations as cbl_prep_x lays them out; `workspace`: the status word of cbl_gemm_b3_status.
+ * cbl_gemm_b3_wide_serves: whether it is faster than cbl_decode_raw + cbl_gemm_dense for matrices of R[0 .. n-1] rows. */
+int32_t cbl_gemm_b3_wide_serves(const int32_t* R, int32_t n, int32_t C, int32_t books, int32_t ntok);
+int cbl_gemm_b3_wide(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, void* const* ys, int ydtype, int64_t ldy,
+                     void* stage, void* workspace, cbl_stream s);
 int cbl_gemm_b3_status(void* workspace, cbl_stream s);
 
 /* Orders a stream for kernels that start early (programmatic dependent launch): the products read tags, books and layouts, and

@@ -95,6 +95,8 @@ SIGNATURES = {
     "cbl_gemm_b3_workspace_bytes": (c_size_t, [POINTER(B3), c_int32, c_int32]),
     "cbl_gemm_b3": (c_int, [POINTER(B3), c_int32, c_void_p, c_int, c_int32, c_int64, c_void_p, POINTER(c_void_p), c_int, c_int64, c_void_p,
                             c_void_p, c_void_p]),
+    "cbl_gemm_b3_wide_serves": (c_int32, [POINTER(c_int32), c_int32, c_int32, c_int32, c_int32]),
+    "cbl_gemm_b3_wide": (c_int, [POINTER(B3), c_int32, c_void_p, c_int, c_int32, c_int64, POINTER(c_void_p), c_int, c_int64, c_void_p, c_void_p, c_void_p]),
     "cbl_gemm_b3_status": (c_int, [c_void_p, c_void_p]),
     "cbl_l8_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "cbl_repack_l8": (c_int, [POINTER(Packed), c_void_p, c_void_p]),

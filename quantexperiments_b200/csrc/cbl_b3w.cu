@@ -1,0 +1,452 @@
+// Products of 129 tokens and more straight from the packed tags (the layout of cbl_gemm_b3 with two copies of the book; one or two summed
+// books, one column order): no decoded copy of the weights in memory.
+//
+// A pair of thread blocks (tcgen05.mma.cta_group::2) computes 256 weight rows x up to 256 tokens.  Each block's decode warps gather the codewords of
+// its 128 rows from shared memory into its tensor memory (operand A), each block brings half of the tokens' activations in by TMA
+// (operand B, read by both), and the accumulators, 128 rows x 256 tokens, lie beside a ring of eight decoded k-blocks of 64 columns.
+//
+// What bounds it: a k-block's MMAs take 2 clocks per token, 512 at 256 tokens.  Shared memory carries a block's gathers (256 clocks with two copies of
+// the book), its half of the activations in and out (256 clocks): the halving is why it runs on pairs.  Decoding again for every 256 tokens costs
+// less than writing the decoded weights to memory and reading them back up to some 900 tokens (cbl_gemm_b3_wide_serves).  Measured with all
+// SMs at work: 0.5 us per k-block and 256 tokens, 0.36 with a fifth of them.
+#include "cbl_tc.cuh"
+
+namespace {
+
+constexpr int BW_ROWS = 128, BW_KB = 64, BW_TOK = 256;
+constexpr int BW_DEC_WARPS = 16, BW_DEC = BW_DEC_WARPS * 32;
+constexpr int BW_X_WARP = 20, BW_MMA_WARP = 21, BW_THREADS = 22 * 32;
+constexpr int BW_SLOTS = 8, BW_STAGES = 6;       // decoded k-blocks in tensor memory, k-blocks of activations in shared memory
+constexpr int BW_STAGE = BW_TOK / 2 * 128;       // bytes of a full stage
+constexpr int BW_SMEM = 131072 + BW_STAGES * BW_STAGE;
+constexpr int BW_MAX_MATS = 4;
+constexpr uint32_t BW_WAIT_LIMIT = 1u << 20;
+
+struct BwMat {
+    const uint4* words;                          // [book][tile][k-block][row]
+    const uint4* table;
+    const uint4* table2;
+    const __half* row_scale;
+    const void* bias;
+    void* y;
+    int R, ntile, item0;                         // item0: number of its first item
+};
+struct BwLaunch {
+    BwMat m[BW_MAX_MATS];
+    int n, books, nkb, ntok, npad, ntb, items;   // ntb blocks of npad tokens; an item: two tiles of rows x a block of tokens
+    int64_t ldy;
+    const float* xinv;
+    unsigned int* status;
+};
+
+__device__ __forceinline__ uint32_t bw_rot1(uint32_t group) { return 1u + group % 7u; }          // cbl_gemm_b3's second copy
+
+__device__ __forceinline__ uint32_t bw_mapa(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void bw_arrive(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void bw_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void bw_tma(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar_cluster) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+                 "l"(map), "r"(c0), "r"(c1), "r"(bar_cluster)
+                 : "memory");
+}
+__device__ __forceinline__ void bw_umma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+__device__ __forceinline__ void bw_commit(uint32_t bar) {                    // arrives at both blocks' barriers
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+                 : "memory");
+}
+__device__ __forceinline__ void bw_st16(uint32_t taddr, const uint4 (&c)[4]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(c[0].x), "r"(c[0].y), "r"(c[0].z), "r"(c[0].w), "r"(c[1].x), "r"(c[1].y), "r"(c[1].z), "r"(c[1].w), "r"(c[2].x), "r"(c[2].y),
+        "r"(c[2].z), "r"(c[2].w), "r"(c[3].x), "r"(c[3].y), "r"(c[3].z), "r"(c[3].w)
+        : "memory");
+}
+__device__ __forceinline__ void bw_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ bool bw_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Bounded wait; one that expires marks the block aborted, after which waits end at once and the roles run out in step.
+__device__ __forceinline__ void bw_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+    for (uint32_t i = 1; i <= BW_WAIT_LIMIT; i++) {
+        if (bw_test(bar, parity) || ((i & 127u) == 0 && *abort)) return;
+    }
+    *abort = 1;
+}
+// The barriers of a ring that have completed their phase, counted from place `at` on (at least one, also when the wait has expired): a lane
+// tests one.  A test queues behind the gathers, some hundred clocks, so it is made for the whole ring.
+__device__ __forceinline__ int bw_run(uint32_t bars, int at, uint32_t parity, int len, volatile int* abort) {
+    const int lane = threadIdx.x & 31, p = at + lane;
+    const bool over = p >= len;
+    const uint32_t bar = bars + 8u * (uint32_t)(over ? p - len : p), ph = parity ^ (uint32_t)over;
+    for (uint32_t i = 1; i <= BW_WAIT_LIMIT; i++) {
+        const uint32_t m = __ballot_sync(0xffffffffu, lane < len && bw_test(bar, ph));
+        if (m & 1u) return __ffs(~m) - 1;
+        if ((i & 127u) == 0 && *abort) return 1;
+    }
+    *abort = 1;
+    return 1;
+}
+template <typename T>
+__global__ void __launch_bounds__(BW_THREADS, 1)
+k_gemm_b3_wide(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ BwLaunch P) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long s_bar[2 * BW_SLOTS + 2 * BW_STAGES + 2];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort;
+    const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int pair = (int)blockIdx.x >> 1, npairs = (int)gridDim.x >> 1;
+    const int i0 = (int)((int64_t)P.items * pair / npairs), i1 = (int)((int64_t)P.items * (pair + 1) / npairs);
+    const int nkb = P.nkb, nu = nkb * P.books;                 // units of an item
+    const uint32_t sbase = cbl_smem_u32(smem), bar0 = cbl_smem_u32(s_bar), x_base = sbase + 131072u;
+    auto full_a = [&](int s) { return bar0 + 8u * s; };                                          // leader's: decode warps of both blocks
+    auto empty_a = [&](int s) { return bar0 + 8u * (BW_SLOTS + s); };                            // each block's
+    auto full_x = [&](int s) { return bar0 + 8u * (2 * BW_SLOTS + s); };                         // leader's
+    auto empty_x = [&](int s) { return bar0 + 8u * (2 * BW_SLOTS + BW_STAGES + s); };            // each block's
+    const uint32_t acc_full = bar0 + 8u * (2 * BW_SLOTS + 2 * BW_STAGES), acc_empty = acc_full + 8u;      // each block's; leader's
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        bw_wait(bar, parity, &s_abort);
+        __syncwarp();
+    };
+    auto mat_of = [&](int item) { int k = 0; while (k + 1 < P.n && item >= P.m[k + 1].item0) k++; return k; };
+    if (tid == 0) {
+        s_abort = 0;
+        for (int s = 0; s < BW_SLOTS; s++) { mbar_init(full_a(s), 8); mbar_init(empty_a(s), 1); }
+        for (int s = 0; s < BW_STAGES; s++) { mbar_init(full_x(s), 1); mbar_init(empty_x(s), 1); }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == BW_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cbl_smem_u32(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    auto load_book = [&](const uint4* __restrict__ tb) {
+        uint4 v[4096 / BW_DEC];
+#pragma unroll
+        for (int k = 0; k < 4096 / BW_DEC; k++) v[k] = __ldg(tb + k * BW_DEC + tid);
+#pragma unroll
+        for (int k = 0; k < 4096 / BW_DEC; k++) {
+            const uint32_t e = (uint32_t)(k * BW_DEC + tid);
+            *(uint4*)(smem + e * 16u) = v[k];
+            *(uint4*)(smem + 65536u + ((e & ~7u) | ((e + bw_rot1(e >> 3)) & 7u)) * 16u) = v[k];
+        }
+    };
+    const uint4* book = nullptr;
+    if (warp < BW_DEC_WARPS && i0 < i1) load_book(book = P.m[mat_of(i0)].table);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    bw_sync();                                                 // both blocks' barriers and tensor memory exist
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0), a_col0 = tmem + BW_TOK;
+
+    if (warp < BW_DEC_WARPS) {
+        // ---------------- decode: a thread a row of this block's tile, a warpgroup every fourth unit
+        const int wg = warp >> 2;
+        const uint32_t lane_addr = a_col0 + ((uint32_t)((warp & 3) * 32) << 16);
+        auto gather = [&](uint32_t w0, uint32_t w1, uint4 (&cw)[4]) {
+            cw[0] = cbl_lds128(sbase + (w0 & 0x1FFF0u));
+            cw[1] = cbl_lds128(sbase + ((w0 >> 14) & 0x1FFF0u));
+            cw[2] = cbl_lds128(sbase + (w1 & 0x1FFF0u));
+            cw[3] = cbl_lds128(sbase + ((w1 >> 14) & 0x1FFF0u));
+        };
+        uint32_t g0 = 0;                                       // number of the run's first unit, over all items
+        for (int it = i0; it < i1; it++) {
+            const BwMat& m = P.m[mat_of(it)];
+            const int tile = (it - m.item0) / P.ntb * 2 + (int)rank;
+            for (int b = 0; b < P.books; b++, g0 += nkb) {
+                const uint4* const tb = b ? m.table2 : m.table;
+                if (tb != book) {                              // everybody is done with the one before
+                    asm volatile("bar.sync 1, %0;" ::"n"(BW_DEC) : "memory");
+                    load_book(book = tb);
+                    asm volatile("bar.sync 1, %0;" ::"n"(BW_DEC) : "memory");
+                }
+                const bool live = tile < m.ntile;              // the second tile of a matrix's last pair may be missing
+                const int first = (wg - (int)(g0 & 3u)) & 3;
+                const uint4* tq = m.words + (((int64_t)b * m.ntile + tile) * nkb + first) * BW_ROWS + (tid & (BW_ROWS - 1));
+                int left = live ? nkb - first : 0;             // units from the next tags on
+                auto tags = [&]() {
+                    const uint4 v = left > 0 ? cbl_ldg_stream(tq) : make_uint4(0, 0, 0, 0);      // slot 0 beyond the end
+                    tq += 4 * BW_ROWS;
+                    left -= 4;
+                    return v;
+                };
+                uint4 q0 = tags(), q1 = tags(), q2 = tags(), q3 = tags();
+                uint4 ca[4], cb[4];
+                if (first < nkb) gather(q0.x, q0.y, ca);
+#pragma unroll 1
+                for (int j = first; j < nkb; j += 4) {
+                    const uint32_t g = g0 + (uint32_t)j;
+                    const int s = (int)(g & (BW_SLOTS - 1));
+                    gather(q0.z, q0.w, cb);
+                    q0 = q1; q1 = q2; q2 = q3; q3 = tags();
+                    wait(empty_a(s), ((g >> 3) & 1u) ^ 1u);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    bw_st16(lane_addr + (uint32_t)s * 32u, ca);
+                    gather(q0.x, q0.y, ca);
+                    bw_st16(lane_addr + (uint32_t)s * 32u + 16u, cb);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bw_arrive(bw_mapa(full_a(s), 0));
+                }
+            }
+        }
+    } else if (warp == BW_X_WARP) {
+        // ---------------- activations: this block's half of the tokens; completion is counted at the leader
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const uint32_t bytes = (uint32_t)P.npad * 64u;         // of a block's half
+        int s = 0, room = 0;
+        uint32_t par = 1;
+        for (int it = i0; it < i1; it++) {
+            const int tok0 = (it - P.m[mat_of(it)].item0) % P.ntb * P.npad + (int)rank * (P.npad >> 1);
+            for (int u = 0; u < nu; u++) {
+                if (room == 0) {
+                    room = bw_run(empty_x(0), s, par, BW_STAGES, &s_abort);
+                    __syncwarp();
+                    if (*(volatile int*)&s_abort) break;
+                }
+                room--;
+                const uint32_t dst = x_base + (uint32_t)(s * BW_STAGE), lead = bw_mapa(full_x(s), 0);
+                const int kb = u < nkb ? u : u - nkb;
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(full_x(s), 2u * bytes);
+                    bw_tma(dst, &xmap, kb * BW_KB, tok0, lead);
+                }
+                __syncwarp();
+                if (++s == BW_STAGES) { s = 0; par ^= 1u; }
+            }
+        }
+    } else if (warp == BW_MMA_WARP) {
+        if (rank == 0) {
+            // ---------------- MMA issue
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(P.npad >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+            const uint64_t x_desc = umma_desc_sw128(x_base);
+            int s = 0, sa = 0, cx = 0, ca = 0;                 // next places of the rings, and how many are known to be full
+            uint32_t px = 0, pa = 0;
+            for (int it = i0; it < i1; it++) {
+                wait(acc_empty, ((uint32_t)(it - i0) & 1u) ^ 1u);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int u = 0; u < nu;) {
+                    if (cx == 0) cx = bw_run(full_x(0), s, px, BW_STAGES, &s_abort);
+                    if (ca == 0) ca = bw_run(full_a(0), sa, pa, BW_SLOTS, &s_abort);
+                    __syncwarp();
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const int n = min(min(cx, ca), nu - u);
+                    const bool last = u + n == nu;
+                    if (elect_one()) {
+                        int xs = s, as = sa;
+                        for (int t = 0; t < n; t++) {
+                            const uint64_t xd = x_desc + (uint64_t)(xs * (BW_STAGE / 16));
+                            const uint32_t a = a_col0 + (uint32_t)as * 32u;
+#pragma unroll
+                            for (int kk = 0; kk < 4; kk++) bw_umma(tmem, a + kk * 8, xd + kk * 2, idesc, (u + t) | kk ? 1u : 0u);
+                            bw_commit(empty_x(xs));
+                            bw_commit(empty_a(as));
+                            if (++xs == BW_STAGES) xs = 0;
+                            if (++as == BW_SLOTS) as = 0;
+                        }
+                        if (last) bw_commit(acc_full);
+                    }
+                    __syncwarp();
+                    u += n; cx -= n; ca -= n;
+                    if ((s += n) >= BW_STAGES) { s -= BW_STAGES; px ^= 1u; }
+                    if ((sa += n) >= BW_SLOTS) { sa -= BW_SLOTS; pa ^= 1u; }
+                }
+            }
+        }
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    } else {
+        // ---------------- epilogue: warp w reads lanes 32 (w & 3) .. (= rows of this block's tile); columns = tokens
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const int q = warp & 3;
+        for (int it = i0; it < i1; it++) {
+            const BwMat& m = P.m[mat_of(it)];
+            const int tile = (it - m.item0) / P.ntb * 2 + (int)rank, tok0 = (it - m.item0) % P.ntb * P.npad;
+            const int r = tile * BW_ROWS + q * 32 + lane, nt = min(P.npad, P.ntok - tok0);
+            const bool put = r < m.R, bias = m.bias != nullptr;
+            const float rs = put ? __half2float(__ldg(m.row_scale + r)) : 0.f, brow = put && bias ? (float)((const T*)m.bias)[r] : 0.f;
+            float xv[BW_TOK / 32];                             // factors that undo the token scales: tokens lane, lane + 32, ..
+#pragma unroll
+            for (int k = 0; k < BW_TOK / 32; k++) xv[k] = lane + 32 * k < nt ? __ldcg(P.xinv + tok0 + lane + 32 * k) : 0.f;
+            T* yr = (T*)m.y + (put ? r : 0) + (int64_t)tok0 * P.ldy;
+            wait(acc_full, (uint32_t)(it - i0) & 1u);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // rolled: instructions that run once per item come from far away (256 tokens unrolled took 20 us)
+#pragma unroll 1
+            for (int k = 0; k * 16 < nt; k++) {
+                uint32_t v[16];
+                bw_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(k * 16), v);
+                float xw = xv[0];
+#pragma unroll
+                for (int h = 1; h < BW_TOK / 32; h++) xw = k >> 1 == h ? xv[h] : xw;
+                // all values, then all stores: a branch between two of them costs a hundred clocks a token
+                T o[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) * __shfl_sync(0xffffffffu, xw, (k & 1) * 16 + j) * rs);
+#pragma unroll
+                for (int j = 0; j < 16; j++) o[j] = cbl_cvt_out<T>(__uint_as_float(v[j]));
+                if (bias) {                                    // two roundings, as two operators would give
+#pragma unroll
+                    for (int j = 0; j < 16; j++) o[j] = cbl_cvt_out<T>((float)o[j] + brow);
+                }
+                const int left = put ? nt - k * 16 : 0;
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (j < left) yr[j * P.ldy] = o[j];
+                yr += 16 * P.ldy;
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bw_arrive(bw_mapa(acc_empty, 0));
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (s_abort && tid == 0) {
+        atomicExch(P.status, 1u);
+        for (int k = 0; k < 100; k++) __nanosleep(1000000);    // copies that are still under way land before the block leaves
+    }
+    __syncthreads();
+    bw_sync();                                                 // the peer no longer reads or signals this block's memory
+    if (warp == BW_MMA_WARP) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+}  // namespace
+
+// Tokens of a block: as even as blocks of at most 256 in steps of 32 can be.
+static int bw_npad(int ntok) {
+    const int nb = cbl_ceil_div(ntok, BW_TOK);
+    return cbl_ceil_div(cbl_ceil_div(ntok, nb), 32) * 32;
+}
+
+// Whether this product is the faster one: estimates of its time and of that of a decode into memory and a GEMM (cbl_gemm_dense), in ns, from
+// measurements of 3584 .. 37888 rows x 896 .. 18944 columns.  Here: 6 us and 12 ns per token of a block, per wave of items 250 ns and 0.9 per
+// token for each k-block and 3 us between waves (a quarter more from four waves on, where the power limit binds).  There: 4.5 us or 4400 GB/s for
+// the decode, 6.3 us, per wave of tiles 120 ns and 1.5 per row of the tile for each k-block; it stays where this one gains less than a tenth.
+// us, here / there: 18944 x 3584, 130 tokens 30 / 63, 256 36 / 65, 512 63 / 84, 700 92 / 105, 1024 138 / 131; 9000 x 2000, 256 24 / 26; 3584 x 3584,
+// 256 32 / 24; 3584 x 18944, 256 123 / 87 (few rows leave pairs idle).
+extern "C" int32_t cbl_gemm_b3_wide_serves(const int32_t* R, int32_t n, int32_t C, int32_t books, int32_t ntok) {
+    if (!R || n < 1 || n > BW_MAX_MATS || C < 8 || (books != 1 && books != 2) || ntok <= 128) return 0;
+    const int64_t pairs = cbl_sm_count() / 2, nkb = cbl_ceil_div(C, BW_KB), npad = bw_npad(ntok), ntb = (ntok + npad - 1) / npad, ntt = (ntok + 255) / 256;
+    int64_t items = 0, rows = 0;
+    for (int i = 0; i < n; i++) {
+        if (R[i] < 0) return 0;
+        rows += R[i];
+        items += cbl_ceil_div(cbl_ceil_div(R[i], BW_ROWS), 2) * ntb;
+    }
+    if (items == 0 || items > (1 << 24)) return 0;
+    const int64_t waves = (items + pairs - 1) / pairs, wave = nkb * books * (250 + npad * 9 / 10);
+    const int64_t here = 6000 + 12 * npad + waves * wave * (waves >= 4 ? 5 : 4) / 4 + (waves - 1) * 3000;
+    int64_t bn = 256, best = -1;
+    for (int64_t b = 256; b >= 64; b -= 32) {
+        const int64_t cost = (ntt * ((rows + b - 1) / b) + pairs - 1) / pairs * (b + 40);
+        if (best < 0 || cost < best) { best = cost; bn = b; }
+    }
+    const int64_t decode = rows * C * 2 / 4400 > 4500 ? rows * C * 2 / 4400 : 4500;
+    const int64_t there = decode + 6300 + (ntt * ((rows + bn - 1) / bn) + pairs - 1) / pairs * nkb * (120 + bn * 3 / 2);
+    return here * 10 < there * 9;
+}
+
+extern "C" int cbl_gemm_b3_wide(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, void* const* ys, int ydtype, int64_t ldy,
+                                void* stage, void* workspace, cbl_stream s) {
+    if (!mats || !ys || !stage || !workspace || n < 1) return CBL_EINVAL;
+    if (n > BW_MAX_MATS) return CBL_EUNSUPPORTED;
+    const int C = mats[0].C, books = mats[0].books;
+    if (ntok < 1 || (x && ldx < C)) return CBL_EINVAL;
+    if (ydtype != CBL_F32 && ydtype != CBL_F16 && ydtype != CBL_BF16) return CBL_EINVAL;
+    if (((uintptr_t)stage % 16) || ((uintptr_t)workspace % 16)) return CBL_EINVAL;
+    BwLaunch P;
+    P.npad = bw_npad(ntok);
+    P.ntb = cbl_ceil_div(ntok, P.npad);
+    P.n = 0;
+    int64_t items = 0;
+    for (int i = 0; i < n; i++) {
+        const cbl_b3& m = mats[i];
+        if (!m.words || !m.table || !m.row_scale || !ys[i] || ldy < m.R) return CBL_EINVAL;
+        if (m.books != 1 && m.books != 2) return CBL_EINVAL;
+        if ((m.books == 2 && !m.table2) || m.R < 0 || m.C <= 0 || m.C % 8) return CBL_EINVAL;
+        if (m.M != 1 || m.copies != 2 || m.tile_rows) return CBL_EUNSUPPORTED;
+        if (m.C != C || m.books != books || m.ntile != cbl_ceil_div(m.R, BW_ROWS)) return CBL_EINVAL;
+        if (((uintptr_t)m.words % 16) || ((uintptr_t)m.table % 16) || (m.table2 && (uintptr_t)m.table2 % 16)) return CBL_EINVAL;
+        if (m.R == 0) continue;
+        P.m[P.n++] = {(const uint4*)m.words, (const uint4*)m.table, (const uint4*)m.table2, (const __half*)m.row_scale, m.bias, ys[i], m.R, m.ntile, (int)items};
+        items += (int64_t)cbl_ceil_div(m.ntile, 2) * P.ntb;
+    }
+    if (items == 0) return CBL_OK;
+    if (items > (1 << 24)) return CBL_EUNSUPPORTED;
+    if (x) {                                                   // x == NULL: the caller has staged the activations
+        const int rc = cbl_prep_x(x, xdtype, ntok, C, ldx, nullptr, 1, stage, s);
+        if (rc) return rc;
+    }
+    const int Mpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
+    P.books = books; P.nkb = cbl_ceil_div(C, BW_KB); P.ntok = ntok; P.items = (int)items; P.ldy = ldy;
+    P.xinv = (const float*)((const __half*)stage + (int64_t)Mpad * Cpad);
+    P.status = (unsigned int*)workspace;
+    encode_tiled_fn enc = get_encode();
+    if (!enc) return CBL_ECUDA;
+    CUtensorMap xmap;
+    const cuuint64_t dims[2] = {(cuuint64_t)Cpad, (cuuint64_t)Mpad};
+    const cuuint64_t strides[1] = {(cuuint64_t)Cpad * 2};
+    const cuuint32_t box[2] = {BW_KB, (cuuint32_t)(P.npad / 2)}, estr[2] = {1, 1};
+    const CUresult cr = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, stage, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
+    typedef void (*kernel_fn)(const CUtensorMap, const BwLaunch);
+    static const kernel_fn fns[3] = {k_gemm_b3_wide<float>, k_gemm_b3_wide<__half>, k_gemm_b3_wide<__nv_bfloat16>};      // by cbl_dtype
+    static bool attr_set[64] = {};
+    int dev = 0;
+    CBL_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        for (int k = 0; k < 3; k++) CBL_CUDA(cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, BW_SMEM));
+        attr_set[dev] = true;
+    }
+    const int pairs = cbl_sm_count() / 2;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (unsigned)(items < pairs ? items : pairs));
+    cfg.blockDim = dim3(BW_THREADS);
+    cfg.dynamicSmemBytes = BW_SMEM;
+    cfg.stream = (cudaStream_t)s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[ydtype], xmap, P));
+    return cbl_check_launch();
+}

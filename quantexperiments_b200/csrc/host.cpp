@@ -162,6 +162,17 @@ int dense_product(const cbl_packed* m, int n, int32_t C, bool wide, const void* 
     return cbl_gemm_dense_bias(w, (int32_t)R, C, row_scale, x, xdt, (int32_t)tokens, ldx, y, ydt, ldy, bias, x ? stage : staged, stage + st.numel() - 16, s);
 }
 
+// Many tokens by codeword gathers (one column order, one number of books).
+bool gathers(const Plan& p, int64_t tokens) {
+    if (p.orders != 1 || tokens <= 128 || tokens > 65535) return false;
+    int32_t rows[MAX_PIECES];
+    for (int i = 0; i < p.n; i++) {
+        if (p.packed[i].books != p.packed[0].books) return false;
+        rows[i] = (int32_t)p.rows[i];
+    }
+    return cbl_gemm_b3_wide_serves(rows, p.n, (int32_t)p.C, p.packed[0].books, (int32_t)tokens);
+}
+
 // One product of `tokens` tokens into y [tokens, R] (row stride ldy); CBL_EUNSUPPORTED when the plan has no layout for them.
 int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* y, int ydt, int64_t ldy, const void* bias, void* stream, const char** fn) {
     const int esz = ydt == CBL_F32 ? 4 : 2;
@@ -199,13 +210,26 @@ int product(Plan& p, const void* x, int xdt, int64_t tokens, int64_t ldx, char* 
         return cbl_gemm_b3(mats, p.n, x, xdt, (int32_t)tokens, ldx, p.perms, ys, ydt, ldy, stage, ws, s);
     }
     if (!p.has_dense || tokens < p.dense_from) return CBL_EUNSUPPORTED;
+    if (gathers(p, tokens)) {
+        if (!p.has_b3[0]) return CBL_EUNSUPPORTED;
+        void* const stage = need(STAGE, cbl_prep_x_bytes((int32_t)tokens, (int32_t)p.C, 1), p.device, stream).data_ptr();
+        void* const ws = need(PARTIAL, 1 << 16, p.device, stream).data_ptr();
+        cbl_b3 mats[MAX_PIECES];
+        for (int i = 0; i < p.n; i++) {
+            mats[i] = p.b3[0][i];
+            mats[i].bias = bias ? (const char*)bias + p.first[i] * esz : nullptr;
+        }
+        *fn = "cbl_gemm_b3_wide";
+        return cbl_gemm_b3_wide(mats, p.n, x, xdt, (int32_t)tokens, ldx, ys, ydt, ldy, stage, ws, s);
+    }
     return dense_product(p.packed, p.n, (int32_t)p.C, false, p.row_scale, x, xdt, tokens, ldx, nullptr, y, ydt, ldy, bias, p.device, stream, fn);
 }
 
 bool layout_for(const Plan& p, int64_t tokens) {
     if ((tokens == 1 && p.has_l8) || (tokens <= 4 && p.direct[tokens])) return true;
     if (tokens <= cbl_gemm_b3_max_tokens(2)) return p.has_b3[tokens <= cbl_gemm_b3_max_tokens(3) ? 1 : 0];
-    return p.has_dense && tokens >= p.dense_from;
+    // (without the layout the caller decides: it builds it, or, in a captured region, decodes)
+    return p.has_dense && tokens >= p.dense_from && (p.has_b3[0] || !gathers(p, tokens));
 }
 
 // Whether the plan's bias can be added by the kernel to products of x: one value per row, x's type and device, nobody's gradient.  Others

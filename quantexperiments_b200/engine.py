@@ -365,17 +365,20 @@ class DecodeEngine:
             add, last = None, len(self.layers) - 1
             st = T > 1 and self._stages_inputs(T)
             sh, si = self._stage_buffers(T) if st else (None, None)
-            ahead = None
+            ahead, decoded = None, []
             if T >= DENSE_MIN_TOKENS and all(S[k].dense is not None for S in self.stacks for k in S):
+                names = ("qkv", "o", "gu", "down")
+                decoded = [S[k] for S in self.stacks for k in names][:4 * last + 1]
+                decoded = [st.dense for st in decoded if not st.gathers(T)]
+            if decoded:
                 if self._side is None:
                     self._side = torch.cuda.Stream(device=self.dev)
-                names = ("qkv", "o", "gu", "down")
-                ahead = _Ahead([S[k].dense for S in self.stacks for k in names][:4 * last + 1], self._side, self._scratch)
+                ahead = _Ahead(decoded, self._side, self._scratch)
 
             def product(stack, x, y, staged=None):
                 """Rows of a prompt are summed in fp32 like each other: no tables of 16-bit entries for the last one (a prompt of one
                 token runs as that token does by itself)."""
-                if ahead is not None:
+                if ahead is not None and not stack.gathers(y.shape[0]):
                     ahead.run(x, y, staged)
                 else:
                     stack.run(x, y, staged, tables=T == 1 and stack.tables and all(l.use_l8() for l in stack.lins))

@@ -2,7 +2,7 @@
 
 DeviceMatrix  the file layout resident on the GPU: dense decode, tag unpacking
 L8Matrix      column-tile re-layout + one-token product by activation-side tables (L8Group: several matrices per launch)
-B3Matrix      slots of rotated book copies + product of 1..128 tokens by codeword gathers (B3Group)
+B3Matrix      slots of rotated book copies + product of 1..128 tokens, or of some hundred, by codeword gathers (B3Group)
 DenseStack    decode once + GEMM, for many tokens
 T16Matrix, X16Matrix, L8Group.gemm_rows, L8Matrix.gemm
               earlier products of small and large batches: callers may use them, nothing in the package does
@@ -525,6 +525,30 @@ class B3Group(_Uncopied):
             stage, x = scratch(self.device, STAGE, need[0]), (X.data_ptr(), _dt(X.dtype), B, X.stride(0) if B > 1 else X.shape[1])
         with _on(self.device):
             _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), *x, _ptr(self.perms), out, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
+        return ys
+
+    @staticmethod
+    def wide_serves(dms: list, n: int) -> bool:
+        """Whether n >= 129 tokens of these matrices run faster by gathers (run_wide) than decoded once and multiplied."""
+        if n <= 128 or len(dms) > B3Group.MAX or any(not dm.fast or dm.M != 1 or dm.C != dms[0].C or dm.books != dms[0].books for dm in dms):
+            return False
+        return bool(lib.cbl_gemm_b3_wide_serves((ctypes.c_int32 * len(dms))(*[dm.R for dm in dms]), len(dms), dms[0].C, dms[0].books, n))
+
+    def run_wide(self, X: torch.Tensor | None, ys: list[torch.Tensor], staged: torch.Tensor | None = None) -> list[torch.Tensor]:
+        """run() for 129 tokens and more (one column order, two copies of the book)."""
+        T = ys[0].shape[0]
+        if X is None and staged is None or X is not None and (X.dim() != 2 or X.shape != (T, self.C) or X.stride(1) != 1 or X.device != self.device):
+            raise ValueError("X must be [T, C] with unit column stride on the matrices' device")
+        if len(ys) != len(self.mats) or len({y.dtype for y in ys}) != 1 or any(y.shape != (T, m.R) or y.stride() != (ys[0].stride(0), 1)
+                                                                             for y, m in zip(ys, self.mats)):
+            raise ValueError("one output [T, R_i] per matrix, one dtype, unit column stride and a common row stride")
+        out = (ctypes.c_void_p * len(ys))(*[y.data_ptr() for y in ys])
+        ws = scratch(self.device, PARTIAL, 1 << 16)
+        stage, x = (staged, (None, 0, T, 0)) if X is None else (scratch(self.device, STAGE, lib.cbl_prep_x_bytes(T, self.C, 1)),
+                                                                 (X.data_ptr(), _dt(X.dtype), T, X.stride(0)))
+        with _on(self.device):
+            _lib.check("cbl_gemm_b3_wide", lib.cbl_gemm_b3_wide(self._structs, len(self.mats), *x, out, _dt(ys[0].dtype), ys[0].stride(0), stage.data_ptr(),
+                                                                ws.data_ptr(), _stream()))
         return ys
 
     def status(self) -> None:

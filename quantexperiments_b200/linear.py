@@ -34,7 +34,8 @@ L8_MIN_ROWS = 2048
 L8_MIN_ROWS_PER_ORDER = 1536
 # Tokens up to which the book lies three times in shared memory (the activations of more tokens need the room: two copies).
 B3_MAX_3COPIES = 16
-# Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM.
+# Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM - or, up to some 900
+# tokens of matrices with rows enough for all SMs, gathers once more (B3Group.wide_serves).
 DENSE_MIN_TOKENS = 129
 
 
@@ -134,6 +135,10 @@ class PackedLinear(_Uncopied, torch.nn.Module):
         least = L8_MIN_ROWS if self.dm.M == 1 else L8_MIN_ROWS_PER_ORDER * self.dm.M
         return self.dm.fast and not self.wide and self.dm.M <= L8Matrix.MAX_ORDERS and self.R >= least
 
+    def gathers(self, n: int) -> bool:
+        """n >= 129 tokens run on codeword gathers.  A captured region builds no layout for them: it decodes."""
+        return not self.wide and B3Group.wide_serves([self.dm], n) and (2 in self._b3 or not torch.cuda.is_current_stream_capturing())
+
     def direct(self, n: int) -> bool:
         """n tokens run straight from the file layout, without a kernel layout: few tokens of a small matrix."""
         return n <= 4 and self.dm.fast and not self.wide and bool(lib.cbl_direct_serves(ctypes.byref(self.dm.struct()), 1, n, self.use_l8()))
@@ -174,6 +179,8 @@ class PackedLinear(_Uncopied, torch.nn.Module):
             self.l8.run(x2[0], y[0])
         elif n < DENSE_MIN_TOKENS:
             self.group(n).run(x2, [y])
+        elif self.gathers(n):
+            self.group(n).run_wide(x2, [y])
         else:
             # many tokens: decode once into the shared 16-bit scratch, then the TMA-fed GEMM
             self.dm.gemm_dense(x2, y)
@@ -236,8 +243,15 @@ class Stack:
             self._b3[copies] = B3Group([l.group(n).mats[0] for l in self.lins])
         return self._b3[copies]
 
+    def gathers(self, n: int) -> bool:
+        """n >= 129 tokens run on codeword gathers (see PackedLinear.gathers)."""
+        return (self.shared and not any(l.wide for l in self.lins) and B3Group.wide_serves([l.dm for l in self.lins], n)
+                and (2 in self._b3 or not torch.cuda.is_current_stream_capturing()))
+
     def ready(self, n: int) -> bool:
         """Whether run() on n tokens builds no layout."""
+        if self.fast and n >= DENSE_MIN_TOKENS and self.gathers(n):
+            return 2 in self._b3
         if not self.fast or n >= DENSE_MIN_TOKENS:
             return True
         if self._direct(n):
@@ -248,6 +262,9 @@ class Stack:
         return copies in self._b3 if self.shared else all(copies in l._b3 for l in self.lins)
 
     def prepare(self, n: int) -> None:
+        if self.fast and n >= DENSE_MIN_TOKENS and self.gathers(n):
+            self.b3(n)._structs
+            return
         if not self.fast or n >= DENSE_MIN_TOKENS or self._direct(n):
             return
         if n == 1 and self.tables:
@@ -268,9 +285,12 @@ class Stack:
     def run(self, x: torch.Tensor | None, y: torch.Tensor, staged: torch.Tensor | None = None, tables: bool | None = None) -> torch.Tensor:
         """tables: whether one token may run on table lookups (None: where the stack's rule says so)."""
         n = y.shape[0]
+        ys = list(y.split(self.Rs, 1))
+        if n >= DENSE_MIN_TOKENS and self.gathers(n):
+            self.b3(n).run_wide(x, ys, staged)
+            return y
         if n >= DENSE_MIN_TOKENS and self.dense is not None:
             return self.dense.gemm(x, y, staged)
-        ys = list(y.split(self.Rs, 1))
         if x is None:
             self.b3(n).run(None, ys, staged)
         elif self._direct(n):

@@ -331,6 +331,65 @@ def test_small_products_straight_from_the_file_layout(R, C, books, M):
             assert torch.equal(biased(xb), lin(xb) + biased.bias)
 
 
+@pytest.mark.parametrize("Rs,C,books,n", [([256], 64, 1, 129), ([300], 1000, 1, 256), ([640, 100, 128], 896, 2, 257), ([128, 1], 72, 1, 513), ([2000], 2048, 2, 1000),
+                                          ([40000], 128, 1, 300)])
+def test_many_tokens_by_gathers(Rs, C, books, n):
+    """Pairs of SMs: one tile of rows and many, a pair with a tile missing, blocks of tokens of every width, several items per pair, two books; outputs
+    side by side with rows between them untouched.  fp32 sums of exact products: C / 16 per book are rounded or truncated at 2^-23 of the running sum.  No
+    further from float64 than the weights decoded to memory and multiplied (which rounds the sum of two books)."""
+    from quantexperiments_b200.kernels import B3Group, B3Matrix, DenseStack
+    lins = [_linear(orc.synth_matrix(R, C, seed=R + C, books=books)) for R in Rs]
+    grp, dense = B3Group([B3Matrix(l.dm, 2) for l in lins]), DenseStack([l.dm for l in lins])
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(n, C, generator=g).bfloat16().cuda()
+    ref = torch.cat([x.double() @ l.dense().double().T for l in lins], 1)
+    y = torch.full((n, sum(Rs) + 5), float("nan"), device="cuda")
+    grp.run_wide(x, list(y[:, :sum(Rs)].split(Rs, 1)))
+    off = (y[:, :sum(Rs)].double() - ref).norm()
+    assert off <= books * max(C / 16, 4) * 2.0 ** -23 * ref.norm() and y[:, sum(Rs):].isnan().all()
+    z = dense.gemm(x, torch.empty(n, sum(Rs), device="cuda"))
+    assert off <= 1.1 * (z.double() - ref).norm() + 2.0 ** -23 * ref.norm()
+    for dt in (torch.float16, torch.bfloat16):
+        h = torch.empty(n, sum(Rs), device="cuda", dtype=dt)
+        grp.run_wide(x, list(h.split(Rs, 1)))
+        assert torch.equal(h, y[:, :sum(Rs)].to(dt))
+    grp.status()
+
+
+@pytest.mark.parametrize("bias", [False, True])
+def test_many_tokens_of_many_rows_take_gathers_on_every_path(bias):
+    """A wide matrix and a stack: first call, native call, serving layer and captured region give the same bits; a capture before the layout exists
+    decodes instead, within rounding."""
+    from quantexperiments_b200.vllm_ext import core
+    ms = [orc.synth_matrix(9216, 256, seed=s) for s in (1, 2)]
+    g = torch.Generator().manual_seed(1)
+    b = torch.randn(9216, generator=g).bfloat16().cuda() if bias else None
+    x = torch.randn(200, 256, generator=g).bfloat16().cuda()
+    lin = _linear(ms[0], bias=b)
+    s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=s):
+        early = lin(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert lin.gathers(200) and not lin.gathers(128) and not lin._b3
+    want = lin(x)
+    assert 2 in lin._b3 and torch.equal(lin(x), want)
+    assert (early.float() - want.float()).abs().max() <= 2.0 ** -6 * want.float().abs().max()
+    y = torch.empty(200, 9216, device="cuda", dtype=torch.bfloat16)
+    assert torch.equal(lin.forward_into(x, y) if b is None else lin.forward_into(x, y) + b, want)
+    with torch.cuda.graph(graph2 := torch.cuda.CUDAGraph(), stream=s):
+        late = lin(x)
+    graph2.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(late, want)
+    ps = core.PackedShards([_linear(m) for m in ms])
+    first, second = ps.forward(x), ps.forward(x)
+    assert ps.stack.gathers(200) and torch.equal(first, second)
+    if b is None:
+        assert torch.equal(first[:, :9216], want)
+
+
 @pytest.mark.parametrize("n,C,M", [(1, 8, 2), (1, 18944, 16), (3, 2056, 4), (9, 3584, 16), (128, 1032, 3)])
 def test_activations_staged_through_column_orders(n, C, M):
     """Rows as long as the orders are picked from shared memory, rows further apart from memory: the same buffer, bit for bit."""
