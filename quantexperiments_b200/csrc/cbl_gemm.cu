@@ -745,8 +745,6 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = uniform_warp(tid), lane = tid & 31;
-    // the decode of the next matrix (launched with programmatic serialization) takes the SMs as this GEMM leaves them
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int nkb = (m.C + GM_BK - 1) / GM_BK;
@@ -773,6 +771,10 @@ k_gemm_dense_2sm(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     __syncthreads();
     cluster_sync_all();                                        // both blocks' barriers and tensor memory exist
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Barriers and tensor memory are set up while the kernels before are still running.  Only behind the wait is the decode of the next matrix
+    // let in, which takes the SMs as this GEMM leaves them: it writes before it waits, into the buffer of the GEMM before this one.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem = s_tmem;
 
     // The producer and the issuing warp wait as whole warps and elect a thread only for straight code: with a wait inside
@@ -1002,18 +1004,20 @@ extern "C" int cbl_gemm_dense_bias(const void* w16, int32_t R, int32_t C, const 
     const int ntiles = cbl_ceil_div(R, bn) * ntt;
     int nclusters = pairs;
     if (nclusters > ntiles) nclusters = ntiles;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * nclusters);
     cfg.blockDim = dim3(G3_THREADS);
     cfg.dynamicSmemBytes = G3_SMEM;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     CBL_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_dense_2sm, xmap, wmap, m, xinv, (int)ntok, y, ydtype, ldy, vec_ok, bias, bn, (unsigned int*)workspace));
     return cbl_check_launch();
 }
