@@ -57,6 +57,7 @@ struct B3Mat {
 };
 struct B3Launch {
     int nseg, nkb, npad, xrows, ntok, NST, RX, XU, PP, Bpad;
+    int flat;                                    // the maps are of rows as they are, k-blocks not set apart: one by one
     int ks, q, rem;                              // ks > 0: ks blocks share a tile; else blocks have q units, the first rem one more
     int64_t ldy;
     const float* xinv;
@@ -363,18 +364,21 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
             credit--;
             const int n = min(XU, nu - i);
             const uint32_t dst = x_base + (uint32_t)xs * xstage;
-            if (kb + n <= nkb) {                               // one copy brings XU k-blocks (at the end of the range more than are used)
+            if (kb + n <= nkb && !P.flat) {                    // one copy brings XU k-blocks (at the end of the range more than are used)
                 if (elect_one()) {
                     mbar_expect_tx(full_x(xs), xstage);
                     b3_tma_3d(dst, &xmap, c1, kb, full_x(xs));
                 }
                 kb += n;
-            } else {                                           // across the border of a tile: one by one
+            } else {                                           // across the border of a tile, or flat: one by one
                 if (elect_one()) mbar_expect_tx(full_x(xs), (uint32_t)n * xbytes);
                 __syncwarp();
                 for (int k = 0; k < n; k++) {
                     if (kb == nkb) { kb = 0; c1 = row_of(++gi); }
-                    if (elect_one()) b3_tma_3d(dst + (uint32_t)k * xbytes, &xmap1, c1, kb, full_x(xs));
+                    if (elect_one()) {
+                        if (P.flat) tma_load_2d(dst + (uint32_t)k * xbytes, &xmap1, kb * B3_KB, c1, full_x(xs));
+                        else b3_tma_3d(dst + (uint32_t)k * xbytes, &xmap1, c1, kb, full_x(xs));
+                    }
                     __syncwarp();
                     kb++;
                 }
@@ -419,9 +423,9 @@ k_gemm_b3(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUte
                 rs = r >= 0 ? __half2float(__ldg(m.row_scale + r)) : 0.f;
             }
             if (pc == 0 || m.tile_order) {
-                const float* xi = P.xinv + (m.tile_order ? __ldg(m.tile_order + tile) * P.Bpad : 0);
+                const float* xi = !P.xinv ? nullptr : P.xinv + (m.tile_order ? __ldg(m.tile_order + tile) * P.Bpad : 0);
 #pragma unroll
-                for (int k = 0; k < B3_NMAX / 32; k++) xv[k] = lane + 32 * k < P.ntok ? __ldcg(xi + lane + 32 * k) : 0.f;
+                for (int k = 0; k < B3_NMAX / 32; k++) xv[k] = lane + 32 * k < P.ntok ? xi ? __ldcg(xi + lane + 32 * k) : 1.f : 0.f;
             }
             float* mine = whole ? nullptr : slot_of(cta, gi) + row;
             int np = 0;                                        // pieces of this output tile
@@ -802,7 +806,7 @@ extern "C" size_t cbl_gemm_b3_workspace_bytes(const cbl_b3* mats, int32_t n, int
     return rc ? 0 : most;
 }
 
-static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, int ntok, int64_t ldy, void* stage, void* workspace, cbl_stream s);
+static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, int ntok, int64_t ldy, void* stage, const void* x16, int64_t ldx, void* workspace, cbl_stream s);
 
 extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdtype, int32_t ntok, int64_t ldx, const int32_t* perms, void* const* ys,
                            int ydtype, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
@@ -817,7 +821,9 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
         if (!ys[i] || (ntok > 1 && ldy < mats[i].R)) return CBL_EINVAL;
     }
     if (mats[0].M > 1 && !perms) return CBL_EINVAL;
-    bool any = false, staged = x == nullptr;                   // x == NULL: the caller has staged the activations
+    // fp16 rows are read as they are (their scale could only cost bits); x == NULL: the caller has staged the activations
+    const bool as_is = x && xdtype == CBL_F16 && mats[0].M == 1 && (uintptr_t)x % 16 == 0 && (ntok == 1 || ldx % 8 == 0);
+    bool any = false, staged = x == nullptr || as_is;
     for (int i = 0; i < n; i++) any |= mats[i].ntile > 0;
     if (!any) return CBL_OK;
     return b3_launches(mats, n, ys, ydtype == CBL_F32 ? 4 : 2, ntok, [&](const B3Part* parts, int k, const B3Plan& pl) {
@@ -826,18 +832,20 @@ extern "C" int cbl_gemm_b3(const cbl_b3* mats, int32_t n, const void* x, int xdt
             if (rc) return rc;
             staged = true;
         }
-        return b3_launch(parts, k, pl, ydtype, ntok, ldy, stage, workspace, s);
+        return b3_launch(parts, k, pl, ydtype, ntok, ldy, stage, as_is ? x : nullptr, ntok == 1 ? mats[0].C : ldx, workspace, s);
     });
 }
 
-static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, int ntok, int64_t ldy, void* stage, void* workspace, cbl_stream s) {
+// x16: fp16 activations that need no staging (one column order, rows on 16-byte boundaries), or NULL.
+static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, int ntok, int64_t ldy, void* stage, const void* x16, int64_t ldx, void* workspace, cbl_stream s) {
     const int C = parts[0].m->C, M = parts[0].m->M, copies = parts[0].m->copies;
     const int Bpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
     B3Launch P;
     P.nkb = cbl_ceil_div(C, B3_KB);
     P.ks = pl.ks; P.q = pl.U / pl.G; P.rem = pl.U % pl.G; P.npad = pl.npad; P.xrows = pl.rows; P.ntok = ntok; P.NST = pl.NST; P.RX = pl.RX; P.XU = pl.XU; P.PP = pl.PP; P.Bpad = Bpad;
     P.ldy = ldy;
-    P.xinv = (const float*)((const __half*)stage + (int64_t)M * Bpad * Cpad);
+    P.xinv = x16 ? nullptr : (const float*)((const __half*)stage + (int64_t)M * Bpad * Cpad);
+    P.flat = x16 && C % B3_KB;
     P.status = (unsigned int*)workspace;
     P.counters = P.status + 64;
     P.partial = (float*)((char*)workspace + (size_t)B3_CTL_WORDS * 4);
@@ -874,21 +882,37 @@ static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, i
     }
     encode_tiled_fn enc = get_encode();
     if (!enc) return CBL_ECUDA;
+    const cuuint32_t estr[3] = {1, 1, 1};
+    // k-blocks set apart as a third dimension, so that one copy brings XU of them
+    auto encode = [&](const void* at, int64_t ld, int rows, int nkb, CUtensorMap* maps) {
+        const cuuint64_t dims[3] = {B3_KB, (cuuint64_t)rows, (cuuint64_t)nkb};
+        const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, B3_KB * 2};
+        const cuuint32_t box[3] = {B3_KB, (cuuint32_t)pl.rows, (cuuint32_t)pl.XU}, box1[3] = {B3_KB, (cuuint32_t)pl.rows, 1};
+        for (int k = 0; k < 2; k++) {
+            const CUresult cr = enc(maps + k, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)at, dims, strides, k ? box1 : box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return false; }
+        }
+        return true;
+    };
     // the maps of the staged activations are a function of these values; a caller that reuses its buffer finds them made
     struct MapKey { void* p; int Cpad, rows, box, XU; };
     static thread_local MapKey key = {nullptr, 0, 0, 0, 0};
-    static thread_local CUtensorMap xmap, xmap1;
-    if (key.p != stage || key.Cpad != Cpad || key.rows != M * Bpad || key.box != pl.rows || key.XU != pl.XU) {
-        const cuuint64_t dims[3] = {B3_KB, (cuuint64_t)M * Bpad, (cuuint64_t)Cpad / B3_KB};
-        const cuuint64_t strides[2] = {(cuuint64_t)Cpad * 2, B3_KB * 2};
-        const cuuint32_t box[3] = {B3_KB, (cuuint32_t)pl.rows, (cuuint32_t)pl.XU}, box1[3] = {B3_KB, (cuuint32_t)pl.rows, 1};
-        const cuuint32_t estr[3] = {1, 1, 1};
+    static thread_local CUtensorMap kept[2];
+    CUtensorMap own[2], *maps = x16 ? own : kept;
+    if (x16 && P.flat) {
+        // columns beyond C are outside the map, and zero, which the third dimension could not say of the last k-block's
+        const cuuint64_t dims[2] = {(cuuint64_t)C, (cuuint64_t)ntok}, strides[1] = {(cuuint64_t)ldx * 2};
+        const cuuint32_t box[2] = {B3_KB, (cuuint32_t)pl.rows};
+        const CUresult cr = enc(own + 1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)x16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
+        own[0] = own[1];
+    } else if (x16) {
+        if (!encode(x16, ldx, ntok, C / B3_KB, own)) return CBL_ECUDA;
+    } else if (key.p != stage || key.Cpad != Cpad || key.rows != M * Bpad || key.box != pl.rows || key.XU != pl.XU) {
         key.p = nullptr;
-        for (int k = 0; k < 2; k++) {
-            CUresult cr = enc(k ? &xmap1 : &xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, stage, dims, strides, k ? box1 : box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
-        }
+        if (!encode(stage, Cpad, M * Bpad, Cpad / B3_KB, kept)) return CBL_ECUDA;
         key = {stage, Cpad, M * Bpad, pl.rows, pl.XU};
     }
     typedef void (*kernel_fn)(const CUtensorMap, const CUtensorMap, const B3Launch);
@@ -911,7 +935,7 @@ static int b3_launch(const B3Part* parts, int n, const B3Plan& pl, int ydtype, i
     cfg.gridDim = dim3(pl.G);
     cfg.blockDim = dim3(B3_THREADS);
     cfg.dynamicSmemBytes = B3_SMEM;
-    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[(copies - 2) * 3 + ydtype], xmap, xmap1, P));
+    CBL_CUDA(cudaLaunchKernelEx(&cfg, fns[(copies - 2) * 3 + ydtype], maps[0], maps[1], P));
     return cbl_check_launch();
 }
 

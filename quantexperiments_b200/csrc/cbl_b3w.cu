@@ -296,7 +296,7 @@ k_gemm_b3_wide(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
             const float rs = put ? __half2float(__ldg(m.row_scale + r)) : 0.f, brow = put && bias ? (float)((const T*)m.bias)[r] : 0.f;
             float xv[BW_TOK / 32];                             // factors that undo the token scales: tokens lane, lane + 32, ..
 #pragma unroll
-            for (int k = 0; k < BW_TOK / 32; k++) xv[k] = lane + 32 * k < nt ? __ldcg(P.xinv + tok0 + lane + 32 * k) : 0.f;
+            for (int k = 0; k < BW_TOK / 32; k++) xv[k] = lane + 32 * k < nt ? P.xinv ? __ldcg(P.xinv + tok0 + lane + 32 * k) : 1.f : 0.f;
             T* yr = (T*)m.y + (put ? r : 0) + (int64_t)tok0 * P.ldy;
             wait(acc_full, (uint32_t)(it - i0) & 1u);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -406,21 +406,23 @@ extern "C" int cbl_gemm_b3_wide(const cbl_b3* mats, int32_t n, const void* x, in
     }
     if (items == 0) return CBL_OK;
     if (items > (1 << 24)) return CBL_EUNSUPPORTED;
-    if (x) {                                                   // x == NULL: the caller has staged the activations
+    // fp16 rows on 16-byte boundaries are read as they are; x == NULL: the caller has staged the activations
+    const bool as_is = x && xdtype == CBL_F16 && (uintptr_t)x % 16 == 0 && ldx % 8 == 0;
+    if (x && !as_is) {
         const int rc = cbl_prep_x(x, xdtype, ntok, C, ldx, nullptr, 1, stage, s);
         if (rc) return rc;
     }
     const int Mpad = (ntok + 7) / 8 * 8, Cpad = (C + 511) / 512 * 512;
     P.books = books; P.nkb = cbl_ceil_div(C, BW_KB); P.ntok = ntok; P.items = (int)items; P.ldy = ldy;
-    P.xinv = (const float*)((const __half*)stage + (int64_t)Mpad * Cpad);
+    P.xinv = as_is ? nullptr : (const float*)((const __half*)stage + (int64_t)Mpad * Cpad);
     P.status = (unsigned int*)workspace;
     encode_tiled_fn enc = get_encode();
     if (!enc) return CBL_ECUDA;
     CUtensorMap xmap;
-    const cuuint64_t dims[2] = {(cuuint64_t)Cpad, (cuuint64_t)Mpad};
-    const cuuint64_t strides[1] = {(cuuint64_t)Cpad * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)(as_is ? C : Cpad), (cuuint64_t)(as_is ? ntok : Mpad)};
+    const cuuint64_t strides[1] = {(cuuint64_t)(as_is ? ldx : Cpad) * 2};
     const cuuint32_t box[2] = {BW_KB, (cuuint32_t)(P.npad / 2)}, estr[2] = {1, 1};
-    const CUresult cr = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, stage, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult cr = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, as_is ? (void*)x : stage, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) { g_cbl_last_cuda_error = (int)cr; return CBL_ECUDA; }
     typedef void (*kernel_fn)(const CUtensorMap, const BwLaunch);

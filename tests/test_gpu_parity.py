@@ -390,6 +390,33 @@ def test_many_tokens_of_many_rows_take_gathers_on_every_path(bias):
         assert torch.equal(first[:, :9216], want)
 
 
+@pytest.mark.parametrize("R,C,books", [(700, 448, 1), (300, 1016, 1), (260, 72, 2), (9216, 136, 1)])
+def test_fp16_activations_are_read_as_they_are(R, C, books):
+    """fp16 rows on 16-byte boundaries are not staged: the same bits as from rows off them, which are (their scale is a power of two), at every
+    token count's ring and with a last k-block that is not whole; rows apart; and no bit is lost beside large values."""
+    lin = _linear(orc.synth_matrix(R, C, seed=R + C, books=books))
+    W = lin.dense().double()
+    g = torch.Generator().manual_seed(C)
+    for n in (1, 5, 8, 9, 16, 17, 37, 64, 65, 128, 200, 300):
+        buf = torch.randn(n * C + 1, generator=g).half().cuda()
+        off = buf[1:].view(n, C)
+        x = off.clone()
+        apart = torch.full((n, C + 8), float("nan"), device="cuda", dtype=torch.float16)
+        apart[:, :C] = x
+        ref = x.double() @ W.T
+        for _ in range(2):
+            y = lin(x)
+            assert (y.double() - ref).norm() <= 2.0 ** -11 * ref.norm() and torch.equal(y, lin(off))
+        assert torch.equal(lin.forward_into(apart[:, :C], torch.empty_like(y)), y)
+        x[:, 1::2] *= 2.0 ** -14
+        x[:, 0] = 60000.0
+        big = torch.empty(n, R, device="cuda")
+        lin.forward_into(x, big)
+        if n >= 5 and (books == 1 or n <= 128):                      # (the decode to memory rounds the sum of two books)
+            bound = books * max(C / 16, 8) * 2.0 ** -23 * (x.double() @ W.T).abs().max()
+            assert (big.double() - x.double() @ W.T).abs().max() <= bound
+
+
 @pytest.mark.parametrize("n,C,M", [(1, 8, 2), (1, 18944, 16), (3, 2056, 4), (9, 3584, 16), (128, 1032, 3)])
 def test_activations_staged_through_column_orders(n, C, M):
     """Rows as long as the orders are picked from shared memory, rows further apart from memory: the same buffer, bit for bit."""
