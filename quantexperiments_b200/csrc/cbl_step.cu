@@ -325,9 +325,13 @@ __global__ void __launch_bounds__(256) k_rope_prompt(const T* __restrict__ qkv, 
 //   values  O[head][dim] += P[head][pos] . V[pos][dim]: the score accumulators ARE the A fragments of this product
 //           (the positions of a score tile are chosen so that they line up), and because the value cache is stored
 //           dimension-major a lane's B fragment is 16 contiguous bytes of a V^T row (8 positions of one dimension).
-// K and V are read once for all heads of the group; nothing is staged in shared memory.  Every warp writes its running
-// max, denominator and un-normalised output per head; k_attn_merge combines the 4 * nsplit partial results.
+// K and V are read once for all heads of the group.  They pass through a warp's own shared memory by asynchronous copies, all 16 KB of 32
+// positions at a time and the next keys while the values are multiplied: in registers a warp had 2 KB under way at most, three blocks of an
+// SM 24 KB (32 sequences of 256 .. 1024 positions, 42 MB: 16.7 us, 14.1 so).
+// Every warp writes its running max, denominator and un-normalised output per head; k_attn_merge combines the 4 * nsplit
+// partial results.
 constexpr int ATT_WARPS = 4, ATT_THREADS = ATT_WARPS * 32;
+constexpr int ATT_K_BYTES = 32 * 256, ATT_WARP_BYTES = ATT_K_BYTES + 128 * 64, ATT_SMEM = ATT_WARPS * ATT_WARP_BYTES;      // keys [position][dim], values [dim][position]
 constexpr int ATT_HD = 128;
 constexpr int ATT_PART = ATT_HD + 4;       // floats per partial result: HD sums, max, denominator, 2 of padding (16-byte rows)
 
@@ -359,8 +363,15 @@ template <> __device__ __forceinline__ uint32_t att_pack<__nv_bfloat16>(float lo
     return *(const uint32_t*)&h;
 }
 
+// 16 bytes from global to shared memory; `bytes` of them are read, the rest is zero.
+__device__ __forceinline__ void att_copy(uint32_t dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// Part c (16 bytes, of 16) of row r of the keys: any two of the eight that a quarter of a warp reads together lie in different banks.
+__device__ __forceinline__ uint32_t att_at(int r, int c) { return (uint32_t)(r * 256 + ((c & 8) | ((c ^ r ^ (c >> 3 << 1)) & 7)) * 16); }
+
 template <typename T, int REP>
-__global__ void __launch_bounds__(ATT_THREADS) k_attn_slice(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
+__global__ void __launch_bounds__(ATT_THREADS, 3) k_attn_slice(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
                                                             const int32_t* __restrict__ pos, int NKV, int max_len, float scale,
                                                             float* __restrict__ part) {
     pdl_enter();
@@ -392,8 +403,31 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_slice(const T* __restrict_
             qa[s][1] = head_ok ? __ldg(qrow + (d0 >> 1) + 1) : 0u;
         }
     }
-    const T* kbase = kc + ((int64_t)b * NKV + kv) * max_len * HD + 32 * t;                  // + position * HD
-    const T* vbase = vc + (((int64_t)b * NKV + kv) * HD + g) * max_len + 8 * t;             // + 8 j * max_len + p0
+    extern __shared__ __align__(128) unsigned char att_smem[];
+    const uint32_t ks = cbl_smem_u32(att_smem) + (uint32_t)(warp * ATT_WARP_BYTES), vs = ks + ATT_K_BYTES;
+    const T* kbase = kc + (((int64_t)b * NKV + kv) * max_len + (lane >> 4)) * HD + (lane & 15) * 8;      // + position * HD
+    const T* vbase = vc + (((int64_t)b * NKV + kv) * HD + (lane >> 2)) * max_len + (lane & 3) * 8;       // + 8 j * max_len + p0
+    auto copy_k = [&](int p) {                                       // (positions beyond the slice are zero)
+        if (p < s1)
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const int r = 2 * i + (lane >> 4);
+                att_copy(ks + att_at(r, lane & 15), kbase + (int64_t)(p + 2 * i) * HD, p + r < s1 ? 16u : 0u);
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto copy_v = [&](int p) {
+        if (p < s1)
+#pragma unroll
+            for (int i = 0; i < 16; i++) att_copy(vs + (uint32_t)(i * 512 + lane * 16), vbase + (int64_t)(8 * i) * max_len + p, 16u);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto landed = [&]() {                                            // the older of the two groups under way
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+    };
+    copy_k(s0 + 32 * warp);
+    copy_v(s0 + 32 * warp);
     float m = -3.0e38f, l = 0.f;
     float o[16][4];
 #pragma unroll
@@ -403,12 +437,12 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_slice(const T* __restrict_
     for (int p0 = s0 + 32 * warp; p0 < s1; p0 += 32 * ATT_WARPS) {
         // ---- scores: tile u, column n <-> position p0 + 8 (n / 2) + 2 u + n % 2; this lane supplies column g and receives columns 2t, 2t + 1
         float sc[4][2];
+        landed();
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const int pk = p0 + 8 * (g >> 1) + 2 * u + (g & 1);
             uint4 kw[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) kw[c] = pk < s1 ? __ldg((const uint4*)(kbase + (int64_t)pk * HD) + c) : make_uint4(0, 0, 0, 0);
+            for (int c = 0; c < 4; c++) kw[c] = cbl_lds128(ks + att_at(8 * (g >> 1) + 2 * u + (g & 1), 4 * t + c));
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int s = 0; s < 8; s++) {
@@ -419,6 +453,8 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_slice(const T* __restrict_
             sc[u][0] = pc < s1 ? acc[0] * scale : -3.0e38f;
             sc[u][1] = pc + 1 < s1 ? acc[1] * scale : -3.0e38f;
         }
+        __syncwarp();
+        copy_k(p0 + 32 * ATT_WARPS);
         // ---- online softmax of head g over the chunk (its 32 positions live in the four lanes t of this g)
         float cm = fmaxf(fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1])), fmaxf(fmaxf(sc[2][0], sc[2][1]), fmaxf(sc[3][0], sc[3][1])));
         cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 1));
@@ -439,11 +475,12 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_slice(const T* __restrict_
         const uint32_t pa0 = att_pack<T>(sc[0][0], sc[0][1]), pa2 = att_pack<T>(sc[1][0], sc[1][1]);
         const uint32_t pb0 = att_pack<T>(sc[2][0], sc[2][1]), pb2 = att_pack<T>(sc[3][0], sc[3][1]);
         // ---- values: dimension tile j = dimensions 8j..8j+7; this lane supplies dimension 8j + g, positions p0 + 8t..8t+7
+        landed();
 #pragma unroll
         for (int j0 = 0; j0 < 16; j0 += 4) {
             uint4 vw[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) vw[j] = __ldg((const uint4*)(vbase + (int64_t)(8 * (j0 + j)) * max_len + p0));
+            for (int j = 0; j < 4; j++) vw[j] = cbl_lds128(vs + (uint32_t)((j0 + j) * 512 + lane * 16));
 #pragma unroll
             for (int j = 0; j < 4; j++) {
 #pragma unroll
@@ -452,6 +489,8 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_slice(const T* __restrict_
                 att_mma<T>(o[j0 + j], pb0, pb2, vw[j].z, vw[j].w);
             }
         }
+        __syncwarp();
+        copy_v(p0 + 32 * ATT_WARPS);
     }
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
@@ -968,7 +1007,14 @@ extern "C" int32_t cbl_attn_decode_max_splits(void) { return ATT_MAX_SPLITS / AT
 template <typename T, int REP>
 static int attn_launch(const void* q, const void* kc, const void* vc, const int32_t* pos, int B, int NKV, int max_len, float scale, void* out,
                        float* part, int nsplit, cudaStream_t st) {
-    int rc = step_launch(k_attn_slice<T, REP>, dim3(nsplit, NKV, B), dim3(ATT_THREADS), 0, st, (const T*)q, (const T*)kc, (const T*)vc, pos,
+    static bool attr_set[64] = {};
+    int dev = 0;
+    CBL_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        CBL_CUDA(cudaFuncSetAttribute(k_attn_slice<T, REP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM));
+        attr_set[dev] = true;
+    }
+    int rc = step_launch(k_attn_slice<T, REP>, dim3(nsplit, NKV, B), dim3(ATT_THREADS), ATT_SMEM, st, (const T*)q, (const T*)kc, (const T*)vc, pos,
                          NKV, max_len, scale, part);
     if (rc != CBL_OK) return rc;
     if (nsplit * ATT_WARPS > 32)
