@@ -378,7 +378,7 @@ class DecodeEngine:
             def product(stack, x, y, staged=None):
                 """Rows of a prompt are summed in fp32 like each other: no tables of 16-bit entries for the last one (a prompt of one
                 token runs as that token does by itself)."""
-                if ahead is not None and not stack.gathers(y.shape[0]):
+                if ahead is not None and not stack.gathers(T):
                     ahead.run(x, y, staged)
                 else:
                     stack.run(x, y, staged, tables=T == 1 and stack.tables and all(l.use_l8() for l in stack.lins))

@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import math
 
 import numpy as np
@@ -468,6 +469,14 @@ class B3Matrix:
         return self.words.numel() * 4 + (0 if self.tile_rows is None else (self.tile_rows.numel() + self.tile_order.numel()) * 4)
 
 
+@functools.lru_cache(maxsize=4096)
+def _wide_serves(n: int, rows: tuple, C: int, books: int, device: int) -> bool:
+    """cbl_gemm_b3_wide_serves: whether n >= 129 tokens of matrices of these sizes run faster by gathers (B3Group.run_wide) than
+    decoded once and multiplied."""
+    with torch.cuda.device(device):
+        return bool(lib.cbl_gemm_b3_wide_serves((ctypes.c_int32 * len(rows))(*rows), len(rows), C, books, n))
+
+
 class B3Group(_Uncopied):
     """Up to four matrices that read the same activations through the same column orders (q|k|v, gate|up), run as one
     launch: run(X [B, >= C], ys) writes ys[i] [B, R_i]; the outputs share one row stride."""
@@ -483,6 +492,7 @@ class B3Group(_Uncopied):
         self.bmax = mats[0].bmax
         self.mats, self.C, self.M, self.device = mats, mats[0].C, mats[0].M, mats[0].device
         self.biases = biases if biases is not None else [None] * len(mats)
+        self.offs = [sum(m.R for m in mats[:i]) for i in range(len(mats) + 1)]
         self._built = None
         self._ws_bytes: dict = {}
 
@@ -527,29 +537,22 @@ class B3Group(_Uncopied):
             _lib.check("cbl_gemm_b3", lib.cbl_gemm_b3(st, len(self.mats), *x, _ptr(self.perms), out, _dt(ys[0].dtype), ldy, stage.data_ptr(), ws.data_ptr(), _stream()))
         return ys
 
-    @staticmethod
-    def wide_serves(dms: list, n: int) -> bool:
-        """Whether n >= 129 tokens of these matrices run faster by gathers (run_wide) than decoded once and multiplied."""
-        if n <= 128 or len(dms) > B3Group.MAX or any(not dm.fast or dm.M != 1 or dm.C != dms[0].C or dm.books != dms[0].books for dm in dms):
-            return False
-        return bool(lib.cbl_gemm_b3_wide_serves((ctypes.c_int32 * len(dms))(*[dm.R for dm in dms]), len(dms), dms[0].C, dms[0].books, n))
-
-    def run_wide(self, X: torch.Tensor | None, ys: list[torch.Tensor], staged: torch.Tensor | None = None) -> list[torch.Tensor]:
-        """run() for 129 tokens and more (one column order, two copies of the book)."""
-        T = ys[0].shape[0]
-        if X is None and staged is None or X is not None and (X.dim() != 2 or X.shape != (T, self.C) or X.stride(1) != 1 or X.device != self.device):
+    def run_wide(self, X: torch.Tensor | None, Y: torch.Tensor, staged: torch.Tensor | None = None) -> torch.Tensor:
+        """run() for 129 tokens and more (one column order, two copies of the book), the outputs side by side in Y [T, sum of R]."""
+        T = Y.shape[0]
+        if X is None and staged is None or X is not None and (X.shape != (T, self.C) or X.stride(1) != 1 or X.device != self.device):
             raise ValueError("X must be [T, C] with unit column stride on the matrices' device")
-        if len(ys) != len(self.mats) or len({y.dtype for y in ys}) != 1 or any(y.shape != (T, m.R) or y.stride() != (ys[0].stride(0), 1)
-                                                                             for y, m in zip(ys, self.mats)):
-            raise ValueError("one output [T, R_i] per matrix, one dtype, unit column stride and a common row stride")
-        out = (ctypes.c_void_p * len(ys))(*[y.data_ptr() for y in ys])
+        if Y.dim() != 2 or Y.shape[1] != self.offs[-1] or Y.stride(1) != 1:
+            raise ValueError("Y must be [T, sum of R] with unit column stride")
+        at, size = Y.data_ptr(), Y.element_size()
+        out = (ctypes.c_void_p * len(self.mats))(*[at + o * size for o in self.offs[:-1]])
         ws = scratch(self.device, PARTIAL, 1 << 16)
         stage, x = (staged, (None, 0, T, 0)) if X is None else (scratch(self.device, STAGE, lib.cbl_prep_x_bytes(T, self.C, 1)),
                                                                  (X.data_ptr(), _dt(X.dtype), T, X.stride(0)))
         with _on(self.device):
-            _lib.check("cbl_gemm_b3_wide", lib.cbl_gemm_b3_wide(self._structs, len(self.mats), *x, out, _dt(ys[0].dtype), ys[0].stride(0), stage.data_ptr(),
+            _lib.check("cbl_gemm_b3_wide", lib.cbl_gemm_b3_wide(self._structs, len(self.mats), *x, out, _dt(Y.dtype), Y.stride(0), stage.data_ptr(),
                                                                 ws.data_ptr(), _stream()))
-        return ys
+        return Y
 
     def status(self) -> None:
         """Synchronises and raises CblError if a bounded device-side wait of an earlier run() expired."""

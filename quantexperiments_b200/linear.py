@@ -16,13 +16,14 @@ pass the plain activation vector, not permuted copies.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 
 import torch
 
 from . import _cblhost, _lib
 from ._lib import lib
-from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix, _Uncopied, epoch
+from .kernels import B3Group, B3Matrix, DeviceMatrix, L8Matrix, T16Matrix, _Uncopied, _wide_serves, epoch
 
 # Rows from which one token runs on activation-side tables (L8Matrix) instead of codeword gathers (B3Matrix); of a matrix with
 # several column orders, rows per order: every order needs tables of its own, and a build costs as much as the lookups of some
@@ -35,8 +36,14 @@ L8_MIN_ROWS_PER_ORDER = 1536
 # Tokens up to which the book lies three times in shared memory (the activations of more tokens need the room: two copies).
 B3_MAX_3COPIES = 16
 # Tokens from which the two-phase path runs: decode the matrix once into a 16-bit scratch + TMA-fed tensor-core GEMM - or, up to some 900
-# tokens of matrices with rows enough for all SMs, gathers once more (B3Group.wide_serves).
+# tokens of matrices with rows enough for all SMs, gathers once more (cbl_gemm_b3_wide_serves).
 DENSE_MIN_TOKENS = 129
+
+
+@functools.lru_cache(maxsize=4096)
+def _direct_serves(R: int, C: int, books: int, M: int, n: int, tables: bool) -> bool:
+    """cbl_direct_serves of one matrix of these sizes (a call through ctypes takes longer than the product)."""
+    return bool(lib.cbl_direct_serves(ctypes.byref(_lib.Packed(R, C, 8, 12, 1, M, books, (C // 8 * 12 + 31) // 32)), 1, n, tables))
 
 
 def _tensors(objs) -> tuple:
@@ -137,11 +144,12 @@ class PackedLinear(_Uncopied, torch.nn.Module):
 
     def gathers(self, n: int) -> bool:
         """n >= 129 tokens run on codeword gathers.  A captured region builds no layout for them: it decodes."""
-        return not self.wide and B3Group.wide_serves([self.dm], n) and (2 in self._b3 or not torch.cuda.is_current_stream_capturing())
+        return (n >= DENSE_MIN_TOKENS and not self.wide and self.dm.fast and self.dm.M == 1
+                and _wide_serves(n, (self.R,), self.C, self.dm.books, self.dm.device.index) and (2 in self._b3 or not torch.cuda.is_current_stream_capturing()))
 
     def direct(self, n: int) -> bool:
         """n tokens run straight from the file layout, without a kernel layout: few tokens of a small matrix."""
-        return n <= 4 and self.dm.fast and not self.wide and bool(lib.cbl_direct_serves(ctypes.byref(self.dm.struct()), 1, n, self.use_l8()))
+        return n <= 4 and self.dm.fast and not self.wide and _direct_serves(self.R, self.C, self.dm.books, self.dm.M, n, self.use_l8())
 
     def gemv(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x [C] (fp16 / bf16 / fp32, contiguous) -> y [R] in x's dtype (or `out`'s)."""
@@ -180,7 +188,7 @@ class PackedLinear(_Uncopied, torch.nn.Module):
         elif n < DENSE_MIN_TOKENS:
             self.group(n).run(x2, [y])
         elif self.gathers(n):
-            self.group(n).run_wide(x2, [y])
+            self.group(n).run_wide(x2, y)
         else:
             # many tokens: decode once into the shared 16-bit scratch, then the TMA-fed GEMM
             self.dm.gemm_dense(x2, y)
@@ -229,6 +237,9 @@ class Stack:
         self.dense = DenseStack([l.dm for l in lins]) if self.fast and len({l.C for l in lins}) == 1 and not any(l.wide for l in lins) else None
         self._l8 = None
         self._b3: dict[int, B3Group] = {}
+        # sizes that the rule for many tokens by gathers goes by
+        self._sizes = (tuple(self.Rs), self.C, lins[0].dm.books, self.device.index) if (
+            self.shared and plain and len(lins) <= B3Group.MAX and len({l.dm.books for l in lins}) == 1 and len({l.C for l in lins}) == 1) else None
 
     @property
     def l8(self):
@@ -245,7 +256,7 @@ class Stack:
 
     def gathers(self, n: int) -> bool:
         """n >= 129 tokens run on codeword gathers (see PackedLinear.gathers)."""
-        return (self.shared and not any(l.wide for l in self.lins) and B3Group.wide_serves([l.dm for l in self.lins], n)
+        return (n >= DENSE_MIN_TOKENS and self._sizes is not None and _wide_serves(n, *self._sizes)
                 and (2 in self._b3 or not torch.cuda.is_current_stream_capturing()))
 
     def ready(self, n: int) -> bool:
@@ -285,12 +296,11 @@ class Stack:
     def run(self, x: torch.Tensor | None, y: torch.Tensor, staged: torch.Tensor | None = None, tables: bool | None = None) -> torch.Tensor:
         """tables: whether one token may run on table lookups (None: where the stack's rule says so)."""
         n = y.shape[0]
-        ys = list(y.split(self.Rs, 1))
         if n >= DENSE_MIN_TOKENS and self.gathers(n):
-            self.b3(n).run_wide(x, ys, staged)
-            return y
+            return self.b3(n).run_wide(x, y, staged)
         if n >= DENSE_MIN_TOKENS and self.dense is not None:
             return self.dense.gemm(x, y, staged)
+        ys = list(y.split(self.Rs, 1))
         if x is None:
             self.b3(n).run(None, ys, staged)
         elif self._direct(n):
